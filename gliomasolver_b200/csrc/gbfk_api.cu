@@ -108,6 +108,14 @@ struct gbfk_ctx {
     bool run_layout_valid = false;
     int *d_run_nbr = nullptr;
     unsigned *d_run_flags = nullptr;
+    // runs with resident blocks (gbfk_resident.cu): per heavy block the list
+    // positions of its face neighbours, the face exchange buffers, the state
+    // count; the number of SMs
+    int *d_res_nbr = nullptr;
+    void *d_res_ex = nullptr;
+    unsigned *d_res_index = nullptr;
+    bool res_ready = false;
+    int sms = 0;
     // phi[cur] is the output of a step: every value +0 <= phi <= 1 or NaN
     // (set only by rd_step; every other writer of phi clears it)
     bool phi_clamped = false;
@@ -217,6 +225,7 @@ void free_topology(gbfk_ctx *c)
     c->faces_valid = false;
     c->lists_valid = false;
     c->run_layout_valid = false;
+    c->res_ready = false;
     c->phi_clamped = false;
 }
 
@@ -227,7 +236,8 @@ void release_topology(gbfk_ctx *c)
     void **ptrs[] = {(void **)&c->d_slot, (void **)&c->d_nbr, &c->d_h, (void **)&c->d_row_ptr, (void **)&c->d_src,
                      &c->d_w, (void **)&c->d_step_rows, (void **)&c->d_all_rows, &c->d_gpw, &c->d_gpg,
                      &c->d_gphi, (void **)&c->d_fwt, &c->d_H, (void **)&c->d_ih2, (void **)&c->d_btype, &c->d_origin,
-                     (void **)&c->d_lists, (void **)&c->d_run_nbr, (void **)&c->d_run_flags};
+                     (void **)&c->d_lists, (void **)&c->d_run_nbr, (void **)&c->d_run_flags,
+                     (void **)&c->d_res_nbr, &c->d_res_ex, (void **)&c->d_res_index};
     for (void **p : ptrs) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -325,6 +335,7 @@ int check_stage_timeout(gbfk_ctx *ctx)
     CK(cudaStreamSynchronize(ctx->stream));
     if (flag) {
         CK(cudaMemsetAsync(ctx->d_nan + 1, 0, sizeof(unsigned), ctx->stream));
+        ctx->res_ready = false;  // a run that gave up leaves its exchange buffers behind
         if (flag & (1u | 256u))
             return fail(ctx, GBFK_E_TIMEOUT, "rd_step: a wait of the pipelined step timed out (1 s; error word 0x%x)",
                         flag);
@@ -523,7 +534,72 @@ int build_step_lists(gbfk_ctx *ctx)
     ctx->lists_gen++;
     ctx->h_lists.swap(lists);
     ctx->run_layout_valid = false;
+    ctx->res_ready = false;
     return GBFK_OK;
+}
+
+// Whether the heavy blocks of the current step lists fit the SMs' shared
+// memory (a uniform grid, lists built).
+template <typename Real>
+bool resident_fits(const gbfk_ctx *ctx)
+{
+    return ctx->uniform && ctx->identity_slots && ctx->lists_valid && ctx->n_heavy > 0 &&
+           ctx->n_heavy <= resident_capacity<Real>(ctx->sms);
+}
+
+// The tables and buffers of resident runs over the current step lists.
+template <typename Real>
+int build_resident(gbfk_ctx *ctx)
+{
+    if (ctx->res_ready) return GBFK_OK;
+    const int n = ctx->n_heavy, nb = ctx->nblocks, bpd = ctx->bpd;
+    std::vector<int> at(nb, -1), nbr((size_t)n * 6);
+    for (int i = 0; i < n; i++) at[ctx->h_lists[i] >> 2] = i;
+    for (int i = 0; i < n; i++) {
+        const int b = ctx->h_lists[i] >> 2;
+        const int p[3] = {b % bpd, (b / bpd) % bpd, b / (bpd * bpd)};
+        for (int f = 0; f < 6; f++) {
+            int q[3] = {p[0], p[1], p[2]};
+            q[f >> 1] = (q[f >> 1] + ((f & 1) ? 1 : bpd - 1)) % bpd;
+            nbr[(size_t)i * 6 + f] = at[q[0] + bpd * (q[1] + bpd * q[2])];
+        }
+    }
+    const size_t ex = (size_t)2 * n * 384 * sizeof(Real);
+    int rc = topo_alloc(ctx, &ctx->d_res_nbr, nbr.size() * sizeof(int));
+    if (!rc) rc = topo_alloc(ctx, &ctx->d_res_ex, ex);
+    if (!rc) rc = topo_alloc(ctx, &ctx->d_res_index, 2 * sizeof(unsigned));
+    if (rc) return rc;
+    CK(cudaMemsetAsync(ctx->d_res_ex, 0, ex, ctx->stream));
+    CK(cudaMemsetAsync(ctx->d_res_index, 0, 2 * sizeof(unsigned), ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_res_nbr, nbr.data(), nbr.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->res_ready = true;
+    return GBFK_OK;
+}
+
+// Arguments of a resident run over the current lists (in, out, stores, nsteps
+// and the empty blocks are the caller's).
+template <typename Real>
+ResidentArgs<Real> resident_args(gbfk_ctx *ctx, double rho, double dt)
+{
+    ResidentArgs<Real> a = {};
+    a.items = ctx->d_lists;
+    a.nbr = ctx->d_res_nbr;
+    a.n = ctx->n_heavy;
+    a.H = (const Real *)ctx->d_H;
+    a.meta = ctx->d_meta;
+    a.pw = (const Real *)ctx->pw;
+    a.pg = (const Real *)ctx->pg;
+    a.bpd = ctx->bpd;
+    a.rho = (Real)rho;
+    a.dt = dt;
+    const double h = sizeof(Real) == 8 ? ctx->h_h[0] : (double)(float)ctx->h_h[0];  // as upload_ih2
+    a.ih2 = 1. / (h * h);
+    a.ex = (Real *)ctx->d_res_ex;
+    a.index = ctx->d_res_index;
+    a.nan_flag = ctx->d_nan;
+    a.err_flag = ctx->d_nan + 1;
+    return a;
 }
 
 // The CTA layout of runs of steps over the current step lists.
@@ -546,6 +622,14 @@ int build_run_layout(gbfk_ctx *ctx, const PoolView<Real> &v)
     return GBFK_OK;
 }
 
+// From how many steps on a call is worth a run: a resident run costs about
+// 14-17 us beside its steps (launch, state and coefficients in, state out),
+// so that against one pipelined launch per step it pays from 6 steps on
+// (64^3 FP32: 14 + 1.2 n against 3.7 n; 128^3: 17 + 2.0 n against 6.3 n),
+// against the per-block kernel (9-28 us per step) from 3; leaving out the
+// empty blocks at 256^3 saves 10 us per step for 23 us.
+constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kSkipSteps = 3;
+
 template <typename Real>
 int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int nsteps, int check_nan)
 {
@@ -560,6 +644,25 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     // a few percent of one launch per step, which programmatic dependent
     // launch already overlaps)
     const bool runs = pipelined && ctx->step_pref == GBFK_STEP_RUN;
+    // AUTO: the steps after the first one of an unclamped state as one run
+    // with resident blocks, where they fit, or as launches that leave out the
+    // empty blocks, whose steps are made up in one launch (nothing couples
+    // them to the others while every coefficient is finite)
+    const bool uncoupled = ctx->step_pref == GBFK_STEP_AUTO && ctx->uniform && ctx->identity_slots &&
+                           std::isfinite(dt) && std::isfinite((double)(Real)Dw) && std::isfinite((double)(Real)Dg);
+    const int clamped_steps = ctx->phi_clamped ? nsteps : nsteps - 1;
+    bool want_run = uncoupled && clamped_steps >= (pipelined ? kResidentSteps : kResidentStepsBlock);
+    if (want_run && (!ctx->res_ready || !ctx->lists_valid)) {
+        // the tables of a run cannot be built inside a stream capture
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(ctx->stream, &st));
+        if (st != cudaStreamCaptureStatusNone) want_run = false;
+    }
+    const bool want_skip = uncoupled && pipelined && clamped_steps >= kSkipSteps;
+    if (want_run && !pipelined) {
+        rc = build_step_lists(ctx);
+        if (rc) return rc;
+    }
     double ih2 = 0;
     if (pipelined) {
         if (!ctx->tma_maps_ready) {
@@ -576,12 +679,39 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     }
     if (check_nan) CK(cudaMemsetAsync(ctx->d_nan, 0, sizeof(unsigned), ctx->stream));
     const BlockLists lists = {ctx->d_lists, ctx->n_heavy, ctx->d_lists + ctx->n_heavy, ctx->n_empty};
-    bool ran_run = false;
+    bool ran_run = false, skip = false;
+    const bool fits = (want_run || want_skip) && resident_fits<Real>(ctx), resident = want_run && fits;
+    if (resident) {
+        rc = build_resident<Real>(ctx);
+        if (rc) return rc;
+    }
     for (int s = 0; s < nsteps;) {
         const Real *in = (const Real *)ctx->phi[ctx->cur];
         Real *out = (Real *)ctx->phi[ctx->cur ^ 1];
         const bool clamped = ctx->phi_clamped || s > 0;
         const int left = nsteps - s;
+        if (resident && clamped) {
+            // in place: every block's state 0 is read by its own CTA alone
+            ResidentArgs<Real> a = resident_args<Real>(ctx, rho, dt);
+            a.in = in;
+            a.out = (Real *)ctx->phi[ctx->cur];
+            a.nsteps = left;
+            a.empty = lists.empty;
+            a.n_empty = lists.n_empty;
+            CK(launch_resident_run<Real>(a, ctx->sms, ctx->stream));
+            ctx->launches++;
+            s += left;
+            ran_run = true;
+            continue;
+        }
+        if (want_skip && !fits && clamped && !skip && lists.n_heavy > 0) {
+            // both buffers get the empty blocks' last state: a heavy block's
+            // halo copies may read either, multiplied by coefficients of 0
+            CK(launch_empty_run<Real>(lists.empty, lists.n_empty, in, (Real *)ctx->phi[ctx->cur], out, left,
+                                      (Real)rho, dt, ctx->d_nan, ctx->stream));
+            ctx->launches++;
+            skip = true;
+        }
         if (runs && clamped && left >= 2) {
             // phi[cur] -> phi[cur ^ 1] -> phi[cur] ..., k steps in one launch
             const int k = left < kMaxRunSteps ? left : kMaxRunSteps;
@@ -599,7 +729,7 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
         }
         if (pipelined) {
             CK(launch_rd_step_tma<Real>(v, lists, (const Real *)ctx->d_H, ctx->d_meta, ih2, in, clamped, out,
-                                        (Real)rho, dt, ctx->d_nan, ctx->d_nan + 1, ctx->tma_maps[ctx->cur], false,
+                                        (Real)rho, dt, ctx->d_nan, ctx->d_nan + 1, ctx->tma_maps[ctx->cur], skip,
                                         ctx->stream));
             ctx->launches++;
             ctx->cur ^= 1;
@@ -795,6 +925,8 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
     cudaMemset(ctx->pw, 0, bytes);
     cudaMemset(ctx->pg, 0, bytes);
     cudaMemset(ctx->d_nan, 0, 2 * sizeof(unsigned));
+    if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
+        return bail(GBFK_E_CUDA);
     if (ensure_table(ctx) != GBFK_OK) return bail(GBFK_E_CUDA);
     *out = ctx;
     return GBFK_OK;

@@ -135,6 +135,48 @@ cudaError_t launch_rd_run_tma(const PoolView<Real> &v, const BlockLists &lists, 
                               unsigned *err_flag, unsigned *flags, const CUtensorMap *maps_in0,
                               const CUtensorMap *maps_buf0, const CUtensorMap *maps_buf1, cudaStream_t s);
 
+// A run of nsteps steps with the heavy blocks resident in shared memory
+// (gbfk_resident.cu): any uniform grid with identity slots whose heavy blocks
+// fit (resident_capacity).  in: the output of a step (every value +0 <= phi
+// <= 1 or NaN).  items: the n heavy blocks (block * 4 + type); nbr: per item
+// the item indices of its six face neighbours (-1: an empty block); stores:
+// NULL (the last state goes to out, which may be in), or nsteps device
+// pointers: where the heavy blocks of state s + 1 go (NULL entries: nowhere).
+// empty: the n_empty empty blocks, whose last state goes to out (n_empty 0:
+// they are left alone).  ex: 2 * n * 384 Real and index: 2 words, both zeroed
+// once per item list and then left to the runs.  dt, Dw and Dg are finite.
+// err_flag as for the pipelined step (bits 0 and 9: a face never came).
+template <typename Real>
+struct ResidentArgs {
+    const int *items, *nbr;
+    int n;
+    const int *empty;
+    int n_empty;
+    const Real *H;
+    const unsigned short *meta;
+    const Real *pw, *pg;
+    int bpd;
+    const Real *in;
+    Real *out;
+    Real *const *stores;
+    int nsteps;
+    Real rho;
+    double dt, ih2;
+    Real *ex;
+    unsigned *index;
+    unsigned *nan_flag, *err_flag;
+    unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
+};
+template <typename Real>
+int resident_capacity(int sms);
+template <typename Real>
+cudaError_t launch_resident_run(const ResidentArgs<Real> &a, int sms, cudaStream_t s);
+// nsteps steps of the empty blocks alone, from `in` into out0 and (unless
+// NULL) out1: the company of nsteps launches that skip them.
+template <typename Real>
+cudaError_t launch_empty_run(const int *empty, int n_empty, const Real *in, Real *out0, Real *out1, int nsteps,
+                             Real rho, double dt, unsigned *nan_flag, cudaStream_t s);
+
 // The same for a step of a TMCMC batch: every active sample (positions
 // 0 .. nactive-1) of one uniform 2^log2_bpd grid.  Per-position fields are
 // consecutive pools of nblocks blocks (phi_in/phi_out, H); per-anatomy ones

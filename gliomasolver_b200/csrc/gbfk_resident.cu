@@ -1,0 +1,769 @@
+// Runs of RD steps with the blocks resident in shared memory, for uniform
+// periodic grids whose blocks sit in consecutive pool slots (any number of
+// blocks per direction).  Results are bit-identical to one launch per step
+// (rd_step_tma_kernel, rd_step_kernel).
+//
+// One CTA per SM, launched cooperatively.  Each heavy block (a block with
+// tissue in it or its face halos) belongs to one CTA for the whole run: its
+// phi (double-buffered), face coefficients and meta words stay in that CTA's
+// shared memory, and a step moves only the block's six faces.  A group of
+// 128 (or 256) threads steps one block, four (two) x-consecutive cells per
+// thread, so that a thread reads its own row, the four neighbouring rows and
+// the y and z coefficients in 16-byte (8-byte) accesses.
+//
+// What bounds it: a step is one exchange of faces through L2 (about 0.9 us
+// from a block's stores to the end of its neighbours' next step, what an 8-
+// block grid takes) plus the issue of its cells' exact-rounding arithmetic
+// (128^3, FP32: 1.69 M warp instructions per step, 67 % of the issue slots).
+// Measured on a B200, us per step over 1000 steps, against one launch per
+// step: 64^3 FP32 1.22 (3.74), FP64 1.40 (3.87); 128^3 FP32 2.02 (6.33),
+// FP64 3.14 (8.59); 120^3, which had the one-CTA-per-block kernel, FP32 12.2
+// before.
+//
+// Faces travel through L2.  After forming state k a block stores its six
+// faces in the exchange buffer k & 1 and its neighbours poll for them there.
+// No flag accompanies the data: every value of a clamped state is +0 <= phi
+// <= 1 or NaN, so the sign bit of each word is free, and it carries the
+// phase (k / 2) & 1 of the buffer's use.  A reader polls until all its words
+// show the expected phase.  Two buffers are enough: each word has one reader,
+// the thread that owns the cell across the face, and that thread writes the
+// word coming back.  A thread stores state k + 2 over state k only after it
+// has read the mirror thread's word of state k + 1, which that thread stored
+// after its own read of state k.  The phase goes on from launch to launch:
+// the state count lives in device memory (index[0]), advanced by the last CTA
+// to leave, so that a launch replayed from a graph finds it right too.
+//
+// Empty blocks (every cell and face-halo cell kEmpty) couple to nothing: all
+// face coefficients of a kEmpty cell are exactly 0 (the harmonic mean with a
+// zero diffusivity), so with finite values its update is the reaction alone,
+// and a heavy block's cell next to an empty block is kEmpty itself.  Their
+// cells run all steps of the call in registers (empty_blocks), usually +0 in
+// and out, and nobody waits for them.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <mutex>
+#include <vector>
+
+#include "gbfk_exact.cuh"
+#include "gbfk_kernels.cuh"
+
+namespace gbfk {
+namespace {
+
+constexpr unsigned long long kPollNs = 1000000000ull;  // a face not seen after 1 s is declared lost
+constexpr unsigned kErrPoll = 1u | 512u;               // error word: a wait gave up, in a resident run
+
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+// ---- words of the exchange buffer -----------------------------------------
+// N consecutive values in 16-, 8- or 4-byte accesses, each value one relaxed
+// access of its own (no order among them is needed: each carries its phase)
+template <int N>
+__device__ __forceinline__ void ld_face(const float *p, float (&v)[N])
+{
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4)
+            asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3])
+                         : "l"(p + i)
+                         : "memory");
+    } else
+        asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void ld_face(const double *p, double (&v)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i += 2)
+        asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];"
+                     : "=d"(v[i]), "=d"(v[i + 1])
+                     : "l"(p + i)
+                     : "memory");
+}
+template <int N>
+__device__ __forceinline__ void st_face(float *p, const float (&v)[N])
+{
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4)
+            asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + i), "f"(v[i]), "f"(v[i + 1]),
+                         "f"(v[i + 2]), "f"(v[i + 3])
+                         : "memory");
+    } else
+        asm volatile("st.relaxed.gpu.global.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v[0]), "f"(v[1]) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void st_face(double *p, const double (&v)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i += 2)
+        asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + i), "d"(v[i]), "d"(v[i + 1]) : "memory");
+}
+__device__ __forceinline__ void st_face1(float *p, float v)
+{
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_face1(double *p, double v)
+{
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+// value with the sign bit set to the phase (m: the sign bit or 0), in one
+// instruction the compiler does not see through: written with bit operators it
+// becomes +-|v| in floating point, which drops the sign of a NaN
+__device__ __forceinline__ unsigned with_phase_bits(unsigned v, unsigned m)
+{
+    unsigned r;
+    asm("lop3.b32 %0, %1, 0x7fffffff, %2, 0xEA;" : "=r"(r) : "r"(v), "r"(m));  // (v & 0x7fffffff) | m
+    return r;
+}
+__device__ __forceinline__ float with_phase(float v, unsigned m)
+{
+    return __uint_as_float(with_phase_bits(__float_as_uint(v), m));
+}
+__device__ __forceinline__ double with_phase(double v, unsigned m)
+{
+    return __hiloint2double((int)with_phase_bits((unsigned)__double2hiint(v), m), __double2loint(v));
+}
+// the sign bit differs from the phase: not there yet
+__device__ __forceinline__ unsigned sign_xor(float v, unsigned m) { return __float_as_uint(v) ^ m; }
+__device__ __forceinline__ unsigned sign_xor(double v, unsigned m) { return (unsigned)__double2hiint(v) ^ m; }
+__device__ __forceinline__ float magnitude(float v) { return __uint_as_float(__float_as_uint(v) & 0x7fffffffu); }
+__device__ __forceinline__ double magnitude(double v)
+{
+    return __hiloint2double(__double2hiint(v) & 0x7fffffff, __double2loint(v));
+}
+
+// The cells of a block are held by kT = 512 / kC threads, kC x-consecutive
+// cells each.  Arrays in shared memory keep 16-byte vectors (or all kC cells,
+// if they are fewer) as [vector][thread], so that a warp's access is one
+// contiguous run of banks for every neighbour offset; rows of a face array
+// count as threads too (kRows rows of 8).
+template <typename Real, int kC>
+struct Tile {
+    static constexpr int V = 16 / (int)sizeof(Real) < kC ? 16 / (int)sizeof(Real) : kC;
+    // where cell x of a row lies in an array of kRows rows
+    template <int kRows>
+    static __device__ __forceinline__ int at(int row, int x)
+    {
+        const int t = row * (8 / kC) + x / kC, v = (x % kC) / V;
+        return (v * (kRows * 8 / kC) + t) * V + x % V;
+    }
+    // the kC cells of "thread" t of such an array
+    template <int kRows>
+    static __device__ __forceinline__ void load(const Real *a, int t, Real (&d)[kC])
+    {
+#pragma unroll
+        for (int v = 0; v < kC / V; v++) {
+            const Real *p = a + (v * (kRows * 8 / kC) + t) * V;
+            if constexpr (sizeof(Real) == 4 && V == 4) {
+                const float4 q = *reinterpret_cast<const float4 *>(p);
+                d[4 * v] = q.x; d[4 * v + 1] = q.y; d[4 * v + 2] = q.z; d[4 * v + 3] = q.w;
+            } else if constexpr (sizeof(Real) == 4) {
+                const float2 q = *reinterpret_cast<const float2 *>(p);
+                d[2 * v] = q.x; d[2 * v + 1] = q.y;
+            } else {
+                const double2 q = *reinterpret_cast<const double2 *>(p);
+                d[2 * v] = q.x; d[2 * v + 1] = q.y;
+            }
+        }
+    }
+    template <int kRows>
+    static __device__ __forceinline__ void store(Real *a, int t, const Real (&d)[kC])
+    {
+#pragma unroll
+        for (int v = 0; v < kC / V; v++) {
+            Real *p = a + (v * (kRows * 8 / kC) + t) * V;
+            if constexpr (sizeof(Real) == 4 && V == 4)
+                *reinterpret_cast<float4 *>(p) = make_float4(d[4 * v], d[4 * v + 1], d[4 * v + 2], d[4 * v + 3]);
+            else if constexpr (sizeof(Real) == 4)
+                *reinterpret_cast<float2 *>(p) = make_float2(d[2 * v], d[2 * v + 1]);
+            else
+                *reinterpret_cast<double2 *>(p) = make_double2(d[2 * v], d[2 * v + 1]);
+        }
+    }
+};
+// kC consecutive cells of a block in global memory (16-byte aligned, or 8 for two floats)
+template <typename Real, int kC>
+__device__ __forceinline__ void ld_cells(const Real *p, Real (&d)[kC])
+{
+#pragma unroll
+    for (int v = 0; v < kC / Tile<Real, kC>::V; v++) {
+        constexpr int V = Tile<Real, kC>::V;
+        if constexpr (sizeof(Real) == 4 && V == 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(p + 4 * v);
+            d[4 * v] = q.x; d[4 * v + 1] = q.y; d[4 * v + 2] = q.z; d[4 * v + 3] = q.w;
+        } else if constexpr (sizeof(Real) == 4) {
+            const float2 q = *reinterpret_cast<const float2 *>(p + 2 * v);
+            d[2 * v] = q.x; d[2 * v + 1] = q.y;
+        } else {
+            const double2 q = *reinterpret_cast<const double2 *>(p + 2 * v);
+            d[2 * v] = q.x; d[2 * v + 1] = q.y;
+        }
+    }
+}
+template <typename Real, int kC>
+__device__ __forceinline__ void st_cells(Real *p, const Real (&d)[kC])
+{
+    // consecutive vectors: a one-thread array
+#pragma unroll
+    for (int v = 0; v < kC / Tile<Real, kC>::V; v++) {
+        constexpr int V = Tile<Real, kC>::V;
+        if constexpr (sizeof(Real) == 4 && V == 4)
+            *reinterpret_cast<float4 *>(p + 4 * v) = make_float4(d[4 * v], d[4 * v + 1], d[4 * v + 2], d[4 * v + 3]);
+        else if constexpr (sizeof(Real) == 4)
+            *reinterpret_cast<float2 *>(p + 2 * v) = make_float2(d[2 * v], d[2 * v + 1]);
+        else
+            *reinterpret_cast<double2 *>(p + 2 * v) = make_double2(d[2 * v], d[2 * v + 1]);
+    }
+}
+
+// One resident block in shared memory: two states, each with its face halos
+// (rows y = -1 .. 8 of planes z = -1 .. 8, and the x faces apart), and the
+// face coefficients: x faces as eight left faces per row and the row's last
+// face apart, y and z faces as in H.  A coefficient carries a set sign bit
+// where either cell of the face is kEmpty (see row_cells).
+constexpr int kRows = 100;
+template <typename Real>
+struct alignas(16) ResidentState {
+    Real phi[kRows * 8];
+    Real xh[2][64];          // [z][y]: the x- and x+ neighbours' cells
+};
+template <typename Real>
+struct alignas(16) ResidentBlock {
+    ResidentState<Real> st[2];
+    Real hx[kBS3], hx8[64], hy[576], hz[576];
+    int nbr[6];              // exchange offset (elements) of the face neighbours, -1: an empty block
+    int e;                   // block * 4 + block type
+    unsigned kinds;          // two bits per warp: the row_cells variant its cells need
+};
+constexpr unsigned kPlain = 0, kEdge = 1, kGeneral = 2;
+
+__device__ __forceinline__ float set_sign(float v, bool s) { return s ? __uint_as_float(__float_as_uint(v) | 0x80000000u) : v; }
+__device__ __forceinline__ double set_sign(double v, bool s) { return s ? -v : v; }
+__device__ __forceinline__ bool sign_of(float v) { return __float_as_int(v) < 0; }
+__device__ __forceinline__ bool sign_of(double v) { return __double2hiint(v) < 0; }
+
+// d = a * b and d += a for two values, each rounded to nearest by itself; one
+// instruction for two floats.  The product is an FMA with -0 (which adds
+// nothing, signs of zero included), and that -0 (neg0: both halves) comes
+// from the host: the assembler contracts a packed multiply, or a packed FMA
+// with a -0 it can see, with the packed add that follows.
+__device__ __forceinline__ unsigned long long packed(const float (&v)[2])
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v[0]), "f"(v[1]));
+    return r;
+}
+__device__ __forceinline__ void pair_mul(float (&d)[2], const float (&a)[2], const float (&b)[2],
+                                         unsigned long long neg0)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(packed(a)), "l"(packed(b)), "l"(neg0));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d[0]), "=f"(d[1]) : "l"(r));
+}
+__device__ __forceinline__ void pair_add(float (&d)[2], const float (&a)[2])
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(packed(d)), "l"(packed(a)));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d[0]), "=f"(d[1]) : "l"(r));
+}
+__device__ __forceinline__ void pair_mul(double (&d)[2], const double (&a)[2], const double (&b)[2],
+                                         unsigned long long)
+{
+    d[0] = rmul(a[0], b[0]);
+    d[1] = rmul(a[1], b[1]);
+}
+__device__ __forceinline__ void pair_add(double (&d)[2], const double (&a)[2])
+{
+    d[0] = radd(d[0], a[0]);
+    d[1] = radd(d[1], a[1]);
+}
+// clamp01 of a rounded result (its NaN is the canonical one): two instructions
+__device__ __forceinline__ float clamp_state(float p)
+{
+    asm("max.NaN.f32 %0, %0, 0f00000000;" : "+f"(p));
+    asm("min.NaN.f32 %0, %0, 0f3F800000;" : "+f"(p));
+    return p;
+}
+__device__ __forceinline__ double clamp_state(double p) { return clamp01(p); }
+
+// p_w, p_g of cell (x, y, z) of block blk, or of the one cell outside it
+// across a face, on the uniform bpd^3 grid
+template <typename Real>
+__device__ __noinline__ void tissue_at(const Real *pw_all, const Real *pg_all, int bpd, int blk, int x, int y, int z,
+                                       Real &pw, Real &pg)
+{
+    int bx = blk % bpd, by = (blk / bpd) % bpd, bz = blk / (bpd * bpd);
+    if (x < 0) bx = bx ? bx - 1 : bpd - 1;
+    if (x > 7) bx = bx + 1 < bpd ? bx + 1 : 0;
+    if (y < 0) by = by ? by - 1 : bpd - 1;
+    if (y > 7) by = by + 1 < bpd ? by + 1 : 0;
+    if (z < 0) bz = bz ? bz - 1 : bpd - 1;
+    if (z > 7) bz = bz + 1 < bpd ? bz + 1 : 0;
+    const int64_t g = ((int64_t)bx + (int64_t)bpd * (by + (int64_t)bpd * bz)) * kBS3 + (x & 7) +
+                      kBS * ((y & 7) + kBS * (z & 7));
+    pw = pw_all[g];
+    pg = pg_all[g];
+}
+
+// What a thread needs to know of its place in a block, fixed for the run.
+struct Place {
+    int t;        // thread of the group
+    int x0, y, z; // its cells: x0 .. x0 + kC - 1 of row (y, z)
+    int tp;       // its place in the padded state array
+    int xl, xr;   // element offsets in ResidentState of the cells before and after them
+    int he;       // element offset from hx of the last cell's right face
+};
+
+// The kC cells of a thread in block b, from the state S with its halos (a
+// clamped state) to out.  kKind, by warp:
+//   kPlain    every cell and neighbour is kTissue: no no-flux doubling, every
+//             cell is inside the domain;
+//   kEdge     kEmpty cells or neighbours among them.  The coefficient of a
+//             face that touches a kEmpty cell is 0, so its sign bit says so
+//             (-0): a neighbour with phi < 0.1 across such a face doubles the
+//             opposite coefficient (for a kEmpty cell itself, whose
+//             coefficients are all 0, whatever is doubled stays 0, and its
+//             formula leaves +0 where phi is +0 and the reaction where it is
+//             not, so that its domain test needs no branch).  -0 for +0 in
+//             the flux sums gives the same sums: (+0) + (-0) = +0 either way;
+//   kGeneral  kOther cells or neighbours: classes from the meta words, p_w
+//             and p_g from global memory.
+template <typename Real, int kC, unsigned kKind>
+__device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, const ResidentBlock<Real> &b,
+                                          const ResidentState<Real> &S, const Place &w, Real (&out)[kC])
+{
+    using TL = Tile<Real, kC>;
+    constexpr int R = 8 / kC;  // threads of a row
+    Real p[kC], ym[kC], yp[kC], zm[kC], zp[kC];
+    TL::template load<kRows>(S.phi, w.tp, p);
+    const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
+    TL::template load<kRows>(S.phi, w.tp - R, ym);
+    TL::template load<kRows>(S.phi, w.tp + R, yp);
+    TL::template load<kRows>(S.phi, w.tp - 10 * R, zm);
+    TL::template load<kRows>(S.phi, w.tp + 10 * R, zp);
+    Real hx[kC], hym[kC], hyp[kC], hzm[kC], hzp[kC];
+    TL::template load<64>(b.hx, w.t, hx);
+    const Real hx_end = b.hx[w.he];
+    const int ty = w.t + w.z * R;  // row z * 9 + y of hy
+    TL::template load<72>(b.hy, ty, hym);
+    TL::template load<72>(b.hy, ty + R, hyp);
+    TL::template load<72>(b.hz, w.t, hzm);
+    TL::template load<72>(b.hz, w.t + 8 * R, hzp);
+    const Real eps = (Real)0.1;
+    constexpr bool kLow = kKind != kPlain;
+    // two cells at a time, so that the single-precision operations of the flux
+    // sums can go in pairs (pair_add, pair_mul: each half rounded by itself)
+#pragma unroll
+    for (int i = 0; i < kC; i += 2) {
+        const Real ph[2] = {p[i], p[i + 1]};
+        const Real xm[2] = {i ? p[i - 1] : xl, p[i]}, xp[2] = {p[i + 1], i + 2 < kC ? p[i + 2] : xr};
+        Real d0[2] = {hx[i], hx[i + 1]}, d1[2] = {hx[i + 1], i + 2 < kC ? hx[i + 2] : hx_end};
+        Real d2[2] = {hym[i], hym[i + 1]}, d3[2] = {hyp[i], hyp[i + 1]}, d4[2] = {hzm[i], hzm[i + 1]},
+             d5[2] = {hzp[i], hzp[i + 1]};
+        const Real y0[2] = {ym[i], ym[i + 1]}, y1[2] = {yp[i], yp[i + 1]}, z0[2] = {zm[i], zm[i + 1]},
+                   z1[2] = {zp[i], zp[i + 1]};
+        bool dom[2] = {true, true};
+        if (kLow) {
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                bool low[6] = {sign_of(d0[j]) && xm[j] < eps, sign_of(d1[j]) && xp[j] < eps,
+                               sign_of(d2[j]) && y0[j] < eps, sign_of(d3[j]) && y1[j] < eps,
+                               sign_of(d4[j]) && z0[j] < eps, sign_of(d5[j]) && z1[j] < eps};
+                if (kKind == kGeneral) {
+                    const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
+                    const int blk = b.e >> 2;
+                    const unsigned mw = a.meta[(int64_t)blk * kBS3 + w.t * kC + i + j];
+                    Real pw, pg;
+                    if ((mw & 3u) == kOther) {
+                        tissue_at(a.pw, a.pg, a.bpd, blk, w.x0 + i + j, w.y, w.z, pw, pg);
+                        dom[j] = in_domain(pw, pg, ph[j]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 6; k++)
+                        if ((mw >> (8 + k)) & 1u) {
+                            tissue_at(a.pw, a.pg, a.bpd, blk, w.x0 + i + j + (k == 1) - (k == 0),
+                                      w.y + (k == 3) - (k == 2), w.z + (k == 5) - (k == 4), pw, pg);
+                            low[k] = domain_chf(phn[k], pw, pg) < eps;
+                        }
+                }
+                // _applyNoFluxBC: neighbour k below 0.1 doubles the opposite coefficient
+                if (low[0]) d1[j] = rmul(d1[j], (Real)2.);
+                if (low[1]) d0[j] = rmul(d0[j], (Real)2.);
+                if (low[2]) d3[j] = rmul(d3[j], (Real)2.);
+                if (low[3]) d2[j] = rmul(d2[j], (Real)2.);
+                if (low[4]) d5[j] = rmul(d5[j], (Real)2.);
+                if (low[5]) d4[j] = rmul(d4[j], (Real)2.);
+            }
+        }
+        // cell_rhs: the same operations in the same order for both cells
+        Real sin_[2] = {rmul(d0[0], xm[0]), rmul(d0[1], xm[1])}, u[2] = {rmul(d1[0], xp[0]), rmul(d1[1], xp[1])};
+        pair_add(sin_, u);
+        pair_mul(u, d2, y0, a.neg0);
+        pair_add(sin_, u);
+        pair_mul(u, d3, y1, a.neg0);
+        pair_add(sin_, u);
+        pair_mul(u, d4, z0, a.neg0);
+        pair_add(sin_, u);
+        pair_mul(u, d5, z1, a.neg0);
+        pair_add(sin_, u);
+        Real sdf[2] = {radd(d0[0], d1[0]), radd(d0[1], d1[1])};
+        pair_add(sdf, d2);
+        pair_add(sdf, d3);
+        pair_add(sdf, d4);
+        pair_add(sdf, d5);
+        pair_mul(sdf, sdf, ph, a.neg0);
+        const Real rr[2] = {a.rho, a.rho};
+        Real rp[2];
+        pair_mul(rp, rr, ph, a.neg0);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const double fluxIn = __dmul_rn(a.ih2, (double)sin_[j]);
+            const double fluxOut = -__dmul_rn((double)sdf[j], a.ih2);
+            const double phid = (double)ph[j];
+            const double reaction = __dmul_rn((double)rp[j], __dadd_rn(1., -phid));
+            const Real dphidt = to_real<Real>(__dadd_rn(__dadd_rn(fluxOut, fluxIn), reaction));
+            const Real q = clamp_state(to_real<Real>(__dadd_rn(phid, __dmul_rn(a.dt, (double)dphidt))));
+            out[i + j] = dom[j] ? q : ph[j];  // outside the domain a clamped value stays (dt is finite)
+        }
+    }
+}
+
+// All steps of an empty block's cell: no coupling, so the reaction alone
+// (cell_rhs with every coefficient +0), until nothing is left of it.
+template <typename Real>
+__device__ __forceinline__ Real empty_cell_steps(Real phi, int nsteps, Real rho, double dt)
+{
+#pragma unroll 1
+    for (int s = 0; s < nsteps; s++) {
+        if (!(phi > (Real)0)) return clamp01(phi);
+        const double reaction = __dmul_rn((double)rmul(rho, phi), __dadd_rn(1., -(double)phi));
+        phi = cell_update(phi, to_real<Real>(__dadd_rn(0., reaction)), dt);
+    }
+    return phi;
+}
+
+// The empty blocks of a run of nsteps steps: state 0 from in, the last state
+// into out0 (and out1, when given), by every thread of the grid.
+template <typename Real>
+__device__ __forceinline__ void empty_blocks(const int *empty, int n_empty, const Real *in, Real *out0, Real *out1,
+                                             int nsteps, Real rho, double dt, unsigned *nan_flag)
+{
+    const int groups = gridDim.x * (blockDim.x >> 7), g = blockIdx.x * (blockDim.x >> 7) + (threadIdx.x >> 7);
+    const int c = (threadIdx.x & 127) * 4;
+    bool bad = false;
+    for (int i = g; i < n_empty; i += groups) {
+        const int64_t at = (int64_t)empty[i] * kBS3 + c;
+        Real v[4];
+        ld_cells(in + at, v);
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < 4; q++) any |= v[q] != (Real)0;
+        if (any) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                v[q] = empty_cell_steps(v[q], nsteps, rho, dt);
+                bad |= v[q] != v[q];
+            }
+        }
+        if (any || out0 != in) st_cells(out0 + at, v);
+        if (out1 && (any || out1 != in)) st_cells(out1 + at, v);
+    }
+    if (bad) atomicOr(nan_flag, 1u);
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(256) empty_run_kernel(const int *empty, int n_empty, const Real *in, Real *out0,
+                                                        Real *out1, int nsteps, Real rho, double dt,
+                                                        unsigned *nan_flag)
+{
+    empty_blocks(empty, n_empty, in, out0, out1, nsteps, rho, dt, nan_flag);
+}
+
+template <typename Real, int kC, int kGroups>
+__global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1) resident_run_kernel(const ResidentArgs<Real> a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ResidentBlock<Real> *blocks = reinterpret_cast<ResidentBlock<Real> *>(smem_raw);
+    using TL = Tile<Real, kC>;
+    constexpr int kT = kBS3 / kC;  // threads of a group
+    constexpr int R = 8 / kC;      // threads of a row
+    const int t = threadIdx.x % kT, group = threadIdx.x / kT, lane = threadIdx.x & 31;
+    const int c = blockIdx.x, G = gridDim.x;
+    const int nlocal = a.n > c ? (a.n - 1 - c) / G + 1 : 0;
+    Place w;
+    w.t = t;
+    w.x0 = (t % R) * kC;
+    w.y = (t / R) & 7;
+    w.z = t / (8 * R);
+    const int row = w.z * 8 + w.y, prow = (w.z + 1) * 10 + w.y + 1;
+    w.tp = prow * R + w.x0 / kC;
+    w.xl = w.x0 ? TL::template at<kRows>(prow, w.x0 - 1) : kRows * 8 + row;
+    w.xr = w.x0 + kC < 8 ? TL::template at<kRows>(prow, w.x0 + kC) : kRows * 8 + 64 + row;
+    w.he = w.x0 + kC < 8 ? TL::template at<64>(row, w.x0 + kC) : kBS3 + row;
+    // the halo vector this thread fetches: kC words of face pf from pw on, to
+    // element pd of the state (vectors pstep elements apart); threads beyond
+    // the 384 halo cells fetch none
+    constexpr bool kAll = kT * kC <= 384;
+    const int pf = t * kC / 64, pw = (t * kC) % 64;
+    const bool fetches = kAll || pf < 6;
+    const int pstep = pf < 2 ? TL::V : kRows * 8 / kC * TL::V;
+    const int pd = pf < 2   ? kRows * 8 + pf * 64 + pw
+                   : pf < 4 ? TL::template at<kRows>((pw / 8 + 1) * 10 + (pf == 2 ? 0 : 9), pw % 8)
+                            : TL::template at<kRows>((pf == 4 ? 0 : 90) + pw / 8 + 1, pw % 8);
+    // the faces its own cells belong to: x (one word), y, z (kC words), -1 none
+    const int sx = w.x0 == 0 ? row : w.x0 + kC == 8 ? 64 + row : -1;
+    const int sy = w.y == 0 ? 128 + w.z * 8 + w.x0 : w.y == 7 ? 192 + w.z * 8 + w.x0 : -1;
+    const int sz = w.z == 0 ? 256 + w.y * 8 + w.x0 : w.z == 7 ? 320 + w.y * 8 + w.x0 : -1;
+    const unsigned k0 = *a.index;  // states stored by earlier launches (mod 4)
+    const int ex_stride = a.n * 384;
+    constexpr unsigned kSign = 0x80000000u;
+    auto phase_of = [&](unsigned k) { return (k & 2u) ? 0u : kSign; };
+    // the faces of a block's state into the exchange buffer
+    auto publish = [&](int item, const Real (&v)[kC], unsigned k) {
+        Real *ex = a.ex + ((k & 1u) ? ex_stride : 0) + item * 384;
+        const unsigned m = phase_of(k);
+        Real u[kC];
+#pragma unroll
+        for (int i = 0; i < kC; i++) u[i] = with_phase(v[i], m);
+        if (kC == 4 || sx >= 0) st_face1(ex + sx, w.x0 ? u[kC - 1] : u[0]);
+        if (sy >= 0) st_face(ex + sy, u);
+        if (sz >= 0) st_face(ex + sz, u);
+    };
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kT) : "memory"); };
+
+    // the group's blocks: state 0, coefficients and cell kinds into shared memory
+    for (int j = group; j < nlocal; j += kGroups) {
+        ResidentBlock<Real> &b = blocks[j];
+        const int item = c + j * G, e = a.items[item];
+        const int64_t blk = e >> 2;
+        const unsigned short *meta = a.meta + blk * kBS3;
+        Real p[kC];
+        ld_cells(a.in + blk * kBS3 + t * kC, p);
+        TL::template store<kRows>(b.st[0].phi, w.tp, p);
+        publish(item, p, k0);
+        const Real *H = a.H + blk * kFacesPerBlock;
+        // face f along a direction touches a kEmpty cell: the cell after it is
+        // kEmpty or has a kEmpty neighbour before it (the last face: the cell
+        // before it, and its neighbour after it)
+        auto touches = [&](int cell, int nb) { return (meta[cell] & 3u) == kEmpty || ((meta[cell] >> (2 + nb)) & 1u); };
+        for (int q = t; q < 576; q += kT) {
+            {
+                const int f = q % 9, row = q / 9;
+                const Real h = set_sign(H[q], f < 8 ? touches(row * 8 + f, 0) : touches(row * 8 + 7, 1));
+                if (f < 8) b.hx[TL::template at<64>(row, f)] = h;
+                else b.hx8[row] = h;
+            }
+            {
+                const int x = q & 7, f = (q >> 3) % 9, zz = q / 72, row = q >> 3;
+                b.hy[TL::template at<72>(row, x)] =
+                    set_sign(H[576 + q], f < 8 ? touches(zz * 64 + f * 8 + x, 2) : touches(zz * 64 + 56 + x, 3));
+            }
+            {
+                const int x = q & 7, yy = (q >> 3) & 7, f = q >> 6, row = q >> 3;
+                b.hz[TL::template at<72>(row, x)] =
+                    set_sign(H[1152 + q], f < 8 ? touches(f * 64 + yy * 8 + x, 4) : touches(448 + yy * 8 + x, 5));
+            }
+        }
+        unsigned kind = kPlain;
+        for (int i = 0; i < kC; i++) {
+            const unsigned m = meta[t * kC + i];
+            if ((m & 3u) == kOther || (m >> 8)) kind = kGeneral;
+            else if (m != kMetaAllTissue && kind == kPlain) kind = kEdge;
+        }
+        if (t == 0) {
+            b.e = e;
+            b.kinds = 0;
+        }
+        if (t < 6) {
+            const int nb = a.nbr[item * 6 + t];
+            b.nbr[t] = nb < 0 ? -1 : nb * 384;
+        }
+        if (fetches && a.nbr[item * 6 + pf] < 0) {  // an empty neighbour: +0 for good
+            for (int v = 0; v < kC / TL::V; v++)
+                for (int i = 0; i < TL::V; i++) b.st[0].phi[pd + v * pstep + i] = b.st[1].phi[pd + v * pstep + i] = (Real)0;
+        }
+        group_sync();
+        const bool general = __any_sync(0xffffffffu, kind == kGeneral), edge = __any_sync(0xffffffffu, kind == kEdge);
+        if (lane == 0) atomicOr(&b.kinds, (general ? kGeneral : edge ? kEdge : kPlain) << (2 * (t >> 5)));
+    }
+    group_sync();
+
+    bool failed = false, bad = false;
+    for (int s = 0; s < a.nsteps; s++) {
+        const unsigned k = k0 + s;
+        const unsigned m = phase_of(k);
+        const Real *ex = a.ex + ((k & 1u) ? ex_stride : 0);
+        const bool last = s == a.nsteps - 1;
+        Real *store = a.stores ? a.stores[s] : (last ? a.out : nullptr);
+        for (int j = group; j < nlocal; j += kGroups) {
+            ResidentBlock<Real> &b = blocks[j];
+            ResidentState<Real> &S = b.st[s & 1];
+            // the halos of state k: the neighbour across face pf stores its face pf ^ 1
+            if (fetches) {
+                const int nb = b.nbr[pf];
+                if (nb >= 0) {
+                    const Real *src = ex + (nb + (pf ^ 1) * 64 + pw);
+                    Real h[kC];
+                    unsigned long long t0 = 0;
+                    for (int it = 0;; it++) {
+                        ld_face(src, h);
+                        unsigned wrong = 0;
+#pragma unroll
+                        for (int i = 0; i < kC; i++) wrong |= sign_xor(h[i], m);
+                        if (!(wrong & kSign)) break;
+                        if ((it & 63) == 63) {
+                            if (t0 == 0) t0 = now_ns();
+                            else if (now_ns() - t0 > kPollNs || it > (1 << 24)) {
+                                failed = true;
+                                break;
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int v = 0; v < kC / TL::V; v++) {
+                        Real g[TL::V];
+#pragma unroll
+                        for (int i = 0; i < TL::V; i++) g[i] = magnitude(h[v * TL::V + i]);
+                        st_cells(S.phi + pd + v * pstep, g);
+                    }
+                }
+            }
+            // the group's halos are in place, its reads of the state before
+            // are over and its writes of state k are seen; a thread that gave
+            // up takes its whole group out
+            unsigned any;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.ne.u32 p, %1, 0;\n\t"
+                "barrier.cta.red.or.pred q, %2, %3, p;\n\t"
+                "selp.u32 %0, 1, 0, q;\n\t}"
+                : "=r"(any)
+                : "r"((unsigned)failed), "r"(group + 1), "n"(kT)
+                : "memory");
+            if (any) {
+                if (t == 0) atomicOr(a.err_flag, kErrPoll);
+                goto out;
+            }
+            Real o[kC];
+            const unsigned kind = (b.kinds >> (2 * (t >> 5))) & 3u;
+            if (kind == kPlain) row_cells<Real, kC, kPlain>(a, b, S, w, o);
+            else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, b, S, w, o);
+            else row_cells<Real, kC, kGeneral>(a, b, S, w, o);
+            if (!last) {
+                publish(c + j * G, o, k + 1);
+                TL::template store<kRows>(b.st[(s + 1) & 1].phi, w.tp, o);
+            } else {
+#pragma unroll
+                for (int i = 0; i < kC; i++) bad |= o[i] != o[i];  // a NaN stays one: the last state shows it
+            }
+            if (store) st_cells(store + (int64_t)(b.e >> 2) * kBS3 + t * kC, o);
+        }
+    }
+out:
+    if (bad) atomicOr(a.nan_flag, 1u);
+    if (a.n_empty > 0)
+        empty_blocks(a.empty, a.n_empty, a.in, a.out, (Real *)nullptr, a.nsteps, a.rho, a.dt, a.nan_flag);
+    // the last CTA to leave advances the state count for the next launch
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (atomicAdd(a.index + 1, 1u) == (unsigned)G - 1) {
+            a.index[1] = 0;
+            a.index[0] = (k0 + (unsigned)a.nsteps) & 3u;
+        }
+    }
+}
+
+constexpr int kMaxSmem = 227 * 1024;
+
+template <typename Real, int kC, int kGroups>
+cudaError_t launch(const ResidentArgs<Real> &a, int ctas, size_t smem, cudaStream_t s)
+{
+    // the kernel's shared memory limit is raised once per device
+    static std::mutex mu;
+    static std::vector<char> raised;
+    auto kernel = resident_run_kernel<Real, kC, kGroups>;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if ((int)raised.size() <= dev) raised.resize(dev + 1, 0);
+        if (!raised[dev]) {
+            if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)) !=
+                cudaSuccess)
+                return e;
+            raised[dev] = 1;
+        }
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kGroups * (kBS3 / kC));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+}  // namespace
+
+template <typename Real>
+int resident_capacity(int sms)
+{
+    return sms * (kMaxSmem / (int)sizeof(ResidentBlock<Real>));
+}
+
+template <typename Real>
+cudaError_t launch_resident_run(const ResidentArgs<Real> &a, int sms, cudaStream_t s)
+{
+    if (a.n <= 0 || a.nsteps <= 0 || a.n > resident_capacity<Real>(sms)) return cudaErrorInvalidValue;
+    const int ctas = a.n < sms ? a.n : sms;
+    const int per = (a.n + ctas - 1) / ctas;
+    const size_t smem = (size_t)per * sizeof(ResidentBlock<Real>);
+    // Threads per block and groups per CTA by the blocks of a CTA, FP32 (us per
+    // step on a B200, 1000 steps): up to two blocks the step is a chain of
+    // latencies, which two cells per thread shorten (64^3, 2 per CTA: 1.22
+    // against 1.32 with four); beyond, four cells per thread cost fewer
+    // instructions and every block gets a group of its own while the registers
+    // last (96^3, 3 per CTA: 1.48 with four groups, 1.56 with seven; 128^3, 7
+    // per CTA: 2.02 with seven, 2.55 with four, 2.13 with eight, whose 64
+    // registers spill; 160^3, 14 per CTA: 3.48 with seven, 4.76 with four).
+    // FP64 needs 128 registers for four cells: four groups (128^3: 3.14; 3.68
+    // with seven, 4.78 with two cells per thread).
+    if (per <= 2) return launch<Real, 2, 2>(a, ctas, smem, s);
+    if constexpr (sizeof(Real) == 4)
+        if (per > 4) return launch<Real, 4, 7>(a, ctas, smem, s);
+    return launch<Real, 4, 4>(a, ctas, smem, s);
+}
+
+template <typename Real>
+cudaError_t launch_empty_run(const int *empty, int n_empty, const Real *in, Real *out0, Real *out1, int nsteps,
+                             Real rho, double dt, unsigned *nan_flag, cudaStream_t s)
+{
+    if (n_empty <= 0) return cudaSuccess;
+    const int grid = (n_empty + 1) / 2 < 148 * 8 ? (n_empty + 1) / 2 : 148 * 8;
+    empty_run_kernel<Real><<<grid, 256, 0, s>>>(empty, n_empty, in, out0, out1, nsteps, rho, dt, nan_flag);
+    return cudaGetLastError();
+}
+
+template int resident_capacity<float>(int);
+template int resident_capacity<double>(int);
+template cudaError_t launch_resident_run<float>(const ResidentArgs<float> &, int, cudaStream_t);
+template cudaError_t launch_resident_run<double>(const ResidentArgs<double> &, int, cudaStream_t);
+template cudaError_t launch_empty_run<float>(const int *, int, const float *, float *, float *, int, float, double,
+                                             unsigned *, cudaStream_t);
+template cudaError_t launch_empty_run<double>(const int *, int, const double *, double *, double *, int, double,
+                                              double, unsigned *, cudaStream_t);
+
+}  // namespace gbfk

@@ -137,16 +137,20 @@ int gbfk_download_dense(gbfk_ctx *ctx, int field, void *host, int n);
 int gbfk_rd_step(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int nsteps,
                  int check_nan);
 /* Which kernel runs the step (no counterpart in the reference: the
- * reference has one CPU operator).  GBFK_STEP_AUTO (the default) runs the
- * persistent TMA-fed pipeline where it applies -- a uniform periodic
- * power-of-two grid from gbfk_set_uniform -- and the one-CTA-per-block kernel
- * elsewhere; all give bit-identical results.  GBFK_STEP_RUN runs the
- * pipeline over all steps of a gbfk_rd_step call in one cooperative launch
- * (the first step alone when phi was uploaded since the last step): each
+ * reference has one CPU operator); all give bit-identical results.
+ * GBFK_STEP_AUTO (the default), for a call of several steps on a uniform
+ * grid from gbfk_set_uniform, runs them in one cooperative launch with the
+ * blocks that hold tissue resident in shared memory (reported as
+ * GBFK_STEP_RUN), where they fit: about 2200 blocks in FP32, 1180 in FP64 on
+ * a B200.  Otherwise it runs the persistent TMA-fed pipeline on uniform
+ * power-of-two grids (in calls of several steps without the blocks that hold
+ * no tissue, whose cells only react and take all steps in a launch of their
+ * own) and the one-CTA-per-block kernel elsewhere.  The first step after phi
+ * was uploaded always runs by itself.  GBFK_STEP_RUN runs the pipeline over
+ * all steps of a gbfk_rd_step call in one cooperative launch: each
  * CTA keeps its blocks and, between steps, waits only for the CTAs that
- * own their face neighbours.  On a B200 it is within a few percent of one
- * launch per step (3% faster at 128^3 in FP32, up to 5% slower in FP64),
- * so AUTO does not pick it.  GBFK_STEP_PIPELINED or GBFK_STEP_RUN on a
+ * own their face neighbours (within a few percent of one launch per step on
+ * a B200).  GBFK_STEP_PIPELINED or GBFK_STEP_RUN on a
  * grid they do not apply to make gbfk_rd_step return GBFK_E_STATE.
  * gbfk_step_kernel reports the kernel of the last gbfk_rd_step (0 before
  * any).  A pipeline stage whose copies never complete, or a neighbour that

@@ -1,0 +1,143 @@
+"""Runs of steps with the blocks resident in shared memory (AUTO, from a few
+steps per call on, any uniform grid) against the one-CTA-per-block kernel, bit
+for bit: one block that is its own neighbour, block counts that are no power
+of two, tumour outside the anatomy (empty blocks whose cells react by
+themselves), values below 0 and above 1, tissue fractions below 0.1 (cells
+that read p_w and p_g), every launch shape and the fallback of grids whose
+blocks do not fit."""
+import threading
+
+import numpy as np
+import pytest
+
+from gliomasolver_b200 import BlockPool, GbfkError
+from gliomasolver_b200.anatomy import make_case
+from gliomasolver_b200.schedule import make_schedule
+
+pytestmark = pytest.mark.gpu
+
+
+def _fields(n, seed, prec):
+    R = np.float64 if prec == "f64" else np.float32
+    pw, pg, c0, _ = make_case(n, seed)
+    rng = np.random.default_rng(seed + 50)
+    c0 = np.maximum(c0, rng.uniform(0, 1, c0.shape) * (rng.uniform(0, 1, c0.shape) < 0.03))
+    c0[0, 0, :] = 1.7
+    c0[1, :, 2] = -0.3
+    pw[n // 2, :, : n // 3] = 0.0
+    pg[n // 2, :, : n // 3] = 0.0
+    thin = rng.uniform(0, 1, c0.shape) < 0.02
+    pw[thin] *= 0.08
+    pg[thin] *= 0.08
+    return [a.astype(R) for a in (pw, pg, c0)]
+
+
+def _pool(n, prec, fields, stream=None):
+    pool = BlockPool((n // 8) ** 3, prec, stream=stream)
+    pool.set_uniform(n // 8)
+    for name, a in zip(("p_w", "p_g", "phi"), fields):
+        pool.upload_dense(name, a)
+    return pool
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("n,seed,steps", [(8, 3, 7), (16, 2, 30), (24, 1, 4), (72, 5, 9), (128, 1, 40), (168, 2, 5)])
+def test_resident_run_equals_block_steps(gbfk_lib, prec, n, seed, steps):
+    fields = _fields(n, seed, prec)
+    s = make_schedule(0.3, 0.2, 300.0, 25.6, n // 8, prec)
+    with _pool(n, prec, fields) as a, _pool(n, prec, fields) as b:
+        b.step_kernel = "block"
+        # the second call starts from a clamped state, the third from an
+        # uploaded one again; the face phase goes on from call to call
+        for k, again in ((steps, False), (steps + 3, False), (steps, True)):
+            for p in (a, b):
+                if again:
+                    p.upload_dense("phi", fields[2])
+                p.rd_step(s.Dw, s.Dg, s.rho, s.dt, k, check_nan=True)
+            assert np.array_equal(a.download_dense("phi"), b.download_dense("phi"))
+        # 168^3 in FP64 has more heavy blocks than the SMs hold
+        if (n, prec) != (168, "f64") and steps > 6:
+            assert a.step_kernel == "run"
+
+
+def test_steps_that_leave_out_the_empty_blocks(gbfk_lib):
+    """256^3 does not fit: launches over the blocks with tissue, the empty
+    blocks' steps (some hold tumour) in one launch, odd and even step counts."""
+    n, prec = 256, "f32"
+    fields = _fields(n, 4, prec)
+    s = make_schedule(0.3, 0.2, 300.0, 25.6, n // 8, prec)
+    with _pool(n, prec, fields) as a, _pool(n, prec, fields) as b:
+        b.step_kernel = "block"
+        for k in (4, 3, 5):
+            for p in (a, b):
+                p.rd_step(s.Dw, s.Dg, s.rho, s.dt, k, check_nan=True)
+            assert np.array_equal(a.download_dense("phi"), b.download_dense("phi"))
+
+
+@pytest.mark.parametrize("n", [32, 56])
+def test_nan_in_a_resident_run_is_reported(gbfk_lib, n):
+    fields = _fields(n, 1, "f32")
+    fields[2][n // 2, n // 2, n // 2] = np.nan
+    s = make_schedule(0.2, 0.05, 300.0, 25.6, n // 8, "f32")
+    with _pool(n, "f32", fields) as pool:
+        with pytest.raises(GbfkError) as e:
+            pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 20, check_nan=True)
+        assert e.value.code == 4
+
+
+def test_resident_run_replayed_from_a_graph(gbfk_lib):
+    """A run captured in a CUDA graph and replayed, with runs outside the
+    graph in between: the state count on the device keeps the face phase."""
+    import torch
+
+    n, prec = 48, "f32"
+    fields = _fields(n, 6, prec)
+    s = make_schedule(0.2, 0.05, 300.0, 25.6, n // 8, prec)
+    st = torch.cuda.Stream()
+    with _pool(n, prec, fields, st.cuda_stream) as a, _pool(n, prec, fields) as b:
+        b.step_kernel = "block"
+        a.rd_step(s.Dw, s.Dg, s.rho, s.dt, 8)
+        a.sync()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            a.rd_step(s.Dw, s.Dg, s.rho, s.dt, 7)
+        total = 8
+        for _ in range(3):
+            with torch.cuda.stream(st):
+                g.replay()
+            a.rd_step(s.Dw, s.Dg, s.rho, s.dt, 9)
+            total += 16
+        b.rd_step(s.Dw, s.Dg, s.rho, s.dt, total)
+        a.sync()
+        assert np.array_equal(a.download_dense("phi"), b.download_dense("phi"))
+        del g
+
+
+def test_two_pools_from_two_threads(gbfk_lib):
+    """Two contexts stepped from two threads at once, each in many runs."""
+    cases = [(64, "f32", 3), (96, "f64", 4)]
+    want, got, errors = {}, {}, []
+
+    def go(n, prec, seed, kind, out):
+        try:
+            fields = _fields(n, seed, prec)
+            s = make_schedule(0.2, 0.05, 300.0, 25.6, n // 8, prec)
+            with _pool(n, prec, fields) as pool:
+                pool.step_kernel = kind
+                for _ in range(25):
+                    pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 20)
+                pool.sync()
+                out[n] = pool.download_dense("phi")
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    for c in cases:
+        go(*c, "block", want)
+    threads = [threading.Thread(target=go, args=(*c, "auto", got)) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for n, _, _ in cases:
+        assert np.array_equal(got[n], want[n])
