@@ -552,18 +552,9 @@ template <typename Real>
 int build_resident(gbfk_ctx *ctx)
 {
     if (ctx->res_ready) return GBFK_OK;
-    const int n = ctx->n_heavy, nb = ctx->nblocks, bpd = ctx->bpd;
-    std::vector<int> at(nb, -1), nbr((size_t)n * 6);
-    for (int i = 0; i < n; i++) at[ctx->h_lists[i] >> 2] = i;
-    for (int i = 0; i < n; i++) {
-        const int b = ctx->h_lists[i] >> 2;
-        const int p[3] = {b % bpd, (b / bpd) % bpd, b / (bpd * bpd)};
-        for (int f = 0; f < 6; f++) {
-            int q[3] = {p[0], p[1], p[2]};
-            q[f >> 1] = (q[f >> 1] + ((f & 1) ? 1 : bpd - 1)) % bpd;
-            nbr[(size_t)i * 6 + f] = at[q[0] + bpd * (q[1] + bpd * q[2])];
-        }
-    }
+    const int n = ctx->n_heavy;
+    std::vector<int> nbr;
+    resident_neighbours(ctx->bpd, ctx->h_lists.data(), n, nbr);
     const size_t ex = (size_t)2 * n * 384 * sizeof(Real);
     int rc = topo_alloc(ctx, &ctx->d_res_nbr, nbr.size() * sizeof(int));
     if (!rc) rc = topo_alloc(ctx, &ctx->d_res_ex, ex);
@@ -649,7 +640,8 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     // empty blocks, whose steps are made up in one launch (nothing couples
     // them to the others while every coefficient is finite)
     const bool uncoupled = ctx->step_pref == GBFK_STEP_AUTO && ctx->uniform && ctx->identity_slots &&
-                           std::isfinite(dt) && std::isfinite((double)(Real)Dw) && std::isfinite((double)(Real)Dg);
+                           std::isfinite(dt) && std::isfinite((double)(Real)Dw) && std::isfinite((double)(Real)Dg) &&
+                           std::isfinite((double)(Real)rho);
     const int clamped_steps = ctx->phi_clamped ? nsteps : nsteps - 1;
     bool want_run = uncoupled && clamped_steps >= (pipelined ? kResidentSteps : kResidentStepsBlock);
     if (want_run && (!ctx->res_ready || !ctx->lists_valid)) {

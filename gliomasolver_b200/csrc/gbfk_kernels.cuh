@@ -165,12 +165,27 @@ struct ResidentArgs {
     Real *ex;
     unsigned *index;
     unsigned *nan_flag, *err_flag;
+    unsigned start = 0;  // resident_teams: states the exchange buffer carried before (mod 4)
     unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
 };
+// appends the table `nbr` of n heavy blocks of a uniform periodic bpd^3 grid
+void resident_neighbours(int bpd, const int *items, int n, std::vector<int> &nbr);
 template <typename Real>
 int resident_capacity(int sms);
+// about how long a step of a run takes with `per` blocks per CTA (to plan with)
+template <typename Real>
+double resident_step_us(int per);
 template <typename Real>
 cudaError_t launch_resident_run(const ResidentArgs<Real> &a, int sms, cudaStream_t s);
+// Many such runs in one launch: `teams` teams of `size` CTAs; team g takes the
+// runs off[g] .. off[g + 1] of the device array `runs`, one after the other
+// (index unused: start instead; n_empty and stores unused).  Runs of one team
+// with the same item list share an exchange buffer, zeroed before the launch,
+// and count its states in `start`.  per: the most blocks of a CTA,
+// ceil(largest n / size); ih2: of all of them.
+template <typename Real>
+cudaError_t launch_resident_teams(const ResidentArgs<Real> *runs, const int *off, int teams, int size, int per,
+                                  double ih2, cudaStream_t s);
 // nsteps steps of the empty blocks alone, from `in` into out0 and (unless
 // NULL) out1: the company of nsteps launches that skip them.
 template <typename Real>

@@ -16,9 +16,10 @@
 // block grid takes) plus the issue of its cells' exact-rounding arithmetic
 // (128^3, FP32: 1.69 M warp instructions per step, 67 % of the issue slots).
 // Measured on a B200, us per step over 1000 steps, against one launch per
-// step: 64^3 FP32 1.22 (3.74), FP64 1.40 (3.87); 128^3 FP32 2.02 (6.33),
-// FP64 3.14 (8.59); 120^3, which had the one-CTA-per-block kernel, FP32 12.2
-// before.
+// step: 64^3 FP32 1.16 (3.74), FP64 1.36 (3.87); 128^3 FP32 1.94 (6.33), FP64
+// 3.06 (8.59); 160^3 FP32 3.27 (17.2, one CTA per block).  A stage by teams
+// of CTAs, 15 blocks per CTA: 128^3 FP32 2.0 us per sample-step (3.7 in
+// launches over all samples), 64^3 0.39 (0.9).
 //
 // Faces travel through L2.  After forming state k a block stores its six
 // faces in the exchange buffer k & 1 and its neighbours poll for them there.
@@ -43,6 +44,7 @@
 
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "gbfk_exact.cuh"
@@ -145,9 +147,9 @@ __device__ __forceinline__ double magnitude(double v)
 // if they are fewer) as [vector][thread], so that a warp's access is one
 // contiguous run of banks for every neighbour offset; rows of a face array
 // count as threads too (kRows rows of 8).
-template <typename Real, int kC>
+template <typename Real, int kC, int kMaxV = 16 / (int)sizeof(Real)>
 struct Tile {
-    static constexpr int V = 16 / (int)sizeof(Real) < kC ? 16 / (int)sizeof(Real) : kC;
+    static constexpr int V = kMaxV < kC ? kMaxV : kC;
     // where cell x of a row lies in an array of kRows rows
     template <int kRows>
     static __device__ __forceinline__ int at(int row, int x)
@@ -172,6 +174,25 @@ struct Tile {
                 const double2 q = *reinterpret_cast<const double2 *>(p);
                 d[2 * v] = q.x; d[2 * v + 1] = q.y;
             }
+        }
+    }
+    // pair v of thread t of an array with two-value vectors
+    template <int kRows>
+    static __device__ __forceinline__ int at2(int t, int v)
+    {
+        static_assert(V == 2, "pairs");
+        return (v * (kRows * 8 / kC) + t) * 2;
+    }
+    template <int kRows>
+    static __device__ __forceinline__ void load2(const Real *a, int t, int v, Real (&d)[2])
+    {
+        const Real *p = a + at2<kRows>(t, v);
+        if constexpr (sizeof(Real) == 4) {
+            const float2 q = *reinterpret_cast<const float2 *>(p);
+            d[0] = q.x; d[1] = q.y;
+        } else {
+            const double2 q = *reinterpret_cast<const double2 *>(p);
+            d[0] = q.x; d[1] = q.y;
         }
     }
     template <int kRows>
@@ -226,8 +247,8 @@ __device__ __forceinline__ void st_cells(Real *p, const Real (&d)[kC])
 
 // One resident block in shared memory: two states, each with its face halos
 // (rows y = -1 .. 8 of planes z = -1 .. 8, and the x faces apart), and the
-// face coefficients: x faces as eight left faces per row and the row's last
-// face apart, y and z faces as in H.  A coefficient carries a set sign bit
+// face coefficients, in two-value vectors: x faces as eight left faces per row
+// and the row's last face apart, y and z faces as in H.  A coefficient carries a set sign bit
 // where either cell of the face is kEmpty (see row_cells).
 constexpr int kRows = 100;
 template <typename Real>
@@ -316,11 +337,27 @@ __device__ __noinline__ void tissue_at(const Real *pw_all, const Real *pg_all, i
 // What a thread needs to know of its place in a block, fixed for the run.
 struct Place {
     int t;        // thread of the group
-    int x0, y, z; // its cells: x0 .. x0 + kC - 1 of row (y, z)
     int tp;       // its place in the padded state array
-    int xl, xr;   // element offsets in ResidentState of the cells before and after them
+    int ty;       // its place in hy
+    int xl, xr;   // element offsets in ResidentState of the cells before and after its own
     int he;       // element offset from hx of the last cell's right face
 };
+template <typename Real, int kC>
+__device__ __forceinline__ Place place_of(int t)
+{
+    using TL = Tile<Real, kC, 2>;
+    constexpr int R = 8 / kC;  // threads of a row
+    const int x0 = (t % R) * kC, y = (t / R) & 7, z = t / (8 * R);
+    const int row = z * 8 + y, prow = (z + 1) * 10 + y + 1;
+    Place w;
+    w.t = t;
+    w.tp = prow * R + x0 / kC;
+    w.ty = t + z * R;  // row z * 9 + y
+    w.xl = x0 ? TL::template at<kRows>(prow, x0 - 1) : kRows * 8 + row;
+    w.xr = x0 + kC < 8 ? TL::template at<kRows>(prow, x0 + kC) : kRows * 8 + 64 + row;
+    w.he = x0 + kC < 8 ? Tile<Real, kC, 2>::template at<64>(row, x0 + kC) : kBS3 + row;
+    return w;
+}
 
 // The kC cells of a thread in block b, from the state S with its halos (a
 // clamped state) to out.  kKind, by warp:
@@ -334,42 +371,41 @@ struct Place {
 //             formula leaves +0 where phi is +0 and the reaction where it is
 //             not, so that its domain test needs no branch).  -0 for +0 in
 //             the flux sums gives the same sums: (+0) + (-0) = +0 either way;
-//   kGeneral  kOther cells or neighbours: classes from the meta words, p_w
-//             and p_g from global memory.
+//   kGeneral  kOther cells or neighbours, or a coefficient that is negative
+//             by itself: classes from the meta words, p_w and p_g from global
+//             memory.
 template <typename Real, int kC, unsigned kKind>
-__device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, const ResidentBlock<Real> &b,
-                                          const ResidentState<Real> &S, const Place &w, Real (&out)[kC])
+__device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, double ih2, unsigned long long neg0,
+                                          const ResidentBlock<Real> &b, const ResidentState<Real> &S, const Place &w,
+                                          Real (&out)[kC])
 {
-    using TL = Tile<Real, kC>;
+    using TL = Tile<Real, kC, 2>;
     constexpr int R = 8 / kC;  // threads of a row
-    Real p[kC], ym[kC], yp[kC], zm[kC], zp[kC];
+    Real p[kC];
     TL::template load<kRows>(S.phi, w.tp, p);
     const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
-    TL::template load<kRows>(S.phi, w.tp - R, ym);
-    TL::template load<kRows>(S.phi, w.tp + R, yp);
-    TL::template load<kRows>(S.phi, w.tp - 10 * R, zm);
-    TL::template load<kRows>(S.phi, w.tp + 10 * R, zp);
-    Real hx[kC], hym[kC], hyp[kC], hzm[kC], hzp[kC];
-    TL::template load<64>(b.hx, w.t, hx);
-    const Real hx_end = b.hx[w.he];
-    const int ty = w.t + w.z * R;  // row z * 9 + y of hy
-    TL::template load<72>(b.hy, ty, hym);
-    TL::template load<72>(b.hy, ty + R, hyp);
-    TL::template load<72>(b.hz, w.t, hzm);
-    TL::template load<72>(b.hz, w.t + 8 * R, hzp);
     const Real eps = (Real)0.1;
     constexpr bool kLow = kKind != kPlain;
     // two cells at a time, so that the single-precision operations of the flux
-    // sums can go in pairs (pair_add, pair_mul: each half rounded by itself)
+    // sums can go in pairs (pair_add, pair_mul: each half rounded by itself),
+    // and only one pair's coefficients are held at once
 #pragma unroll
     for (int i = 0; i < kC; i += 2) {
         const Real ph[2] = {p[i], p[i + 1]};
         const Real xm[2] = {i ? p[i - 1] : xl, p[i]}, xp[2] = {p[i + 1], i + 2 < kC ? p[i + 2] : xr};
-        Real d0[2] = {hx[i], hx[i + 1]}, d1[2] = {hx[i + 1], i + 2 < kC ? hx[i + 2] : hx_end};
-        Real d2[2] = {hym[i], hym[i + 1]}, d3[2] = {hyp[i], hyp[i + 1]}, d4[2] = {hzm[i], hzm[i + 1]},
-             d5[2] = {hzp[i], hzp[i + 1]};
-        const Real y0[2] = {ym[i], ym[i + 1]}, y1[2] = {yp[i], yp[i + 1]}, z0[2] = {zm[i], zm[i + 1]},
-                   z1[2] = {zp[i], zp[i + 1]};
+        Real d0[2], d1[2], d2[2], d3[2], d4[2], d5[2];
+        TL::template load2<64>(b.hx, w.t, i / 2, d0);
+        d1[0] = d0[1];
+        d1[1] = i + 2 < kC ? b.hx[TL::template at2<64>(w.t, i / 2 + 1)] : b.hx[w.he];
+        TL::template load2<72>(b.hy, w.ty, i / 2, d2);
+        TL::template load2<72>(b.hy, w.ty + R, i / 2, d3);
+        TL::template load2<72>(b.hz, w.t, i / 2, d4);
+        TL::template load2<72>(b.hz, w.t + 8 * R, i / 2, d5);
+        Real y0[2], y1[2], z0[2], z1[2];
+        TL::template load2<kRows>(S.phi, w.tp - R, i / 2, y0);
+        TL::template load2<kRows>(S.phi, w.tp + R, i / 2, y1);
+        TL::template load2<kRows>(S.phi, w.tp - 10 * R, i / 2, z0);
+        TL::template load2<kRows>(S.phi, w.tp + 10 * R, i / 2, z1);
         bool dom[2] = {true, true};
         if (kLow) {
 #pragma unroll
@@ -379,18 +415,20 @@ __device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, const Res
                                sign_of(d4[j]) && z0[j] < eps, sign_of(d5[j]) && z1[j] < eps};
                 if (kKind == kGeneral) {
                     const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
-                    const int blk = b.e >> 2;
-                    const unsigned mw = a.meta[(int64_t)blk * kBS3 + w.t * kC + i + j];
+                    const int blk = b.e >> 2, cell = w.t * kC + i + j, x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
+                    const unsigned mw = a.meta[(int64_t)blk * kBS3 + cell];
+#pragma unroll
+                    for (int k = 0; k < 6; k++) low[k] = ((mw >> (2 + k)) & 1u) && phn[k] < eps;
                     Real pw, pg;
                     if ((mw & 3u) == kOther) {
-                        tissue_at(a.pw, a.pg, a.bpd, blk, w.x0 + i + j, w.y, w.z, pw, pg);
+                        tissue_at(a.pw, a.pg, a.bpd, blk, x, y, z, pw, pg);
                         dom[j] = in_domain(pw, pg, ph[j]);
                     }
 #pragma unroll
                     for (int k = 0; k < 6; k++)
                         if ((mw >> (8 + k)) & 1u) {
-                            tissue_at(a.pw, a.pg, a.bpd, blk, w.x0 + i + j + (k == 1) - (k == 0),
-                                      w.y + (k == 3) - (k == 2), w.z + (k == 5) - (k == 4), pw, pg);
+                            tissue_at(a.pw, a.pg, a.bpd, blk, x + (k == 1) - (k == 0), y + (k == 3) - (k == 2),
+                                      z + (k == 5) - (k == 4), pw, pg);
                             low[k] = domain_chf(phn[k], pw, pg) < eps;
                         }
                 }
@@ -406,33 +444,34 @@ __device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, const Res
         // cell_rhs: the same operations in the same order for both cells
         Real sin_[2] = {rmul(d0[0], xm[0]), rmul(d0[1], xm[1])}, u[2] = {rmul(d1[0], xp[0]), rmul(d1[1], xp[1])};
         pair_add(sin_, u);
-        pair_mul(u, d2, y0, a.neg0);
+        pair_mul(u, d2, y0, neg0);
         pair_add(sin_, u);
-        pair_mul(u, d3, y1, a.neg0);
+        pair_mul(u, d3, y1, neg0);
         pair_add(sin_, u);
-        pair_mul(u, d4, z0, a.neg0);
+        pair_mul(u, d4, z0, neg0);
         pair_add(sin_, u);
-        pair_mul(u, d5, z1, a.neg0);
+        pair_mul(u, d5, z1, neg0);
         pair_add(sin_, u);
         Real sdf[2] = {radd(d0[0], d1[0]), radd(d0[1], d1[1])};
         pair_add(sdf, d2);
         pair_add(sdf, d3);
         pair_add(sdf, d4);
         pair_add(sdf, d5);
-        pair_mul(sdf, sdf, ph, a.neg0);
+        pair_mul(sdf, sdf, ph, neg0);
         const Real rr[2] = {a.rho, a.rho};
         Real rp[2];
-        pair_mul(rp, rr, ph, a.neg0);
+        pair_mul(rp, rr, ph, neg0);
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const double fluxIn = __dmul_rn(a.ih2, (double)sin_[j]);
-            const double fluxOut = -__dmul_rn((double)sdf[j], a.ih2);
+            const double fluxIn = __dmul_rn(ih2, (double)sin_[j]);
+            const double fluxOut = -__dmul_rn((double)sdf[j], ih2);
             const double phid = (double)ph[j];
             const double reaction = __dmul_rn((double)rp[j], __dadd_rn(1., -phid));
             const Real dphidt = to_real<Real>(__dadd_rn(__dadd_rn(fluxOut, fluxIn), reaction));
             const Real q = clamp_state(to_real<Real>(__dadd_rn(phid, __dmul_rn(a.dt, (double)dphidt))));
             out[i + j] = dom[j] ? q : ph[j];  // outside the domain a clamped value stays (dt is finite)
         }
+        if (i + 2 < kC) asm volatile("" ::: "memory");
     }
 }
 
@@ -487,27 +526,26 @@ __global__ void __launch_bounds__(256) empty_run_kernel(const int *empty, int n_
     empty_blocks(empty, n_empty, in, out0, out1, nsteps, rho, dt, nan_flag);
 }
 
-template <typename Real, int kC, int kGroups>
-__global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1) resident_run_kernel(const ResidentArgs<Real> a)
+// One run: the blocks of CTA c of G, from state 0 (a.in) to state a.nsteps;
+// k0: the states these words of the exchange buffer have carried before (mod
+// 4).  False when a face never came (the caller's CTA then leaves).
+// The run's arguments lie in constant or shared memory and are read where they
+// are used (the waits in between keep the compiler from holding them): with
+// 72 registers a thread, what is held spills, and beside 200 KB of blocks the
+// spills of 896 threads do not fit in L1 (a 128^3 FP32 stage by teams took 3.7
+// us per sample-step with 120 bytes spilled, 2.0 with none).
+template <typename Real, int kC, int kGroups, bool kStores>
+__device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double ih2, unsigned long long neg0,
+                                           ResidentBlock<Real> *blocks, const int &c, const int &G,
+                                           const unsigned &k0)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ResidentBlock<Real> *blocks = reinterpret_cast<ResidentBlock<Real> *>(smem_raw);
-    using TL = Tile<Real, kC>;
+    using TL = Tile<Real, kC, 2>;
     constexpr int kT = kBS3 / kC;  // threads of a group
     constexpr int R = 8 / kC;      // threads of a row
     const int t = threadIdx.x % kT, group = threadIdx.x / kT, lane = threadIdx.x & 31;
-    const int c = blockIdx.x, G = gridDim.x;
     const int nlocal = a.n > c ? (a.n - 1 - c) / G + 1 : 0;
-    Place w;
-    w.t = t;
-    w.x0 = (t % R) * kC;
-    w.y = (t / R) & 7;
-    w.z = t / (8 * R);
-    const int row = w.z * 8 + w.y, prow = (w.z + 1) * 10 + w.y + 1;
-    w.tp = prow * R + w.x0 / kC;
-    w.xl = w.x0 ? TL::template at<kRows>(prow, w.x0 - 1) : kRows * 8 + row;
-    w.xr = w.x0 + kC < 8 ? TL::template at<kRows>(prow, w.x0 + kC) : kRows * 8 + 64 + row;
-    w.he = w.x0 + kC < 8 ? TL::template at<64>(row, w.x0 + kC) : kBS3 + row;
+    const Place w = place_of<Real, kC>(t);
+    const int x0 = (t % R) * kC, y = (t / R) & 7, z = t / (8 * R), row = z * 8 + y;
     // the halo vector this thread fetches: kC words of face pf from pw on, to
     // element pd of the state (vectors pstep elements apart); threads beyond
     // the 384 halo cells fetch none
@@ -519,26 +557,25 @@ __global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1) resident_run_kernel(
                    : pf < 4 ? TL::template at<kRows>((pw / 8 + 1) * 10 + (pf == 2 ? 0 : 9), pw % 8)
                             : TL::template at<kRows>((pf == 4 ? 0 : 90) + pw / 8 + 1, pw % 8);
     // the faces its own cells belong to: x (one word), y, z (kC words), -1 none
-    const int sx = w.x0 == 0 ? row : w.x0 + kC == 8 ? 64 + row : -1;
-    const int sy = w.y == 0 ? 128 + w.z * 8 + w.x0 : w.y == 7 ? 192 + w.z * 8 + w.x0 : -1;
-    const int sz = w.z == 0 ? 256 + w.y * 8 + w.x0 : w.z == 7 ? 320 + w.y * 8 + w.x0 : -1;
-    const unsigned k0 = *a.index;  // states stored by earlier launches (mod 4)
-    const int ex_stride = a.n * 384;
+    const int sx = x0 == 0 ? row : x0 + kC == 8 ? 64 + row : -1;
+    const int sy = y == 0 ? 128 + z * 8 + x0 : y == 7 ? 192 + z * 8 + x0 : -1;
+    const int sz = z == 0 ? 256 + y * 8 + x0 : z == 7 ? 320 + y * 8 + x0 : -1;
     constexpr unsigned kSign = 0x80000000u;
     auto phase_of = [&](unsigned k) { return (k & 2u) ? 0u : kSign; };
     // the faces of a block's state into the exchange buffer
     auto publish = [&](int item, const Real (&v)[kC], unsigned k) {
-        Real *ex = a.ex + ((k & 1u) ? ex_stride : 0) + item * 384;
+        Real *ex = a.ex + (((k & 1u) ? a.n : 0) + item) * 384;
         const unsigned m = phase_of(k);
         Real u[kC];
 #pragma unroll
         for (int i = 0; i < kC; i++) u[i] = with_phase(v[i], m);
-        if (kC == 4 || sx >= 0) st_face1(ex + sx, w.x0 ? u[kC - 1] : u[0]);
+        if (kC == 4 || sx >= 0) st_face1(ex + sx, x0 ? u[kC - 1] : u[0]);
         if (sy >= 0) st_face(ex + sy, u);
         if (sz >= 0) st_face(ex + sz, u);
     };
     auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kT) : "memory"); };
 
+    group_sync();  // a run before this one has left the group's blocks
     // the group's blocks: state 0, coefficients and cell kinds into shared memory
     for (int j = group; j < nlocal; j += kGroups) {
         ResidentBlock<Real> &b = blocks[j];
@@ -591,18 +628,27 @@ __global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1) resident_run_kernel(
                 for (int i = 0; i < TL::V; i++) b.st[0].phi[pd + v * pstep + i] = b.st[1].phi[pd + v * pstep + i] = (Real)0;
         }
         group_sync();
+        // a coefficient that is negative by itself (a negative tissue fraction)
+        // has a sign that says nothing of kEmpty cells
+        for (int i = 0; i < kC; i++) {
+            const unsigned m = meta[t * kC + i];
+            const int x = x0 + i;
+            const Real d[6] = {b.hx[TL::template at<64>(row, x)],
+                               x < 7 ? b.hx[TL::template at<64>(row, x + 1)] : b.hx8[row],
+                               b.hy[TL::template at<72>(row + z, x)], b.hy[TL::template at<72>(row + z + 1, x)],
+                               b.hz[TL::template at<72>(row, x)], b.hz[TL::template at<72>(row + 8, x)]};
+            for (int k = 0; k < 6; k++)
+                if (sign_of(d[k]) != ((m & 3u) == kEmpty || ((m >> (2 + k)) & 1u))) kind = kGeneral;
+        }
         const bool general = __any_sync(0xffffffffu, kind == kGeneral), edge = __any_sync(0xffffffffu, kind == kEdge);
         if (lane == 0) atomicOr(&b.kinds, (general ? kGeneral : edge ? kEdge : kPlain) << (2 * (t >> 5)));
     }
     group_sync();
 
-    bool failed = false, bad = false;
+    bool failed = false;
     for (int s = 0; s < a.nsteps; s++) {
         const unsigned k = k0 + s;
         const unsigned m = phase_of(k);
-        const Real *ex = a.ex + ((k & 1u) ? ex_stride : 0);
-        const bool last = s == a.nsteps - 1;
-        Real *store = a.stores ? a.stores[s] : (last ? a.out : nullptr);
         for (int j = group; j < nlocal; j += kGroups) {
             ResidentBlock<Real> &b = blocks[j];
             ResidentState<Real> &S = b.st[s & 1];
@@ -610,7 +656,7 @@ __global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1) resident_run_kernel(
             if (fetches) {
                 const int nb = b.nbr[pf];
                 if (nb >= 0) {
-                    const Real *src = ex + (nb + (pf ^ 1) * 64 + pw);
+                    const Real *src = a.ex + (((k & 1u) ? a.n * 384 : 0) + nb + (pf ^ 1) * 64 + pw);
                     Real h[kC];
                     unsigned long long t0 = 0;
                     for (int it = 0;; it++) {
@@ -650,46 +696,101 @@ __global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1) resident_run_kernel(
                 : "memory");
             if (any) {
                 if (t == 0) atomicOr(a.err_flag, kErrPoll);
-                goto out;
+                return false;
             }
             Real o[kC];
             const unsigned kind = (b.kinds >> (2 * (t >> 5))) & 3u;
-            if (kind == kPlain) row_cells<Real, kC, kPlain>(a, b, S, w, o);
-            else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, b, S, w, o);
-            else row_cells<Real, kC, kGeneral>(a, b, S, w, o);
-            if (!last) {
+            if (kind == kPlain) row_cells<Real, kC, kPlain>(a, ih2, neg0, b, S, w, o);
+            else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, ih2, neg0, b, S, w, o);
+            else row_cells<Real, kC, kGeneral>(a, ih2, neg0, b, S, w, o);
+            if (s + 1 < a.nsteps) {
                 publish(c + j * G, o, k + 1);
                 TL::template store<kRows>(b.st[(s + 1) & 1].phi, w.tp, o);
             } else {
+                bool bad = false;
 #pragma unroll
-                for (int i = 0; i < kC; i++) bad |= o[i] != o[i];  // a NaN stays one: the last state shows it
+                for (int i = 0; i < kC; i++) bad |= o[i] != o[i];
+                if (bad) atomicOr(a.nan_flag, 1u);  // a NaN stays one: the last state shows it
+                if (!kStores || !a.stores) st_cells(a.out + (int64_t)(b.e >> 2) * kBS3 + t * kC, o);
             }
-            if (store) st_cells(store + (int64_t)(b.e >> 2) * kBS3 + t * kC, o);
+            if (kStores && a.stores) {
+                Real *store = a.stores[s];
+                if (store) st_cells(store + (int64_t)(b.e >> 2) * kBS3 + t * kC, o);
+            }
         }
     }
-out:
-    if (bad) atomicOr(a.nan_flag, 1u);
+    return true;
+}
+
+template <typename Real, int kC, int kGroups>
+__global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1)
+resident_run_kernel(const __grid_constant__ ResidentArgs<Real> a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const unsigned k0 = *a.index;  // states stored by earlier launches (mod 4)
+    const int c = blockIdx.x, G = gridDim.x;
+    run_blocks<Real, kC, kGroups, true>(a, a.ih2, a.neg0, reinterpret_cast<ResidentBlock<Real> *>(smem_raw), c, G, k0);
     if (a.n_empty > 0)
         empty_blocks(a.empty, a.n_empty, a.in, a.out, (Real *)nullptr, a.nsteps, a.rho, a.dt, a.nan_flag);
     // the last CTA to leave advances the state count for the next launch
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (atomicAdd(a.index + 1, 1u) == (unsigned)G - 1) {
+        if (atomicAdd(a.index + 1, 1u) == gridDim.x - 1) {
             a.index[1] = 0;
             a.index[0] = (k0 + (unsigned)a.nsteps) & 3u;
         }
     }
 }
 
+// Many runs at once: team g of the grid's `teams` teams of `size` CTAs takes
+// runs off[g] .. off[g + 1], one after the other.  Teams share nothing; a
+// run's k0 (start) counts the states its team's exchange buffer carried
+// before.
+template <typename Real>
+struct alignas(16) TeamState {  // at a fixed place in shared memory: no register holds its address
+    ResidentArgs<Real> a;
+    int run, rank, size, failed;
+};
+constexpr int kTeamHead = 256;  // bytes of shared memory before the blocks
+static_assert(sizeof(TeamState<double>) <= kTeamHead, "team state");
+template <typename Real, int kC, int kGroups>
+__global__ void __launch_bounds__(kGroups * (kBS3 / kC), 1)
+resident_teams_kernel(const ResidentArgs<Real> *runs, const int *off, const int size, double ih2,
+                      unsigned long long neg0)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TeamState<Real> &me = *reinterpret_cast<TeamState<Real> *>(smem_raw);
+    if (threadIdx.x == 0) {
+        me.run = off[blockIdx.x / size];
+        me.rank = blockIdx.x % size;
+        me.size = size;
+        me.failed = 0;
+    }
+    __syncthreads();
+    while (me.run < off[blockIdx.x / size + 1] && !me.failed) {
+        // the arguments, word by word
+        for (int i = threadIdx.x; i < (int)(sizeof(me.a) / 4); i += blockDim.x)
+            reinterpret_cast<unsigned *>(&me.a)[i] = reinterpret_cast<const unsigned *>(runs + me.run)[i];
+        __syncthreads();
+        if (!run_blocks<Real, kC, kGroups, false>(me.a, ih2, neg0,
+                                                  reinterpret_cast<ResidentBlock<Real> *>(smem_raw + kTeamHead),
+                                                  me.rank, me.size, me.a.start))
+            me.failed = 1;
+        __syncthreads();
+        if (threadIdx.x == 0) me.run++;
+        __syncthreads();
+    }
+}
+
 constexpr int kMaxSmem = 227 * 1024;
 
-template <typename Real, int kC, int kGroups>
-cudaError_t launch(const ResidentArgs<Real> &a, int ctas, size_t smem, cudaStream_t s)
+// A cooperative launch (CTAs wait for one another, so all must be resident)
+// with the kernel's shared memory limit raised once per device.
+template <auto kernel, typename... Args>
+cudaError_t launch_coop(int ctas, int threads, size_t smem, cudaStream_t s, Args... args)
 {
-    // the kernel's shared memory limit is raised once per device
     static std::mutex mu;
     static std::vector<char> raised;
-    auto kernel = resident_run_kernel<Real, kC, kGroups>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -705,7 +806,7 @@ cudaError_t launch(const ResidentArgs<Real> &a, int ctas, size_t smem, cudaStrea
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kGroups * (kBS3 / kC));
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -713,15 +814,88 @@ cudaError_t launch(const ResidentArgs<Real> &a, int ctas, size_t smem, cudaStrea
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Cells per thread and groups per CTA by the blocks of a CTA (`per`).  Up to
+// two blocks the step is a chain of latencies, which two cells per thread
+// shorten (64^3 FP32, 2 per CTA: 1.16 us per step against 1.32 with four).
+// Beyond, four cells per thread cost fewer instructions, and a step takes the
+// rounds the groups need for the blocks, each round longer the more groups
+// share the SM: on a B200 in FP32 about 1.23, 1.35, 1.40 and 1.62 us with 4, 5,
+// 6 and 7 groups (15 blocks: 4.9 us with four, 4.05 with five, 4.1 with six,
+// 4.5 with seven; 14 blocks: 3.26 with seven, 3.75 with five; 7 blocks: 1.94
+// with seven, 2.42 with four).  Eight groups leave 64 registers a thread,
+// which spill.  FP64 needs 124 registers for four cells: four groups (128^3:
+// 3.07; 3.68 with seven, 4.78 with two cells per thread).
+constexpr double kRoundUs[4] = {1.23, 1.35, 1.40, 1.62};
+constexpr double kRoundUs64 = 1.5;
+template <typename Real>
+int groups_for(int per, double &us)
+{
+    if (per <= 2) {
+        us = sizeof(Real) == 8 ? 1.33 : 1.15;
+        return 2;
+    }
+    if (sizeof(Real) == 8) {
+        us = kRoundUs64 * ((per + 3) / 4);
+        return 4;
+    }
+    int best = 4;
+    us = 1e9;
+    for (int g = 4; g <= 7; g++) {
+        const double u = kRoundUs[g - 4] * ((per + g - 1) / g);
+        if (u < us) {
+            us = u;
+            best = g;
+        }
+    }
+    return best;
+}
+template <typename Real, typename F>
+cudaError_t with_shape(int per, F &&f)
+{
+    using std::integral_constant;
+    double us;
+    const int g = groups_for<Real>(per, us);
+    if (g == 2) return f(integral_constant<int, 2>(), integral_constant<int, 2>());
+    if constexpr (sizeof(Real) == 4) {
+        if (g == 5) return f(integral_constant<int, 4>(), integral_constant<int, 5>());
+        if (g == 6) return f(integral_constant<int, 4>(), integral_constant<int, 6>());
+        if (g == 7) return f(integral_constant<int, 4>(), integral_constant<int, 7>());
+    }
+    return f(integral_constant<int, 4>(), integral_constant<int, 4>());
 }
 
 }  // namespace
 
+void resident_neighbours(int bpd, const int *items, int n, std::vector<int> &nbr)
+{
+    std::vector<int> at((size_t)bpd * bpd * bpd, -1);
+    for (int i = 0; i < n; i++) at[items[i] >> 2] = i;
+    for (int i = 0; i < n; i++) {
+        const int b = items[i] >> 2;
+        const int p[3] = {b % bpd, (b / bpd) % bpd, b / (bpd * bpd)};
+        for (int f = 0; f < 6; f++) {
+            int q[3] = {p[0], p[1], p[2]};
+            q[f >> 1] = (q[f >> 1] + ((f & 1) ? 1 : bpd - 1)) % bpd;
+            nbr.push_back(at[q[0] + bpd * (q[1] + bpd * q[2])]);
+        }
+    }
+}
+
 template <typename Real>
 int resident_capacity(int sms)
 {
-    return sms * (kMaxSmem / (int)sizeof(ResidentBlock<Real>));
+    return sms * ((kMaxSmem - kTeamHead) / (int)sizeof(ResidentBlock<Real>));
+}
+
+template <typename Real>
+double resident_step_us(int per)
+{
+    double us;
+    groups_for<Real>(per, us);
+    return us + 0.15;
 }
 
 template <typename Real>
@@ -730,21 +904,25 @@ cudaError_t launch_resident_run(const ResidentArgs<Real> &a, int sms, cudaStream
     if (a.n <= 0 || a.nsteps <= 0 || a.n > resident_capacity<Real>(sms)) return cudaErrorInvalidValue;
     const int ctas = a.n < sms ? a.n : sms;
     const int per = (a.n + ctas - 1) / ctas;
-    const size_t smem = (size_t)per * sizeof(ResidentBlock<Real>);
-    // Threads per block and groups per CTA by the blocks of a CTA, FP32 (us per
-    // step on a B200, 1000 steps): up to two blocks the step is a chain of
-    // latencies, which two cells per thread shorten (64^3, 2 per CTA: 1.22
-    // against 1.32 with four); beyond, four cells per thread cost fewer
-    // instructions and every block gets a group of its own while the registers
-    // last (96^3, 3 per CTA: 1.48 with four groups, 1.56 with seven; 128^3, 7
-    // per CTA: 2.02 with seven, 2.55 with four, 2.13 with eight, whose 64
-    // registers spill; 160^3, 14 per CTA: 3.48 with seven, 4.76 with four).
-    // FP64 needs 128 registers for four cells: four groups (128^3: 3.14; 3.68
-    // with seven, 4.78 with two cells per thread).
-    if (per <= 2) return launch<Real, 2, 2>(a, ctas, smem, s);
-    if constexpr (sizeof(Real) == 4)
-        if (per > 4) return launch<Real, 4, 7>(a, ctas, smem, s);
-    return launch<Real, 4, 4>(a, ctas, smem, s);
+    return with_shape<Real>(per, [&](auto c, auto g) {
+        constexpr int kC = decltype(c)::value, kGroups = decltype(g)::value;
+        return launch_coop<resident_run_kernel<Real, kC, kGroups>>(ctas, kGroups * (kBS3 / kC),
+                                                                   (size_t)per * sizeof(ResidentBlock<Real>), s, a);
+    });
+}
+
+template <typename Real>
+cudaError_t launch_resident_teams(const ResidentArgs<Real> *runs, const int *off, int teams, int size, int per,
+                                  double ih2, cudaStream_t s)
+{
+    if (teams <= 0 || size <= 0 || per <= 0 || per > resident_capacity<Real>(1))
+        return cudaErrorInvalidValue;
+    return with_shape<Real>(per, [&](auto c, auto g) {
+        constexpr int kC = decltype(c)::value, kGroups = decltype(g)::value;
+        return launch_coop<resident_teams_kernel<Real, kC, kGroups>>(
+            teams * size, kGroups * (kBS3 / kC), kTeamHead + (size_t)per * sizeof(ResidentBlock<Real>), s, runs, off, size,
+            ih2, ResidentArgs<Real>().neg0);
+    });
 }
 
 template <typename Real>
@@ -757,10 +935,16 @@ cudaError_t launch_empty_run(const int *empty, int n_empty, const Real *in, Real
     return cudaGetLastError();
 }
 
+template double resident_step_us<float>(int);
+template double resident_step_us<double>(int);
 template int resident_capacity<float>(int);
 template int resident_capacity<double>(int);
 template cudaError_t launch_resident_run<float>(const ResidentArgs<float> &, int, cudaStream_t);
 template cudaError_t launch_resident_run<double>(const ResidentArgs<double> &, int, cudaStream_t);
+template cudaError_t launch_resident_teams<float>(const ResidentArgs<float> *, const int *, int, int, int, double,
+                                                  cudaStream_t);
+template cudaError_t launch_resident_teams<double>(const ResidentArgs<double> *, const int *, int, int, int, double,
+                                                   cudaStream_t);
 template cudaError_t launch_empty_run<float>(const int *, int, const float *, float *, float *, int, float, double,
                                              unsigned *, cudaStream_t);
 template cudaError_t launch_empty_run<double>(const int *, int, const double *, double *, double *, int, double,

@@ -245,21 +245,26 @@ int gbfk_batch_set_samples(gbfk_batch *b, int nsamples, const gbfk_sample *sampl
 /* Build every sample's initial condition and face coefficients, then run all
  * samples to their horizons.  samples_per_cta: -1 for the persistent
  * pipelined step over all active samples (a power-of-two bpd only), 1, 2 or
- * 4 for the one-CTA-per-block kernel with that many samples per CTA, or 0 to
- * let the autotuner time the candidates on the first steps and keep the
- * fastest (the results do not depend on it).  GBFK_E_NAN if a sample became
- * NaN; GBFK_E_STATE for -1 on a grid it does not apply to. */
+ * 4 for the one-CTA-per-block kernel with that many samples per CTA, or 0:
+ * where the blocks with tissue of a sample fit in the SMs' shared memory, all
+ * steps of all samples in one launch, each sample resident on a team of SMs;
+ * elsewhere the autotuner times the candidates on the first steps and keeps
+ * the fastest (the results do not depend on it).  GBFK_E_NAN if a sample
+ * became NaN; GBFK_E_STATE for -1 on a grid it does not apply to. */
 int gbfk_batch_run(gbfk_batch *b, int samples_per_cta);
-/* The samples_per_cta choice the last run used (-1: the pipelined step). */
+/* The samples_per_cta choice the last run used (-1: the pipelined step, or
+ * the samples resident in shared memory). */
 int gbfk_batch_samples_per_cta(const gbfk_batch *b);
 /* The launch shape of the pipelined step the last run used: consumer warps
  * per CTA, heavy-block ring slots, empty-block ring slots (all 0 when it
  * used the per-block kernel).  With samples_per_cta 0 the autotuner times
- * every compiled shape; otherwise the shape is the default (or the
- * GBFK_TMA_SHAPE="warps,heavy,empty" environment variable). */
+ * every compiled shape; otherwise (resident samples included) the shape is
+ * the default (or the GBFK_TMA_SHAPE="warps,heavy,empty" environment
+ * variable). */
 int gbfk_batch_tile_shape(const gbfk_batch *b, int shape[3]);
 /* gbfk_batch_run replays its steps after the autotuner and the first step as
- * CUDA graphs of up to 512 launches captured on the batch's stream; this is
+ * CUDA graphs of up to 512 launches (resident samples: all steps as one)
+ * captured on the batch's stream; this is
  * how many the last run replayed (0 when the stream could not be captured,
  * e.g. the legacy default stream). */
 int gbfk_batch_graph_count(const gbfk_batch *b);

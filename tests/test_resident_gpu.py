@@ -141,3 +141,36 @@ def test_two_pools_from_two_threads(gbfk_lib):
     assert not errors
     for n, _, _ in cases:
         assert np.array_equal(got[n], want[n])
+
+
+@pytest.mark.parametrize("prec,bpd,samples", [("f64", 5, 9), ("f32", 12, 3), ("f32", 3, 40)])
+def test_stage_of_resident_runs_equals_steps_by_launches(gbfk_lib, prec, bpd, samples):
+    """A stage by teams of CTAs (block counts that are no power of two, two
+    anatomies per team, both initial conditions, horizons from 0 steps on)
+    against the per-block kernel, twice on one batch."""
+    from gliomasolver_b200.tmcmc import Batch, sample_stage, to_gbfk_samples
+
+    R = np.float64 if prec == "f64" else np.float32
+    n = 8 * bpd
+    anat = [make_case(n, seed)[:2] for seed in (0, 5)]
+    anat[1] = tuple(a * 0.9 for a in anat[1])
+    stage = sample_stage(samples, anat[0][0], seed=2, tend_range=(1.0, 60.0))
+    recs, _ = to_gbfk_samples(stage, bpd, prec, anatomy=[i % 2 for i in range(samples)])
+    for i, r in enumerate(recs):
+        r.nsteps = min(r.nsteps, 60) * (i != 1)
+        r.ic = i % 3 == 2
+    with Batch(bpd, samples, prec, max_anatomies=2) as b:
+        for i, (pw, pg) in enumerate(anat):
+            b.set_anatomy(i, pw.astype(R), pg.astype(R))
+        for _ in range(2):
+            b.set_samples(recs)
+            b.run(1)
+            want = [b.download(i) for i in range(samples)]
+            b.set_samples(recs)
+            b.run(0)
+            assert b.samples_per_cta == -1 and b.graph_count == 1
+            for i in range(samples):
+                assert np.array_equal(b.download(i), want[i]), i
+            for r in recs:  # other step counts and horizons the second time
+                r.nsteps += 3
+    assert max(w.max() for w in want) > 0.1
