@@ -1296,7 +1296,7 @@ template <typename Real>
 static int cfl_impl(gbfk_ctx *ctx, double Dw, double Dg, double *out)
 {
     const int nparts = 148 * 4;
-    if (!ctx->d_partial) CK(cudaMalloc(&ctx->d_partial, (size_t)148 * 4 * 7 * sizeof(double)));
+    if (!ctx->d_partial) CK(cudaMalloc(&ctx->d_partial, (size_t)kLikelihoodMaxParts * kLikelihoodPartBytes));
     const Real dw = (Real)Dw, dg = (Real)Dg;
     CK(launch_cfl<Real>(view<Real>(ctx), dw, dg, ctx->d_partial, nparts, ctx->stream));
     ctx->launches++;
@@ -1442,10 +1442,13 @@ int gbfk_log_likelihood(gbfk_ctx *ctx, const gbfk_likelihood_params *p, double o
     if (p->step_pet <= 0 || p->step_mri <= 0 || !(p->slope != 0))
         return fail(ctx, GBFK_E_INVALID, "log_likelihood: bad parameters");
     CK(cudaSetDevice(ctx->device));
-    int rc = dump_to_device(ctx, ctx->obs_n);
-    if (rc) return rc;
-    const int nparts = 148 * 4;
-    if (!ctx->d_partial) CK(cudaMalloc(&ctx->d_partial, (size_t)nparts * 7 * sizeof(double)));
+    // a uniform grid's dump at its own resolution is its own cells
+    const bool own = ctx->have_topology && ctx->have_origin && ctx->uniform && ctx->obs_n == 8 * ctx->bpd;
+    if (!own) {
+        const int rc = dump_to_device(ctx, ctx->obs_n);
+        if (rc) return rc;
+    }
+    if (!ctx->d_partial) CK(cudaMalloc(&ctx->d_partial, (size_t)kLikelihoodMaxParts * kLikelihoodPartBytes));
     if (!ctx->d_lik) CK(cudaMalloc(&ctx->d_lik, 4 * sizeof(double)));
     LikelihoodParams lp;
     lp.pet_sigma2 = p->pet_sigma2;
@@ -1455,9 +1458,16 @@ int gbfk_log_likelihood(gbfk_ctx *ctx, const gbfk_likelihood_params *p, double o
     lp.slope = p->slope;
     lp.step_pet = p->step_pet;
     lp.step_mri = p->step_mri;
-    CK(launch_likelihood(ctx->d_model, ctx->obs_n, ctx->d_t1c, ctx->d_flair, ctx->d_pet,
-                         ctx->nroi ? ctx->d_roi : nullptr, ctx->nroi, lp, ctx->d_partial, nparts, ctx->d_lik,
-                         ctx->stream));
+    const int *roi = ctx->nroi ? ctx->d_roi : nullptr;
+    if (!own)
+        CK(launch_likelihood_dense(ctx->d_model, ctx->obs_n, ctx->d_t1c, ctx->d_flair, ctx->d_pet, roi, ctx->nroi, lp,
+                                   ctx->d_partial, ctx->d_lik, ctx->stream));
+    else if (ctx->precision == GBFK_F64)
+        CK(launch_likelihood_pool<double>(nullptr, {ctx->phi[ctx->cur], lp}, 1, ctx->obs_n, ctx->d_t1c, ctx->d_flair,
+                                          ctx->d_pet, roi, ctx->nroi, ctx->d_partial, ctx->d_lik, ctx->stream));
+    else
+        CK(launch_likelihood_pool<float>(nullptr, {ctx->phi[ctx->cur], lp}, 1, ctx->obs_n, ctx->d_t1c, ctx->d_flair,
+                                         ctx->d_pet, roi, ctx->nroi, ctx->d_partial, ctx->d_lik, ctx->stream));
     ctx->launches += 2;
     CK(cudaMemcpyAsync(out, ctx->d_lik, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1936,19 +1946,10 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     }
     double lik[4] = {0, 0, 0, 0};
     if (e == cudaSuccess) {
-        if (!ctx->d_partial) e = cudaMalloc(&ctx->d_partial, (size_t)148 * 4 * 7 * sizeof(double));
+        if (!ctx->d_partial)
+            e = cudaMalloc(&ctx->d_partial, (size_t)kLikelihoodMaxParts * kLikelihoodPartBytes);
         if (e == cudaSuccess && !ctx->d_lik) e = cudaMalloc(&ctx->d_lik, 4 * sizeof(double));
-        if (e == cudaSuccess && ctx->model_bytes < (size_t)n * n * n * sizeof(double)) {
-            if (ctx->d_model) cudaFree(ctx->d_model);
-            ctx->d_model = nullptr;
-            ctx->model_bytes = 0;
-            e = cudaMalloc(&ctx->d_model, (size_t)n * n * n * sizeof(double));
-            if (e == cudaSuccess) ctx->model_bytes = (size_t)n * n * n * sizeof(double);
-        }
     }
-    if (e == cudaSuccess)
-        e = launch_uq_dump<Real>(ctx->d_slot, (const Real *)ctx->d_origin, (const Real *)ctx->d_h, nb, F, n,
-                                 ctx->d_model, ctx->stream);
     if (e == cudaSuccess) {
         LikelihoodParams lp;
         lp.pet_sigma2 = 1;
@@ -1959,9 +1960,10 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         lp.step_pet = 1;
         lp.step_mri = 1;
         // with a ROI (HGG_Likelihood.cpp:97-124) the loss sums over its voxels only
-        e = launch_likelihood(ctx->d_model, n, ctx->d_t1c, ctx->d_flair, nullptr, ctx->nroi ? ctx->d_roi : nullptr,
-                              ctx->nroi, lp, ctx->d_partial, 148 * 4, ctx->d_lik, ctx->stream);
-        ctx->launches += 3;
+        e = launch_likelihood_pool<Real>(nullptr, {F, lp}, 1, n, ctx->d_t1c, ctx->d_flair, nullptr,
+                                         ctx->nroi ? ctx->d_roi : nullptr, ctx->nroi, ctx->d_partial, ctx->d_lik,
+                                         ctx->stream);
+        ctx->launches += 2;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(lik, ctx->d_lik, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     int *roi_count = nullptr;

@@ -99,8 +99,8 @@ struct gbfk_batch {
     int *d_roi = nullptr;
     int nroi = 0;
     bool have_obs = false;
-    double *d_model = nullptr;   // one sample's dump grid
     double *d_partial = nullptr; // likelihood partial sums
+    LikelihoodSample *d_lik_in = nullptr;  // the samples' states and parameters
     double *d_lik = nullptr;     // 4 per sample
     // GBFK_IC_BALL samples: band cells (int64 pool index) and their values
     void *d_ball = nullptr;
@@ -129,21 +129,6 @@ int bfail(gbfk_batch *b, int code, const char *fmt, ...)
             return bfail(b, e_ == cudaErrorMemoryAllocation ? GBFK_E_OOM : GBFK_E_CUDA, "%s: %s (%s:%d)", \
                          #call, cudaGetErrorString(e_), __FILE__, __LINE__);                              \
     } while (0)
-
-// One sample's phi (block-pool order of a uniform bpd^3 grid) as doubles on
-// the n^3 grid, x fastest: the dump of a uniform grid at its own resolution
-// (each cell written once, Glioma_ReactionDiffusion.cpp:208-262).
-template <typename Real>
-__global__ void pool_to_dense_kernel(const Real *__restrict__ pool, int n, double *__restrict__ out)
-{
-    const int64_t N = (int64_t)n * n * n;
-    const int bpd = n / kBS;
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < N; g += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(g % n), y = (int)((g / n) % n), z = (int)(g / ((int64_t)n * n));
-        const int64_t slot = (x >> 3) + (int64_t)bpd * ((y >> 3) + (int64_t)bpd * (z >> 3));
-        out[g] = (double)pool[slot * kBS3 + (x & 7) + kBS * ((y & 7) + kBS * (z & 7))];
-    }
-}
 
 template <typename Real>
 PoolView<Real> batch_pool(gbfk_batch *b)
@@ -751,17 +736,20 @@ int batch_run(gbfk_batch *b, int spc)
 template <typename Real>
 int batch_likelihood(gbfk_batch *b, const gbfk_likelihood_params *params, int per_sample, double *out)
 {
-    const int n = b->n, nparts = 148 * 4;
-    const size_t N = (size_t)n * n * n;
-    if (!b->d_model) BK(cudaMalloc(&b->d_model, N * sizeof(double)));
-    if (!b->d_partial) BK(cudaMalloc(&b->d_partial, (size_t)nparts * 7 * sizeof(double)));
+    const int n = b->n, parts = likelihood_parts(n);
+    if (b->nsamples == 0) return GBFK_OK;
+    // parameters and results of every sample and the partial sums of as many
+    // as 16 MiB hold (a launch's worth), kept for the next call
+    const size_t part_bytes = (size_t)parts * kLikelihoodPartBytes;
+    const int most = std::max(1, std::min(b->max_samples, (int)(((size_t)16 << 20) / part_bytes)));
+    if (!b->d_partial) BK(cudaMalloc(&b->d_partial, (size_t)most * part_bytes));
+    if (!b->d_lik_in) BK(cudaMalloc(&b->d_lik_in, (size_t)b->max_samples * sizeof(LikelihoodSample)));
     if (!b->d_lik) BK(cudaMalloc(&b->d_lik, (size_t)b->max_samples * 4 * sizeof(double)));
     const size_t field = (size_t)b->nblocks * kBS3;
-    int64_t grid = (N + 255) / 256;
-    if (grid > 148 * 32) grid = 148 * 32;
+    std::vector<LikelihoodSample> in(b->nsamples);
     for (int s = 0; s < b->nsamples; s++) {
         const gbfk_likelihood_params *p = params + (per_sample ? s : 0);
-        LikelihoodParams lp;
+        LikelihoodParams &lp = in[s].p;
         lp.pet_sigma2 = p->pet_sigma2;
         lp.pet_scale = p->pet_scale;
         lp.t1_uc = p->t1_uc;
@@ -769,12 +757,15 @@ int batch_likelihood(gbfk_batch *b, const gbfk_likelihood_params *params, int pe
         lp.slope = p->slope;
         lp.step_pet = p->step_pet;
         lp.step_mri = p->step_mri;
-        const Real *final = (const Real *)b->phi_all[b->final_in_0 ? 0 : b->params[s].nsteps & 1] + (size_t)b->pos[s] * field;
-        pool_to_dense_kernel<Real><<<(int)grid, 256, 0, b->stream>>>(final, n, b->d_model);
-        BK(cudaGetLastError());
-        BK(launch_likelihood(b->d_model, n, b->d_t1c, b->d_flair, b->d_pet, b->nroi ? b->d_roi : nullptr, b->nroi,
-                             lp, b->d_partial, nparts, b->d_lik + 4 * (size_t)s, b->stream));
-        b->launches += 3;
+        in[s].state = (const Real *)b->phi_all[b->final_in_0 ? 0 : b->params[s].nsteps & 1] + (size_t)b->pos[s] * field;
+    }
+    BK(cudaMemcpyAsync(b->d_lik_in, in.data(), in.size() * sizeof(in[0]), cudaMemcpyHostToDevice, b->stream));
+    for (int s = 0; s < b->nsamples; s += most) {
+        const int count = std::min(most, b->nsamples - s);
+        BK(launch_likelihood_pool<Real>(b->d_lik_in + s, LikelihoodSample{}, count, n, b->d_t1c, b->d_flair, b->d_pet,
+                                        b->nroi ? b->d_roi : nullptr, b->nroi, b->d_partial, b->d_lik + 4 * (size_t)s,
+                                        b->stream));
+        b->launches += 2;
     }
     BK(cudaMemcpyAsync(out, b->d_lik, (size_t)b->nsamples * 4 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
@@ -878,7 +869,7 @@ int gbfk_batch_destroy(gbfk_batch *b)
     if (b->stream) cudaStreamSynchronize(b->stream);
     void *ptrs[] = {b->d_nbr,       b->d_ih2,    b->d_views, b->d_nan,      b->d_err,     b->d_rho, b->d_dt,
                     b->d_lists,     b->pw_all,   b->pg_all,  b->meta_all,   b->btype_all, b->phi_all[0],
-                    b->phi_all[1],  b->H_all,    b->d_t1c,   b->d_flair,    b->d_pet,     b->d_roi, b->d_model,
+                    b->phi_all[1],  b->H_all,    b->d_t1c,   b->d_flair,    b->d_pet,     b->d_roi, b->d_lik_in,
                     b->d_partial,   b->d_lik,    b->d_ball,  b->d_dec,      b->d_res};
     for (void *p : ptrs)
         if (p) cudaFree(p);

@@ -248,10 +248,27 @@ struct LikelihoodParams {
     int step_pet, step_mri;
 };
 
-// out[0..3] = L_PET, L_T1c, L_FLAIR, their sum; partial holds nparts * 7 doubles.
-cudaError_t launch_likelihood(const double *model, int n, const unsigned char *t1c, const unsigned char *flair,
-                              const double *pet, const int *roi, int nroi, const LikelihoodParams &p,
-                              double *partial, int nparts, double *out, cudaStream_t s);
+// One state and its parameters: the dump grid's doubles, or the block pool of
+// a uniform grid.
+struct LikelihoodSample {
+    const void *state;
+    LikelihoodParams p;
+};
+// out[4 * k .. 4 * k + 3] = L_PET, L_T1c, L_FLAIR, their sum of state k on the
+// n^3 grid; partial: likelihood_parts(n) (at most kLikelihoodMaxParts) *
+// kLikelihoodPartBytes per state.
+constexpr int kLikelihoodMaxParts = 148 * 8;
+constexpr int kLikelihoodPartBytes = 88;
+int likelihood_parts(int n);
+cudaError_t launch_likelihood_dense(const double *model, int n, const unsigned char *t1c, const unsigned char *flair,
+                                    const double *pet, const int *roi, int nroi, const LikelihoodParams &p,
+                                    void *partial, double *out, cudaStream_t s);
+// count states in block pools of the uniform n^3 grid: the device array
+// samples, or (samples NULL, count 1) `one`
+template <typename Real>
+cudaError_t launch_likelihood_pool(const LikelihoodSample *samples, const LikelihoodSample &one, int count, int n,
+                                   const unsigned char *t1c, const unsigned char *flair, const double *pet,
+                                   const int *roi, int nroi, void *partial, double *out, cudaStream_t s);
 
 // Discrete adjoint (uniform grids): one adjoint step per launch
 // (adj_fused_kernel).  The state of an adjoint step kept between launches,

@@ -102,3 +102,46 @@ def test_log_likelihood_matches_oracle(gbfk_lib, use_roi, use_pet):
         got = pool.log_likelihood(step_pet=3, step_mri=2, **PARAMS)
     assert np.allclose(got[:3], want, rtol=1e-12, atol=1e-9)
     assert got[3] == pytest.approx(got[:3].sum(), rel=1e-15)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec,n", [("f64", 8), ("f32", 16), ("f32", 64)])
+@pytest.mark.parametrize("slope", [2.0, 0.05])
+def test_likelihood_of_a_pool_term_by_term(gbfk_lib, prec, n, slope):
+    """Every kind of voxel (0, a tail that rounds away against the threshold, at
+    the threshold, between, above, 1), both labels, rows of zeros between full
+    ones, against sums of the terms in extended precision.  Each device term
+    is exp and log1p in FP64 (a few units in the last place, 1e-15) and the
+    sums are compensated: 1e-13 relative."""
+    from gliomasolver_b200 import BlockPool
+
+    R = np.float64 if prec == "f64" else np.float32
+    rng = np.random.default_rng(n)
+    kinds = np.array([0.0, 1e-40, 1e-20, 0.1, 0.25, 0.5, 0.7, 0.8, 1.0], dtype=R)
+    u = kinds[rng.integers(0, kinds.size, (n, n, n))]
+    u = np.where(rng.random((n, n, n)) < 0.3, rng.random((n, n, n)), u).astype(R)
+    u[:, ::3, :] = 0
+    t1, fl = ((rng.random((n, n, n)) < f).astype(float) for f in (0.3, 0.6))
+    pet = rng.random((n, n, n)) * (rng.random((n, n, n)) < 0.5)
+    t1uc, t2uc = float(R(0.7)), float(R(0.25))
+    s2, scale = 0.02, 0.85
+    with BlockPool((n // 8) ** 3, prec) as pool:
+        pool.set_uniform(n // 8)
+        pool.upload_dense("phi", u)
+        pool.set_observations(t1, fl, pet)
+        got = pool.log_likelihood(pet_sigma2=s2, pet_scale=scale, t1_uc=t1uc, t2_uc=t2uc, slope=slope)
+    x = u.astype(np.longdouble)
+
+    def term(mask, uc):
+        d = x - np.longdouble(uc)
+        t = np.where(d > 0, np.longdouble(1), d * d) / np.longdouble(slope)
+        near, far = np.log1p(-np.exp(-t) / 2), np.log(np.longdouble(0.5)) - t
+        la, lb = np.where(d > 0, near, far), np.where(d > 0, far, near)
+        return np.where(d == 0, np.log(np.longdouble(0.5)), np.where(mask == 1, la, lb)).sum()
+
+    on = pet > 0
+    r = x[on] - scale * pet[on].astype(np.longdouble)
+    lpet = -0.5 * on.sum() * np.log(2 * np.pi * s2) - 0.5 / s2 * float((r * r).sum())
+    want = [lpet, float(term(t1, t1uc)), float(term(fl, t2uc))]
+    assert np.allclose(got[:3], want, rtol=1e-13, atol=0)
+    assert got[3] == pytest.approx(sum(want), rel=1e-12)
