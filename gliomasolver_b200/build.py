@@ -20,7 +20,7 @@ NVCC_FLAGS = [
     "-lineinfo",
     # the RD arithmetic must round exactly like the reference's CPU code
     "-fmad=false",
-    "-Xcompiler", "-fPIC,-ffp-contract=off", "-shared",
+    "-Xcompiler", "-fPIC,-ffp-contract=off,-pthread", "-shared",
 ]
 
 
@@ -36,7 +36,7 @@ def needs_build() -> bool:
     if not OUT.exists():
         return True
     mt = OUT.stat().st_mtime
-    deps = [HERE / s for s in SOURCES] + list((HERE / "csrc").glob("*.cuh")) + [ROOT / "include" / "gbfk.h"]
+    deps = [HERE / s for s in SOURCES] + list((HERE / "csrc").glob("*.cuh")) + list((HERE / "csrc").glob("*.h")) + [ROOT / "include" / "gbfk.h"]
     return any(d.stat().st_mtime > mt for d in deps if d.exists())
 
 

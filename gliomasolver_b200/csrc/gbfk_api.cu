@@ -2,6 +2,7 @@
 // movement and the hot-path entry points.  Host code only; kernels live in
 // gbfk_kernels.cu.
 #include "gbfk.h"
+#include "gbfk_hostio.h"
 #include "gbfk_kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -124,6 +125,7 @@ struct gbfk_ctx {
     unsigned *d_nan = nullptr;        // [0]: NaN seen in a step, [1]: a pipeline stage wait timed out
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
+    gbfk_host::StagedCopy staged;     // copies of pageable host memory
     // gbfk_forward_adjoint's device buffers, kept from one call to the next
     // (freed by gbfk_destroy, or replaced when a call needs other sizes or
     // more checkpoint buffers)
@@ -955,6 +957,7 @@ int gbfk_destroy(gbfk_ctx *ctx)
     for (auto *m : {&ctx->adj_ev_write, &ctx->adj_ev_read})
         for (auto &kv : *m) cudaEventDestroy(kv.second);
     if (ctx->adj_ev_join) cudaEventDestroy(ctx->adj_ev_join);
+    ctx->staged.release();
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return GBFK_OK;
@@ -1137,8 +1140,7 @@ int gbfk_upload_field(gbfk_ctx *ctx, int field, const void *host, int64_t first,
     if (!p || !host || first < 0 || ncells < 0 || first + ncells > (int64_t)ctx->max_blocks * kBS3)
         return fail(ctx, GBFK_E_INVALID, "upload_field: bad field or range");
     CK(cudaSetDevice(ctx->device));
-    CK(cudaMemcpyAsync((char *)p + first * ctx->rsize, host, ncells * ctx->rsize, cudaMemcpyHostToDevice,
-                       ctx->stream));
+    CK(ctx->staged.to_device((char *)p + first * ctx->rsize, host, ncells * ctx->rsize, ctx->device, ctx->stream));
     if (field != GBFK_PHI) invalidate_static(ctx);
     return GBFK_OK;
 }
@@ -1150,8 +1152,7 @@ int gbfk_download_field(gbfk_ctx *ctx, int field, void *host, int64_t first, int
     if (!p || !host || first < 0 || ncells < 0 || first + ncells > (int64_t)ctx->max_blocks * kBS3)
         return fail(ctx, GBFK_E_INVALID, "download_field: bad field or range");
     CK(cudaSetDevice(ctx->device));
-    CK(cudaMemcpyAsync(host, (const char *)p + first * ctx->rsize, ncells * ctx->rsize, cudaMemcpyDeviceToHost,
-                       ctx->stream));
+    CK(ctx->staged.to_host(host, (const char *)p + first * ctx->rsize, ncells * ctx->rsize, ctx->device, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return GBFK_OK;
 }
@@ -1173,7 +1174,7 @@ static int dense_io(gbfk_ctx *ctx, int field, void *host, int n, bool up)
         ctx->stage_bytes = bytes;
     }
     if (up) {
-        CK(cudaMemcpyAsync(ctx->d_stage, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
+        CK(ctx->staged.to_device(ctx->d_stage, host, bytes, ctx->device, ctx->stream));
         if (ctx->precision == GBFK_F64)
             CK(launch_dense_scatter<double>((const double *)ctx->d_stage, (double *)p, n, true, ctx->stream));
         else
@@ -1186,7 +1187,7 @@ static int dense_io(gbfk_ctx *ctx, int field, void *host, int n, bool up)
         else
             CK(launch_dense_scatter<float>((const float *)p, (float *)ctx->d_stage, n, false, ctx->stream));
         ctx->launches++;
-        CK(cudaMemcpyAsync(host, ctx->d_stage, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx->staged.to_host(host, ctx->d_stage, bytes, ctx->device, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
     }
     return GBFK_OK;
@@ -1389,8 +1390,7 @@ int gbfk_uq_dump(gbfk_ctx *ctx, int n, double *host_out)
     CK(cudaSetDevice(ctx->device));
     int rc = dump_to_device(ctx, n);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(host_out, ctx->d_model, (size_t)n * n * n * sizeof(double), cudaMemcpyDeviceToHost,
-                       ctx->stream));
+    CK(ctx->staged.to_host(host_out, ctx->d_model, (size_t)n * n * n * sizeof(double), ctx->device, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return GBFK_OK;
 }
@@ -2014,7 +2014,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
             if (e == cudaSuccess) ctx->stage_bytes = A.fbytes;
         }
         if (e == cudaSuccess) e = launch_dense_scatter<Real>(A.LAM, (Real *)ctx->d_stage, n, false, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(grad_c0, ctx->d_stage, A.fbytes, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = ctx->staged.to_host(grad_c0, ctx->d_stage, A.fbytes, ctx->device, ctx->stream);
         ctx->launches++;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

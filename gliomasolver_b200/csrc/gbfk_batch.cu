@@ -15,6 +15,7 @@
 #include "gbfk.h"
 #include "gbfk_exact.cuh"
 #include "gbfk_host.h"
+#include "gbfk_hostio.h"
 #include "gbfk_kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -105,6 +106,9 @@ struct gbfk_batch {
     // GBFK_IC_BALL samples: band cells (int64 pool index) and their values
     void *d_ball = nullptr;
     size_t ball_cap = 0;
+    // one dense volume on the device, and the copies of pageable host memory
+    void *d_stage = nullptr;
+    gbfk_host::StagedCopy staged;
     int64_t launches = 0;
     std::string err;
 };
@@ -870,9 +874,11 @@ int gbfk_batch_destroy(gbfk_batch *b)
     void *ptrs[] = {b->d_nbr,       b->d_ih2,    b->d_views, b->d_nan,      b->d_err,     b->d_rho, b->d_dt,
                     b->d_lists,     b->pw_all,   b->pg_all,  b->meta_all,   b->btype_all, b->phi_all[0],
                     b->phi_all[1],  b->H_all,    b->d_t1c,   b->d_flair,    b->d_pet,     b->d_roi, b->d_lik_in,
-                    b->d_partial,   b->d_lik,    b->d_ball,  b->d_dec,      b->d_res};
+                    b->d_partial,   b->d_lik,    b->d_ball,  b->d_dec,      b->d_res,
+                    b->d_stage};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    b->staged.release();
     if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return GBFK_OK;
@@ -889,24 +895,18 @@ int gbfk_batch_set_anatomy(gbfk_batch *b, int anatomy, const void *pw_dense, con
         return bfail(b, GBFK_E_INVALID, "set_anatomy: bad anatomy index or null field");
     BK(cudaSetDevice(b->device));
     const size_t bytes = (size_t)b->n * b->n * b->n * b->rsize;
-    void *stage = nullptr;
-    BK(cudaMalloc(&stage, bytes));
+    if (!b->d_stage) BK(cudaMalloc(&b->d_stage, bytes));
     const void *src[2] = {pw_dense, pg_dense};
     void *dst[2] = {b->pw[anatomy], b->pg[anatomy]};
     for (int f = 0; f < 2; f++) {
-        cudaError_t e = cudaMemcpyAsync(stage, src[f], bytes, cudaMemcpyHostToDevice, b->stream);
-        if (e == cudaSuccess)
-            e = b->precision == GBFK_F64
-                    ? launch_dense_scatter<double>((const double *)stage, (double *)dst[f], b->n, true, b->stream)
-                    : launch_dense_scatter<float>((const float *)stage, (float *)dst[f], b->n, true, b->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-        if (e != cudaSuccess) {
-            cudaFree(stage);
-            BK(e);
-        }
+        BK(b->staged.to_device(b->d_stage, src[f], bytes, b->device, b->stream));
+        if (b->precision == GBFK_F64)
+            BK(launch_dense_scatter<double>((const double *)b->d_stage, (double *)dst[f], b->n, true, b->stream));
+        else
+            BK(launch_dense_scatter<float>((const float *)b->d_stage, (float *)dst[f], b->n, true, b->stream));
+        BK(cudaStreamSynchronize(b->stream));
         b->launches++;
     }
-    cudaFree(stage);
     b->anatomy_set[anatomy] = true;
     return GBFK_OK;
 }
@@ -965,19 +965,17 @@ int gbfk_batch_download(gbfk_batch *b, int sample, void *dense_out)
     if (sample < 0 || sample >= b->nsamples || !dense_out) return bfail(b, GBFK_E_INVALID, "download: bad sample");
     BK(cudaSetDevice(b->device));
     const size_t bytes = (size_t)b->n * b->n * b->n * b->rsize;
-    void *stage = nullptr;
-    BK(cudaMalloc(&stage, bytes));
     if (b->pos.size() != (size_t)b->nsamples) return bfail(b, GBFK_E_STATE, "download: the batch has not run");
+    if (!b->d_stage) BK(cudaMalloc(&b->d_stage, bytes));
     const size_t field = (size_t)b->nblocks * kBS3 * b->rsize;
     const void *src = (const char *)b->phi_all[b->final_in_0 ? 0 : b->params[sample].nsteps & 1] +
                       (size_t)b->pos[sample] * field;
-    cudaError_t e = b->precision == GBFK_F64
-                        ? launch_dense_scatter<double>((const double *)src, (double *)stage, b->n, false, b->stream)
-                        : launch_dense_scatter<float>((const float *)src, (float *)stage, b->n, false, b->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dense_out, stage, bytes, cudaMemcpyDeviceToHost, b->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-    cudaFree(stage);
-    BK(e);
+    if (b->precision == GBFK_F64)
+        BK(launch_dense_scatter<double>((const double *)src, (double *)b->d_stage, b->n, false, b->stream));
+    else
+        BK(launch_dense_scatter<float>((const float *)src, (float *)b->d_stage, b->n, false, b->stream));
+    BK(b->staged.to_host(dense_out, b->d_stage, bytes, b->device, b->stream));
+    BK(cudaStreamSynchronize(b->stream));
     b->launches++;
     return GBFK_OK;
 }

@@ -320,3 +320,18 @@ def test_bounded_wait_gives_up_and_the_device_stays_usable(gbfk_lib):
         pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 4, check_nan=True)
         got = pool.download_dense("phi")
     assert np.array_equal(got, O.rd_steps_dense(pw, pg, c0, s.Dw, s.Dg, s.rho, s.h, s.dt, 4))
+
+
+@pytest.mark.parametrize("prec,cells,first", [("f32", 9_000_001, 3), ("f64", 4_194_305, 0), ("f32", 1000, 5)])
+def test_copies_of_pageable_memory_round_trip(gbfk_lib, prec, cells, first):
+    """Ranges that go through the staging threads (32 MiB and more, odd chunk
+    counts and offsets) and one that does not, twice in a row from buffers
+    that change as soon as the call returns."""
+    rng = np.random.default_rng(cells)
+    with BlockPool((cells + first) // 512 + 1, prec) as pool:
+        for _ in range(2):
+            a = rng.random(cells).astype(pool.dtype)
+            want = a.copy()
+            pool.upload("phi", a, first_cell=first)
+            a[:] = -1
+            assert np.array_equal(pool.download("phi", cells, first_cell=first), want)
