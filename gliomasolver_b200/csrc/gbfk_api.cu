@@ -117,6 +117,12 @@ struct gbfk_ctx {
     unsigned *d_res_index = nullptr;
     bool res_ready = false;
     int sms = 0;
+    // adjoint runs with resident blocks: exchange buffers, gradient sums of
+    // threads and CTAs, face count (one buffer, zeroed per item list); the
+    // pointer tables of a sweep
+    void *d_adj_run = nullptr;
+    bool adj_run_ready = false;
+    void *d_adj_table = nullptr;
     // phi[cur] is the output of a step: every value +0 <= phi <= 1 or NaN
     // (set only by rd_step; every other writer of phi clears it)
     bool phi_clamped = false;
@@ -227,7 +233,7 @@ void free_topology(gbfk_ctx *c)
     c->faces_valid = false;
     c->lists_valid = false;
     c->run_layout_valid = false;
-    c->res_ready = false;
+    c->res_ready = c->adj_run_ready = false;
     c->phi_clamped = false;
 }
 
@@ -239,7 +245,7 @@ void release_topology(gbfk_ctx *c)
                      &c->d_w, (void **)&c->d_step_rows, (void **)&c->d_all_rows, &c->d_gpw, &c->d_gpg,
                      &c->d_gphi, (void **)&c->d_fwt, &c->d_H, (void **)&c->d_ih2, (void **)&c->d_btype, &c->d_origin,
                      (void **)&c->d_lists, (void **)&c->d_run_nbr, (void **)&c->d_run_flags,
-                     (void **)&c->d_res_nbr, &c->d_res_ex, (void **)&c->d_res_index};
+                     (void **)&c->d_res_nbr, &c->d_res_ex, (void **)&c->d_res_index, &c->d_adj_run, &c->d_adj_table};
     for (void **p : ptrs) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -337,7 +343,7 @@ int check_stage_timeout(gbfk_ctx *ctx)
     CK(cudaStreamSynchronize(ctx->stream));
     if (flag) {
         CK(cudaMemsetAsync(ctx->d_nan + 1, 0, sizeof(unsigned), ctx->stream));
-        ctx->res_ready = false;  // a run that gave up leaves its exchange buffers behind
+        ctx->res_ready = ctx->adj_run_ready = false;  // a run that gave up leaves its exchange buffers behind
         if (flag & (1u | 256u))
             return fail(ctx, GBFK_E_TIMEOUT, "rd_step: a wait of the pipelined step timed out (1 s; error word 0x%x)",
                         flag);
@@ -536,7 +542,7 @@ int build_step_lists(gbfk_ctx *ctx)
     ctx->lists_gen++;
     ctx->h_lists.swap(lists);
     ctx->run_layout_valid = false;
-    ctx->res_ready = false;
+    ctx->res_ready = ctx->adj_run_ready = false;
     return GBFK_OK;
 }
 
@@ -1599,10 +1605,23 @@ struct Adjoint {
         fsteps++;
         ctx->launches++;
     }
+    // The operations of a sweep, recorded for runs with resident blocks: k
+    // forward steps from src into dst, or (dst NULL) an adjoint step from src.
+    struct Op {
+        const Real *src;
+        Real *dst;
+        int k;
+    };
+    bool record = false;
+    std::vector<Op> ops;
     // k forward steps from src into dst; intermediate states alternate
     // between T0 and T1 (src and dst are never T0/T1 and never equal)
     void advance(const Real *src, Real *dst, int k)
     {
+        if (record) {
+            ops.push_back({src, dst, k});
+            return;
+        }
         if (err != cudaSuccess) return;
         if (k == 0) {
             if (src != dst) {
@@ -1645,6 +1664,10 @@ struct Adjoint {
     // one adjoint step through the forward step from phi_k (one launch)
     void adjoint_step(const Real *phi_k)
     {
+        if (record) {
+            ops.push_back({phi_k, nullptr, 0});
+            return;
+        }
         if (err != cudaSuccess) return;
         adjoint_reads(phi_k);
         if (err != cudaSuccess) return;
@@ -1667,6 +1690,91 @@ struct Adjoint {
                                          sets[latest], sets[latest ^ 1], 2, false, blocks, nlaunch, rho, dt, Dw,
                                          grad_acc, ctx->stream);
         ctx->launches++;
+    }
+    // Runs the recorded operations on ctx->stream: forward steps that follow
+    // one another as one resident run that stores the states in between,
+    // adjoint steps that follow one another as one resident run over the
+    // stored states.  (A sweep's steps come in such groups: the schedule
+    // advances far, then step by step through the buffers that are left, then
+    // goes back through them.)  Every state buffer's empty blocks hold +0.
+    AdjRunArgs<Real> run{};  // the arguments that all adjoint runs share
+    Real *lam_out = nullptr;
+    int64_t total_steps = 0;
+    int resident_sweep(double rho_, double dt_)
+    {
+        record = false;
+        std::vector<Op> todo;
+        todo.swap(ops);
+        const int rc = run_ops(todo, rho_, dt_);
+        record = true;
+        return rc;
+    }
+    int run_ops(const std::vector<Op> &ops, double rho_, double dt_)
+    {
+        std::vector<const Real *> table;
+        struct Group {
+            size_t from, to, table;  // operations, first pointer
+            int steps;
+            bool adjoint, resident;
+        };
+        std::vector<Group> groups;
+        for (size_t i = 0; i < ops.size();) {
+            Group g = {i, i + 1, table.size(), 0, ops[i].dst == nullptr, true};
+            if (g.adjoint) {
+                while (g.to < ops.size() && !ops[g.to].dst) g.to++;
+                g.steps = (int)(g.to - g.from);
+                for (size_t q = g.from; q < g.to; q++) table.push_back(ops[q].src);
+            } else if (ops[i].k > 0) {
+                while (g.to < ops.size() && ops[g.to].dst && ops[g.to].k > 0 && ops[g.to].src == ops[g.to - 1].dst) g.to++;
+                for (size_t q = g.from; q < g.to; q++) {
+                    for (int k = 1; k < ops[q].k; k++) table.push_back(nullptr);
+                    table.push_back(ops[q].dst);
+                    g.steps += ops[q].k;
+                    g.resident &= clean(ops[q].dst);
+                }
+                g.resident &= g.steps >= kResidentSteps;
+            } else {
+                g.resident = false;  // a copy
+            }
+            groups.push_back(g);
+            i = g.to;
+        }
+        if (table.empty()) return GBFK_OK;
+        int rc = topo_alloc(ctx, &ctx->d_adj_table, table.size() * sizeof(table[0]));
+        if (rc) return rc;
+        CK(cudaMemcpyAsync(ctx->d_adj_table, table.data(), table.size() * sizeof(table[0]), cudaMemcpyHostToDevice,
+                           ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));  // the table is the host's until then
+        Real *const *d_table = (Real *const *)ctx->d_adj_table;
+        for (const Group &g : groups) {
+            if (g.adjoint) {
+                AdjRunArgs<Real> a = run;
+                a.states = d_table + g.table;
+                a.nsteps = g.steps;
+                a.first = asteps == 0;
+                a.final = asteps + g.steps == total_steps;
+                if (a.final) {
+                    a.lam_out = lam_out;
+                    CK(cudaMemsetAsync(lam_out, 0, fbytes, ctx->stream));
+                }
+                CK(launch_adjoint_run<Real>(a, abs_terms, ctx->sms, ctx->stream));
+                ctx->launches++;
+                asteps += g.steps;
+            } else if (g.resident) {
+                ResidentArgs<Real> a = resident_args<Real>(ctx, rho_, dt_);
+                a.in = ops[g.from].src;
+                a.out = nullptr;
+                a.stores = d_table + g.table;
+                a.nsteps = g.steps;
+                CK(launch_resident_run<Real>(a, ctx->sms, ctx->stream));
+                ctx->launches++;
+                fsteps += g.steps;
+            } else {
+                for (size_t q = g.from; q < g.to; q++) advance(ops[q].src, ops[q].dst, ops[q].k);
+                CK(err);
+            }
+        }
+        return GBFK_OK;
     }
     static double beta(int c, int r)  // C(c + r, c) = C(c + r, r), capped; 0 for r < 0
     {
@@ -1901,7 +2009,8 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     // and face halos have p_w = p_g = 0, so both diffusivities of such a face
     // are 0 and its harmonic mean is 0), so no neighbour feeds their lambda.
     // They keep status kAdjMuZero in both sets and lambda 0.
-    bool ic_clean = false;  // every empty block of the initial condition holds +0
+    bool ic_clean = false;    // every empty block of the initial condition holds +0
+    bool ic_clamped = false;  // and every value of it is one of a clamped state
     if (e == cudaSuccess && ctx->identity_slots) {
         int *d_list = (int *)ctx->adj_mem[15];
         unsigned char *d_pos = (unsigned char *)(d_list + nb);
@@ -1912,9 +2021,12 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         ctx->launches++;
         if (e == cudaSuccess) {
-            ic_clean = true;
-            for (int b = 0; b < nb; b++)
+            ic_clean = ic_clamped = true;
+            for (int b = 0; b < nb; b++) {
+                if (pos[b] & 2) ic_clamped = false;
+                pos[b] &= 1;
                 if (bt[b] == kBlockEmpty && pos[b]) ic_clean = false;
+            }
             // blocks with tissue first, then empty blocks with a positive
             // initial value (a tumour outside the anatomy)
             std::vector<int> list;
@@ -1937,10 +2049,66 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     // after which no buffer is known to hold +0 there
     A.skip_empty = e == cudaSuccess && A.pipelined && ic_clean && std::isfinite(p->dt);
     if (!A.skip_empty) ctx->adj_clean.clear();  // full steps: nothing is tracked
+    // runs with resident blocks, where the blocks fit with their adjoint state
+    // (FP32 1184 on a B200, FP64 592) and nothing couples the empty ones
+    const bool resident = e == cudaSuccess && A.skip_empty && ic_clamped && p->nsteps > 0 &&
+                          ctx->step_pref == GBFK_STEP_AUTO && std::isfinite((double)(Real)p->Dw) &&
+                          std::isfinite((double)(Real)p->Dg) && std::isfinite((double)A.rho) &&
+                          resident_fits<Real>(ctx) && ctx->n_heavy <= adjoint_run_capacity<Real>(ctx->sms);
+    double *run_sums = nullptr;
+    if (resident) {
+        rc = build_resident<Real>(ctx);
+        const size_t n = (size_t)ctx->n_heavy, ex = 2 * n * 384 * 2 * sizeof(Real),
+                     acc = (size_t)adjoint_run_threads((int)n, ctx->sms) * 6 * sizeof(double),
+                     sums = (size_t)ctx->sms * 6 * sizeof(double), bytes = ex + acc + sums + 2 * sizeof(unsigned);
+        if (!rc) rc = topo_alloc(ctx, &ctx->d_adj_run, bytes);
+        if (rc) {
+            cleanup();
+            return rc;
+        }
+        char *d = (char *)ctx->d_adj_run;
+        if (!ctx->adj_run_ready) {
+            CK(cudaMemsetAsync(d, 0, bytes, ctx->stream));
+            ctx->adj_run_ready = true;
+        }
+        A.fs = ctx->stream;
+        A.record = true;
+        A.total_steps = p->nsteps;
+        A.lam_out = F;  // the horizon state is no longer needed by then
+        AdjRunArgs<Real> &r = A.run;
+        const ResidentArgs<Real> f = resident_args<Real>(ctx, p->rho, p->dt);
+        r.items = f.items;
+        r.nbr = f.nbr;
+        r.n = f.n;
+        r.H = f.H;
+        r.meta = f.meta;
+        r.pw = f.pw;
+        r.pg = f.pg;
+        r.bpd = f.bpd;
+        r.lam = A.LAM;
+        r.mu = A.sets[0].mu;
+        r.self = A.sets[0].self;
+        r.flags = A.sets[0].flags;
+        r.acc = (double *)(d + ex);
+        r.sums = run_sums = (double *)(d + ex + acc);
+        r.rho = A.rho;
+        r.dt = p->dt;
+        r.ih2 = f.ih2;
+        r.ex = (uint2 *)d;
+        r.index = (unsigned *)(d + ex + acc + sums);
+        r.err_flag = ctx->d_nan + 1;
+    }
     // forward to the horizon (storing the first chain of checkpoints), loss and its gradient
     if (e == cudaSuccess) {
         A.join(ctx->stream, A.fs);
         A.sweep(X0, F, p->nsteps, p->nsnapshots);
+        if (resident) {
+            rc = A.resident_sweep(p->rho, p->dt);
+            if (rc) {
+                cleanup();
+                return rc;
+            }
+        }
         A.adjoint_reads(F);
         e = A.err;
     }
@@ -1987,18 +2155,29 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     // reverse sweep, then lambda_0 into LAM
     if (e == cudaSuccess) {
         A.reverse_chain(0, p->nsteps, p->nsnapshots, X0);
+        if (resident) {
+            rc = A.resident_sweep(p->rho, p->dt);
+            if (rc) {
+                cleanup();
+                return rc;
+            }
+            A.LAM = A.lam_out;
+        }
         e = A.err;
     }
     if (e == cudaSuccess) {
-        A.finish();
+        if (!resident) A.finish();
         A.join(A.fs, ctx->stream);
         e = A.err;
     }
     // parameter gradients
-    std::vector<double> acc((size_t)nb * kGradSlots);
+    // per block, or (resident) per CTA
+    const size_t parts = resident ? (size_t)std::min(ctx->n_heavy, ctx->sms) : (size_t)nb;
+    std::vector<double> acc(parts * kGradSlots);
     std::vector<double> xp((size_t)xparts * 6, 0.0);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(acc.data(), A.grad_acc, acc.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(acc.data(), resident ? run_sums : A.grad_acc, acc.size() * sizeof(double),
+                            cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess && p->sigma > 0) {
         e = launch_x0_grad<Real>(bpd, X0, A.LAM, p->x0, p->sigma, xpart, xparts, ctx->stream);
         ctx->launches++;
@@ -2020,6 +2199,10 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cleanup();
     if (e != cudaSuccess) return fail(ctx, GBFK_E_CUDA, "forward_adjoint: %s", cudaGetErrorString(e));
+    if (resident) {
+        rc = check_stage_timeout(ctx);
+        if (rc) return rc;
+    }
     auto nsum = [](const double *v, size_t stride, size_t count) {
         double s = 0, c = 0;
         for (size_t i = 0; i < count; i++)
@@ -2033,14 +2216,20 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         return s + c;
     };
     res->loss = -(lik[1] + lik[2]);
-    res->drho = nsum(acc.data(), kGradSlots, nb);
-    res->dDw = nsum(acc.data() + 2, kGradSlots, nb);
+    res->drho = nsum(acc.data(), kGradSlots, parts);
+    res->dDw = nsum(acc.data() + 2, kGradSlots, parts);
     res->drho_abs = res->dDw_abs = 0;
     if (A.abs_terms)
-        for (int b = 0; b < nb; b++) {
-            res->drho_abs += acc[(size_t)b * kGradSlots + 4];
-            res->dDw_abs += acc[(size_t)b * kGradSlots + 5];
+        for (size_t b = 0; b < parts; b++) {
+            res->drho_abs += acc[b * kGradSlots + 4];
+            res->dDw_abs += acc[b * kGradSlots + 5];
         }
+    if (resident) {
+        res->drho *= p->dt;
+        res->dDw *= p->dt / A.Dw;
+        res->drho_abs *= p->dt;
+        res->dDw_abs *= fabs(p->dt / A.Dw);
+    }
     for (int d = 0; d < 3; d++) res->dx0[d] = p->sigma > 0 ? nsum(xp.data() + 2 * d, 6, xparts) : 0.0;
     res->forward_steps = A.fsteps;
     res->adjoint_steps = A.asteps;

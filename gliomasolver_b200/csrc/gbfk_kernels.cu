@@ -1453,16 +1453,21 @@ cudaError_t upload_ghost_table()
     return cudaMemcpyToSymbol(c_ghost_id, table, sizeof(table));
 }
 
-// out[b] = 1 when a cell of block b (pool order, identity slots) is > 0
+// out[b]: bit 0 a cell of block b (pool order, identity slots) is > 0, bit 1 a
+// cell is negative, -0 or above 1
 template <typename Real>
 __global__ void block_any_positive_kernel(const Real *__restrict__ phi, int nblocks, unsigned char *__restrict__ out)
 {
     for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
         const Real *q = phi + (int64_t)b * kBS3;
-        bool any = false;
-        for (int c = threadIdx.x; c < kBS3; c += blockDim.x) any |= q[c] > (Real)0;
+        bool any = false, off = false;
+        for (int c = threadIdx.x; c < kBS3; c += blockDim.x) {
+            any |= q[c] > (Real)0;
+            off |= q[c] > (Real)1 || (signbit(q[c]) && q[c] == q[c]);
+        }
         any = __syncthreads_or(any);
-        if (threadIdx.x == 0) out[b] = any ? 1 : 0;
+        off = __syncthreads_or(off);
+        if (threadIdx.x == 0) out[b] = (any ? 1 : 0) | (off ? 2 : 0);
     }
 }
 

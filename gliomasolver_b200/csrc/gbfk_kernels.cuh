@@ -300,7 +300,49 @@ cudaError_t launch_adjoint_fused(const PoolView<Real> &v, const Real *H, const u
                                  const double *ih2, const Real *phi, Real *lam, const AdjBuffers &prev,
                                  const AdjBuffers &out, int mode, bool abs_terms, const int *blocks, int nlaunch,
                                  Real rho, double dt, double Dw, double *grad_acc, cudaStream_t s);
-// out[b] = 1 when a cell of block b (identity slots) is > 0
+// A run of nsteps adjoint steps with the heavy blocks resident in shared memory
+// (gbfk_resident_adjoint.cu), for sweeps whose empty blocks hold +0 in every
+// state: items, nbr, H, meta, pw, pg, bpd as in ResidentArgs.  states: nsteps
+// device pointers, phi_k of the steps in the order they run (k descending).
+// first: lambda' of the first step is lam; otherwise the run goes on from mu
+// (n * 512 Real), self (n * 512) and flags (n * 512), which a run leaves for
+// the next one, and from acc (adjoint_run_threads * 6 doubles).  final: after
+// the steps lambda_0 goes to the heavy blocks of lam_out and the sums of every CTA
+// (rho sum, compensation, Dw sum, compensation, magnitudes of rho and Dw, to be
+// multiplied by dt, those of Dw also by 1 / Dw) to sums (6 per CTA, at most one
+// CTA per SM).  ex: 2 * n * 384 words of 8 bytes
+// (FP64: 16), index: 2 words, both zeroed once per item list.
+template <typename Real>
+struct AdjRunArgs {
+    const int *items, *nbr;
+    int n;
+    const Real *H;
+    const unsigned short *meta;
+    const Real *pw, *pg;
+    int bpd;
+    const Real *const *states;
+    int nsteps;
+    int first, final;
+    const Real *lam;
+    Real *lam_out;
+    void *mu;
+    double *self;
+    unsigned char *flags;
+    double *acc, *sums;
+    Real rho;
+    double dt, ih2;
+    uint2 *ex;
+    unsigned *index;
+    unsigned *err_flag;
+    unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
+};
+template <typename Real>
+int adjoint_run_capacity(int sms);
+int adjoint_run_threads(int n, int sms);
+template <typename Real>
+cudaError_t launch_adjoint_run(const AdjRunArgs<Real> &a, bool abs_terms, int sms, cudaStream_t s);
+// out[b]: bit 0 a cell of block b (identity slots) is > 0, bit 1 a cell is no
+// value of a clamped state (+0 <= phi <= 1, or NaN)
 template <typename Real>
 cudaError_t launch_block_any_positive(const Real *phi, int nblocks, unsigned char *out, cudaStream_t s);
 // dL/dphi of loss = -(L_T1c + L_FLAIR) in pool order; roi_count: NULL (every

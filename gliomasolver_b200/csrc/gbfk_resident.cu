@@ -40,222 +40,16 @@
 // and a heavy block's cell next to an empty block is kEmpty itself.  Their
 // cells run all steps of the call in registers (empty_blocks), usually +0 in
 // and out, and nobody waits for them.
-#include <cuda_runtime.h>
-
-#include <cstdint>
-#include <mutex>
-#include <type_traits>
-#include <vector>
-
-#include "gbfk_exact.cuh"
-#include "gbfk_kernels.cuh"
+#include "gbfk_resident.cuh"
 
 namespace gbfk {
 namespace {
-
-constexpr unsigned long long kPollNs = 1000000000ull;  // a face not seen after 1 s is declared lost
-constexpr unsigned kErrPoll = 1u | 512u;               // error word: a wait gave up, in a resident run
-
-__device__ __forceinline__ unsigned long long now_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-// ---- words of the exchange buffer -----------------------------------------
-// N consecutive values in 16-, 8- or 4-byte accesses, each value one relaxed
-// access of its own (no order among them is needed: each carries its phase)
-template <int N>
-__device__ __forceinline__ void ld_face(const float *p, float (&v)[N])
-{
-    if constexpr (N % 4 == 0) {
-#pragma unroll
-        for (int i = 0; i < N; i += 4)
-            asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3])
-                         : "l"(p + i)
-                         : "memory");
-    } else
-        asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p) : "memory");
-}
-template <int N>
-__device__ __forceinline__ void ld_face(const double *p, double (&v)[N])
-{
-#pragma unroll
-    for (int i = 0; i < N; i += 2)
-        asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];"
-                     : "=d"(v[i]), "=d"(v[i + 1])
-                     : "l"(p + i)
-                     : "memory");
-}
-template <int N>
-__device__ __forceinline__ void st_face(float *p, const float (&v)[N])
-{
-    if constexpr (N % 4 == 0) {
-#pragma unroll
-        for (int i = 0; i < N; i += 4)
-            asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + i), "f"(v[i]), "f"(v[i + 1]),
-                         "f"(v[i + 2]), "f"(v[i + 3])
-                         : "memory");
-    } else
-        asm volatile("st.relaxed.gpu.global.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v[0]), "f"(v[1]) : "memory");
-}
-template <int N>
-__device__ __forceinline__ void st_face(double *p, const double (&v)[N])
-{
-#pragma unroll
-    for (int i = 0; i < N; i += 2)
-        asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + i), "d"(v[i]), "d"(v[i + 1]) : "memory");
-}
-__device__ __forceinline__ void st_face1(float *p, float v)
-{
-    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_face1(double *p, double v)
-{
-    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-}
-// value with the sign bit set to the phase (m: the sign bit or 0), in one
-// instruction the compiler does not see through: written with bit operators it
-// becomes +-|v| in floating point, which drops the sign of a NaN
-__device__ __forceinline__ unsigned with_phase_bits(unsigned v, unsigned m)
-{
-    unsigned r;
-    asm("lop3.b32 %0, %1, 0x7fffffff, %2, 0xEA;" : "=r"(r) : "r"(v), "r"(m));  // (v & 0x7fffffff) | m
-    return r;
-}
-__device__ __forceinline__ float with_phase(float v, unsigned m)
-{
-    return __uint_as_float(with_phase_bits(__float_as_uint(v), m));
-}
-__device__ __forceinline__ double with_phase(double v, unsigned m)
-{
-    return __hiloint2double((int)with_phase_bits((unsigned)__double2hiint(v), m), __double2loint(v));
-}
-// the sign bit differs from the phase: not there yet
-__device__ __forceinline__ unsigned sign_xor(float v, unsigned m) { return __float_as_uint(v) ^ m; }
-__device__ __forceinline__ unsigned sign_xor(double v, unsigned m) { return (unsigned)__double2hiint(v) ^ m; }
-__device__ __forceinline__ float magnitude(float v) { return __uint_as_float(__float_as_uint(v) & 0x7fffffffu); }
-__device__ __forceinline__ double magnitude(double v)
-{
-    return __hiloint2double(__double2hiint(v) & 0x7fffffff, __double2loint(v));
-}
-
-// The cells of a block are held by kT = 512 / kC threads, kC x-consecutive
-// cells each.  Arrays in shared memory keep 16-byte vectors (or all kC cells,
-// if they are fewer) as [vector][thread], so that a warp's access is one
-// contiguous run of banks for every neighbour offset; rows of a face array
-// count as threads too (kRows rows of 8).
-template <typename Real, int kC, int kMaxV = 16 / (int)sizeof(Real)>
-struct Tile {
-    static constexpr int V = kMaxV < kC ? kMaxV : kC;
-    // where cell x of a row lies in an array of kRows rows
-    template <int kRows>
-    static __device__ __forceinline__ int at(int row, int x)
-    {
-        const int t = row * (8 / kC) + x / kC, v = (x % kC) / V;
-        return (v * (kRows * 8 / kC) + t) * V + x % V;
-    }
-    // the kC cells of "thread" t of such an array
-    template <int kRows>
-    static __device__ __forceinline__ void load(const Real *a, int t, Real (&d)[kC])
-    {
-#pragma unroll
-        for (int v = 0; v < kC / V; v++) {
-            const Real *p = a + (v * (kRows * 8 / kC) + t) * V;
-            if constexpr (sizeof(Real) == 4 && V == 4) {
-                const float4 q = *reinterpret_cast<const float4 *>(p);
-                d[4 * v] = q.x; d[4 * v + 1] = q.y; d[4 * v + 2] = q.z; d[4 * v + 3] = q.w;
-            } else if constexpr (sizeof(Real) == 4) {
-                const float2 q = *reinterpret_cast<const float2 *>(p);
-                d[2 * v] = q.x; d[2 * v + 1] = q.y;
-            } else {
-                const double2 q = *reinterpret_cast<const double2 *>(p);
-                d[2 * v] = q.x; d[2 * v + 1] = q.y;
-            }
-        }
-    }
-    // pair v of thread t of an array with two-value vectors
-    template <int kRows>
-    static __device__ __forceinline__ int at2(int t, int v)
-    {
-        static_assert(V == 2, "pairs");
-        return (v * (kRows * 8 / kC) + t) * 2;
-    }
-    template <int kRows>
-    static __device__ __forceinline__ void load2(const Real *a, int t, int v, Real (&d)[2])
-    {
-        const Real *p = a + at2<kRows>(t, v);
-        if constexpr (sizeof(Real) == 4) {
-            const float2 q = *reinterpret_cast<const float2 *>(p);
-            d[0] = q.x; d[1] = q.y;
-        } else {
-            const double2 q = *reinterpret_cast<const double2 *>(p);
-            d[0] = q.x; d[1] = q.y;
-        }
-    }
-    template <int kRows>
-    static __device__ __forceinline__ void store(Real *a, int t, const Real (&d)[kC])
-    {
-#pragma unroll
-        for (int v = 0; v < kC / V; v++) {
-            Real *p = a + (v * (kRows * 8 / kC) + t) * V;
-            if constexpr (sizeof(Real) == 4 && V == 4)
-                *reinterpret_cast<float4 *>(p) = make_float4(d[4 * v], d[4 * v + 1], d[4 * v + 2], d[4 * v + 3]);
-            else if constexpr (sizeof(Real) == 4)
-                *reinterpret_cast<float2 *>(p) = make_float2(d[2 * v], d[2 * v + 1]);
-            else
-                *reinterpret_cast<double2 *>(p) = make_double2(d[2 * v], d[2 * v + 1]);
-        }
-    }
-};
-// kC consecutive cells of a block in global memory (16-byte aligned, or 8 for two floats)
-template <typename Real, int kC>
-__device__ __forceinline__ void ld_cells(const Real *p, Real (&d)[kC])
-{
-#pragma unroll
-    for (int v = 0; v < kC / Tile<Real, kC>::V; v++) {
-        constexpr int V = Tile<Real, kC>::V;
-        if constexpr (sizeof(Real) == 4 && V == 4) {
-            const float4 q = *reinterpret_cast<const float4 *>(p + 4 * v);
-            d[4 * v] = q.x; d[4 * v + 1] = q.y; d[4 * v + 2] = q.z; d[4 * v + 3] = q.w;
-        } else if constexpr (sizeof(Real) == 4) {
-            const float2 q = *reinterpret_cast<const float2 *>(p + 2 * v);
-            d[2 * v] = q.x; d[2 * v + 1] = q.y;
-        } else {
-            const double2 q = *reinterpret_cast<const double2 *>(p + 2 * v);
-            d[2 * v] = q.x; d[2 * v + 1] = q.y;
-        }
-    }
-}
-template <typename Real, int kC>
-__device__ __forceinline__ void st_cells(Real *p, const Real (&d)[kC])
-{
-    // consecutive vectors: a one-thread array
-#pragma unroll
-    for (int v = 0; v < kC / Tile<Real, kC>::V; v++) {
-        constexpr int V = Tile<Real, kC>::V;
-        if constexpr (sizeof(Real) == 4 && V == 4)
-            *reinterpret_cast<float4 *>(p + 4 * v) = make_float4(d[4 * v], d[4 * v + 1], d[4 * v + 2], d[4 * v + 3]);
-        else if constexpr (sizeof(Real) == 4)
-            *reinterpret_cast<float2 *>(p + 2 * v) = make_float2(d[2 * v], d[2 * v + 1]);
-        else
-            *reinterpret_cast<double2 *>(p + 2 * v) = make_double2(d[2 * v], d[2 * v + 1]);
-    }
-}
 
 // One resident block in shared memory: two states, each with its face halos
 // (rows y = -1 .. 8 of planes z = -1 .. 8, and the x faces apart), and the
 // face coefficients, in two-value vectors: x faces as eight left faces per row
 // and the row's last face apart, y and z faces as in H.  A coefficient carries a set sign bit
 // where either cell of the face is kEmpty (see row_cells).
-constexpr int kRows = 100;
-template <typename Real>
-struct alignas(16) ResidentState {
-    Real phi[kRows * 8];
-    Real xh[2][64];          // [z][y]: the x- and x+ neighbours' cells
-};
 template <typename Real>
 struct alignas(16) ResidentBlock {
     ResidentState<Real> st[2];
@@ -264,116 +58,9 @@ struct alignas(16) ResidentBlock {
     int e;                   // block * 4 + block type
     unsigned kinds;          // two bits per warp: the row_cells variant its cells need
 };
-constexpr unsigned kPlain = 0, kEdge = 1, kGeneral = 2;
-
-__device__ __forceinline__ float set_sign(float v, bool s) { return s ? __uint_as_float(__float_as_uint(v) | 0x80000000u) : v; }
-__device__ __forceinline__ double set_sign(double v, bool s) { return s ? -v : v; }
-__device__ __forceinline__ bool sign_of(float v) { return __float_as_int(v) < 0; }
-__device__ __forceinline__ bool sign_of(double v) { return __double2hiint(v) < 0; }
-
-// d = a * b and d += a for two values, each rounded to nearest by itself; one
-// instruction for two floats.  The product is an FMA with -0 (which adds
-// nothing, signs of zero included), and that -0 (neg0: both halves) comes
-// from the host: the assembler contracts a packed multiply, or a packed FMA
-// with a -0 it can see, with the packed add that follows.
-__device__ __forceinline__ unsigned long long packed(const float (&v)[2])
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v[0]), "f"(v[1]));
-    return r;
-}
-__device__ __forceinline__ void pair_mul(float (&d)[2], const float (&a)[2], const float (&b)[2],
-                                         unsigned long long neg0)
-{
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(packed(a)), "l"(packed(b)), "l"(neg0));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d[0]), "=f"(d[1]) : "l"(r));
-}
-__device__ __forceinline__ void pair_add(float (&d)[2], const float (&a)[2])
-{
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(packed(d)), "l"(packed(a)));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d[0]), "=f"(d[1]) : "l"(r));
-}
-__device__ __forceinline__ void pair_mul(double (&d)[2], const double (&a)[2], const double (&b)[2],
-                                         unsigned long long)
-{
-    d[0] = rmul(a[0], b[0]);
-    d[1] = rmul(a[1], b[1]);
-}
-__device__ __forceinline__ void pair_add(double (&d)[2], const double (&a)[2])
-{
-    d[0] = radd(d[0], a[0]);
-    d[1] = radd(d[1], a[1]);
-}
-// clamp01 of a rounded result (its NaN is the canonical one): two instructions
-__device__ __forceinline__ float clamp_state(float p)
-{
-    asm("max.NaN.f32 %0, %0, 0f00000000;" : "+f"(p));
-    asm("min.NaN.f32 %0, %0, 0f3F800000;" : "+f"(p));
-    return p;
-}
-__device__ __forceinline__ double clamp_state(double p) { return clamp01(p); }
-
-// p_w, p_g of cell (x, y, z) of block blk, or of the one cell outside it
-// across a face, on the uniform bpd^3 grid
-template <typename Real>
-__device__ __noinline__ void tissue_at(const Real *pw_all, const Real *pg_all, int bpd, int blk, int x, int y, int z,
-                                       Real &pw, Real &pg)
-{
-    int bx = blk % bpd, by = (blk / bpd) % bpd, bz = blk / (bpd * bpd);
-    if (x < 0) bx = bx ? bx - 1 : bpd - 1;
-    if (x > 7) bx = bx + 1 < bpd ? bx + 1 : 0;
-    if (y < 0) by = by ? by - 1 : bpd - 1;
-    if (y > 7) by = by + 1 < bpd ? by + 1 : 0;
-    if (z < 0) bz = bz ? bz - 1 : bpd - 1;
-    if (z > 7) bz = bz + 1 < bpd ? bz + 1 : 0;
-    const int64_t g = ((int64_t)bx + (int64_t)bpd * (by + (int64_t)bpd * bz)) * kBS3 + (x & 7) +
-                      kBS * ((y & 7) + kBS * (z & 7));
-    pw = pw_all[g];
-    pg = pg_all[g];
-}
-
-// What a thread needs to know of its place in a block, fixed for the run.
-struct Place {
-    int t;        // thread of the group
-    int tp;       // its place in the padded state array
-    int ty;       // its place in hy
-    int xl, xr;   // element offsets in ResidentState of the cells before and after its own
-    int he;       // element offset from hx of the last cell's right face
-};
-template <typename Real, int kC>
-__device__ __forceinline__ Place place_of(int t)
-{
-    using TL = Tile<Real, kC, 2>;
-    constexpr int R = 8 / kC;  // threads of a row
-    const int x0 = (t % R) * kC, y = (t / R) & 7, z = t / (8 * R);
-    const int row = z * 8 + y, prow = (z + 1) * 10 + y + 1;
-    Place w;
-    w.t = t;
-    w.tp = prow * R + x0 / kC;
-    w.ty = t + z * R;  // row z * 9 + y
-    w.xl = x0 ? TL::template at<kRows>(prow, x0 - 1) : kRows * 8 + row;
-    w.xr = x0 + kC < 8 ? TL::template at<kRows>(prow, x0 + kC) : kRows * 8 + 64 + row;
-    w.he = x0 + kC < 8 ? Tile<Real, kC, 2>::template at<64>(row, x0 + kC) : kBS3 + row;
-    return w;
-}
-
 // The kC cells of a thread in block b, from the state S with its halos (a
-// clamped state) to out.  kKind, by warp:
-//   kPlain    every cell and neighbour is kTissue: no no-flux doubling, every
-//             cell is inside the domain;
-//   kEdge     kEmpty cells or neighbours among them.  The coefficient of a
-//             face that touches a kEmpty cell is 0, so its sign bit says so
-//             (-0): a neighbour with phi < 0.1 across such a face doubles the
-//             opposite coefficient (for a kEmpty cell itself, whose
-//             coefficients are all 0, whatever is doubled stays 0, and its
-//             formula leaves +0 where phi is +0 and the reaction where it is
-//             not, so that its domain test needs no branch).  -0 for +0 in
-//             the flux sums gives the same sums: (+0) + (-0) = +0 either way;
-//   kGeneral  kOther cells or neighbours, or a coefficient that is negative
-//             by itself: classes from the meta words, p_w and p_g from global
-//             memory.
+// clamped state) to out; kKind: the cells of the thread's warp (kPlain, kEdge
+// or kGeneral).
 template <typename Real, int kC, unsigned kKind>
 __device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, double ih2, unsigned long long neg0,
                                           const ResidentBlock<Real> &b, const ResidentState<Real> &S, const Place &w,
@@ -384,7 +71,6 @@ __device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, double ih
     Real p[kC];
     TL::template load<kRows>(S.phi, w.tp, p);
     const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
-    const Real eps = (Real)0.1;
     constexpr bool kLow = kKind != kPlain;
     // two cells at a time, so that the single-precision operations of the flux
     // sums can go in pairs (pair_add, pair_mul: each half rounded by itself),
@@ -410,28 +96,11 @@ __device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, double ih
         if (kLow) {
 #pragma unroll
             for (int j = 0; j < 2; j++) {
-                bool low[6] = {sign_of(d0[j]) && xm[j] < eps, sign_of(d1[j]) && xp[j] < eps,
-                               sign_of(d2[j]) && y0[j] < eps, sign_of(d3[j]) && y1[j] < eps,
-                               sign_of(d4[j]) && z0[j] < eps, sign_of(d5[j]) && z1[j] < eps};
-                if (kKind == kGeneral) {
-                    const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
-                    const int blk = b.e >> 2, cell = w.t * kC + i + j, x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-                    const unsigned mw = a.meta[(int64_t)blk * kBS3 + cell];
-#pragma unroll
-                    for (int k = 0; k < 6; k++) low[k] = ((mw >> (2 + k)) & 1u) && phn[k] < eps;
-                    Real pw, pg;
-                    if ((mw & 3u) == kOther) {
-                        tissue_at(a.pw, a.pg, a.bpd, blk, x, y, z, pw, pg);
-                        dom[j] = in_domain(pw, pg, ph[j]);
-                    }
-#pragma unroll
-                    for (int k = 0; k < 6; k++)
-                        if ((mw >> (8 + k)) & 1u) {
-                            tissue_at(a.pw, a.pg, a.bpd, blk, x + (k == 1) - (k == 0), y + (k == 3) - (k == 2),
-                                      z + (k == 5) - (k == 4), pw, pg);
-                            low[k] = domain_chf(phn[k], pw, pg) < eps;
-                        }
-                }
+                const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
+                const Real df[6] = {d0[j], d1[j], d2[j], d3[j], d4[j], d5[j]};
+                bool low[6];
+                dom[j] = no_flux_tests<Real, kKind>(a.meta, a.pw, a.pg, a.bpd, b.e >> 2, w.t * kC + i + j, ph[j], phn, df,
+                                                    low);
                 // _applyNoFluxBC: neighbour k below 0.1 doubles the opposite coefficient
                 if (low[0]) d1[j] = rmul(d1[j], (Real)2.);
                 if (low[1]) d0[j] = rmul(d0[j], (Real)2.);
@@ -542,7 +211,7 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
     using TL = Tile<Real, kC, 2>;
     constexpr int kT = kBS3 / kC;  // threads of a group
     constexpr int R = 8 / kC;      // threads of a row
-    const int t = threadIdx.x % kT, group = threadIdx.x / kT, lane = threadIdx.x & 31;
+    const int t = threadIdx.x % kT, group = threadIdx.x / kT;
     const int nlocal = a.n > c ? (a.n - 1 - c) / G + 1 : 0;
     const Place w = place_of<Real, kC>(t);
     const int x0 = (t % R) * kC, y = (t / R) & 7, z = t / (8 * R), row = z * 8 + y;
@@ -581,44 +250,11 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
         ResidentBlock<Real> &b = blocks[j];
         const int item = c + j * G, e = a.items[item];
         const int64_t blk = e >> 2;
-        const unsigned short *meta = a.meta + blk * kBS3;
         Real p[kC];
         ld_cells(a.in + blk * kBS3 + t * kC, p);
         TL::template store<kRows>(b.st[0].phi, w.tp, p);
         publish(item, p, k0);
-        const Real *H = a.H + blk * kFacesPerBlock;
-        // face f along a direction touches a kEmpty cell: the cell after it is
-        // kEmpty or has a kEmpty neighbour before it (the last face: the cell
-        // before it, and its neighbour after it)
-        auto touches = [&](int cell, int nb) { return (meta[cell] & 3u) == kEmpty || ((meta[cell] >> (2 + nb)) & 1u); };
-        for (int q = t; q < 576; q += kT) {
-            {
-                const int f = q % 9, row = q / 9;
-                const Real h = set_sign(H[q], f < 8 ? touches(row * 8 + f, 0) : touches(row * 8 + 7, 1));
-                if (f < 8) b.hx[TL::template at<64>(row, f)] = h;
-                else b.hx8[row] = h;
-            }
-            {
-                const int x = q & 7, f = (q >> 3) % 9, zz = q / 72, row = q >> 3;
-                b.hy[TL::template at<72>(row, x)] =
-                    set_sign(H[576 + q], f < 8 ? touches(zz * 64 + f * 8 + x, 2) : touches(zz * 64 + 56 + x, 3));
-            }
-            {
-                const int x = q & 7, yy = (q >> 3) & 7, f = q >> 6, row = q >> 3;
-                b.hz[TL::template at<72>(row, x)] =
-                    set_sign(H[1152 + q], f < 8 ? touches(f * 64 + yy * 8 + x, 4) : touches(448 + yy * 8 + x, 5));
-            }
-        }
-        unsigned kind = kPlain;
-        for (int i = 0; i < kC; i++) {
-            const unsigned m = meta[t * kC + i];
-            if ((m & 3u) == kOther || (m >> 8)) kind = kGeneral;
-            else if (m != kMetaAllTissue && kind == kPlain) kind = kEdge;
-        }
-        if (t == 0) {
-            b.e = e;
-            b.kinds = 0;
-        }
+        if (t == 0) b.e = e;
         if (t < 6) {
             const int nb = a.nbr[item * 6 + t];
             b.nbr[t] = nb < 0 ? -1 : nb * 384;
@@ -627,21 +263,7 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
             for (int v = 0; v < kC / TL::V; v++)
                 for (int i = 0; i < TL::V; i++) b.st[0].phi[pd + v * pstep + i] = b.st[1].phi[pd + v * pstep + i] = (Real)0;
         }
-        group_sync();
-        // a coefficient that is negative by itself (a negative tissue fraction)
-        // has a sign that says nothing of kEmpty cells
-        for (int i = 0; i < kC; i++) {
-            const unsigned m = meta[t * kC + i];
-            const int x = x0 + i;
-            const Real d[6] = {b.hx[TL::template at<64>(row, x)],
-                               x < 7 ? b.hx[TL::template at<64>(row, x + 1)] : b.hx8[row],
-                               b.hy[TL::template at<72>(row + z, x)], b.hy[TL::template at<72>(row + z + 1, x)],
-                               b.hz[TL::template at<72>(row, x)], b.hz[TL::template at<72>(row + 8, x)]};
-            for (int k = 0; k < 6; k++)
-                if (sign_of(d[k]) != ((m & 3u) == kEmpty || ((m >> (2 + k)) & 1u))) kind = kGeneral;
-        }
-        const bool general = __any_sync(0xffffffffu, kind == kGeneral), edge = __any_sync(0xffffffffu, kind == kEdge);
-        if (lane == 0) atomicOr(&b.kinds, (general ? kGeneral : edge ? kEdge : kPlain) << (2 * (t >> 5)));
+        load_coefficients<Real, kC>(b, a.H + blk * kFacesPerBlock, a.meta + blk * kBS3, t, group_sync);
     }
     group_sync();
 
@@ -780,41 +402,6 @@ resident_teams_kernel(const ResidentArgs<Real> *runs, const int *off, const int 
         if (threadIdx.x == 0) me.run++;
         __syncthreads();
     }
-}
-
-constexpr int kMaxSmem = 227 * 1024;
-
-// A cooperative launch (CTAs wait for one another, so all must be resident)
-// with the kernel's shared memory limit raised once per device.
-template <auto kernel, typename... Args>
-cudaError_t launch_coop(int ctas, int threads, size_t smem, cudaStream_t s, Args... args)
-{
-    static std::mutex mu;
-    static std::vector<char> raised;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if ((int)raised.size() <= dev) raised.resize(dev + 1, 0);
-        if (!raised[dev]) {
-            if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)) !=
-                cudaSuccess)
-                return e;
-            raised[dev] = 1;
-        }
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // Cells per thread and groups per CTA by the blocks of a CTA (`per`).  Up to

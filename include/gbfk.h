@@ -321,8 +321,12 @@ int gbfk_batch_log_likelihood(gbfk_batch *b, const gbfk_likelihood_params *param
  * States are kept with binomial checkpointing in nsnapshots device buffers;
  * these and seven work fields stay allocated in the context until
  * gbfk_destroy, so that later calls on the same grid with at most as many
- * checkpoints allocate nothing.  The forward steps of the reverse sweep run
- * on a second stream of the context (created at the first call, ordered
+ * checkpoints allocate nothing.  Where the blocks that hold tissue fit in the
+ * SMs' shared memory with their adjoint state (about 1180 in FP32, 590 in FP64
+ * on a B200) and the initial state lies in [0, 1] and is +0 in the others, the
+ * steps that follow one another in the sweep run in one cooperative launch,
+ * on the context's stream.  Elsewhere the forward steps of the reverse sweep
+ * run on a second stream of the context (created at the first call, ordered
  * after the work already on the context's stream) next to the adjoint steps;
  * the call returns when both are done.  GBFK_ADJ_STREAMS=1 keeps everything
  * on the context's stream (the same results). */

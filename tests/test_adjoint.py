@@ -450,3 +450,49 @@ def test_adjoint_with_a_roi_matches_central_differences():
     assert np.linalg.norm(dev["grad_c0"] - lam0) <= 1e-13 * np.linalg.norm(lam0)
     assert dev["dDw"] == pytest.approx(ddw, rel=1e-12)
     pool.close()
+
+
+@pytest.mark.parametrize("prec,n,steps", [("f64", 8, 9), ("f64", 64, 21), ("f32", 64, 40), ("f32", 128, 30)])
+def test_resident_sweep_equals_launches_per_step(prec, n, steps):
+    """The sweep with resident blocks (AUTO) against the one that launches each
+    step (the pipelined kernel forced), with tissue fractions below 0.1, from
+    one block (its own neighbour) to seven blocks per SM, few and all
+    checkpoints.  Both evaluate the same terms; only the compensated sums of
+    the gradients are grouped otherwise, and lambda_0 is the same number in
+    every cell.  An initial field outside [0, 1] takes the launches."""
+    from gliomasolver_b200 import BlockPool
+
+    R = np.float64 if prec == "f64" else np.float32
+    bpd = n // 8
+    pw, pg, _ = make_anatomy(n, 3)
+    rng = np.random.default_rng(n)
+    thin = rng.random(pw.shape) < 0.02
+    pw[thin] *= 0.08
+    pg[thin] *= 0.08
+    sched = make_schedule(0.2, 0.1, 100.0, L, bpd, prec)
+    dt = min(sched.dt, 0.2)  # at 8^3 the schedule's step saturates every cell, which ends every gradient
+    c0 = tumor_ic(n, (0.5, 0.45, 0.5), pw, pg).astype(R)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
+    with BlockPool(bpd ** 3, prec) as pool:
+        pool.set_uniform(bpd)
+        pool.upload_dense("p_w", pw.astype(R))
+        pool.upload_dense("p_g", pg.astype(R))
+        pool.set_observations(t1, fl)
+        for scale, shots in ((1.0, (4, steps + 1)), (1.5, (4,))):
+            for k in shots:
+                out = {}
+                for kind in ("pipelined", "auto"):
+                    pool.step_kernel = kind
+                    pool.upload_dense("phi", (scale * c0).astype(R))
+                    before = pool.launches
+                    out[kind] = pool.forward_adjoint(sched.Dw, sched.Dg, sched.rho, dt, steps, sigma=0.0,
+                                                     nsnapshots=k, grad_c0=True, term_magnitudes=True, **UC)
+                    out[kind]["launches"] = pool.launches - before
+                a, b = out["auto"], out["pipelined"]
+                assert np.array_equal(a["grad_c0"], b["grad_c0"]) and np.count_nonzero(b["grad_c0"]) > n
+                assert a["loss"] == b["loss"] and a["forward_steps"] == b["forward_steps"]
+                for key in ("dDw", "drho", "dDw_abs", "drho_abs"):
+                    bound = 1e-14 * b[key.replace("_abs", "") + "_abs"]
+                    assert abs(a[key] - b[key]) <= bound + 1e-13 * abs(b[key]), key
+                if scale == 1.0 and k > 4:
+                    assert a["launches"] < steps < b["launches"]
