@@ -52,7 +52,7 @@ enum gbfk_status {
     GBFK_E_NAN = 4,     /* a step produced NaN/Inf in phi */
     GBFK_E_TIMEOUT = 5, /* a bounded device wait gave up */
     GBFK_E_STATE = 6,   /* required data (topology, fields) not uploaded */
-    GBFK_E_TOO_LARGE = 7, /* grid larger than gbfk_rd_step_static's fixed scratch */
+    GBFK_E_TOO_LARGE = 7, /* grid larger than gbfk_rd_step_static takes */
     GBFK_E_IO = 8         /* a file could not be opened, read or written, or is malformed */
 };
 
@@ -418,9 +418,7 @@ int gbfk_probe_bounded_wait(int device, double *seconds);
  * cannot let the library call cudaMalloc: code whose device memory belongs to
  * another allocator that reserved it up front, or a time loop that must not
  * pay cudaMalloc's device-wide synchronisation.  It allocates nothing and
- * frees nothing: its scratch (face coefficients, meta words, block types,
- * neighbour table) is one fixed device array of about 7.3 MiB that every GPU
- * loading the library holds until the process exits.
+ * frees nothing: one kernel forms the face coefficients and takes the step.
  *   pw, pg, phi_in : device arrays of bpd^3 * 512 Real in block-pool order
  *                    (block (bx,by,bz) at slot bx + bpd*(by + bpd*bz));
  *   phi_out        : device array of the same size that overlaps phi_in
@@ -428,12 +426,8 @@ int gbfk_probe_bounded_wait(int device, double *seconds);
  *   Dw, Dg, rho, dt: as for gbfk_rd_step; stream: a cudaStream_t of `device`
  *                    (GBFK_E_INVALID for another device's stream) or NULL for
  *                    the legacy default stream; device: CUDA ordinal.
- * Returns GBFK_E_TOO_LARGE when bpd^3 > GBFK_STATIC_MAX_BLOCKS.  Every call
- * on a device shares the scratch array (it keeps the last call's contents and
- * is fully rewritten by each call), so calls that overlap on the GPU race:
- * serialise them.  The first call on a device (and the first after its
- * context was reset) looks up the array's address with that device current;
- * make it before any stream capture.  The work is asynchronous on the stream.
+ * Returns GBFK_E_TOO_LARGE when bpd^3 > GBFK_STATIC_MAX_BLOCKS.  Calls share
+ * nothing but the caller's buffers.  The work is asynchronous on the stream.
  * No NaN check: a step that produces NaN or Inf still returns GBFK_OK (check
  * the output where that matters).  The caller's current device is restored;
  * an error the caller's earlier work left pending is returned as GBFK_E_CUDA

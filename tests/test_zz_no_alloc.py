@@ -106,3 +106,38 @@ def test_static_step_argument_checks(gbfk_lib):
         other = torch.cuda.Stream(device=1)
         assert L.gbfk_rd_step_static(_lib.GBFK_F32, 2, at(0), at(0), at(0), at(n), 1e-4, 1e-5, 0.1, 0.1,
                                      ctypes.c_void_p(other.cuda_stream), 0) == 1
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("bpd", [1, 2, 3, 7, 8])
+@pytest.mark.parametrize("dt", [None, float("inf")])
+def test_static_step_equals_rd_step_on_any_values(gbfk_lib, prec, bpd, dt):
+    """Every block count per direction at the edges of its range (one block is its own neighbour), and states and
+    tissue that no clamp has seen: negative, above 1, minus zero, NaN.  Bit for bit, NaN in the same cells."""
+    import torch
+
+    n, R = 8 * bpd, np.float64 if prec == "f64" else np.float32
+    r = np.random.default_rng(bpd)
+    pw, pg, c0 = (np.where(r.random((n, n, n)) < 0.5, 0.0, r.uniform(-0.05, 1.2, (n, n, n))).astype(R) for _ in range(3))
+    c0[r.random(c0.shape) < 0.1] = -0.0
+    c0[r.random(c0.shape) < 0.002] = np.nan
+    s = make_schedule(0.2, 0.05, 300.0, 25.6, bpd, prec)
+    dt = s.dt if dt is None else dt
+    with BlockPool(bpd ** 3, prec) as pool:
+        pool.set_uniform(bpd)
+        pool.upload_dense("p_w", pw)
+        pool.upload_dense("p_g", pg)
+        pool.upload_dense("phi", c0)
+        pool.rd_step(s.Dw, s.Dg, s.rho, dt, 1, check_nan=False)
+        want = _pool_order(pool.download_dense("phi"))
+    d_pw, d_pg, d_in = (torch.from_numpy(_pool_order(a)).cuda() for a in (pw, pg, c0))
+    d_out = torch.empty_like(d_in)
+    at = ctypes.c_void_p
+    assert _lib.load().gbfk_rd_step_static(
+        _lib.GBFK_F64 if prec == "f64" else _lib.GBFK_F32, bpd, at(d_pw.data_ptr()), at(d_pg.data_ptr()),
+        at(d_in.data_ptr()), at(d_out.data_ptr()), s.Dw, s.Dg, s.rho, dt,
+        at(torch.cuda.current_stream().cuda_stream), 0) == _lib.GBFK_OK
+    torch.cuda.synchronize()
+    got = d_out.cpu().numpy()
+    assert np.array_equal(got, want, equal_nan=True)
+    assert np.array_equal(np.signbit(got), np.signbit(want)) or np.isnan(want).any()
