@@ -128,7 +128,7 @@ struct gbfk_ctx {
     bool phi_clamped = false;
 
     // scratch
-    unsigned *d_nan = nullptr;        // [0]: NaN seen in a step, [1]: a pipeline stage wait timed out
+    unsigned *d_nan = nullptr;        // [0]: NaN seen in a step, [1]: a wait timed out, [2], [3]: a levels run's barrier
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
     gbfk_host::StagedCopy staged;     // copies of pageable host memory
@@ -680,6 +680,9 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     if (check_nan) CK(cudaMemsetAsync(ctx->d_nan, 0, sizeof(unsigned), ctx->stream));
     const BlockLists lists = {ctx->d_lists, ctx->n_heavy, ctx->d_lists + ctx->n_heavy, ctx->n_empty};
     bool ran_run = false, skip = false;
+    // AUTO: a multi-level grid whose blocks fit takes its steps in one launch
+    const bool levels = ctx->step_pref == GBFK_STEP_AUTO && !ctx->uniform && ctx->have_csr &&
+                        levels_run_fits<Real>(ctx->nblocks, ctx->sms);
     const bool fits = (want_run || want_skip) && resident_fits<Real>(ctx), resident = want_run && fits;
     if (resident) {
         rc = build_resident<Real>(ctx);
@@ -734,6 +737,17 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
             ctx->launches++;
             ctx->cur ^= 1;
             s++;
+            continue;
+        }
+        if (levels && left >= 2) {
+            const int k = left < kMaxRunSteps ? left : kMaxRunSteps;
+            CK(launch_levels_run<Real>(v, (const Real *)ctx->d_H, ctx->d_meta, ctx->d_ih2, ctx->d_row_ptr, ctx->d_src,
+                                       (const Real *)ctx->d_w, (Real *)ctx->phi[ctx->cur], out, k, (Real)rho, dt,
+                                       ctx->d_nan, ctx->d_nan + 1, ctx->d_nan + 2, ctx->sms, ctx->stream));
+            ctx->launches++;
+            ctx->cur ^= (k & 1);
+            s += k;
+            ran_run = true;
             continue;
         }
         if (ctx->n_step_rows > 0) {
@@ -915,7 +929,7 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
     const size_t bytes = (size_t)cfg->max_blocks * kBS3 * ctx->rsize;
     if (cudaMalloc(&ctx->phi[0], bytes) != cudaSuccess || cudaMalloc(&ctx->phi[1], bytes) != cudaSuccess ||
         cudaMalloc(&ctx->pw, bytes) != cudaSuccess || cudaMalloc(&ctx->pg, bytes) != cudaSuccess ||
-        cudaMalloc(&ctx->d_nan, 2 * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&ctx->d_nan, 4 * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&ctx->d_meta, (size_t)cfg->max_blocks * kBS3 * sizeof(unsigned short)) != cudaSuccess) {
         cudaGetLastError();
         return bail(GBFK_E_OOM);
@@ -924,7 +938,7 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
     cudaMemset(ctx->phi[1], 0, bytes);
     cudaMemset(ctx->pw, 0, bytes);
     cudaMemset(ctx->pg, 0, bytes);
-    cudaMemset(ctx->d_nan, 0, 2 * sizeof(unsigned));
+    cudaMemset(ctx->d_nan, 0, 4 * sizeof(unsigned));
     if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
         return bail(GBFK_E_CUDA);
     if (ensure_table(ctx) != GBFK_OK) return bail(GBFK_E_CUDA);

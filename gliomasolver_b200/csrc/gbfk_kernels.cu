@@ -2,6 +2,7 @@
 // details, split/collapse and the dense <-> block-pool permutation.
 #include "gbfk_exact.cuh"
 #include "gbfk_kernels.cuh"
+#include "gbfk_resident.cuh"
 
 #include <type_traits>
 
@@ -288,6 +289,38 @@ __device__ __forceinline__ int face_neighbour(const PoolView<Real> &v, int blk, 
 #define GBFK_STEP_MIN_BLOCKS_F64 5
 #endif
 
+// The no-flux test of neighbour k (value phn) of cell (x, y, z), by the cell's
+// meta word and the block's type.
+template <typename Real>
+__device__ __forceinline__ bool neighbour_low(const PoolView<Real> &v, int blk, int64_t base, unsigned char bt,
+                                              unsigned mw, int k, Real phn, int x, int y, int z)
+{
+    const Real eps = (Real)0.1;
+    bool low, slow;
+    if (bt == kBlockTissue) {
+        low = false;
+        slow = !(phn >= (Real)0);
+    } else if (bt == kBlockEmpty) {
+        low = phn < eps;
+        slow = false;
+    } else if ((mw >> (2 + k)) & 1u) {
+        low = phn < eps;
+        slow = false;
+    } else {
+        low = false;
+        slow = ((mw >> (8 + k)) & 1u) || !(phn >= (Real)0);
+    }
+    if (slow) {
+        const int nx = x + (k == 0 ? -1 : k == 1 ? 1 : 0);
+        const int ny = y + (k == 2 ? -1 : k == 3 ? 1 : 0);
+        const int nz = z + (k == 4 ? -1 : k == 5 ? 1 : 0);
+        Real pw, pg;
+        lab_pwpg(v, blk, base, nx, ny, nz, pw, pg);
+        low = domain_chf(phn, pw, pg) < eps;
+    }
+    return low;
+}
+
 // The step for one block `blk` (all 128 threads of the CTA call it together;
 // it synchronises the CTA).  v.pw/v.pg/v.btype and meta describe the anatomy,
 // H the face coefficients of the coefficient pair, phi_in/phi_out the field.
@@ -385,7 +418,6 @@ __device__ __forceinline__ void step_block(const PoolView<Real> &v, int blk, Rea
     __syncthreads();
 
     const double ih2 = ih2blk[blk];
-    const Real eps = (Real)0.1;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const Real phi = p.v[i];
@@ -401,31 +433,7 @@ __device__ __forceinline__ void step_block(const PoolView<Real> &v, int blk, Rea
             phn[5] = ph[l + kPlane];
             bool low[6];
 #pragma unroll
-            for (int k = 0; k < 6; k++) {
-                bool slow;
-                if (bt == kBlockTissue) {
-                    low[k] = false;
-                    slow = !(phn[k] >= (Real)0);
-                } else if (bt == kBlockEmpty) {
-                    low[k] = phn[k] < eps;
-                    slow = false;
-                } else if ((mw[i] >> (2 + k)) & 1u) {
-                    low[k] = phn[k] < eps;
-                    slow = false;
-                } else {
-                    low[k] = false;
-                    slow = ((mw[i] >> (8 + k)) & 1u) || !(phn[k] >= (Real)0);
-                }
-                if (slow) {
-                    const int x = x4 + i;
-                    const int nx = x + (k == 0 ? -1 : k == 1 ? 1 : 0);
-                    const int ny = y + (k == 2 ? -1 : k == 3 ? 1 : 0);
-                    const int nz = z + (k == 4 ? -1 : k == 5 ? 1 : 0);
-                    Real pw, pg;
-                    lab_pwpg(v, blk, base, nx, ny, nz, pw, pg);
-                    low[k] = domain_chf(phn[k], pw, pg) < eps;
-                }
-            }
+            for (int k = 0; k < 6; k++) low[k] = neighbour_low(v, blk, base, bt, mw[i], k, phn[k], x4 + i, y, z);
             dphidt = cell_rhs_flags<Real>(hx[i], hx[i + 1], hym.v[i], hyp.v[i], hzm.v[i], hzp.v[i], low, phn, phi,
                                           rho, ih2);
         }
@@ -509,6 +517,234 @@ cudaError_t launch_rd_step(const PoolView<Real> &v, const Real *H, const unsigne
     return launch_pdl(rd_step_kernel<Real, false>, v.nblocks, 128, s, v, H, meta, ih2, phi_in, phi_out, dphidt_out,
                       rho, dt, dt_finite, nan_flag);
 }
+
+// ---------------------------------------------------------------------------
+// A run of steps of a multi-level grid in one cooperative launch: one block
+// per CTA, its cells, meta words and face coefficients kept on the SM, the
+// states published to the two phi buffers, and a grid barrier between steps.
+// Halo cells of the same level are read from their block's state, the others
+// are formed from their ghost row, entries in list order as fill_ghosts_kernel
+// does it, so every value is the same as with a launch per step.
+//
+// What bounds a step is its chain (barrier, gather, exchange, update), not
+// issue or bandwidth: a small grid has one or two blocks per SM.  A launch
+// pair per step (ghost fill, step) had two launch gaps, loaded the
+// coefficients anew and gathered through a ghost buffer.  kC cells per thread:
+// as few as leave every block its CTA (levels_shape).  Per step, FP32, before
+// and now: 190 leaves 9.9 -> 3.2 us, 960 leaves 10.9 -> 6.9; 314 leaves take
+// 3.9 and 34 leaves, all chain, 2.5.  With each row's entries in
+// their own loop instead of the first ones of all rows in flight together:
+// 3.6, 5.4 and 8.1 us.
+
+// CTAs an SM holds with `cells` cells per thread: at most 64 registers a
+// thread, 80 for FP64 with four cells (it spills below that).
+template <typename Real>
+constexpr int levels_min_ctas(int cells)
+{
+    return sizeof(Real) == 4 || cells < 4 ? 2 * cells : 6;
+}
+
+struct LevelsSync {
+    unsigned arrived, left;
+};
+
+template <typename Real, int kC>
+__global__ void __launch_bounds__(512 / kC, levels_min_ctas<Real>(kC))
+rd_levels_run_kernel(PoolView<Real> v, const Real *__restrict__ H, const unsigned short *__restrict__ meta,
+                     const double *__restrict__ ih2blk, const int64_t *__restrict__ row_ptr,
+                     const int *__restrict__ src, const Real *__restrict__ w, Real *state0, Real *state1, int nsteps,
+                     Real rho, double dt, int dt_finite, unsigned *nan_flag, unsigned *err_flag, LevelsSync *sync)
+{
+    constexpr int kT = 512 / kC, kHalo = (384 + kT - 1) / kT, kPre = kC == 1 ? 8 : 4;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Real *ph = reinterpret_cast<Real *>(smem_raw), *sH = ph + kStepLab;
+    const int t = threadIdx.x, blk = blockIdx.x;
+    const int64_t base = slot_of(v, blk) * kBS3;
+    const int c0 = t * kC, x0 = c0 & 7, y = (c0 >> 3) & 7, z = c0 >> 6;
+    const int l0 = lab_p(x0, y, z);
+    for (int q = t; q < kFacesPerBlock; q += kT) sH[q] = H[(int64_t)blk * kFacesPerBlock + q];
+    const unsigned char bt = v.btype[blk];
+    unsigned mw[kC];
+    Real p[kC];
+#pragma unroll
+    for (int i = 0; i < kC; i++) {
+        mw[i] = meta[base + c0 + i];
+        p[i] = state0[base + c0 + i];
+    }
+    // halo cell q of face q / 64: a neighbour's cell, or a ghost row's entries
+    int64_t from[kHalo];
+    int terms[kHalo], hlab[kHalo];
+    bool direct[kHalo];
+#pragma unroll
+    for (int i = 0; i < kHalo; i++) {
+        const int q = t + kT * i;
+        terms[i] = hlab[i] = 0;
+        from[i] = 0;
+        direct[i] = false;
+        if (q >= 384) continue;
+        int lx, ly, lz, sc;
+        face_cell(q >> 6, q & 63, lx, ly, lz, sc);
+        hlab[i] = lab_p(lx, ly, lz);
+        const int nb = v.nbr[blk * 6 + (q >> 6)];
+        direct[i] = nb >= 0;
+        if (direct[i]) {
+            from[i] = (int64_t)nb * kBS3 + sc;
+            terms[i] = 1;
+        } else {
+            const int64_t r = (int64_t)blk * kLabGhosts + c_ghost_id[lab_index(lx, ly, lz)];
+            from[i] = row_ptr[r];
+            terms[i] = (int)(row_ptr[r + 1] - from[i]);
+        }
+    }
+    const double ih2 = ih2blk[blk];
+    bool bad = false;
+    for (int s = 0; s < nsteps; s++) {
+        const Real *in = (s & 1) ? state1 : state0;
+        Real *out = (s & 1) ? state0 : state1;
+        bool dom[kC], any = false;
+#pragma unroll
+        for (int i = 0; i < kC; i++) {
+            const unsigned cls = mw[i] & 3u;
+            if (cls == kTissue && p[i] >= (Real)0) dom[i] = true;
+            else if (cls == kEmpty) dom[i] = p[i] > (Real)0;
+            else dom[i] = in_domain(v.pw[base + c0 + i], v.pg[base + c0 + i], p[i]);
+            any |= dom[i];
+        }
+        const bool work = __syncthreads_or(any);  // and the lab's readers of the last step are done
+        if (work) {
+            // published by other CTAs in this launch: past the L1; the first
+            // entries of all rows are in flight together
+            Real g[kHalo][kPre], gw[kHalo][kPre];
+#pragma unroll
+            for (int i = 0; i < kHalo; i++)
+#pragma unroll
+                for (int k = 0; k < kPre; k++) {
+                    g[i][k] = gw[i][k] = (Real)0;
+                    if (k < terms[i]) {
+                        const int64_t c = direct[i] ? from[i] : (int64_t)__ldg(src + from[i] + k);
+                        g[i][k] = __ldcg(in + c);
+                        if (!direct[i]) gw[i][k] = __ldg(w + from[i] + k);
+                    }
+                }
+#pragma unroll
+            for (int i = 0; i < kHalo; i++) {
+                if (t + kT * i >= 384) continue;
+                Real sum = g[i][0];
+                if (!direct[i]) {
+                    sum = (Real)0;
+#pragma unroll
+                    for (int k = 0; k < kPre; k++)
+                        if (k < terms[i]) sum = radd(sum, rmul(g[i][k], gw[i][k]));
+                    for (int k = kPre; k < terms[i]; k++)
+                        sum = radd(sum, rmul(__ldcg(in + __ldg(src + from[i] + k)), __ldg(w + from[i] + k)));
+                }
+                ph[hlab[i]] = sum;
+            }
+#pragma unroll
+            for (int i = 0; i < kC; i++) ph[l0 + i] = p[i];
+            __syncthreads();
+        }
+        Real next[kC];
+#pragma unroll
+        for (int i = 0; i < kC; i++) {
+            Real dphidt = (Real)0.;
+            if (dom[i]) {
+                const int l = l0 + i, x = x0 + i;
+                const Real phn[6] = {ph[l - 1], ph[l + 1], ph[l - kPitch], ph[l + kPitch], ph[l - kPlane],
+                                     ph[l + kPlane]};
+                bool low[6];
+#pragma unroll
+                for (int k = 0; k < 6; k++) low[k] = neighbour_low(v, blk, base, bt, mw[i], k, phn[k], x, y, z);
+                const int rx = (z * 8 + y) * 9 + x, ry = 576 + (z * 9 + y) * 8 + x, rz = 1152 + (z * 8 + y) * 8 + x;
+                dphidt = cell_rhs_flags<Real>(sH[rx], sH[rx + 1], sH[ry], sH[ry + 8], sH[rz], sH[rz + 64], low, phn,
+                                              p[i], rho, ih2);
+            }
+            next[i] = (!dom[i] && dt_finite) ? clamp01(p[i]) : cell_update(p[i], dphidt, dt);
+            bad |= (next[i] != next[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kC; i++) {
+            p[i] = next[i];
+            __stcg(out + base + c0 + i, p[i]);
+        }
+        if (s + 1 == nsteps) break;
+        // every block's state s + 1 is there, and state s has been read
+        __syncthreads();
+        bool lost = false;
+        if (t == 0) {
+            const unsigned target = (unsigned)(s + 1) * gridDim.x;
+            unsigned seen;
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync->arrived) : "memory");
+            unsigned long long since = 0;
+            for (unsigned n = 0;; n++) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&sync->arrived) : "memory");
+                if (seen >= target) break;
+                if ((n & 1023u) == 1023u) {
+                    const unsigned long long now = now_ns();
+                    if (!since) since = now;
+                    else if (now - since > kPollNs) {
+                        lost = true;
+                        break;
+                    }
+                }
+            }
+        }
+        if (__syncthreads_or(lost)) {
+            if (t == 0) atomicOr(err_flag, kErrPoll);
+            break;
+        }
+    }
+    if (bad) atomicOr(nan_flag, 1u);
+    // the last CTA to leave readies the counters for the next launch
+    if (t == 0 && atomicAdd(&sync->left, 1u) == gridDim.x - 1) {
+        sync->arrived = 0;
+        sync->left = 0;
+    }
+}
+
+// Cells per thread of a run over nblocks blocks, 0 if they do not fit (a
+// launch pair per step then).
+template <typename Real>
+int levels_shape(int nblocks, int sms)
+{
+    for (int c = 1; c <= 4; c *= 2)
+        if (nblocks <= sms * levels_min_ctas<Real>(c)) return c;
+    return 0;
+}
+
+template <typename Real>
+bool levels_run_fits(int nblocks, int sms) { return levels_shape<Real>(nblocks, sms) > 0; }
+
+template <typename Real>
+cudaError_t launch_levels_run(const PoolView<Real> &v, const Real *H, const unsigned short *meta, const double *ih2,
+                              const int64_t *row_ptr, const int *src, const Real *w, Real *state0, Real *state1,
+                              int nsteps, Real rho, double dt, unsigned *nan_flag, unsigned *err_flag, void *sync,
+                              int sms, cudaStream_t s)
+{
+    const int c = levels_shape<Real>(v.nblocks, sms), fin = isfinite(dt) ? 1 : 0;
+    const size_t smem = (kStepLab + kFacesPerBlock) * sizeof(Real);
+    LevelsSync *y = (LevelsSync *)sync;
+    if (c == 1)
+        return launch_coop<rd_levels_run_kernel<Real, 1>>(v.nblocks, 512, smem, s, v, H, meta, ih2, row_ptr, src, w,
+                                                          state0, state1, nsteps, rho, dt, fin, nan_flag, err_flag, y);
+    if (c == 2)
+        return launch_coop<rd_levels_run_kernel<Real, 2>>(v.nblocks, 256, smem, s, v, H, meta, ih2, row_ptr, src, w,
+                                                          state0, state1, nsteps, rho, dt, fin, nan_flag, err_flag, y);
+    if (c == 4)
+        return launch_coop<rd_levels_run_kernel<Real, 4>>(v.nblocks, 128, smem, s, v, H, meta, ih2, row_ptr, src, w,
+                                                          state0, state1, nsteps, rho, dt, fin, nan_flag, err_flag, y);
+    return cudaErrorInvalidConfiguration;
+}
+template bool levels_run_fits<float>(int, int);
+template bool levels_run_fits<double>(int, int);
+template cudaError_t launch_levels_run<float>(const PoolView<float> &, const float *, const unsigned short *,
+                                              const double *, const int64_t *, const int *, const float *, float *,
+                                              float *, int, float, double, unsigned *, unsigned *, void *, int,
+                                              cudaStream_t);
+template cudaError_t launch_levels_run<double>(const PoolView<double> &, const double *, const unsigned short *,
+                                               const double *, const int64_t *, const int *, const double *, double *,
+                                               double *, int, double, double, unsigned *, unsigned *, void *, int,
+                                               cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Discrete adjoint of the fused step (uniform grids).  The forward step is

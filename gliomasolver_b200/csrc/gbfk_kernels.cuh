@@ -223,6 +223,17 @@ cudaError_t launch_rd_batch_step_tma(const BatchLists &bl, int nactive, int tota
 int tma_batch_shapes(int *codes, int max_codes);
 int tma_shape_effective(int code, int real_bytes);
 
+// nsteps steps of a grid of any topology in one launch, state0 -> state1 ->
+// state0 ..., ghost rows as launch_fill_ghosts reads them.  `sync`: two zeroed
+// words of the context's, left zeroed.
+template <typename Real>
+bool levels_run_fits(int nblocks, int sms);
+template <typename Real>
+cudaError_t launch_levels_run(const PoolView<Real> &v, const Real *H, const unsigned short *meta, const double *ih2,
+                              const int64_t *row_ptr, const int *src, const Real *w, Real *state0, Real *state1,
+                              int nsteps, Real rho, double dt, unsigned *nan_flag, unsigned *err_flag, void *sync,
+                              int sms, cudaStream_t s);
+
 template <typename Real>
 cudaError_t launch_fill_ghosts(const int *rows, int64_t nrows, const int64_t *row_ptr, const int *src,
                                const Real *w, const Real *field, Real *ghosts, cudaStream_t s);

@@ -146,7 +146,11 @@ int gbfk_rd_step(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
  * power-of-two grids (in calls of several steps without the blocks that hold
  * no tissue, whose cells only react and take all steps in a launch of their
  * own) and the one-CTA-per-block kernel elsewhere.  The first step after phi
- * was uploaded always runs by itself.  GBFK_STEP_RUN runs the pipeline over
+ * was uploaded always runs by itself there.  On a grid from
+ * gbfk_set_topology with up to about 1180 blocks in FP32, 890 in FP64, a call
+ * of several steps is one cooperative launch with a block per CTA (also
+ * reported as GBFK_STEP_RUN); larger ones launch a ghost fill and the
+ * one-CTA-per-block kernel per step.  GBFK_STEP_RUN runs the pipeline over
  * all steps of a gbfk_rd_step call in one cooperative launch: each
  * CTA keeps its blocks and, between steps, waits only for the CTAs that
  * own their face neighbours (within a few percent of one launch per step on

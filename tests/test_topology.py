@@ -151,3 +151,52 @@ def test_cfl_step_on_the_device(gbfk_lib, prec):
         mx = max(R(s.Dw), R(s.Dg))
         assert c["h_min"] == float(h)
         assert c["dt"] == float(R(0.99 * np.float64(h) * np.float64(h) / (6.0 * np.float64(mx))))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("bpd", [2, 6, 7, 9, 11])
+def test_run_of_ghost_list_steps_equals_launches(gbfk_lib, prec, bpd):
+    """A ghost-list grid's steps in one launch (one, two and four cells per thread; the last size does not fit) against a
+    launch pair per step: permuted slots, ghost rows of 0 to 9 arbitrary entries, an unclamped state with NaN, odd and
+    even step counts, twice on one pool."""
+    from gliomasolver_b200 import BlockPool
+
+    R, n, nb = np.float64 if prec == "f64" else np.float32, 8 * bpd, bpd ** 3
+    r = np.random.default_rng(bpd)
+    slots = r.permutation(nb + 3)[:nb]
+    blocks, csr = uniform_topology(bpd, slots)
+    rows = np.flatnonzero(r.random(nb * LAB_GHOSTS) < 0.1)
+    count = np.ones(nb * LAB_GHOSTS, dtype=np.int64)
+    count[rows] = r.integers(0, 10, rows.size)
+    odd = np.repeat(np.isin(np.arange(count.size), rows), count)
+    src = np.repeat(csr["src"], count)
+    src[odd] = slots[r.integers(0, nb, odd.sum())] * 512 + r.integers(0, 512, odd.sum())
+    w = [np.where(odd, r.uniform(0.1, 0.7, src.size), 1.0) for _ in range(3)]
+    csr = {"row_ptr": np.concatenate([[0], np.cumsum(count)]), "src": src, "w0": w[0], "w1": w[1], "w2": w[2]}
+    pw, pg, c0, fields = _pool_inputs(n, 3, R, slots)
+    php = fields[2] + r.uniform(-0.05, 0.1, fields[2].size).astype(R)
+    php[slots[nb // 2] * 512 + 77] = np.nan
+    s = make_schedule(0.3, 0.1, 150.0, 25.6, bpd, prec)
+    out = {}
+    for kind in ("block", "auto"):
+        with BlockPool(nb + 3, prec) as pool:
+            pool.set_topology(blocks, csr)
+            for name, a in (("p_w", fields[0]), ("p_g", fields[1]), ("phi", php)):
+                pool.upload(name, np.concatenate([a, np.zeros((nb + 3) * 512 - a.size, R)]))
+            pool.step_kernel = kind
+            got = []
+            for steps in (1, 2, 5, 12):
+                pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, steps, check_nan=False)
+                got.append(pool.download("phi", (nb + 3) * 512))
+            got.append(pool.fwt_details())
+            with pytest.raises(Exception):
+                pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 2, check_nan=True)
+            used = pool.step_kernel
+        out[kind] = got
+    assert used == ("run" if nb <= 148 * 6 else "block")
+    order = (np.asarray(slots)[:, None] * 512 + np.arange(512)).ravel()
+    for a, b in zip(out["auto"][:-1], out["block"][:-1]):
+        assert np.array_equal(a[order], b[order], equal_nan=True)
+    assert np.array_equal(out["auto"][-1], out["block"][-1], equal_nan=True)
+    assert not np.array_equal(out["auto"][0][order], out["auto"][3][order], equal_nan=True)
