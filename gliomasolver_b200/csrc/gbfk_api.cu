@@ -116,6 +116,10 @@ struct gbfk_ctx {
     void *d_res_ex = nullptr;
     unsigned *d_res_index = nullptr;
     bool res_ready = false;
+    // step by step over the heavy blocks (launch_stream_step)
+    void *d_stream_image = nullptr, *d_stream_faces[2] = {};
+    int *d_stream_from = nullptr;
+    bool stream_ready = false;
     int sms = 0;
     // adjoint runs with resident blocks: exchange buffers, gradient sums of
     // threads and CTAs, face count (one buffer, zeroed per item list); the
@@ -233,7 +237,7 @@ void free_topology(gbfk_ctx *c)
     c->faces_valid = false;
     c->lists_valid = false;
     c->run_layout_valid = false;
-    c->res_ready = c->adj_run_ready = false;
+    c->res_ready = c->adj_run_ready = c->stream_ready = false;
     c->phi_clamped = false;
 }
 
@@ -245,7 +249,8 @@ void release_topology(gbfk_ctx *c)
                      &c->d_w, (void **)&c->d_step_rows, (void **)&c->d_all_rows, &c->d_gpw, &c->d_gpg,
                      &c->d_gphi, (void **)&c->d_fwt, &c->d_H, (void **)&c->d_ih2, (void **)&c->d_btype, &c->d_origin,
                      (void **)&c->d_lists, (void **)&c->d_run_nbr, (void **)&c->d_run_flags,
-                     (void **)&c->d_res_nbr, &c->d_res_ex, (void **)&c->d_res_index, &c->d_adj_run, &c->d_adj_table};
+                     (void **)&c->d_res_nbr, &c->d_res_ex, (void **)&c->d_res_index, &c->d_adj_run, &c->d_adj_table,
+                     &c->d_stream_image, &c->d_stream_faces[0], &c->d_stream_faces[1], (void **)&c->d_stream_from};
     for (void **p : ptrs) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -542,7 +547,7 @@ int build_step_lists(gbfk_ctx *ctx)
     ctx->lists_gen++;
     ctx->h_lists.swap(lists);
     ctx->run_layout_valid = false;
-    ctx->res_ready = ctx->adj_run_ready = false;
+    ctx->res_ready = ctx->adj_run_ready = ctx->stream_ready = false;
     return GBFK_OK;
 }
 
@@ -601,6 +606,54 @@ ResidentArgs<Real> resident_args(gbfk_ctx *ctx, double rho, double dt)
     return a;
 }
 
+// The tables of steps over the heavy blocks alone; false without room for them
+// (the caller has another way).
+template <typename Real>
+bool build_stream(gbfk_ctx *ctx)
+{
+    if (ctx->stream_ready) return true;
+    const size_t n = (size_t)ctx->n_heavy, faces = (n + 1) * stream_face_values * sizeof(Real);
+    std::vector<int> from;
+    stream_sources(ctx->bpd, ctx->h_lists.data(), (int)n, from);
+    if (topo_alloc(ctx, &ctx->d_stream_image, n * stream_image_bytes<Real>()) ||
+        topo_alloc(ctx, &ctx->d_stream_faces[0], faces) || topo_alloc(ctx, &ctx->d_stream_faces[1], faces) ||
+        topo_alloc(ctx, &ctx->d_stream_from, from.size() * sizeof(int)) ||
+        cudaMemsetAsync(ctx->d_stream_faces[0], 0, faces, ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(ctx->d_stream_faces[1], 0, faces, ctx->stream) != cudaSuccess ||
+        cudaMemcpyAsync(ctx->d_stream_from, from.data(), from.size() * sizeof(int), cudaMemcpyHostToDevice,
+                        ctx->stream) != cudaSuccess ||
+        launch_stream_pack<Real>(ctx->d_lists, (int)n, (const Real *)ctx->d_H, ctx->d_meta, ctx->d_stream_image,
+                                 ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    ctx->launches++;
+    ctx->stream_ready = true;
+    return true;
+}
+
+template <typename Real>
+StreamArgs<Real> stream_args(gbfk_ctx *ctx, double rho, double dt)
+{
+    StreamArgs<Real> a = {};
+    a.items = ctx->d_lists;
+    a.from = ctx->d_stream_from;
+    a.n = ctx->n_heavy;
+    a.image = ctx->d_stream_image;
+    a.meta = ctx->d_meta;
+    a.pw = (const Real *)ctx->pw;
+    a.pg = (const Real *)ctx->pg;
+    a.bpd = ctx->bpd;
+    a.rho = (Real)rho;
+    a.dt = dt;
+    const double h = sizeof(Real) == 8 ? ctx->h_h[0] : (double)(float)ctx->h_h[0];  // as upload_ih2
+    a.ih2 = 1. / (h * h);
+    a.nan_flag = ctx->d_nan;
+    a.err_flag = ctx->d_nan + 1;
+    return a;
+}
+
 // The CTA layout of runs of steps over the current step lists.
 template <typename Real>
 int build_run_layout(gbfk_ctx *ctx, const PoolView<Real> &v)
@@ -627,7 +680,7 @@ int build_run_layout(gbfk_ctx *ctx, const PoolView<Real> &v)
 // (64^3 FP32: 14 + 1.2 n against 3.7 n; 128^3: 17 + 2.0 n against 6.3 n),
 // against the per-block kernel (9-28 us per step) from 3; leaving out the
 // empty blocks at 256^3 saves 10 us per step for 23 us.
-constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kSkipSteps = 3;
+constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kStreamSteps = 3;
 
 template <typename Real>
 int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int nsteps, int check_nan)
@@ -644,22 +697,26 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     // launch already overlaps)
     const bool runs = pipelined && ctx->step_pref == GBFK_STEP_RUN;
     // AUTO: the steps after the first one of an unclamped state as one run
-    // with resident blocks, where they fit, or as launches that leave out the
-    // empty blocks, whose steps are made up in one launch (nothing couples
+    // with resident blocks, where they fit, or as launches over the heavy
+    // blocks, with the empty ones' steps made up in one launch (nothing couples
     // them to the others while every coefficient is finite)
     const bool uncoupled = ctx->step_pref == GBFK_STEP_AUTO && ctx->uniform && ctx->identity_slots &&
                            std::isfinite(dt) && std::isfinite((double)(Real)Dw) && std::isfinite((double)(Real)Dg) &&
                            std::isfinite((double)(Real)rho);
     const int clamped_steps = ctx->phi_clamped ? nsteps : nsteps - 1;
     bool want_run = uncoupled && clamped_steps >= (pipelined ? kResidentSteps : kResidentStepsBlock);
-    if (want_run && (!ctx->res_ready || !ctx->lists_valid)) {
-        // the tables of a run cannot be built inside a stream capture
+    bool want_stream = uncoupled && clamped_steps >= kStreamSteps;
+    // the tables of either cannot be built inside a stream capture
+    const bool run_ready = ctx->lists_valid && ctx->res_ready, stream_ready = ctx->lists_valid && ctx->stream_ready;
+    if ((want_run && !run_ready) || (want_stream && !stream_ready)) {
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
         CK(cudaStreamIsCapturing(ctx->stream, &st));
-        if (st != cudaStreamCaptureStatusNone) want_run = false;
+        if (st != cudaStreamCaptureStatusNone) {
+            want_run = want_run && run_ready;
+            want_stream = want_stream && stream_ready;
+        }
     }
-    const bool want_skip = uncoupled && pipelined && clamped_steps >= kSkipSteps;
-    if (want_run && !pipelined) {
+    if ((want_run || want_stream) && !pipelined) {
         rc = build_step_lists(ctx);
         if (rc) return rc;
     }
@@ -679,15 +736,17 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     }
     if (check_nan) CK(cudaMemsetAsync(ctx->d_nan, 0, sizeof(unsigned), ctx->stream));
     const BlockLists lists = {ctx->d_lists, ctx->n_heavy, ctx->d_lists + ctx->n_heavy, ctx->n_empty};
-    bool ran_run = false, skip = false;
+    bool ran_run = false, skip = false, streamed = false;
     // AUTO: a multi-level grid whose blocks fit takes its steps in one launch
     const bool levels = ctx->step_pref == GBFK_STEP_AUTO && !ctx->uniform && ctx->have_csr &&
                         levels_run_fits<Real>(ctx->nblocks, ctx->sms);
-    const bool fits = (want_run || want_skip) && resident_fits<Real>(ctx), resident = want_run && fits;
+    const bool fits = (want_run || want_stream) && resident_fits<Real>(ctx), resident = want_run && fits;
     if (resident) {
         rc = build_resident<Real>(ctx);
         if (rc) return rc;
     }
+    // without room for the images, the steps run as they do for short calls
+    const bool stream = want_stream && !fits && ctx->n_heavy > 0 && build_stream<Real>(ctx);
     for (int s = 0; s < nsteps;) {
         const Real *in = (const Real *)ctx->phi[ctx->cur];
         Real *out = (Real *)ctx->phi[ctx->cur ^ 1];
@@ -707,13 +766,30 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
             ran_run = true;
             continue;
         }
-        if (want_skip && !fits && clamped && !skip && lists.n_heavy > 0) {
+        if (stream && clamped && !skip) {
             // both buffers get the empty blocks' last state: a heavy block's
             // halo copies may read either, multiplied by coefficients of 0
             CK(launch_empty_run<Real>(lists.empty, lists.n_empty, in, (Real *)ctx->phi[ctx->cur], out, left,
                                       (Real)rho, dt, ctx->d_nan, ctx->stream));
             ctx->launches++;
             skip = true;
+        }
+        if (stream && clamped) {
+            StreamArgs<Real> a = stream_args<Real>(ctx, rho, dt);
+            a.in = in;
+            a.out = out;
+            a.faces_in = (const Real *)ctx->d_stream_faces[s & 1];
+            a.faces_out = (Real *)ctx->d_stream_faces[(s & 1) ^ 1];
+            if (!streamed) {
+                CK(launch_stream_faces<Real>(a.items, a.n, in, (Real *)ctx->d_stream_faces[s & 1], ctx->stream));
+                ctx->launches++;
+            }
+            CK(launch_stream_step<Real>(a, !streamed, ctx->sms, ctx->stream));
+            ctx->launches++;
+            ctx->cur ^= 1;
+            s++;
+            streamed = true;
+            continue;
         }
         if (runs && clamped && left >= 2) {
             // phi[cur] -> phi[cur ^ 1] -> phi[cur] ..., k steps in one launch
@@ -732,7 +808,7 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
         }
         if (pipelined) {
             CK(launch_rd_step_tma<Real>(v, lists, (const Real *)ctx->d_H, ctx->d_meta, ih2, in, clamped, out,
-                                        (Real)rho, dt, ctx->d_nan, ctx->d_nan + 1, ctx->tma_maps[ctx->cur], skip,
+                                        (Real)rho, dt, ctx->d_nan, ctx->d_nan + 1, ctx->tma_maps[ctx->cur], false,
                                         ctx->stream));
             ctx->launches++;
             ctx->cur ^= 1;
@@ -762,7 +838,7 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
         s++;
     }
     if (nsteps > 0) {
-        ctx->step_used = ran_run ? GBFK_STEP_RUN : pipelined ? GBFK_STEP_PIPELINED : GBFK_STEP_BLOCK;
+        ctx->step_used = ran_run ? GBFK_STEP_RUN : pipelined || streamed ? GBFK_STEP_PIPELINED : GBFK_STEP_BLOCK;
         ctx->phi_clamped = true;
     }
     if (check_nan) {

@@ -168,6 +168,39 @@ struct ResidentArgs {
     unsigned start = 0;  // resident_teams: states the exchange buffer carried before (mod 4)
     unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
 };
+// One step of the n heavy blocks of a uniform grid of any size (gbfk_stream.cu).
+// image: their coefficients in the layout of the kernel's shared memory
+// (stream_image_bytes each, launch_stream_pack); from: eight words per block
+// that say where its copies come from (stream_sources);
+// faces_in: the x and y faces of phi_in's heavy blocks (stream_face_values each,
+// launch_stream_faces), a record of zeros after the last; faces_out: the next
+// state's.  first: nothing of the launch before may overlap.
+template <typename Real>
+struct StreamArgs {
+    const int *items, *from;
+    int n;
+    const void *image;
+    const unsigned short *meta;
+    const Real *pw, *pg;
+    int bpd;
+    const Real *in, *faces_in;
+    Real *out, *faces_out;
+    Real rho;
+    double dt, ih2;
+    unsigned *nan_flag, *err_flag;
+    unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
+};
+constexpr int stream_face_values = 256;
+void stream_sources(int bpd, const int *items, int n, std::vector<int> &from);
+template <typename Real>
+size_t stream_image_bytes();
+template <typename Real>
+cudaError_t launch_stream_pack(const int *items, int n, const Real *H, const unsigned short *meta, void *image,
+                               cudaStream_t s);
+template <typename Real>
+cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, cudaStream_t s);
+template <typename Real>
+cudaError_t launch_stream_step(const StreamArgs<Real> &a, bool first, int sms, cudaStream_t s);
 // appends the table `nbr` of n heavy blocks of a uniform periodic bpd^3 grid
 void resident_neighbours(int bpd, const int *items, int n, std::vector<int> &nbr);
 template <typename Real>

@@ -58,92 +58,6 @@ struct alignas(16) ResidentBlock {
     int e;                   // block * 4 + block type
     unsigned kinds;          // two bits per warp: the row_cells variant its cells need
 };
-// The kC cells of a thread in block b, from the state S with its halos (a
-// clamped state) to out; kKind: the cells of the thread's warp (kPlain, kEdge
-// or kGeneral).
-template <typename Real, int kC, unsigned kKind>
-__device__ __forceinline__ void row_cells(const ResidentArgs<Real> &a, double ih2, unsigned long long neg0,
-                                          const ResidentBlock<Real> &b, const ResidentState<Real> &S, const Place &w,
-                                          Real (&out)[kC])
-{
-    using TL = Tile<Real, kC, 2>;
-    constexpr int R = 8 / kC;  // threads of a row
-    Real p[kC];
-    TL::template load<kRows>(S.phi, w.tp, p);
-    const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
-    constexpr bool kLow = kKind != kPlain;
-    // two cells at a time, so that the single-precision operations of the flux
-    // sums can go in pairs (pair_add, pair_mul: each half rounded by itself),
-    // and only one pair's coefficients are held at once
-#pragma unroll
-    for (int i = 0; i < kC; i += 2) {
-        const Real ph[2] = {p[i], p[i + 1]};
-        const Real xm[2] = {i ? p[i - 1] : xl, p[i]}, xp[2] = {p[i + 1], i + 2 < kC ? p[i + 2] : xr};
-        Real d0[2], d1[2], d2[2], d3[2], d4[2], d5[2];
-        TL::template load2<64>(b.hx, w.t, i / 2, d0);
-        d1[0] = d0[1];
-        d1[1] = i + 2 < kC ? b.hx[TL::template at2<64>(w.t, i / 2 + 1)] : b.hx[w.he];
-        TL::template load2<72>(b.hy, w.ty, i / 2, d2);
-        TL::template load2<72>(b.hy, w.ty + R, i / 2, d3);
-        TL::template load2<72>(b.hz, w.t, i / 2, d4);
-        TL::template load2<72>(b.hz, w.t + 8 * R, i / 2, d5);
-        Real y0[2], y1[2], z0[2], z1[2];
-        TL::template load2<kRows>(S.phi, w.tp - R, i / 2, y0);
-        TL::template load2<kRows>(S.phi, w.tp + R, i / 2, y1);
-        TL::template load2<kRows>(S.phi, w.tp - 10 * R, i / 2, z0);
-        TL::template load2<kRows>(S.phi, w.tp + 10 * R, i / 2, z1);
-        bool dom[2] = {true, true};
-        if (kLow) {
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
-                const Real df[6] = {d0[j], d1[j], d2[j], d3[j], d4[j], d5[j]};
-                bool low[6];
-                dom[j] = no_flux_tests<Real, kKind>(a.meta, a.pw, a.pg, a.bpd, b.e >> 2, w.t * kC + i + j, ph[j], phn, df,
-                                                    low);
-                // _applyNoFluxBC: neighbour k below 0.1 doubles the opposite coefficient
-                if (low[0]) d1[j] = rmul(d1[j], (Real)2.);
-                if (low[1]) d0[j] = rmul(d0[j], (Real)2.);
-                if (low[2]) d3[j] = rmul(d3[j], (Real)2.);
-                if (low[3]) d2[j] = rmul(d2[j], (Real)2.);
-                if (low[4]) d5[j] = rmul(d5[j], (Real)2.);
-                if (low[5]) d4[j] = rmul(d4[j], (Real)2.);
-            }
-        }
-        // cell_rhs: the same operations in the same order for both cells
-        Real sin_[2] = {rmul(d0[0], xm[0]), rmul(d0[1], xm[1])}, u[2] = {rmul(d1[0], xp[0]), rmul(d1[1], xp[1])};
-        pair_add(sin_, u);
-        pair_mul(u, d2, y0, neg0);
-        pair_add(sin_, u);
-        pair_mul(u, d3, y1, neg0);
-        pair_add(sin_, u);
-        pair_mul(u, d4, z0, neg0);
-        pair_add(sin_, u);
-        pair_mul(u, d5, z1, neg0);
-        pair_add(sin_, u);
-        Real sdf[2] = {radd(d0[0], d1[0]), radd(d0[1], d1[1])};
-        pair_add(sdf, d2);
-        pair_add(sdf, d3);
-        pair_add(sdf, d4);
-        pair_add(sdf, d5);
-        pair_mul(sdf, sdf, ph, neg0);
-        const Real rr[2] = {a.rho, a.rho};
-        Real rp[2];
-        pair_mul(rp, rr, ph, neg0);
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const double fluxIn = __dmul_rn(ih2, (double)sin_[j]);
-            const double fluxOut = -__dmul_rn((double)sdf[j], ih2);
-            const double phid = (double)ph[j];
-            const double reaction = __dmul_rn((double)rp[j], __dadd_rn(1., -phid));
-            const Real dphidt = to_real<Real>(__dadd_rn(__dadd_rn(fluxOut, fluxIn), reaction));
-            const Real q = clamp_state(to_real<Real>(__dadd_rn(phid, __dmul_rn(a.dt, (double)dphidt))));
-            out[i + j] = dom[j] ? q : ph[j];  // outside the domain a clamped value stays (dt is finite)
-        }
-        if (i + 2 < kC) asm volatile("" ::: "memory");
-    }
-}
-
 // All steps of an empty block's cell: no coupling, so the reaction alone
 // (cell_rhs with every coefficient +0), until nothing is left of it.
 template <typename Real>
@@ -322,9 +236,18 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
             }
             Real o[kC];
             const unsigned kind = (b.kinds >> (2 * (t >> 5))) & 3u;
-            if (kind == kPlain) row_cells<Real, kC, kPlain>(a, ih2, neg0, b, S, w, o);
-            else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, ih2, neg0, b, S, w, o);
-            else row_cells<Real, kC, kGeneral>(a, ih2, neg0, b, S, w, o);
+            Real p[kC];
+            TL::template load<kRows>(S.phi, w.tp, p);
+            const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
+            auto rows = [&](int i, Real (&y0)[2], Real (&y1)[2], Real (&z0)[2], Real (&z1)[2]) {
+                TL::template load2<kRows>(S.phi, w.tp - R, i, y0);
+                TL::template load2<kRows>(S.phi, w.tp + R, i, y1);
+                TL::template load2<kRows>(S.phi, w.tp - 10 * R, i, z0);
+                TL::template load2<kRows>(S.phi, w.tp + 10 * R, i, z1);
+            };
+            if (kind == kPlain) row_cells<Real, kC, kPlain>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
+            else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
+            else row_cells<Real, kC, kGeneral>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
             if (s + 1 < a.nsteps) {
                 publish(c + j * G, o, k + 1);
                 TL::template store<kRows>(b.st[(s + 1) & 1].phi, w.tp, o);

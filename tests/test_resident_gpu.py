@@ -174,3 +174,32 @@ def test_stage_of_resident_runs_equals_steps_by_launches(gbfk_lib, prec, bpd, sa
             for r in recs:  # other step counts and horizons the second time
                 r.nsteps += 3
     assert max(w.max() for w in want) > 0.1
+
+
+@pytest.mark.parametrize("prec,n", [("f32", 176), ("f64", 144), ("f64", 160)])
+def test_steps_over_the_heavy_blocks_equal_the_block_kernel(gbfk_lib, prec, n):
+    """Grids whose heavy blocks do not fit the SMs: calls too short for their own tables, odd and even step counts, an
+    unclamped first state, tumour in empty blocks, cells of every class, and new coefficients on the same pool."""
+    pw, pg, c0, _ = make_case(n, 3)
+    rng = np.random.default_rng(n)
+    c0 = np.maximum(c0, rng.uniform(0, 1, c0.shape) * (rng.uniform(0, 1, c0.shape) < 0.03))
+    c0[0, 0, :], c0[1, :, 2] = 1.7, -0.3
+    sel = rng.uniform(0, 1, c0.shape) < 0.02
+    pw[sel] *= 0.08
+    pg[sel] *= 0.08
+    R = np.float64 if prec == "f64" else np.float32
+    pw, pg, c0 = (a.astype(R) for a in (pw, pg, c0))
+    out = {}
+    for kind in ("block", "auto"):
+        with _pool(n, prec, (pw, pg, c0)) as pool:
+            pool.step_kernel = kind
+            got = []
+            for Dw, steps in ((0.3, 7), (0.3, 4), (0.3, 2), (0.15, 5)):
+                s = make_schedule(Dw, 0.2, 300.0, 25.6, n // 8, prec)
+                pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, steps, check_nan=True)
+                got.append(pool.download_dense("phi"))
+                if steps > 3:
+                    assert pool.step_kernel == ("block" if kind == "block" else "pipelined")
+        out[kind] = got
+    for a, b in zip(out["auto"], out["block"]):
+        assert np.array_equal(a, b)
