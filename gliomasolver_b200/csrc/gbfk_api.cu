@@ -622,7 +622,7 @@ bool build_stream(gbfk_ctx *ctx)
         cudaMemsetAsync(ctx->d_stream_faces[1], 0, faces, ctx->stream) != cudaSuccess ||
         cudaMemcpyAsync(ctx->d_stream_from, from.data(), from.size() * sizeof(int), cudaMemcpyHostToDevice,
                         ctx->stream) != cudaSuccess ||
-        launch_stream_pack<Real>(ctx->d_lists, (int)n, (const Real *)ctx->d_H, ctx->d_meta, ctx->d_stream_image,
+        launch_stream_pack<Real>(ctx->d_lists, (int)n, ctx->bpd, (const Real *)ctx->d_H, ctx->d_meta, ctx->d_stream_image,
                                  ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         cudaGetLastError();
@@ -641,10 +641,8 @@ StreamArgs<Real> stream_args(gbfk_ctx *ctx, double rho, double dt)
     a.from = ctx->d_stream_from;
     a.n = ctx->n_heavy;
     a.image = ctx->d_stream_image;
-    a.meta = ctx->d_meta;
     a.pw = (const Real *)ctx->pw;
     a.pg = (const Real *)ctx->pg;
-    a.bpd = ctx->bpd;
     a.rho = (Real)rho;
     a.dt = dt;
     const double h = sizeof(Real) == 8 ? ctx->h_h[0] : (double)(float)ctx->h_h[0];  // as upload_ih2

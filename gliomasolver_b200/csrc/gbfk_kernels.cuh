@@ -180,9 +180,7 @@ struct StreamArgs {
     const int *items, *from;
     int n;
     const void *image;
-    const unsigned short *meta;
     const Real *pw, *pg;
-    int bpd;
     const Real *in, *faces_in;
     Real *out, *faces_out;
     Real rho;
@@ -195,7 +193,7 @@ void stream_sources(int bpd, const int *items, int n, std::vector<int> &from);
 template <typename Real>
 size_t stream_image_bytes();
 template <typename Real>
-cudaError_t launch_stream_pack(const int *items, int n, const Real *H, const unsigned short *meta, void *image,
+cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta, void *image,
                                cudaStream_t s);
 template <typename Real>
 cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, cudaStream_t s);

@@ -55,6 +55,7 @@ struct alignas(16) ResidentBlock {
     ResidentState<Real> st[2];
     Real hx[kBS3], hx8[64], hy[576], hz[576];
     int nbr[6];              // exchange offset (elements) of the face neighbours, -1: an empty block
+    int at[6];               // their pool blocks
     int e;                   // block * 4 + block type
     unsigned kinds;          // two bits per warp: the row_cells variant its cells need
 };
@@ -172,6 +173,7 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
         if (t < 6) {
             const int nb = a.nbr[item * 6 + t];
             b.nbr[t] = nb < 0 ? -1 : nb * 384;
+            b.at[t] = block_across(a.bpd, e >> 2, t);
         }
         if (fetches && a.nbr[item * 6 + pf] < 0) {  // an empty neighbour: +0 for good
             for (int v = 0; v < kC / TL::V; v++)

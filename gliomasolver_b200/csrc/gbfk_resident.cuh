@@ -228,8 +228,7 @@ struct alignas(16) ResidentState {
 //             not, so that its domain test needs no branch).  -0 for +0 in
 //             the flux sums gives the same sums: (+0) + (-0) = +0 either way;
 //   kGeneral  kOther cells or neighbours, or a coefficient that is negative
-//             by itself: classes from the meta words, p_w and p_g from global
-//             memory.
+//             by itself: the tests as written, p_w and p_g from global memory.
 constexpr unsigned kPlain = 0, kEdge = 1, kGeneral = 2;
 
 __device__ __forceinline__ float set_sign(float v, bool s) { return s ? __uint_as_float(__float_as_uint(v) | 0x80000000u) : v; }
@@ -281,23 +280,13 @@ __device__ __forceinline__ float clamp_state(float p)
 }
 __device__ __forceinline__ double clamp_state(double p) { return clamp01(p); }
 
-// p_w, p_g of cell (x, y, z) of block blk, or of the one cell outside it
-// across a face, on the uniform bpd^3 grid
-template <typename Real>
-__device__ __noinline__ void tissue_at(const Real *pw_all, const Real *pg_all, int bpd, int blk, int x, int y, int z,
-                                       Real &pw, Real &pg)
+// The pool blocks across the faces of block blk of the uniform periodic bpd^3 grid.
+__device__ __forceinline__ int block_across(int bpd, int blk, int f)
 {
-    int bx = blk % bpd, by = (blk / bpd) % bpd, bz = blk / (bpd * bpd);
-    if (x < 0) bx = bx ? bx - 1 : bpd - 1;
-    if (x > 7) bx = bx + 1 < bpd ? bx + 1 : 0;
-    if (y < 0) by = by ? by - 1 : bpd - 1;
-    if (y > 7) by = by + 1 < bpd ? by + 1 : 0;
-    if (z < 0) bz = bz ? bz - 1 : bpd - 1;
-    if (z > 7) bz = bz + 1 < bpd ? bz + 1 : 0;
-    const int64_t g = ((int64_t)bx + (int64_t)bpd * (by + (int64_t)bpd * bz)) * kBS3 + (x & 7) +
-                      kBS * ((y & 7) + kBS * (z & 7));
-    pw = pw_all[g];
-    pg = pg_all[g];
+    int q[3] = {blk % bpd, (blk / bpd) % bpd, blk / (bpd * bpd)};
+    const int v = q[f >> 1] + ((f & 1) ? 1 : -1);
+    q[f >> 1] = v < 0 ? bpd - 1 : v == bpd ? 0 : v;
+    return q[0] + bpd * (q[1] + bpd * q[2]);
 }
 
 // What a thread needs to know of its place in a block, fixed for the run.
@@ -325,37 +314,55 @@ __device__ __forceinline__ Place place_of(int t)
     return w;
 }
 
-// The no-flux tests of a cell of a clamped state (low[k]: neighbour k has chf <
-// 0.1) and whether it is inside the domain.
-template <typename Real, unsigned kKind>
-__device__ __forceinline__ bool no_flux_tests(const unsigned short *meta, const Real *pw_all, const Real *pg_all,
-                                              int bpd, int blk, int cell, Real phi, const Real (&phn)[6],
-                                              const Real (&df)[6], bool (&low)[6])
+// The no-flux tests of the pair of cells i, i + 1 of a thread of a clamped state
+// (low[j][k]: neighbour k has chf < 0.1) and whether they are inside the
+// domain (dom). kGeneral evaluates the tests as they are written, with p_w
+// and p_g of the row and its neighbours from global memory; its loads do not
+// wait for one another. (One load per cell that is kOther, each behind the
+// test that finds it: 26 us per step for a 128^3 FP32 brain with a partial
+// volume rim, of which 3 cells in 1000 are kOther.)
+template <typename Real, int kC, unsigned kKind, typename Args, typename Block>
+__device__ __forceinline__ void no_flux_tests(const Args &a, const Block &b, int t, int i, const Real (&ph)[2],
+                                              const Real (&phn)[6][2], const Real (&df)[6][2], bool (&low)[2][6],
+                                              bool (&dom)[2])
 {
     const Real eps = (Real)0.1;
-    if (kKind != kGeneral) {
+    if constexpr (kKind != kGeneral) {
 #pragma unroll
-        for (int k = 0; k < 6; k++) low[k] = kKind == kEdge && sign_of(df[k]) && phn[k] < eps;
-        return true;
-    }
-    const unsigned mw = meta[(int64_t)blk * kBS3 + cell];
-    const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-    bool dom = true;
-    Real pw, pg;
+        for (int j = 0; j < 2; j++)
 #pragma unroll
-    for (int k = 0; k < 6; k++) low[k] = ((mw >> (2 + k)) & 1u) && phn[k] < eps;
-    if ((mw & 3u) == kOther) {
-        tissue_at(pw_all, pg_all, bpd, blk, x, y, z, pw, pg);
-        dom = in_domain(pw, pg, phi);
-    }
+            for (int k = 0; k < 6; k++) low[j][k] = kKind == kEdge && sign_of(df[k][j]) && phn[k][j] < eps;
+    } else {
+        constexpr int R = 8 / kC;
+        const int x0 = (t % R) * kC, y = (t / R) & 7, z = t / (8 * R), row = z * 8 + y, c = t * kC + i;
+        auto cell = [&](int f, int in) { return (int64_t)(f < 0 ? b.e >> 2 : b.at[f]) * kBS3 + in; };
+        const int64_t at[6] = {i || x0 ? cell(-1, c - 1) : cell(0, row * 8 + 7),
+                               i + 2 < kC || x0 + kC < 8 ? cell(-1, c + 2) : cell(1, row * 8),
+                               y ? cell(-1, c - 8) : cell(2, c + 56),
+                               y < 7 ? cell(-1, c + 8) : cell(3, c - 56),
+                               z ? cell(-1, c - 64) : cell(4, c + 448),
+                               z < 7 ? cell(-1, c + 64) : cell(5, c - 448)};
+        Real w[6][2], g[6][2], ow[2], og[2];
+        ld_cells(a.pw + cell(-1, c), ow);
+        ld_cells(a.pg + cell(-1, c), og);
+        w[0][0] = a.pw[at[0]];
+        g[0][0] = a.pg[at[0]];
+        w[1][1] = a.pw[at[1]];
+        g[1][1] = a.pg[at[1]];
 #pragma unroll
-    for (int k = 0; k < 6; k++)
-        if ((mw >> (8 + k)) & 1u) {
-            tissue_at(pw_all, pg_all, bpd, blk, x + (k == 1) - (k == 0), y + (k == 3) - (k == 2),
-                      z + (k == 5) - (k == 4), pw, pg);
-            low[k] = domain_chf(phn[k], pw, pg) < eps;
+        for (int k = 2; k < 6; k++) {
+            ld_cells(a.pw + at[k], w[k]);
+            ld_cells(a.pg + at[k], g[k]);
         }
-    return dom;
+        w[0][1] = ow[0]; g[0][1] = og[0];
+        w[1][0] = ow[1]; g[1][0] = og[1];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            dom[j] = in_domain(ow[j], og[j], ph[j]);
+#pragma unroll
+            for (int k = 0; k < 6; k++) low[j][k] = domain_chf(phn[k][j], w[k][j], g[k][j]) < eps;
+        }
+    }
 }
 
 // The coefficients of a block into shared memory (members hx, hx8, hy, hz of b,
@@ -410,8 +417,8 @@ __device__ __forceinline__ void load_coefficients(Block &b, const Real *H, const
     if ((t & 31) == 0) atomicOr(&b.kinds, (general ? kGeneral : edge ? kEdge : kPlain) << (2 * (t >> 5)));
 }
 
-// The kC cells p of a thread in block b (hx, hx8, hy, hz and e as in
-// ResidentBlock) of a clamped state to out; xl, xr: the cells before and after
+// The kC cells p of a thread in block b (hx, hx8, hy, hz, e and at as
+// in ResidentBlock) of a clamped state to out; xl, xr: the cells before and after
 // them; rows(i, y0, y1, z0, z1): the neighbours of pair i; kKind: the cells of
 // the thread's warp (kPlain, kEdge or kGeneral).
 template <typename Real, int kC, unsigned kKind, typename Args, typename Block, typename Rows>
@@ -441,13 +448,15 @@ __device__ __forceinline__ void row_cells(const Args &a, double ih2, unsigned lo
         rows(i / 2, y0, y1, z0, z1);
         bool dom[2] = {true, true};
         if (kLow) {
+            const Real phn[6][2] = {{xm[0], xm[1]}, {xp[0], xp[1]}, {y0[0], y0[1]},
+                                    {y1[0], y1[1]}, {z0[0], z0[1]}, {z1[0], z1[1]}};
+            const Real df[6][2] = {{d0[0], d0[1]}, {d1[0], d1[1]}, {d2[0], d2[1]},
+                                   {d3[0], d3[1]}, {d4[0], d4[1]}, {d5[0], d5[1]}};
+            bool lows[2][6];
+            no_flux_tests<Real, kC, kKind>(a, b, w.t, i, ph, phn, df, lows, dom);
 #pragma unroll
             for (int j = 0; j < 2; j++) {
-                const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
-                const Real df[6] = {d0[j], d1[j], d2[j], d3[j], d4[j], d5[j]};
-                bool low[6];
-                dom[j] = no_flux_tests<Real, kKind>(a.meta, a.pw, a.pg, a.bpd, b.e >> 2, w.t * kC + i + j, ph[j], phn, df,
-                                                    low);
+                const bool (&low)[6] = lows[j];
                 // _applyNoFluxBC: neighbour k below 0.1 doubles the opposite coefficient
                 if (low[0]) d1[j] = rmul(d1[j], (Real)2.);
                 if (low[1]) d0[j] = rmul(d0[j], (Real)2.);

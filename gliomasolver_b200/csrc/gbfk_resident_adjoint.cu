@@ -108,7 +108,7 @@ struct alignas(16) AdjBlock {
     unsigned char fl[2][kRows * 8 + 128];
     double self[kBS3];
     Real hx[kBS3], hx8[64], hy[576], hz[576];
-    int nbr[6], nbrblk[6];  // face neighbours: item (-1: an empty block), pool block
+    int nbr[6], at[6];  // face neighbours: item (-1: an empty block), pool block
     int e;
     unsigned kinds;
 };
@@ -150,13 +150,15 @@ __device__ __forceinline__ void adj_forward(const AdjRunArgs<Real> &a, double ih
     bool dom[2] = {true, true};
     unsigned fl[2] = {0, 0};
     if (kKind != kPlain) {
+        const Real phn[6][2] = {{xm[0], xm[1]}, {xp[0], xp[1]}, {y0[0], y0[1]},
+                                {y1[0], y1[1]}, {z0[0], z0[1]}, {z1[0], z1[1]}};
+        const Real df[6][2] = {{d0[0], d0[1]}, {d1[0], d1[1]}, {d2[0], d2[1]},
+                               {d3[0], d3[1]}, {d4[0], d4[1]}, {d5[0], d5[1]}};
+        bool lows[2][6];
+        no_flux_tests<Real, kC, kKind>(a, b, w.t, i, ph, phn, df, lows, dom);
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const Real phn[6] = {xm[j], xp[j], y0[j], y1[j], z0[j], z1[j]};
-            const Real df[6] = {d0[j], d1[j], d2[j], d3[j], d4[j], d5[j]};
-            bool low[6];
-            dom[j] = no_flux_tests<Real, kKind>(a.meta, a.pw, a.pg, a.bpd, b.e >> 2, w.t * kC + i + j, ph[j], phn, df,
-                                                low);
+            const bool (&low)[6] = lows[j];
             // _applyNoFluxBC: neighbour k below 0.1 doubles the opposite coefficient
             if (low[0]) { d1[j] = rmul(d1[j], (Real)2.); fl[j] |= 4u; }
             if (low[1]) { d0[j] = rmul(d0[j], (Real)2.); fl[j] |= 2u; }
@@ -377,7 +379,7 @@ adj_run_kernel(const __grid_constant__ AdjRunArgs<Real> a)
         if (t < 6) {
             const int nb = a.nbr[item * 6 + t];
             b.nbr[t] = nb;
-            b.nbrblk[t] = nb < 0 ? -1 : a.items[nb] >> 2;
+            b.at[t] = block_across(a.bpd, e >> 2, t);
         }
         if (fetches && a.nbr[item * 6 + pf] < 0)  // an empty neighbour: phi = mu = 0
             for (int s = 0; s < 2; s++)
@@ -412,9 +414,8 @@ adj_run_kernel(const __grid_constant__ AdjRunArgs<Real> a)
         const Real *phi = a.states[s];
         ld_cells(phi + (int64_t)(b.e >> 2) * kBS3 + t * kC, pn);
         if (fetches) {
-            const int nb = b.nbrblk[pf];
-            if (nb >= 0) {
-                const Real *q = phi + (int64_t)nb * kBS3 + pc;
+            if (b.nbr[pf] >= 0) {
+                const Real *q = phi + (int64_t)b.at[pf] * kBS3 + pc;
 #pragma unroll
                 for (int i = 0; i < kC; i++) hn[i] = q[i * pcs];
             }

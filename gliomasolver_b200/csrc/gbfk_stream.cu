@@ -15,7 +15,15 @@
 // images of a group's first blocks are on their way before the step before has
 // finished.
 //
-// @FIGURES@
+// What bounds it, per step: about 4 us from one launch's last block to the next
+// one's first (the state cannot be copied before it is complete), then 0.25 us
+// (FP32; FP64 0.46) per block of an SM, three quarters of it instruction issue.
+// Measured: 256^3 FP32, 7184 heavy blocks, 16.4 us (20.2 with one column of
+// cells per thread and tensor boxes as halos, 30 with the empty blocks);
+// 216^3 FP32 11.7, 160^3 FP64 8.7, 192^3 FP64 12.7.  Copies by every thread
+// (16-, 8- and 4-byte asynchronous ones) took 20.2 at 256^3, their issue queue
+// full; six groups 17.1; the sources of the copies through two dependent
+// loads instead of a table 20.2.
 #include "gbfk_async.cuh"
 #include "gbfk_resident.cuh"
 
@@ -28,9 +36,8 @@ constexpr unsigned kErrStream = 1u | 1024u;          // error word: a copy never
 template <typename Real>
 struct alignas(16) StreamImage {
     Real hx[kBS3], hx8[64], hy[576], hz[576];  // as in ResidentBlock
+    int at[6], e;
     unsigned kinds;
-    int e;
-    int pad[2];
 };
 // x-, x+, y-, y+, z-, z+ halos, as the neighbours' faces: [z][y], [z][x], [y][x]
 template <typename Real>
@@ -47,7 +54,7 @@ constexpr int kStreamHead = 256;  // bytes of shared memory for the barriers
 
 template <typename Real>
 __global__ void __launch_bounds__(kThreads)
-stream_pack_kernel(const int *items, const Real *H, const unsigned short *meta, StreamImage<Real> *image)
+stream_pack_kernel(const int *items, int bpd, const Real *H, const unsigned short *meta, StreamImage<Real> *image)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StreamImage<Real> &b = *reinterpret_cast<StreamImage<Real> *>(smem_raw);
@@ -55,6 +62,7 @@ stream_pack_kernel(const int *items, const Real *H, const unsigned short *meta, 
     const int64_t blk = e >> 2;
     load_coefficients<Real, kCells>(b, H + blk * kFacesPerBlock, meta + blk * kBS3, t, [] { __syncthreads(); });
     if (t == 0) b.e = e;
+    if (t < 6) b.at[t] = block_across(bpd, e >> 2, t);
     __syncthreads();
     const int4 *from = reinterpret_cast<const int4 *>(&b);
     int4 *to = reinterpret_cast<int4 *>(image + blockIdx.x);
@@ -223,11 +231,12 @@ template <typename Real>
 size_t stream_image_bytes() { return sizeof(StreamImage<Real>); }
 
 template <typename Real>
-cudaError_t launch_stream_pack(const int *items, int n, const Real *H, const unsigned short *meta, void *image,
+cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta, void *image,
                                cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    stream_pack_kernel<Real><<<n, kThreads, sizeof(StreamImage<Real>), s>>>(items, H, meta, (StreamImage<Real> *)image);
+    stream_pack_kernel<Real><<<n, kThreads, sizeof(StreamImage<Real>), s>>>(items, bpd, H, meta,
+                                                                            (StreamImage<Real> *)image);
     return cudaGetLastError();
 }
 
@@ -263,9 +272,9 @@ cudaError_t launch_stream_step(const StreamArgs<Real> &a, bool first, int sms, c
 
 template size_t stream_image_bytes<float>();
 template size_t stream_image_bytes<double>();
-template cudaError_t launch_stream_pack<float>(const int *, int, const float *, const unsigned short *, void *,
+template cudaError_t launch_stream_pack<float>(const int *, int, int, const float *, const unsigned short *, void *,
                                                cudaStream_t);
-template cudaError_t launch_stream_pack<double>(const int *, int, const double *, const unsigned short *, void *,
+template cudaError_t launch_stream_pack<double>(const int *, int, int, const double *, const unsigned short *, void *,
                                                 cudaStream_t);
 template cudaError_t launch_stream_faces<float>(const int *, int, const float *, float *, cudaStream_t);
 template cudaError_t launch_stream_faces<double>(const int *, int, const double *, double *, cudaStream_t);
