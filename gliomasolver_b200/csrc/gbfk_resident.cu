@@ -126,6 +126,9 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
     using TL = Tile<Real, kC, 2>;
     constexpr int kT = kBS3 / kC;  // threads of a group
     constexpr int R = 8 / kC;      // threads of a row
+    // skip kStill warps: 128^3 FP32 2.51 -> 2.38 us per step, FP64 3.27 -> 3.11,
+    // 64^3 FP64 1.37 -> 1.32; two cells in FP32 lost by it (1.12 -> 1.16)
+    constexpr bool kSkips = kC == 4 || sizeof(Real) == 8;
     const int t = threadIdx.x % kT, group = threadIdx.x / kT;
     const int nlocal = a.n > c ? (a.n - 1 - c) / G + 1 : 0;
     const Place w = place_of<Real, kC>(t);
@@ -179,7 +182,10 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
             for (int v = 0; v < kC / TL::V; v++)
                 for (int i = 0; i < TL::V; i++) b.st[0].phi[pd + v * pstep + i] = b.st[1].phi[pd + v * pstep + i] = (Real)0;
         }
-        load_coefficients<Real, kC>(b, a.H + blk * kFacesPerBlock, a.meta + blk * kBS3, t, group_sync);
+        bool zero = kSkips;
+#pragma unroll
+        for (int i = 0; i < kC; i++) zero = zero && p[i] == (Real)0;
+        load_coefficients<Real, kC>(b, a.H + blk * kFacesPerBlock, a.meta + blk * kBS3, t, zero, group_sync);
     }
     group_sync();
 
@@ -238,18 +244,23 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
             }
             Real o[kC];
             const unsigned kind = (b.kinds >> (2 * (t >> 5))) & 3u;
-            Real p[kC];
-            TL::template load<kRows>(S.phi, w.tp, p);
-            const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
-            auto rows = [&](int i, Real (&y0)[2], Real (&y1)[2], Real (&z0)[2], Real (&z1)[2]) {
-                TL::template load2<kRows>(S.phi, w.tp - R, i, y0);
-                TL::template load2<kRows>(S.phi, w.tp + R, i, y1);
-                TL::template load2<kRows>(S.phi, w.tp - 10 * R, i, z0);
-                TL::template load2<kRows>(S.phi, w.tp + 10 * R, i, z1);
-            };
-            if (kind == kPlain) row_cells<Real, kC, kPlain>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
-            else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
-            else row_cells<Real, kC, kGeneral>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
+            if (kSkips && kind == kStill) {
+#pragma unroll
+                for (int i = 0; i < kC; i++) o[i] = (Real)0;
+            } else {
+                Real p[kC];
+                TL::template load<kRows>(S.phi, w.tp, p);
+                const Real xl = S.phi[w.xl], xr = S.phi[w.xr];
+                auto rows = [&](int i, Real (&y0)[2], Real (&y1)[2], Real (&z0)[2], Real (&z1)[2]) {
+                    TL::template load2<kRows>(S.phi, w.tp - R, i, y0);
+                    TL::template load2<kRows>(S.phi, w.tp + R, i, y1);
+                    TL::template load2<kRows>(S.phi, w.tp - 10 * R, i, z0);
+                    TL::template load2<kRows>(S.phi, w.tp + 10 * R, i, z1);
+                };
+                if (kind == kPlain) row_cells<Real, kC, kPlain>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
+                else if (kind == kEdge) row_cells<Real, kC, kEdge>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
+                else row_cells<Real, kC, kGeneral>(a, ih2, neg0, b, w, p, xl, xr, rows, o);
+            }
             if (s + 1 < a.nsteps) {
                 publish(c + j * G, o, k + 1);
                 TL::template store<kRows>(b.st[(s + 1) & 1].phi, w.tp, o);
@@ -332,16 +343,16 @@ resident_teams_kernel(const ResidentArgs<Real> *runs, const int *off, const int 
 // Cells per thread and groups per CTA by the blocks of a CTA (`per`).  Up to
 // two blocks the step is a chain of latencies, which two cells per thread
 // shorten (64^3 FP32, 2 per CTA: 1.16 us per step against 1.32 with four).
-// Beyond, four cells per thread cost fewer instructions, and a step takes the
-// rounds the groups need for the blocks, each round longer the more groups
-// share the SM: on a B200 in FP32 about 1.23, 1.35, 1.40 and 1.62 us with 4, 5,
-// 6 and 7 groups (15 blocks: 4.9 us with four, 4.05 with five, 4.1 with six,
-// 4.5 with seven; 14 blocks: 3.26 with seven, 3.75 with five; 7 blocks: 1.94
-// with seven, 2.42 with four).  Eight groups leave 64 registers a thread,
-// which spill.  FP64 needs 124 registers for four cells: four groups (128^3:
-// 3.07; 3.68 with seven, 4.78 with two cells per thread).
-constexpr double kRoundUs[4] = {1.23, 1.35, 1.40, 1.62};
-constexpr double kRoundUs64 = 1.5;
+// Beyond, four cells per thread cost fewer instructions. In FP32 a step takes
+// about 0.70 us per round of the groups over the blocks and 0.155 us per block
+// (4 blocks 1.33 us, 6 1.59, 7 1.73, 8 1.94), so the blocks go in as few
+// rounds as eight groups allow (64 registers a thread, none spilled), with no
+// more groups than those rounds need: 8 blocks 1.94 us with eight groups, 2.58
+// with seven, 2.38 with four; 9 blocks 2.58 with five, 2.76 with eight; 12
+// blocks 2.94 with six, 3.11 with eight, 3.49 with four. FP64 needs 124
+// registers for four cells: four groups (128^3: 3.07; 3.68 with seven, 4.78
+// with two cells per thread).
+constexpr double kRoundUs = 0.70, kBlockUs = 0.155, kRoundUs64 = 1.5;
 template <typename Real>
 int groups_for(int per, double &us)
 {
@@ -353,16 +364,9 @@ int groups_for(int per, double &us)
         us = kRoundUs64 * ((per + 3) / 4);
         return 4;
     }
-    int best = 4;
-    us = 1e9;
-    for (int g = 4; g <= 7; g++) {
-        const double u = kRoundUs[g - 4] * ((per + g - 1) / g);
-        if (u < us) {
-            us = u;
-            best = g;
-        }
-    }
-    return best;
+    const int rounds = (per + 7) / 8, g = (per + rounds - 1) / rounds;
+    us = kRoundUs * rounds + kBlockUs * per;
+    return g < 4 ? 4 : g;
 }
 template <typename Real, typename F>
 cudaError_t with_shape(int per, F &&f)
@@ -375,6 +379,7 @@ cudaError_t with_shape(int per, F &&f)
         if (g == 5) return f(integral_constant<int, 4>(), integral_constant<int, 5>());
         if (g == 6) return f(integral_constant<int, 4>(), integral_constant<int, 6>());
         if (g == 7) return f(integral_constant<int, 4>(), integral_constant<int, 7>());
+        if (g == 8) return f(integral_constant<int, 4>(), integral_constant<int, 8>());
     }
     return f(integral_constant<int, 4>(), integral_constant<int, 4>());
 }

@@ -401,7 +401,7 @@ adj_run_kernel(const __grid_constant__ AdjRunArgs<Real> a)
             store_flags(b.fl[0], f);
             publish(item, v, f, tag0 + 1);
         }
-        load_coefficients<Real, kC>(b, a.H + blk * kFacesPerBlock, a.meta + blk * kBS3, t, group_sync);
+        load_coefficients<Real, kC>(b, a.H + blk * kFacesPerBlock, a.meta + blk * kBS3, t, false, group_sync);
     }
     group_sync();
 

@@ -60,7 +60,8 @@ stream_pack_kernel(const int *items, int bpd, const Real *H, const unsigned shor
     StreamImage<Real> &b = *reinterpret_cast<StreamImage<Real> *>(smem_raw);
     const int t = threadIdx.x, e = items[blockIdx.x];
     const int64_t blk = e >> 2;
-    load_coefficients<Real, kCells>(b, H + blk * kFacesPerBlock, meta + blk * kBS3, t, [] { __syncthreads(); });
+    load_coefficients<Real, kCells>(b, H + blk * kFacesPerBlock, meta + blk * kBS3, t, false,
+                                    [] { __syncthreads(); });
     if (t == 0) b.e = e;
     if (t < 6) b.at[t] = block_across(bpd, e >> 2, t);
     __syncthreads();
