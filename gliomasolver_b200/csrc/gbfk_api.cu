@@ -112,12 +112,13 @@ struct gbfk_ctx {
     // runs with resident blocks (gbfk_resident.cu): per heavy block the list
     // positions of its face neighbours, the face exchange buffers, the state
     // count; the number of SMs
-    int *d_res_nbr = nullptr;
-    void *d_res_ex = nullptr;
-    unsigned *d_res_index = nullptr;
+    void *d_res = nullptr;            // one buffer: the exchange words, then
+    int *d_res_nbr = nullptr;         // the neighbour table and
+    unsigned *d_res_index = nullptr;  // the state count
     bool res_ready = false;
     // step by step over the heavy blocks (launch_stream_step)
-    void *d_stream_image = nullptr, *d_stream_faces[2] = {};
+    void *d_stream = nullptr;         // one buffer: the images, the faces of two states, the sources
+    void *d_stream_faces[2] = {};
     int *d_stream_from = nullptr;
     bool stream_ready = false;
     int sms = 0;
@@ -249,8 +250,7 @@ void release_topology(gbfk_ctx *c)
                      &c->d_w, (void **)&c->d_step_rows, (void **)&c->d_all_rows, &c->d_gpw, &c->d_gpg,
                      &c->d_gphi, (void **)&c->d_fwt, &c->d_H, (void **)&c->d_ih2, (void **)&c->d_btype, &c->d_origin,
                      (void **)&c->d_lists, (void **)&c->d_run_nbr, (void **)&c->d_run_flags,
-                     (void **)&c->d_res_nbr, &c->d_res_ex, (void **)&c->d_res_index, &c->d_adj_run, &c->d_adj_table,
-                     &c->d_stream_image, &c->d_stream_faces[0], &c->d_stream_faces[1], (void **)&c->d_stream_from};
+                     &c->d_res, &c->d_adj_run, &c->d_adj_table, &c->d_stream};
     for (void **p : ptrs) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -569,11 +569,11 @@ int build_resident(gbfk_ctx *ctx)
     std::vector<int> nbr;
     resident_neighbours(ctx->bpd, ctx->h_lists.data(), n, nbr);
     const size_t ex = (size_t)2 * n * 384 * sizeof(Real);
-    int rc = topo_alloc(ctx, &ctx->d_res_nbr, nbr.size() * sizeof(int));
-    if (!rc) rc = topo_alloc(ctx, &ctx->d_res_ex, ex);
-    if (!rc) rc = topo_alloc(ctx, &ctx->d_res_index, 2 * sizeof(unsigned));
+    const int rc = topo_alloc(ctx, &ctx->d_res, ex + (nbr.size() + 2) * sizeof(int));
     if (rc) return rc;
-    CK(cudaMemsetAsync(ctx->d_res_ex, 0, ex, ctx->stream));
+    ctx->d_res_nbr = (int *)((char *)ctx->d_res + ex);
+    ctx->d_res_index = (unsigned *)(ctx->d_res_nbr + nbr.size());
+    CK(cudaMemsetAsync(ctx->d_res, 0, ex, ctx->stream));
     CK(cudaMemsetAsync(ctx->d_res_index, 0, 2 * sizeof(unsigned), ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_res_nbr, nbr.data(), nbr.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -599,7 +599,7 @@ ResidentArgs<Real> resident_args(gbfk_ctx *ctx, double rho, double dt)
     a.dt = dt;
     const double h = sizeof(Real) == 8 ? ctx->h_h[0] : (double)(float)ctx->h_h[0];  // as upload_ih2
     a.ih2 = 1. / (h * h);
-    a.ex = (Real *)ctx->d_res_ex;
+    a.ex = (Real *)ctx->d_res;
     a.index = ctx->d_res_index;
     a.nan_flag = ctx->d_nan;
     a.err_flag = ctx->d_nan + 1;
@@ -612,23 +612,22 @@ template <typename Real>
 bool build_stream(gbfk_ctx *ctx)
 {
     if (ctx->stream_ready) return true;
-    const size_t n = (size_t)ctx->n_heavy, faces = (n + 1) * stream_face_values * sizeof(Real);
-    std::vector<int> from;
-    stream_sources(ctx->bpd, ctx->h_lists.data(), (int)n, from);
-    if (topo_alloc(ctx, &ctx->d_stream_image, n * stream_image_bytes<Real>()) ||
-        topo_alloc(ctx, &ctx->d_stream_faces[0], faces) || topo_alloc(ctx, &ctx->d_stream_faces[1], faces) ||
-        topo_alloc(ctx, &ctx->d_stream_from, from.size() * sizeof(int)) ||
-        cudaMemsetAsync(ctx->d_stream_faces[0], 0, faces, ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(ctx->d_stream_faces[1], 0, faces, ctx->stream) != cudaSuccess ||
-        cudaMemcpyAsync(ctx->d_stream_from, from.data(), from.size() * sizeof(int), cudaMemcpyHostToDevice,
-                        ctx->stream) != cudaSuccess ||
-        launch_stream_pack<Real>(ctx->d_lists, (int)n, ctx->bpd, (const Real *)ctx->d_H, ctx->d_meta, ctx->d_stream_image,
-                                 ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    const size_t n = (size_t)ctx->n_heavy, record = stream_face_values * sizeof(Real);
+    auto zeros = [&](void *faces) {  // the record after the last
+        return cudaMemsetAsync((char *)faces + n * record, 0, record, ctx->stream) == cudaSuccess;
+    };
+    const size_t image = n * stream_image_bytes<Real>(), faces = (n + 1) * record;
+    if (topo_alloc(ctx, &ctx->d_stream, image + 2 * faces + (n * 8 + ctx->nblocks) * sizeof(int))) return false;
+    for (int i = 0; i < 2; i++) ctx->d_stream_faces[i] = (char *)ctx->d_stream + image + i * faces;
+    ctx->d_stream_from = (int *)((char *)ctx->d_stream + image + 2 * faces);
+    if (!zeros(ctx->d_stream_faces[0]) || !zeros(ctx->d_stream_faces[1]) ||
+        launch_stream_pack<Real>(ctx->d_lists, (int)n, ctx->bpd, (const Real *)ctx->d_H, ctx->d_meta,
+                                 ctx->d_stream, ctx->d_stream_from, ctx->d_stream_from + n * 8,
+                                 ctx->stream) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    ctx->launches++;
+    ctx->launches += 2;
     ctx->stream_ready = true;
     return true;
 }
@@ -640,7 +639,7 @@ StreamArgs<Real> stream_args(gbfk_ctx *ctx, double rho, double dt)
     a.items = ctx->d_lists;
     a.from = ctx->d_stream_from;
     a.n = ctx->n_heavy;
-    a.image = ctx->d_stream_image;
+    a.image = ctx->d_stream;
     a.pw = (const Real *)ctx->pw;
     a.pg = (const Real *)ctx->pg;
     a.rho = (Real)rho;
@@ -676,9 +675,10 @@ int build_run_layout(gbfk_ctx *ctx, const PoolView<Real> &v)
 // 14-17 us beside its steps (launch, state and coefficients in, state out),
 // so that against one pipelined launch per step it pays from 6 steps on
 // (64^3 FP32: 14 + 1.2 n against 3.7 n; 128^3: 17 + 2.0 n against 6.3 n),
-// against the per-block kernel (9-28 us per step) from 3; leaving out the
-// empty blocks at 256^3 saves 10 us per step for 23 us.
-constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kStreamSteps = 3;
+// against the per-block kernel (9-28 us per step) from 3.  Steps over the heavy
+// blocks alone (256^3: 16.4 us instead of 30) cost 23 us per call for the empty
+// blocks' steps and the faces, and 51 us for the image of new coefficients.
+constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kStreamSteps = 3, kStreamStepsNew = 6;
 
 template <typename Real>
 int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int nsteps, int check_nan)
@@ -703,7 +703,7 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
                            std::isfinite((double)(Real)rho);
     const int clamped_steps = ctx->phi_clamped ? nsteps : nsteps - 1;
     bool want_run = uncoupled && clamped_steps >= (pipelined ? kResidentSteps : kResidentStepsBlock);
-    bool want_stream = uncoupled && clamped_steps >= kStreamSteps;
+    bool want_stream = uncoupled && clamped_steps >= (ctx->lists_valid && ctx->stream_ready ? kStreamSteps : kStreamStepsNew);
     // the tables of either cannot be built inside a stream capture
     const bool run_ready = ctx->lists_valid && ctx->res_ready, stream_ready = ctx->lists_valid && ctx->stream_ready;
     if ((want_run && !run_ready) || (want_stream && !stream_ready)) {
@@ -738,10 +738,12 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     // AUTO: a multi-level grid whose blocks fit takes its steps in one launch
     const bool levels = ctx->step_pref == GBFK_STEP_AUTO && !ctx->uniform && ctx->have_csr &&
                         levels_run_fits<Real>(ctx->nblocks, ctx->sms);
-    const bool fits = (want_run || want_stream) && resident_fits<Real>(ctx), resident = want_run && fits;
+    const bool fits = (want_run || want_stream) && resident_fits<Real>(ctx);
+    bool resident = want_run && fits;
     if (resident) {
         rc = build_resident<Real>(ctx);
-        if (rc) return rc;
+        if (rc == GBFK_E_OOM) resident = false;  // one launch per step needs none of it
+        else if (rc) return rc;
     }
     // without room for the images, the steps run as they do for short calls
     const bool stream = want_stream && !fits && ctx->n_heavy > 0 && build_stream<Real>(ctx);
@@ -2139,21 +2141,25 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     if (!A.skip_empty) ctx->adj_clean.clear();  // full steps: nothing is tracked
     // runs with resident blocks, where the blocks fit with their adjoint state
     // (FP32 1184 on a B200, FP64 592) and nothing couples the empty ones
-    const bool resident = e == cudaSuccess && A.skip_empty && ic_clamped && p->nsteps > 0 &&
+    bool resident = e == cudaSuccess && A.skip_empty && ic_clamped && p->nsteps > 0 &&
                           ctx->step_pref == GBFK_STEP_AUTO && std::isfinite((double)(Real)p->Dw) &&
                           std::isfinite((double)(Real)p->Dg) && std::isfinite((double)A.rho) &&
                           resident_fits<Real>(ctx) && ctx->n_heavy <= adjoint_run_capacity<Real>(ctx->sms);
     double *run_sums = nullptr;
+    const size_t ex = 2 * (size_t)ctx->n_heavy * 384 * 2 * sizeof(Real),
+                 acc_bytes = resident ? (size_t)adjoint_run_threads(ctx->n_heavy, ctx->sms) * 6 * sizeof(double) : 0,
+                 sums = (size_t)ctx->sms * 6 * sizeof(double), bytes = ex + acc_bytes + sums + 2 * sizeof(unsigned);
     if (resident) {
         rc = build_resident<Real>(ctx);
-        const size_t n = (size_t)ctx->n_heavy, ex = 2 * n * 384 * 2 * sizeof(Real),
-                     acc = (size_t)adjoint_run_threads((int)n, ctx->sms) * 6 * sizeof(double),
-                     sums = (size_t)ctx->sms * 6 * sizeof(double), bytes = ex + acc + sums + 2 * sizeof(unsigned);
         if (!rc) rc = topo_alloc(ctx, &ctx->d_adj_run, bytes);
-        if (rc) {
+        if (rc && rc != GBFK_E_OOM) {
             cleanup();
             return rc;
         }
+        if (rc) resident = false;  // one launch per step needs none of it
+        rc = GBFK_OK;
+    }
+    if (resident) {
         char *d = (char *)ctx->d_adj_run;
         if (!ctx->adj_run_ready) {
             CK(cudaMemsetAsync(d, 0, bytes, ctx->stream));
@@ -2178,12 +2184,12 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         r.self = A.sets[0].self;
         r.flags = A.sets[0].flags;
         r.acc = (double *)(d + ex);
-        r.sums = run_sums = (double *)(d + ex + acc);
+        r.sums = run_sums = (double *)(d + ex + acc_bytes);
         r.rho = A.rho;
         r.dt = p->dt;
         r.ih2 = f.ih2;
         r.ex = (uint2 *)d;
-        r.index = (unsigned *)(d + ex + acc + sums);
+        r.index = (unsigned *)(d + ex + acc_bytes + sums);
         r.err_flag = ctx->d_nan + 1;
     }
     // forward to the horizon (storing the first chain of checkpoints), loss and its gradient

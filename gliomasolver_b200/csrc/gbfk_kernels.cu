@@ -4,6 +4,7 @@
 #include "gbfk_kernels.cuh"
 #include "gbfk_resident.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace gbfk {
@@ -115,10 +116,12 @@ face_kernel(PoolView<Real> v, Real Dw, Real Dg, Real *__restrict__ H, unsigned s
     const int blk = blockIdx.x;
     const int t = threadIdx.x;
     const int64_t base = slot_of(v, blk) * kBS3;
+    bool tissue = false;
     for (int c = t; c < kBS3; c += 256) {
         const int l = lab_index(c & 7, (c >> 3) & 7, c >> 6);
         S.pw[l] = v.pw[base + c];
         S.pg[l] = v.pg[base + c];
+        tissue |= S.pw[l] != (Real)0 || S.pg[l] != (Real)0;
     }
     for (int q = t; q < 6 * kFaceCells; q += 256) {
         const int f = q >> 6, p = q & 63;
@@ -134,8 +137,18 @@ face_kernel(PoolView<Real> v, Real Dw, Real Dg, Real *__restrict__ H, unsigned s
             S.pw[l] = v.gpw[g];
             S.pg[l] = v.gpg[g];
         }
+        tissue |= S.pw[l] != (Real)0 || S.pg[l] != (Real)0;
     }
-    __syncthreads();
+    // no tissue in the block or its face halos (four blocks of five of a
+    // brain's box): every coefficient is +0.  128^3 FP32: 28 -> 22 us
+    if (!__syncthreads_or(tissue) && isfinite(Dw) && isfinite(Dg)) {
+        const int4 zero = make_int4(0, 0, 0, 0);
+        int4 *h = reinterpret_cast<int4 *>(H + (int64_t)blk * kFacesPerBlock);
+        for (int q = t; q < (int)(kFacesPerBlock * sizeof(Real) / 16); q += 256) h[q] = zero;
+        for (int c = t; c < kBS3; c += 256) meta[base + c] = kMetaAllEmpty;
+        if (t == 0) btype[blk] = kBlockEmpty;
+        return;
+    }
     for (int c = t; c < kBS3; c += 256) {
         const int l = lab_index(c & 7, (c >> 3) & 7, c >> 6);
         S.df[l] = diffusivity(S.pw[l], S.pg[l], Dw, Dg);
@@ -1324,13 +1337,18 @@ __global__ void gaussian_ic_kernel(int bpd, const Real *__restrict__ pw, const R
     const int n = 8 * bpd;
     const int64_t N = (int64_t)n * n * n;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+        // the divisions and exp only where there is tissue
+        if (!(pw[i] + pg[i] > (Real)0)) {
+            out[i] = (Real)0;
+            continue;
+        }
         const int64_t b = i >> 9;
         const int c = (int)(i & 511);
         const int bx = (int)(b % bpd), by = (int)((b / bpd) % bpd), bz = (int)(b / ((int64_t)bpd * bpd));
         const double x = (double)(bx * 8 + (c & 7)) / n, y = (double)(by * 8 + ((c >> 3) & 7)) / n,
                      z = (double)(bz * 8 + (c >> 6)) / n;
         const double r2 = (x - x0) * (x - x0) + (y - y0) * (y - y0) + (z - z0) * (z - z0);
-        out[i] = (pw[i] + pg[i] > (Real)0) ? (Real)exp(-r2 / (2. * sigma * sigma)) : (Real)0;
+        out[i] = (Real)exp(-r2 / (2. * sigma * sigma));
     }
 }
 
@@ -1588,17 +1606,28 @@ cudaError_t launch_collapse(int ncollapse, const int *children, const int *paren
 // ---------------------------------------------------------------------------
 // Dense n^3 volume <-> uniform block pool (block (bx,by,bz) in slot
 // bx + bpd*(by + bpd*bz)).
+// A thread moves four x-consecutive cells; rows are counted in 32 bits (n^2 <
+// 2^32).  A 64-bit division per index of each cell took 17 us at 128^3 FP32
+// and 78 at 256^3; this takes 6.6 and 24.
 template <typename Real>
-__global__ void dense_scatter_kernel(const Real *__restrict__ src, Real *__restrict__ dst, int n, bool to_pool)
+__global__ void __launch_bounds__(256) dense_scatter_kernel(const Real *__restrict__ src, Real *__restrict__ dst,
+                                                            unsigned n, bool to_pool)
 {
-    const int64_t N = (int64_t)n * n * n;
-    const int bpd = n / kBS;
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < N; g += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(g % n), y = (int)((g / n) % n), z = (int)(g / ((int64_t)n * n));
-        const int64_t slot = (x >> 3) + (int64_t)bpd * ((y >> 3) + (int64_t)bpd * (z >> 3));
-        const int64_t p = slot * kBS3 + (x & 7) + kBS * ((y & 7) + kBS * (z & 7));
-        if (to_pool) dst[p] = src[g];
-        else dst[g] = src[p];
+    const unsigned bpd = n / kBS, per = n / 4, rows = n * n;
+    const unsigned lanes = min(per, 256u), lane = threadIdx.x % lanes, group = threadIdx.x / lanes,
+                   groups = blockDim.x / lanes;
+    if (group >= groups) return;
+    for (unsigned row = blockIdx.x * groups + group; row < rows; row += gridDim.x * groups) {
+        const unsigned y = row % n, z = row / n;
+        const int64_t pool = ((int64_t)bpd * ((y >> 3) + (int64_t)bpd * (z >> 3))) * kBS3 + kBS * ((y & 7) + kBS * (z & 7));
+        const int64_t dense = (int64_t)row * n;
+        for (unsigned v = lane; v < per; v += lanes) {
+            const int64_t p = pool + (int64_t)(v >> 1) * kBS3 + (v & 1) * 4, g = dense + 4 * v;
+            Vec4<Real> c;
+            c.load(src + (to_pool ? g : p));
+            c.store(dst + (to_pool ? p : g));
+        }
+        if (row + gridDim.x * groups < row) break;  // the next row's number would not fit
     }
 }
 
@@ -1656,10 +1685,8 @@ cudaError_t launch_cfl(const PoolView<Real> &v, Real Dw, Real Dg, double *partia
 template <typename Real>
 cudaError_t launch_dense_scatter(const Real *src, Real *dst, int n, bool to_pool, cudaStream_t s)
 {
-    const int64_t N = (int64_t)n * n * n;
-    int64_t nb = (N + 255) / 256;
-    if (nb > 148 * 64) nb = 148 * 64;
-    dense_scatter_kernel<Real><<<(int)nb, 256, 0, s>>>(src, dst, n, to_pool);
+    const int64_t nb = std::min<int64_t>(((int64_t)n * n * (n / 4) + 255) / 256, 148 * 32);
+    dense_scatter_kernel<Real><<<(int)nb, 256, 0, s>>>(src, dst, (unsigned)n, to_pool);
     return cudaGetLastError();
 }
 

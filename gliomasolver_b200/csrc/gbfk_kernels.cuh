@@ -170,8 +170,9 @@ struct ResidentArgs {
 };
 // One step of the n heavy blocks of a uniform grid of any size (gbfk_stream.cu).
 // image: their coefficients in the layout of the kernel's shared memory
-// (stream_image_bytes each, launch_stream_pack); from: eight words per block
-// that say where its copies come from (stream_sources);
+// (stream_image_bytes each) and from: eight words per block that say where its
+// copies come from, both by launch_stream_pack (at: a word per block of the grid,
+// scratch);
 // faces_in: the x and y faces of phi_in's heavy blocks (stream_face_values each,
 // launch_stream_faces), a record of zeros after the last; faces_out: the next
 // state's.  first: nothing of the launch before may overlap.
@@ -189,12 +190,11 @@ struct StreamArgs {
     unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
 };
 constexpr int stream_face_values = 256;
-void stream_sources(int bpd, const int *items, int n, std::vector<int> &from);
 template <typename Real>
 size_t stream_image_bytes();
 template <typename Real>
-cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta, void *image,
-                               cudaStream_t s);
+cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta,
+                               void *image, int *from, int *at, cudaStream_t s);
 template <typename Real>
 cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, cudaStream_t s);
 template <typename Real>

@@ -52,9 +52,17 @@ template <typename Real>
 constexpr int kStreamSlots = sizeof(Real) == 4 ? 3 : 2;
 constexpr int kStreamHead = 256;  // bytes of shared memory for the barriers
 
+// at[block] = its item (the rest: -1)
+__global__ void stream_index_kernel(const int *items, int n, int *at)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) at[items[i] >> 2] = i;
+}
+
 template <typename Real>
 __global__ void __launch_bounds__(kThreads)
-stream_pack_kernel(const int *items, int bpd, const Real *H, const unsigned short *meta, StreamImage<Real> *image)
+stream_pack_kernel(const int *items, int n, int bpd, const Real *H, const unsigned short *meta, const int *at,
+                   StreamImage<Real> *image, int *from)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StreamImage<Real> &b = *reinterpret_cast<StreamImage<Real> *>(smem_raw);
@@ -62,12 +70,24 @@ stream_pack_kernel(const int *items, int bpd, const Real *H, const unsigned shor
     const int64_t blk = e >> 2;
     load_coefficients<Real, kCells>(b, H + blk * kFacesPerBlock, meta + blk * kBS3, t, false,
                                     [] { __syncthreads(); });
-    if (t == 0) b.e = e;
-    if (t < 6) b.at[t] = block_across(bpd, e >> 2, t);
+    if (t == 0) {
+        b.e = e;
+        from[blockIdx.x * 8] = blockIdx.x;
+        from[blockIdx.x * 8 + 1] = (e >> 2) * 8;
+    }
+    if (t < 6) {
+        const int across = block_across(bpd, e >> 2, t), item = at[across];
+        b.at[t] = across;
+        // in records of 64 cells: x and y faces of the faces array, z faces of
+        // the state; an empty neighbour's are the zeros after the last faces
+        from[blockIdx.x * 8 + 2 + t] = item < 0 ? (int)(n * 4u | (t < 4 ? 0u : 0x80000000u))
+                                       : t < 4  ? item * 4 + (t ^ 1)
+                                                : across * 8 + (t == 4 ? 7 : 0);
+    }
     __syncthreads();
-    const int4 *from = reinterpret_cast<const int4 *>(&b);
+    const int4 *src = reinterpret_cast<const int4 *>(&b);
     int4 *to = reinterpret_cast<int4 *>(image + blockIdx.x);
-    for (int q = t; q < (int)(sizeof(b) / 16); q += kThreads) to[q] = from[q];
+    for (int q = t; q < (int)(sizeof(b) / 16); q += kThreads) to[q] = src[q];
 }
 
 // The x and y faces of a thread's cells (x0 .. x0 + 3 of row z * 8 + y).
@@ -211,33 +231,19 @@ stream_step_kernel(const __grid_constant__ StreamArgs<Real> a)
 
 }  // namespace
 
-void stream_sources(int bpd, const int *items, int n, std::vector<int> &from)
-{
-    std::vector<int> nbr;
-    resident_neighbours(bpd, items, n, nbr);
-    from.clear();
-    for (int i = 0; i < n; i++) {
-        from.push_back(i);
-        from.push_back((items[i] >> 2) * 8);
-        for (int f = 0; f < 6; f++) {
-            const int nb = nbr[(size_t)i * 6 + f];
-            if (nb < 0) from.push_back((int)(n * 4u | (f < 4 ? 0u : 0x80000000u)));  // zeros
-            else if (f < 4) from.push_back(nb * 4 + (f ^ 1));
-            else from.push_back((items[nb] >> 2) * 8 + (f == 4 ? 7 : 0));
-        }
-    }
-}
-
 template <typename Real>
 size_t stream_image_bytes() { return sizeof(StreamImage<Real>); }
 
 template <typename Real>
-cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta, void *image,
-                               cudaStream_t s)
+cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta,
+                               void *image, int *from, int *at, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    stream_pack_kernel<Real><<<n, kThreads, sizeof(StreamImage<Real>), s>>>(items, bpd, H, meta,
-                                                                            (StreamImage<Real> *)image);
+    cudaError_t e = cudaMemsetAsync(at, 0xff, (size_t)bpd * bpd * bpd * sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    stream_index_kernel<<<(n + 255) / 256, 256, 0, s>>>(items, n, at);
+    stream_pack_kernel<Real><<<n, kThreads, sizeof(StreamImage<Real>), s>>>(items, n, bpd, H, meta, at,
+                                                                            (StreamImage<Real> *)image, from);
     return cudaGetLastError();
 }
 
@@ -274,9 +280,9 @@ cudaError_t launch_stream_step(const StreamArgs<Real> &a, bool first, int sms, c
 template size_t stream_image_bytes<float>();
 template size_t stream_image_bytes<double>();
 template cudaError_t launch_stream_pack<float>(const int *, int, int, const float *, const unsigned short *, void *,
-                                               cudaStream_t);
+                                               int *, int *, cudaStream_t);
 template cudaError_t launch_stream_pack<double>(const int *, int, int, const double *, const unsigned short *, void *,
-                                                cudaStream_t);
+                                               int *, int *, cudaStream_t);
 template cudaError_t launch_stream_faces<float>(const int *, int, const float *, float *, cudaStream_t);
 template cudaError_t launch_stream_faces<double>(const int *, int, const double *, double *, cudaStream_t);
 template cudaError_t launch_stream_step<float>(const StreamArgs<float> &, bool, int, cudaStream_t);

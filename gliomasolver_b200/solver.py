@@ -143,10 +143,10 @@ class BlockPool:
     # -- hot path ---------------------------------------------------------
     @property
     def step_kernel(self) -> str:
-        """Kernel of the last rd_step: "pipelined" (persistent TMA pipeline,
-        uniform power-of-two grids, one launch per step), "run" (several
-        steps in one launch, with the blocks resident in shared memory or,
-        where "run" was assigned, the same pipeline over all steps of the
+        """Kernel of the last rd_step: "pipelined" (persistent kernels fed
+        by bulk copies, uniform grids, one launch per step), "run" (several
+        steps in one launch: on "auto" with the blocks resident on the SMs;
+        where "run" was assigned, the TMA pipeline over all steps of the
         call), "block" (one CTA per block) or "" before any step.  Assign "auto", "block",
         "pipelined" or "run" to choose."""
         k = int(self.lib.gbfk_step_kernel(self.ctx))

@@ -141,12 +141,12 @@ int gbfk_rd_step(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
  * GBFK_STEP_AUTO (the default), for a call of several steps on a uniform
  * grid from gbfk_set_uniform, runs them in one cooperative launch with the
  * blocks that hold tissue resident in shared memory (reported as
- * GBFK_STEP_RUN), where they fit: about 2200 blocks in FP32, 1180 in FP64 on
- * a B200.  Otherwise it runs the persistent TMA-fed pipeline on uniform
- * power-of-two grids (in calls of several steps without the blocks that hold
- * no tissue, whose cells only react and take all steps in a launch of their
- * own) and the one-CTA-per-block kernel elsewhere.  The first step after phi
- * was uploaded always runs by itself there.  On a grid from
+ * GBFK_STEP_RUN), where they fit: about 2300 blocks in FP32, 1180 in FP64 on
+ * a B200. Beyond, each step is a launch over the blocks that hold tissue
+ * (reported as GBFK_STEP_PIPELINED); the others, whose cells only react, take
+ * all steps in a launch of their own. Short calls, and the first step after
+ * phi was uploaded, run the persistent TMA-fed pipeline on power-of-two grids
+ * and the one-CTA-per-block kernel elsewhere.  On a grid from
  * gbfk_set_topology with up to about 1180 blocks in FP32, 890 in FP64, a call
  * of several steps is one cooperative launch with a block per CTA (also
  * reported as GBFK_STEP_RUN); larger ones launch a ghost fill and the

@@ -194,7 +194,7 @@ def test_steps_over_the_heavy_blocks_equal_the_block_kernel(gbfk_lib, prec, n):
         with _pool(n, prec, (pw, pg, c0)) as pool:
             pool.step_kernel = kind
             got = []
-            for Dw, steps in ((0.3, 7), (0.3, 4), (0.3, 2), (0.15, 5)):
+            for Dw, steps in ((0.3, 7), (0.3, 4), (0.3, 2), (0.15, 7)):
                 s = make_schedule(Dw, 0.2, 300.0, 25.6, n // 8, prec)
                 pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, steps, check_nan=True)
                 got.append(pool.download_dense("phi"))
