@@ -14,12 +14,14 @@
 // What bounds it: a step is one exchange of faces through L2 (about 0.9 us
 // from a block's stores to the end of its neighbours' next step, what an 8-
 // block grid takes) plus the issue of its cells' exact-rounding arithmetic
-// (128^3, FP32: 1.69 M warp instructions per step, 67 % of the issue slots).
-// Measured on a B200, us per step over 1000 steps, against one launch per
-// step: 64^3 FP32 1.16 (3.74), FP64 1.36 (3.87); 128^3 FP32 1.94 (6.33), FP64
-// 3.06 (8.59); 160^3 FP32 3.27 (17.2, one CTA per block).  A stage by teams
-// of CTAs, 15 blocks per CTA: 128^3 FP32 2.0 us per sample-step (3.7 in
-// launches over all samples), 64^3 0.39 (0.9).
+// (128^3, FP32, 860 blocks with tissue: 1.35 M warp instructions per step, 61 %
+// of the issue slots).
+// Measured on a B200, us per step over 2000 steps, against one launch per
+// step, a brain of 18 % of its box: 64^3 FP32 1.11 (3.74), FP64 1.37 (3.85);
+// 96^3 FP32 1.32 (9.3, one CTA per block); 128^3 FP32 1.94 (6.41), FP64 3.12
+// (8.82); 160^3 FP32 3.24 (17.5, one CTA per block). A stage by teams of CTAs:
+// 128^3 FP32 1.93 us per sample-step (3.7 in launches over all samples), 64^3
+// 0.42 (0.95).
 //
 // Faces travel through L2.  After forming state k a block stores its six
 // faces in the exchange buffer k & 1 and its neighbours poll for them there.
