@@ -225,8 +225,9 @@ struct alignas(16) ResidentState {
 //             opposite coefficient (for a kEmpty cell itself, whose
 //             coefficients are all 0, whatever is doubled stays 0, and its
 //             formula leaves +0 where phi is +0 and the reaction where it is
-//             not, so that its domain test needs no branch).  -0 for +0 in
-//             the flux sums gives the same sums: (+0) + (-0) = +0 either way;
+//             not, so that its domain test needs no branch unless the result
+//             is NaN).  -0 for +0 in the flux sums gives the same sums:
+//             (+0) + (-0) = +0 either way;
 //   kGeneral  kOther cells or neighbours, or a coefficient that is negative
 //             by itself: the tests as written, p_w and p_g from global memory;
 //   kStill    kEmpty cells that hold +0, which stay so: nothing flows into a
@@ -502,6 +503,18 @@ __device__ __forceinline__ void row_cells(const Args &a, double ih2, unsigned lo
             const Real dphidt = to_real<Real>(__dadd_rn(__dadd_rn(fluxOut, fluxIn), reaction));
             const Real q = clamp_state(to_real<Real>(__dadd_rn(phid, __dmul_rn(a.dt, (double)dphidt))));
             out[i + j] = dom[j] ? q : ph[j];  // outside the domain a clamped value stays (dt is finite)
+        }
+        // kEdge takes every cell for one inside the domain, which a kEmpty cell
+        // at +0 is not: with finite values its formula leaves +0, but a NaN
+        // neighbour gives NaN through a coefficient of 0 too.  So a new value
+        // that is NaN goes through the domain test as it is written.
+        if constexpr (kKind == kEdge) {
+            if (out[i] != out[i] || out[i + 1] != out[i + 1]) {
+                const int64_t c = (int64_t)(b.e >> 2) * kBS3 + w.t * kC + i;
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    if (!in_domain(a.pw[c + j], a.pg[c + j], ph[j])) out[i + j] = ph[j];
+            }
         }
         if (i + 2 < kC) asm volatile("" ::: "memory");
     }

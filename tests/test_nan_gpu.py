@@ -1,0 +1,131 @@
+"""Where a NaN goes: every way of taking several steps leaves it in the same
+cells as the one-CTA-per-block kernel, which evaluates the domain test
+p_w + p_g + phi > 0 of every cell as it is written (a CSF cell at +0 is outside
+the domain and keeps its +0 next to a NaN)."""
+import numpy as np
+import pytest
+
+from gliomasolver_b200 import BlockPool, GbfkError
+from gliomasolver_b200.schedule import make_schedule
+
+pytestmark = pytest.mark.gpu
+
+
+def layered(n, seed, prec, thin=False):
+    """p_w, p_g, phi: tissue cut into rooms by CSF sheets one to three cells
+    thick, a corner of CSF (whole blocks of it from 32^3 on), phi in the
+    tissue only, NaN in tissue cells of one room in front of a sheet; with
+    `thin` also cells whose p_w + p_g is below 0.1."""
+    R = np.float64 if prec == "f64" else np.float32
+    rng = np.random.default_rng(seed)
+    tissue = np.ones((n, n, n), dtype=bool)
+    at = 5
+    for k in range(n):
+        width = 1 + k % 3
+        if at + width + 3 > n:
+            break
+        tissue[:, :, at:at + width] = False
+        tissue[at:at + width, :, :] &= rng.random((width, n, n)) < 0.5
+        at += width + 6
+    tissue[: n // 2, : n // 2, : n // 2] = False
+    pw = np.where(tissue, rng.uniform(0.3, 0.7, tissue.shape), 0.0)
+    pg = np.where(tissue, 1.0 - pw, 0.0)
+    if thin:
+        few = rng.random(tissue.shape) < 0.02
+        pw, pg = np.where(few, 0.06 * pw, pw), np.where(few, 0.06 * pg, pg)
+    phi = np.where(tissue & (rng.random(tissue.shape) < 0.4), rng.uniform(0, 1, tissue.shape), 0.0)
+    spot = np.argwhere(tissue[:, :, 4])[:: max(1, n)][:4]
+    for z, y in spot:
+        phi[z, y, 4] = np.nan
+    return [a.astype(R) for a in (pw, pg, phi)]
+
+
+def _pool(n, prec, fields):
+    pool = BlockPool((n // 8) ** 3, prec)
+    pool.set_uniform(n // 8)
+    for name, a in zip(("p_w", "p_g", "phi"), fields):
+        pool.upload_dense(name, a)
+    return pool
+
+
+def same_as_block_steps(n, prec, fields, calls, used):
+    s = make_schedule(0.3, 0.2, 300.0, 25.6, n // 8, prec)
+    with _pool(n, prec, fields) as a, _pool(n, prec, fields) as b:
+        b.step_kernel = "block"
+        for steps in calls:
+            for p in (a, b):
+                p.rd_step(s.Dw, s.Dg, s.rho, s.dt, steps)
+            got, want = a.download_dense("phi"), b.download_dense("phi")
+            assert a.step_kernel == used
+            assert np.array_equal(got, want, equal_nan=True), (steps, np.isnan(got).sum(), np.isnan(want).sum())
+        assert 0 < np.isnan(want).sum() < want.size
+        for p in (a, b):
+            with pytest.raises(GbfkError) as e:
+                p.rd_step(s.Dw, s.Dg, s.rho, s.dt, 8, check_nan=True)
+            assert e.value.code == 4
+
+
+@pytest.mark.parametrize("thin", [False, True])
+@pytest.mark.parametrize("prec,n", [("f32", 24), ("f64", 32), ("f32", 64), ("f32", 104), ("f64", 72)])
+def test_nan_beside_csf_in_a_resident_run(gbfk_lib, prec, n, thin):
+    same_as_block_steps(n, prec, layered(n, n, prec, thin), (8, 13, 40), "run")
+
+
+@pytest.mark.parametrize("prec,n", [("f32", 152), ("f64", 120)])
+def test_nan_beside_csf_in_steps_over_the_heavy_blocks(gbfk_lib, prec, n):
+    same_as_block_steps(n, prec, layered(n, n, prec), (8, 13), "pipelined")
+
+
+@pytest.mark.parametrize("prec,bpd", [("f32", 4), ("f64", 3), ("f32", 12)])
+def test_nan_beside_csf_in_a_stage(gbfk_lib, prec, bpd):
+    """Initial conditions that are NaN: everywhere in the tissue (a NaN
+    origin), or at the origin alone (0 / 0 with a width whose square is 0)."""
+    from gliomasolver_b200.tmcmc import Batch, sample_stage, to_gbfk_samples
+
+    n = 8 * bpd
+    pw, pg, _ = layered(n, 7, prec)
+    recs, _ = to_gbfk_samples(sample_stage(4, pw, seed=2, tend_range=(5.0, 30.0)), bpd, prec)
+    for i, r in enumerate(recs):
+        r.nsteps = 9 + 4 * i
+    recs[1].x0[0] = np.nan
+    z, y = np.argwhere(pw[:, :, 4] > 0)[n]
+    recs[2].x0[0], recs[2].x0[1], recs[2].x0[2] = 4 / n, y / n, z / n
+    recs[2].sigma = 1e-200
+    with Batch(bpd, 4, prec, max_anatomies=1) as b:
+        b.set_anatomy(0, pw, pg)
+        out = []
+        for kind in (1, 0):
+            b.set_samples(recs)
+            with pytest.raises(GbfkError) as e:
+                b.run(kind)
+            assert e.value.code == 4
+            out.append([b.download(i) for i in range(4)])
+        assert b.samples_per_cta == -1
+    for i, (want, got) in enumerate(zip(*out)):
+        assert np.array_equal(got, want, equal_nan=True), i
+        assert np.isnan(want).any() == (i in (1, 2))
+
+
+@pytest.mark.parametrize("prec,bpd", [("f64", 4), ("f32", 8)])
+def test_nan_beside_csf_in_a_resident_sweep(gbfk_lib, prec, bpd):
+    """The gradient with NaN in the initial field: the same cells of lambda_0
+    as with a launch per step."""
+    n, steps = 8 * bpd, 14
+    pw, pg, phi = layered(n, 3, prec, thin=True)
+    rng = np.random.default_rng(1)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
+    s = make_schedule(0.2, 0.1, 100.0, 25.6, bpd, prec)
+    out = {}
+    with _pool(n, prec, (pw, pg, phi)) as pool:
+        pool.set_observations(t1, fl)
+        for kind in ("pipelined", "auto"):
+            pool.step_kernel = kind
+            out[kind] = pool.forward_adjoint(s.Dw, s.Dg, s.rho, min(s.dt, 0.2), steps, sigma=0.0, nsnapshots=4,
+                                             grad_c0=True, term_magnitudes=True, t1_uc=0.7, t2_uc=0.25, slope=2.0)
+    a, b = out["auto"], out["pipelined"]
+    assert np.array_equal(a["grad_c0"], b["grad_c0"], equal_nan=True)
+    assert np.isnan(a["loss"]) == np.isnan(b["loss"])
+    for key in ("dDw", "drho", "dDw_abs", "drho_abs"):
+        scale = b[key.replace("_abs", "") + "_abs"]
+        assert np.isnan(a[key]) == np.isnan(b[key]), key
+        assert np.isnan(b[key]) or abs(a[key] - b[key]) <= 1e-14 * scale + 1e-13 * abs(b[key]), key
