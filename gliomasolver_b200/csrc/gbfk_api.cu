@@ -117,8 +117,9 @@ struct gbfk_ctx {
     unsigned *d_res_index = nullptr;  // the state count
     bool res_ready = false;
     // step by step over the heavy blocks (launch_stream_step)
-    void *d_stream = nullptr;         // one buffer: the images, the faces of two states, the sources
+    void *d_stream = nullptr;         // one buffer: the images, the faces of two states, state 0, the sources
     void *d_stream_faces[2] = {};
+    void *d_stream_save = nullptr;
     int *d_stream_from = nullptr;
     bool stream_ready = false;
     int sms = 0;
@@ -133,7 +134,8 @@ struct gbfk_ctx {
     bool phi_clamped = false;
 
     // scratch
-    unsigned *d_nan = nullptr;        // [0]: NaN seen in a step, [1]: a wait timed out, [2], [3]: a levels run's barrier
+    // [0]: NaN seen in a step, [1]: a wait timed out, [2], [3]: a grid barrier, [4], [5]: SettleWords
+    unsigned *d_nan = nullptr;
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
     gbfk_host::StagedCopy staged;     // copies of pageable host memory
@@ -616,10 +618,12 @@ bool build_stream(gbfk_ctx *ctx)
     auto zeros = [&](void *faces) {  // the record after the last
         return cudaMemsetAsync((char *)faces + n * record, 0, record, ctx->stream) == cudaSuccess;
     };
-    const size_t image = n * stream_image_bytes<Real>(), faces = (n + 1) * record;
-    if (topo_alloc(ctx, &ctx->d_stream, image + 2 * faces + (n * 8 + ctx->nblocks) * sizeof(int))) return false;
+    const size_t image = n * stream_image_bytes<Real>(), faces = (n + 1) * record,
+                 save = n * kBS3 * sizeof(Real);
+    if (topo_alloc(ctx, &ctx->d_stream, image + 2 * faces + save + (n * 8 + ctx->nblocks) * sizeof(int))) return false;
     for (int i = 0; i < 2; i++) ctx->d_stream_faces[i] = (char *)ctx->d_stream + image + i * faces;
-    ctx->d_stream_from = (int *)((char *)ctx->d_stream + image + 2 * faces);
+    ctx->d_stream_save = (char *)ctx->d_stream + image + 2 * faces;
+    ctx->d_stream_from = (int *)((char *)ctx->d_stream_save + save);
     if (!zeros(ctx->d_stream_faces[0]) || !zeros(ctx->d_stream_faces[1]) ||
         launch_stream_pack<Real>(ctx->d_lists, (int)n, ctx->bpd, (const Real *)ctx->d_H, ctx->d_meta,
                                  ctx->d_stream, ctx->d_stream_from, ctx->d_stream_from + n * 8,
@@ -648,6 +652,33 @@ StreamArgs<Real> stream_args(gbfk_ctx *ctx, double rho, double dt)
     a.ih2 = 1. / (h * h);
     a.nan_flag = ctx->d_nan;
     a.err_flag = ctx->d_nan + 1;
+    a.settle = (SettleWords *)(ctx->d_nan + 4);
+    return a;
+}
+
+// What is left to do after a run or a chain over the heavy blocks (state, save,
+// nsteps and last are the caller's).
+template <typename Real>
+SettleArgs<Real> settle_args(gbfk_ctx *ctx, double rho, double dt)
+{
+    const ResidentArgs<Real> r = resident_args<Real>(ctx, rho, dt);
+    SettleArgs<Real> a = {};
+    a.bpd = ctx->bpd;
+    a.nblocks = ctx->nblocks;
+    a.items = ctx->d_lists;
+    a.n = ctx->n_heavy;
+    a.empty = ctx->d_lists + ctx->n_heavy;
+    a.n_empty = ctx->n_empty;
+    a.H = r.H;
+    a.pw = r.pw;
+    a.pg = r.pg;
+    a.rho = r.rho;
+    a.dt = r.dt;
+    a.ih2 = r.ih2;
+    a.words = (SettleWords *)(ctx->d_nan + 4);
+    a.nan_flag = ctx->d_nan;
+    a.err_flag = ctx->d_nan + 1;
+    a.sync = ctx->d_nan + 2;
     return a;
 }
 
@@ -672,12 +703,13 @@ int build_run_layout(gbfk_ctx *ctx, const PoolView<Real> &v)
 }
 
 // From how many steps on a call is worth a run: a resident run costs about
-// 14-17 us beside its steps (launch, state and coefficients in, state out),
-// so that against one pipelined launch per step it pays from 6 steps on
-// (64^3 FP32: 14 + 1.2 n against 3.7 n; 128^3: 17 + 2.0 n against 6.3 n),
-// against the per-block kernel (9-28 us per step) from 3.  Steps over the heavy
-// blocks alone (256^3: 16.4 us instead of 30) cost 23 us per call for the empty
-// blocks' steps and the faces, and 51 us for the image of new coefficients.
+// 11-15 us beside its steps (launch, state and coefficients in, state out, and
+// 3 us of launch_settle), so that against one pipelined launch per step it is
+// even at 4 steps and pays from 6 on (64^3 FP32: 10.5 + 1.17 n against 3.85 n;
+// 128^3: 14.6 + 1.88 n against 6.4 n), against the per-block kernel (9-28 us per
+// step) from 3.  Steps over the heavy blocks alone (256^3: 15.7 us instead of
+// 30) cost 39 us per call (the empty blocks, the faces and state 0, the first
+// launch, launch_settle), and 51 us for the image of new coefficients.
 constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kStreamSteps = 3, kStreamStepsNew = 6;
 
 template <typename Real>
@@ -734,7 +766,10 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     }
     if (check_nan) CK(cudaMemsetAsync(ctx->d_nan, 0, sizeof(unsigned), ctx->stream));
     const BlockLists lists = {ctx->d_lists, ctx->n_heavy, ctx->d_lists + ctx->n_heavy, ctx->n_empty};
-    bool ran_run = false, skip = false, streamed = false;
+    bool ran_run = false;
+    int streamed = 0;  // steps of the chain over the heavy blocks
+    Real *const buffer[2] = {(Real *)ctx->phi[0], (Real *)ctx->phi[1]};
+    int chain = 0;  // the buffer of the chain's state 0
     // AUTO: a multi-level grid whose blocks fit takes its steps in one launch
     const bool levels = ctx->step_pref == GBFK_STEP_AUTO && !ctx->uniform && ctx->have_csr &&
                         levels_run_fits<Real>(ctx->nblocks, ctx->sms);
@@ -756,23 +791,23 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
             // in place: every block's state 0 is read by its own CTA alone
             ResidentArgs<Real> a = resident_args<Real>(ctx, rho, dt);
             a.in = in;
-            a.out = (Real *)ctx->phi[ctx->cur];
+            a.out = buffer[ctx->cur];
             a.nsteps = left;
             a.empty = lists.empty;
             a.n_empty = lists.n_empty;
+            a.settle = (SettleWords *)(ctx->d_nan + 4);
+            a.save = out;
             CK(launch_resident_run<Real>(a, ctx->sms, ctx->stream));
-            ctx->launches++;
+            SettleArgs<Real> f = settle_args<Real>(ctx, rho, dt);
+            f.state[0] = a.out;
+            f.state[1] = out;
+            f.save = out;
+            f.nsteps = left;
+            CK(launch_settle<Real>(f, ctx->sms, ctx->stream));
+            ctx->launches += 2;
             s += left;
             ran_run = true;
             continue;
-        }
-        if (stream && clamped && !skip) {
-            // both buffers get the empty blocks' last state: a heavy block's
-            // halo copies may read either, multiplied by coefficients of 0
-            CK(launch_empty_run<Real>(lists.empty, lists.n_empty, in, (Real *)ctx->phi[ctx->cur], out, left,
-                                      (Real)rho, dt, ctx->d_nan, ctx->stream));
-            ctx->launches++;
-            skip = true;
         }
         if (stream && clamped) {
             StreamArgs<Real> a = stream_args<Real>(ctx, rho, dt);
@@ -781,14 +816,27 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
             a.faces_in = (const Real *)ctx->d_stream_faces[s & 1];
             a.faces_out = (Real *)ctx->d_stream_faces[(s & 1) ^ 1];
             if (!streamed) {
-                CK(launch_stream_faces<Real>(a.items, a.n, in, (Real *)ctx->d_stream_faces[s & 1], ctx->stream));
-                ctx->launches++;
+                chain = ctx->cur;
+                CK(launch_empty_scan<Real>(lists.empty, lists.n_empty, in, out, a.settle, ctx->d_nan, ctx->stream));
+                CK(launch_stream_faces<Real>(a.items, a.n, in, (Real *)ctx->d_stream_faces[s & 1],
+                                             (Real *)ctx->d_stream_save, ctx->stream));
+                ctx->launches += lists.n_empty > 0 ? 2 : 1;
             }
             CK(launch_stream_step<Real>(a, !streamed, ctx->sms, ctx->stream));
             ctx->launches++;
             ctx->cur ^= 1;
             s++;
-            streamed = true;
+            streamed++;
+            if (s == nsteps) {
+                SettleArgs<Real> f = settle_args<Real>(ctx, rho, dt);
+                f.state[0] = buffer[chain];
+                f.state[1] = buffer[chain ^ 1];
+                f.save = (const Real *)ctx->d_stream_save;
+                f.nsteps = streamed;
+                f.last = streamed & 1;
+                CK(launch_settle<Real>(f, ctx->sms, ctx->stream));
+                ctx->launches++;
+            }
             continue;
         }
         if (runs && clamped && left >= 2) {
@@ -1005,7 +1053,7 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
     const size_t bytes = (size_t)cfg->max_blocks * kBS3 * ctx->rsize;
     if (cudaMalloc(&ctx->phi[0], bytes) != cudaSuccess || cudaMalloc(&ctx->phi[1], bytes) != cudaSuccess ||
         cudaMalloc(&ctx->pw, bytes) != cudaSuccess || cudaMalloc(&ctx->pg, bytes) != cudaSuccess ||
-        cudaMalloc(&ctx->d_nan, 4 * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&ctx->d_nan, 8 * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&ctx->d_meta, (size_t)cfg->max_blocks * kBS3 * sizeof(unsigned short)) != cudaSuccess) {
         cudaGetLastError();
         return bail(GBFK_E_OOM);
@@ -1014,7 +1062,7 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
     cudaMemset(ctx->phi[1], 0, bytes);
     cudaMemset(ctx->pw, 0, bytes);
     cudaMemset(ctx->pg, 0, bytes);
-    cudaMemset(ctx->d_nan, 0, 4 * sizeof(unsigned));
+    cudaMemset(ctx->d_nan, 0, 8 * sizeof(unsigned));
     if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
         return bail(GBFK_E_CUDA);
     if (ensure_table(ctx) != GBFK_OK) return bail(GBFK_E_CUDA);
@@ -1856,6 +1904,7 @@ struct Adjoint {
                 a.out = nullptr;
                 a.stores = d_table + g.table;
                 a.nsteps = g.steps;
+                a.settle = (SettleWords *)(ctx->d_nan + 4);
                 CK(launch_resident_run<Real>(a, ctx->sms, ctx->stream));
                 ctx->launches++;
                 fsteps += g.steps;
@@ -1958,7 +2007,8 @@ struct Adjoint {
 };
 
 template <typename Real>
-int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoint_result *res, void *grad_c0)
+int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoint_result *res, void *grad_c0,
+                         bool finite = true)
 {
     int rc = prepare_static<Real>(ctx, p->Dw, p->Dg);
     if (rc) return rc;
@@ -2100,7 +2150,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     // are 0 and its harmonic mean is 0), so no neighbour feeds their lambda.
     // They keep status kAdjMuZero in both sets and lambda 0.
     bool ic_clean = false;    // every empty block of the initial condition holds +0
-    bool ic_clamped = false;  // and every value of it is one of a clamped state
+    bool ic_clamped = false;  // and every value of it is one of a clamped state, none NaN
     if (e == cudaSuccess && ctx->identity_slots) {
         int *d_list = (int *)ctx->adj_mem[15];
         unsigned char *d_pos = (unsigned char *)(d_list + nb);
@@ -2141,7 +2191,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     if (!A.skip_empty) ctx->adj_clean.clear();  // full steps: nothing is tracked
     // runs with resident blocks, where the blocks fit with their adjoint state
     // (FP32 1184 on a B200, FP64 592) and nothing couples the empty ones
-    bool resident = e == cudaSuccess && A.skip_empty && ic_clamped && p->nsteps > 0 &&
+    bool resident = e == cudaSuccess && finite && A.skip_empty && ic_clamped && p->nsteps > 0 &&
                           ctx->step_pref == GBFK_STEP_AUTO && std::isfinite((double)(Real)p->Dw) &&
                           std::isfinite((double)(Real)p->Dg) && std::isfinite((double)A.rho) &&
                           resident_fits<Real>(ctx) && ctx->n_heavy <= adjoint_run_capacity<Real>(ctx->sms);
@@ -2290,12 +2340,19 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         if (e == cudaSuccess) e = ctx->staged.to_host(grad_c0, ctx->d_stage, A.fbytes, ctx->device, ctx->stream);
         ctx->launches++;
     }
+    SettleWords words = {};
+    if (resident && e == cudaSuccess)
+        e = cudaMemcpyAsync(&words, ctx->d_nan + 4, sizeof(words), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cleanup();
     if (e != cudaSuccess) return fail(ctx, GBFK_E_CUDA, "forward_adjoint: %s", cudaGetErrorString(e));
     if (resident) {
         rc = check_stage_timeout(ctx);
         if (rc) return rc;
+        if (words.nan) {  // the runs' steps are those of finite states only: once more, a launch per step
+            CK(cudaMemsetAsync(ctx->d_nan + 4, 0, sizeof(words), ctx->stream));
+            return forward_adjoint_impl<Real>(ctx, p, res, grad_c0, false);
+        }
     }
     auto nsum = [](const double *v, size_t stride, size_t count) {
         double s = 0, c = 0;

@@ -625,7 +625,13 @@ int batch_run(gbfk_batch *b, int spc)
             b->chosen_spc = -1;
             b->chosen_shape = -1;
             b->final_in_0 = true;
-            return batch_finish(b);
+            rc = batch_finish(b);
+            if (rc != GBFK_E_NAN) return rc;
+            // a run's steps are those of finite states only (a NaN would spread
+            // through CSF): once more, by launches
+            rc = batch_prepare<Real>(b);
+            if (rc) return rc;
+            b->final_in_0 = false;
         }
     }
     if (spc == -1 && b->log2_bpd < 0)

@@ -685,22 +685,7 @@ rd_levels_run_kernel(PoolView<Real> v, const Real *__restrict__ H, const unsigne
         __syncthreads();
         bool lost = false;
         if (t == 0) {
-            const unsigned target = (unsigned)(s + 1) * gridDim.x;
-            unsigned seen;
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync->arrived) : "memory");
-            unsigned long long since = 0;
-            for (unsigned n = 0;; n++) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&sync->arrived) : "memory");
-                if (seen >= target) break;
-                if ((n & 1023u) == 1023u) {
-                    const unsigned long long now = now_ns();
-                    if (!since) since = now;
-                    else if (now - since > kPollNs) {
-                        lost = true;
-                        break;
-                    }
-                }
-            }
+            lost = !arrive_and_wait(&sync->arrived, (unsigned)(s + 1) * gridDim.x, kPollNs);
         }
         if (__syncthreads_or(lost)) {
             if (t == 0) atomicOr(err_flag, kErrPoll);
@@ -1717,7 +1702,7 @@ cudaError_t upload_ghost_table()
 }
 
 // out[b]: bit 0 a cell of block b (pool order, identity slots) is > 0, bit 1 a
-// cell is negative, -0 or above 1
+// cell is negative, -0, above 1 or NaN
 template <typename Real>
 __global__ void block_any_positive_kernel(const Real *__restrict__ phi, int nblocks, unsigned char *__restrict__ out)
 {
@@ -1726,7 +1711,7 @@ __global__ void block_any_positive_kernel(const Real *__restrict__ phi, int nblo
         bool any = false, off = false;
         for (int c = threadIdx.x; c < kBS3; c += blockDim.x) {
             any |= q[c] > (Real)0;
-            off |= q[c] > (Real)1 || (signbit(q[c]) && q[c] == q[c]);
+            off |= !(q[c] <= (Real)1) || signbit(q[c]);
         }
         any = __syncthreads_or(any);
         off = __syncthreads_or(off);

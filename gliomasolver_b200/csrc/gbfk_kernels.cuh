@@ -135,6 +135,13 @@ cudaError_t launch_rd_run_tma(const PoolView<Real> &v, const BlockLists &lists, 
                               unsigned *err_flag, unsigned *flags, const CUtensorMap *maps_in0,
                               const CUtensorMap *maps_buf0, const CUtensorMap *maps_buf1, cudaStream_t s);
 
+// What a run or a chain of steps over the heavy blocks alone leaves for
+// launch_settle, all 0 between calls.
+struct SettleWords {
+    unsigned outside;  // an empty block of state 0 holds a value that is not +0
+    unsigned nan;      // a NaN in state 0 or a later one
+};
+
 // A run of nsteps steps with the heavy blocks resident in shared memory
 // (gbfk_resident.cu): any uniform grid with identity slots whose heavy blocks
 // fit (resident_capacity).  in: the output of a step (every value +0 <= phi
@@ -142,10 +149,11 @@ cudaError_t launch_rd_run_tma(const PoolView<Real> &v, const BlockLists &lists, 
 // the item indices of its six face neighbours (-1: an empty block); stores:
 // NULL (the last state goes to out, which may be in), or nsteps device
 // pointers: where the heavy blocks of state s + 1 go (NULL entries: nowhere).
-// empty: the n_empty empty blocks, whose last state goes to out (n_empty 0:
-// they are left alone).  ex: 2 * n * 384 Real and index: 2 words, both zeroed
-// once per item list and then left to the runs.  dt, Dw and Dg are finite.
-// err_flag as for the pipelined step (bits 0 and 9: a face never came).
+// empty: the n_empty empty blocks, of which the run only notes in `settle` what
+// launch_settle has to know; settle: NULL, or its words; save: NULL, or where the
+// heavy blocks of state 0 are kept, one after the other.  ex: 2 * n * 384 Real and index: 2 words,
+// both zeroed once per item list and then left to the runs.  dt, Dw and Dg are
+// finite.  err_flag as for the pipelined step (bits 0 and 9: a face never came).
 template <typename Real>
 struct ResidentArgs {
     const int *items, *nbr;
@@ -165,6 +173,8 @@ struct ResidentArgs {
     Real *ex;
     unsigned *index;
     unsigned *nan_flag, *err_flag;
+    Real *save;
+    SettleWords *settle;
     unsigned start = 0;  // resident_teams: states the exchange buffer carried before (mod 4)
     unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
 };
@@ -187,6 +197,7 @@ struct StreamArgs {
     Real rho;
     double dt, ih2;
     unsigned *nan_flag, *err_flag;
+    SettleWords *settle;
     unsigned long long neg0 = 0x8000000080000000ull;  // -0 twice (pair_mul)
 };
 constexpr int stream_face_values = 256;
@@ -196,7 +207,7 @@ template <typename Real>
 cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, const unsigned short *meta,
                                void *image, int *from, int *at, cudaStream_t s);
 template <typename Real>
-cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, cudaStream_t s);
+cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, Real *save, cudaStream_t s);
 template <typename Real>
 cudaError_t launch_stream_step(const StreamArgs<Real> &a, bool first, int sms, cudaStream_t s);
 // appends the table `nbr` of n heavy blocks of a uniform periodic bpd^3 grid
@@ -217,11 +228,32 @@ cudaError_t launch_resident_run(const ResidentArgs<Real> &a, int sms, cudaStream
 template <typename Real>
 cudaError_t launch_resident_teams(const ResidentArgs<Real> *runs, const int *off, int teams, int size, int per,
                                   double ih2, cudaStream_t s);
-// nsteps steps of the empty blocks alone, from `in` into out0 and (unless
-// NULL) out1: the company of nsteps launches that skip them.
+// Before a chain of steps over the heavy blocks: the empty blocks of state 0
+// (in) noted in `settle` and copied to the other state buffer
+// (launch_stream_faces keeps the heavy ones in `save`, one after the other).
 template <typename Real>
-cudaError_t launch_empty_run(const int *empty, int n_empty, const Real *in, Real *out0, Real *out1, int nsteps,
-                             Real rho, double dt, unsigned *nan_flag, cudaStream_t s);
+cudaError_t launch_empty_scan(const int *empty, int n_empty, const Real *in, Real *other, SettleWords *settle,
+                              unsigned *nan_flag, cudaStream_t s);
+// After a run or a chain: the empty blocks' steps where they hold more than +0;
+// where a NaN was seen, all blocks' steps from state 0 on (gbfk_resident.cu).
+// sync: two zeroed words, left zeroed.
+template <typename Real>
+struct SettleArgs {
+    int bpd, nblocks;
+    const int *items, *empty;
+    int n, n_empty;
+    const Real *H;
+    const Real *pw, *pg;
+    Real *state[2];    // state[0] holds the empty blocks of state 0; the last state goes to state[last]
+    const Real *save;  // the heavy blocks of state 0 (state[1] may hold them)
+    int nsteps, last;
+    Real rho;
+    double dt, ih2;
+    SettleWords *words;
+    unsigned *nan_flag, *err_flag, *sync;
+};
+template <typename Real>
+cudaError_t launch_settle(const SettleArgs<Real> &a, int sms, cudaStream_t s);
 
 // The same for a step of a TMCMC batch: every active sample (positions
 // 0 .. nactive-1) of one uniform 2^log2_bpd grid.  Per-position fields are
@@ -383,8 +415,8 @@ int adjoint_run_capacity(int sms);
 int adjoint_run_threads(int n, int sms);
 template <typename Real>
 cudaError_t launch_adjoint_run(const AdjRunArgs<Real> &a, bool abs_terms, int sms, cudaStream_t s);
-// out[b]: bit 0 a cell of block b (identity slots) is > 0, bit 1 a cell is no
-// value of a clamped state (+0 <= phi <= 1, or NaN)
+// out[b]: bit 0 a cell of block b (identity slots) is > 0, bit 1 a cell is not
+// in +0 <= phi <= 1
 template <typename Real>
 cudaError_t launch_block_any_positive(const Real *phi, int nblocks, unsigned char *out, cudaStream_t s);
 // dL/dphi of loss = -(L_T1c + L_FLAIR) in pool order; roi_count: NULL (every

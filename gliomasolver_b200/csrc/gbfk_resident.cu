@@ -39,9 +39,9 @@
 // Empty blocks (every cell and face-halo cell kEmpty) couple to nothing: all
 // face coefficients of a kEmpty cell are exactly 0 (the harmonic mean with a
 // zero diffusivity), so with finite values its update is the reaction alone,
-// and a heavy block's cell next to an empty block is kEmpty itself.  Their
-// cells run all steps of the call in registers (empty_blocks), usually +0 in
-// and out, and nobody waits for them.
+// and a heavy block's cell next to an empty block is kEmpty itself.  They
+// usually hold +0, which stays; what else they hold, and a NaN, which does
+// couple them, is settled after the run (settle_kernel).
 #include "gbfk_resident.cuh"
 
 namespace gbfk {
@@ -75,41 +75,124 @@ __device__ __forceinline__ Real empty_cell_steps(Real phi, int nsteps, Real rho,
     return phi;
 }
 
-// The empty blocks of a run of nsteps steps: state 0 from in, the last state
-// into out0 (and out1, when given), by every thread of the grid.
+// Whether the empty blocks hold anything but +0 in state 0, noted in `settle` by
+// every thread of the grid; other: NULL, or the state buffer that gets them too.
 template <typename Real>
-__device__ __forceinline__ void empty_blocks(const int *empty, int n_empty, const Real *in, Real *out0, Real *out1,
-                                             int nsteps, Real rho, double dt, unsigned *nan_flag)
+__device__ __forceinline__ void scan_empty(const int *empty, int n_empty, const Real *in, Real *other,
+                                           SettleWords *settle, unsigned *nan_flag)
 {
     const int groups = gridDim.x * (blockDim.x >> 7), g = blockIdx.x * (blockDim.x >> 7) + (threadIdx.x >> 7);
     const int c = (threadIdx.x & 127) * 4;
-    bool bad = false;
+    bool any = false, bad = false;
     for (int i = g; i < n_empty; i += groups) {
         const int64_t at = (int64_t)empty[i] * kBS3 + c;
         Real v[4];
         ld_cells(in + at, v);
-        bool any = false;
 #pragma unroll
-        for (int q = 0; q < 4; q++) any |= v[q] != (Real)0;
-        if (any) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                v[q] = empty_cell_steps(v[q], nsteps, rho, dt);
-                bad |= v[q] != v[q];
-            }
+        for (int q = 0; q < 4; q++) {
+            any |= v[q] != (Real)0;
+            bad |= v[q] != v[q];
         }
-        if (any || out0 != in) st_cells(out0 + at, v);
-        if (out1 && (any || out1 != in)) st_cells(out1 + at, v);
+        if (other) st_cells(other + at, v);
     }
-    if (bad) atomicOr(nan_flag, 1u);
+    if (any) settle->outside = 1;
+    if (bad) {
+        settle->nan = 1;
+        atomicOr(nan_flag, 1u);
+    }
 }
 
 template <typename Real>
-__global__ void __launch_bounds__(256) empty_run_kernel(const int *empty, int n_empty, const Real *in, Real *out0,
-                                                        Real *out1, int nsteps, Real rho, double dt,
-                                                        unsigned *nan_flag)
+__global__ void __launch_bounds__(256) empty_scan_kernel(const int *empty, int n_empty, const Real *in, Real *other,
+                                                         SettleWords *settle, unsigned *nan_flag)
 {
-    empty_blocks(empty, n_empty, in, out0, out1, nsteps, rho, dt, nan_flag);
+    scan_empty(empty, n_empty, in, other, settle, nan_flag);
+}
+
+// After a run or a chain of steps over the heavy blocks.  With every empty block
+// at +0 (every tumour inside the anatomy) and no NaN there is nothing to do, and
+// a launch that finds that out costs a call about 3 us.  Else, without a NaN, the
+// empty blocks' cells take their steps here, each by itself: a coefficient of 0
+// times a finite neighbour is 0.  A NaN does cross such a face into a cell that
+// is inside the domain (phi > 0), and stays out of one that is not, which the
+// kernels before this one do not tell apart; a NaN stays a NaN, so the last state
+// shows that there was one, and all steps of the call are taken again from state
+// 0 over all blocks, each cell by the expressions as they are written.
+template <typename Real>
+__global__ void __launch_bounds__(512, 1) settle_kernel(const __grid_constant__ SettleArgs<Real> a)
+{
+    constexpr unsigned long long kSettleNs = 10000000000ull;  // the longest any CTA is behind, by far
+    __shared__ SettleWords w;
+    const int t = threadIdx.x;
+    if (t == 0) {
+        w.outside = *(volatile unsigned *)&a.words->outside;
+        w.nan = *(volatile unsigned *)&a.words->nan;
+    }
+    __syncthreads();
+    if (!w.outside && !w.nan) return;
+    const int64_t threads = (int64_t)gridDim.x * blockDim.x, me = (int64_t)blockIdx.x * blockDim.x + t;
+    bool bad = false, lost = false, ok = true;
+    if (!w.nan) {
+        for (int64_t i = me; i < (int64_t)a.n_empty * kBS3; i += threads) {
+            Real *p = a.state[a.last] + (int64_t)a.empty[i >> 9] * kBS3 + (i & 511);
+            if (*p != (Real)0) *p = empty_cell_steps(*p, a.nsteps, a.rho, a.dt);
+        }
+    } else {
+        Real *here = a.state[0], *there = a.state[1];
+        unsigned waits = 0;
+        auto grid_sync = [&] {  // false: someone never came
+            __threadfence();
+            __syncthreads();
+            waits++;
+            if (t == 0) lost = !arrive_and_wait(a.sync, waits * gridDim.x, kSettleNs);
+            return !__syncthreads_or(lost);
+        };
+        for (int64_t i = me; i < (int64_t)a.n * kBS3; i += threads)
+            __stcg(here + (int64_t)(a.items[i >> 9] >> 2) * kBS3 + (i & 511), a.save[i]);
+        for (int s = 0; s < a.nsteps && ok; s++) {
+            ok = grid_sync();
+            for (int64_t i = me; ok && i < (int64_t)a.nblocks * kBS3; i += threads) {
+                const int blk = (int)(i >> 9), c = (int)i & 511, x = c & 7, y = (c >> 3) & 7, z = c >> 6;
+                const Real phi = __ldcg(here + i);
+                Real dphidt = (Real)0.;
+                if (in_domain(a.pw[i], a.pg[i], phi)) {
+                    auto across = [&](int f, int in) { return (int64_t)block_across(a.bpd, blk, f) * kBS3 + in; };
+                    const int64_t at[6] = {x ? i - 1 : across(0, c + 7), x < 7 ? i + 1 : across(1, c - 7),
+                                           y ? i - 8 : across(2, c + 56), y < 7 ? i + 8 : across(3, c - 56),
+                                           z ? i - 64 : across(4, c + 448), z < 7 ? i + 64 : across(5, c - 448)};
+                    Real phn[6];
+                    bool low[6];
+#pragma unroll
+                    for (int k = 0; k < 6; k++) {
+                        phn[k] = __ldcg(here + at[k]);
+                        low[k] = domain_chf(phn[k], a.pw[at[k]], a.pg[at[k]]) < (Real)0.1;
+                    }
+                    const Real *h = a.H + (int64_t)blk * kFacesPerBlock;
+                    const int rx = (z * 8 + y) * 9 + x, ry = 576 + (z * 9 + y) * 8 + x, rz = 1152 + (z * 8 + y) * 8 + x;
+                    dphidt = cell_rhs_flags<Real>(h[rx], h[rx + 1], h[ry], h[ry + 8], h[rz], h[rz + 64], low, phn, phi,
+                                                  a.rho, a.ih2);
+                }
+                const Real next = cell_update(phi, dphidt, a.dt);
+                bad |= next != next;
+                __stcg(there + i, next);
+            }
+            Real *const next = here;
+            here = there;
+            there = next;
+        }
+        if (ok && here != a.state[a.last]) {
+            ok = grid_sync();
+            for (int64_t i = me; ok && i < (int64_t)a.nblocks * kBS3; i += threads) __stcg(there + i, __ldcg(here + i));
+        }
+    }
+    if (bad) atomicOr(a.nan_flag, 1u);
+    if (!ok && t == 0) atomicOr(a.err_flag, kErrPoll);
+    // the last CTA to leave readies the words for the next call
+    __syncthreads();
+    if (t == 0 && atomicAdd(a.sync + 1, 1u) == gridDim.x - 1) {
+        a.sync[0] = a.sync[1] = 0;
+        *a.words = SettleWords{};
+    }
 }
 
 // One run: the blocks of CTA c of G, from state 0 (a.in) to state a.nsteps;
@@ -174,6 +257,7 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
         ld_cells(a.in + blk * kBS3 + t * kC, p);
         TL::template store<kRows>(b.st[0].phi, w.tp, p);
         publish(item, p, k0);
+        if (a.save) st_cells(a.save + (int64_t)item * kBS3 + t * kC, p);
         if (t == 0) b.e = e;
         if (t < 6) {
             const int nb = a.nbr[item * 6 + t];
@@ -270,7 +354,10 @@ __device__ __forceinline__ bool run_blocks(const ResidentArgs<Real> &a, double i
                 bool bad = false;
 #pragma unroll
                 for (int i = 0; i < kC; i++) bad |= o[i] != o[i];
-                if (bad) atomicOr(a.nan_flag, 1u);  // a NaN stays one: the last state shows it
+                if (bad) {  // a NaN stays one: the last state shows it
+                    atomicOr(a.nan_flag, 1u);
+                    if (a.settle) a.settle->nan = 1;
+                }
                 if (!kStores || !a.stores) st_cells(a.out + (int64_t)(b.e >> 2) * kBS3 + t * kC, o);
             }
             if (kStores && a.stores) {
@@ -290,8 +377,7 @@ resident_run_kernel(const __grid_constant__ ResidentArgs<Real> a)
     const unsigned k0 = *a.index;  // states stored by earlier launches (mod 4)
     const int c = blockIdx.x, G = gridDim.x;
     run_blocks<Real, kC, kGroups, true>(a, a.ih2, a.neg0, reinterpret_cast<ResidentBlock<Real> *>(smem_raw), c, G, k0);
-    if (a.n_empty > 0)
-        empty_blocks(a.empty, a.n_empty, a.in, a.out, (Real *)nullptr, a.nsteps, a.rho, a.dt, a.nan_flag);
+    if (a.n_empty > 0) scan_empty(a.empty, a.n_empty, a.in, (Real *)nullptr, a.settle, a.nan_flag);
     // the last CTA to leave advances the state count for the next launch
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -445,13 +531,19 @@ cudaError_t launch_resident_teams(const ResidentArgs<Real> *runs, const int *off
 }
 
 template <typename Real>
-cudaError_t launch_empty_run(const int *empty, int n_empty, const Real *in, Real *out0, Real *out1, int nsteps,
-                             Real rho, double dt, unsigned *nan_flag, cudaStream_t s)
+cudaError_t launch_empty_scan(const int *empty, int n_empty, const Real *in, Real *other, SettleWords *settle,
+                              unsigned *nan_flag, cudaStream_t s)
 {
     if (n_empty <= 0) return cudaSuccess;
     const int grid = (n_empty + 1) / 2 < 148 * 8 ? (n_empty + 1) / 2 : 148 * 8;
-    empty_run_kernel<Real><<<grid, 256, 0, s>>>(empty, n_empty, in, out0, out1, nsteps, rho, dt, nan_flag);
+    empty_scan_kernel<Real><<<grid, 256, 0, s>>>(empty, n_empty, in, other, settle, nan_flag);
     return cudaGetLastError();
+}
+
+template <typename Real>
+cudaError_t launch_settle(const SettleArgs<Real> &a, int sms, cudaStream_t s)
+{
+    return launch_coop<settle_kernel<Real>>(sms, 512, 0, s, a);
 }
 
 template double resident_step_us<float>(int);
@@ -464,9 +556,11 @@ template cudaError_t launch_resident_teams<float>(const ResidentArgs<float> *, c
                                                   cudaStream_t);
 template cudaError_t launch_resident_teams<double>(const ResidentArgs<double> *, const int *, int, int, int, double,
                                                    cudaStream_t);
-template cudaError_t launch_empty_run<float>(const int *, int, const float *, float *, float *, int, float, double,
-                                             unsigned *, cudaStream_t);
-template cudaError_t launch_empty_run<double>(const int *, int, const double *, double *, double *, int, double,
-                                              double, unsigned *, cudaStream_t);
+template cudaError_t launch_empty_scan<float>(const int *, int, const float *, float *, SettleWords *, unsigned *,
+                                              cudaStream_t);
+template cudaError_t launch_empty_scan<double>(const int *, int, const double *, double *, SettleWords *, unsigned *,
+                                               cudaStream_t);
+template cudaError_t launch_settle<float>(const SettleArgs<float> &, int, cudaStream_t);
+template cudaError_t launch_settle<double>(const SettleArgs<double> &, int, cudaStream_t);
 
 }  // namespace gbfk

@@ -26,6 +26,24 @@ __device__ __forceinline__ unsigned long long now_ns()
     return t;
 }
 
+// One thread's wait until `arrived` counts `target` arrivals (its own among
+// them); false when that took longer than limit_ns.
+__device__ __forceinline__ bool arrive_and_wait(unsigned *arrived, unsigned target, unsigned long long limit_ns)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+    unsigned long long since = 0;
+    for (unsigned n = 0;; n++) {
+        unsigned seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
+        if (seen >= target) return true;
+        if ((n & 1023u) == 1023u) {
+            const unsigned long long now = now_ns();
+            if (!since) since = now;
+            else if (now - since > limit_ns) return false;
+        }
+    }
+}
+
 // ---- words of the exchange buffer -----------------------------------------
 // N consecutive values in 16-, 8- or 4-byte accesses, each value one relaxed
 // access of its own (no order among them is needed: each carries its phase)
@@ -225,9 +243,11 @@ struct alignas(16) ResidentState {
 //             opposite coefficient (for a kEmpty cell itself, whose
 //             coefficients are all 0, whatever is doubled stays 0, and its
 //             formula leaves +0 where phi is +0 and the reaction where it is
-//             not, so that its domain test needs no branch unless the result
-//             is NaN).  -0 for +0 in the flux sums gives the same sums:
-//             (+0) + (-0) = +0 either way;
+//             not, so that its domain test needs no branch).  -0 for +0 in
+//             the flux sums gives the same sums: (+0) + (-0) = +0 either way.
+//             With a NaN among the neighbours that formula gives NaN where the
+//             test keeps +0: the steps of a state with a NaN in it are not
+//             these kernels' (see settle_kernel);
 //   kGeneral  kOther cells or neighbours, or a coefficient that is negative
 //             by itself: the tests as written, p_w and p_g from global memory;
 //   kStill    kEmpty cells that hold +0, which stay so: nothing flows into a
@@ -504,18 +524,6 @@ __device__ __forceinline__ void row_cells(const Args &a, double ih2, unsigned lo
             const Real q = clamp_state(to_real<Real>(__dadd_rn(phid, __dmul_rn(a.dt, (double)dphidt))));
             out[i + j] = dom[j] ? q : ph[j];  // outside the domain a clamped value stays (dt is finite)
         }
-        // kEdge takes every cell for one inside the domain, which a kEmpty cell
-        // at +0 is not: with finite values its formula leaves +0, but a NaN
-        // neighbour gives NaN through a coefficient of 0 too.  So a new value
-        // that is NaN goes through the domain test as it is written.
-        if constexpr (kKind == kEdge) {
-            if (out[i] != out[i] || out[i + 1] != out[i + 1]) {
-                const int64_t c = (int64_t)(b.e >> 2) * kBS3 + w.t * kC + i;
-#pragma unroll
-                for (int j = 0; j < 2; j++)
-                    if (!in_domain(a.pw[c + j], a.pg[c + j], ph[j])) out[i + j] = ph[j];
-            }
-        }
         if (i + 2 < kC) asm volatile("" ::: "memory");
     }
 }
@@ -542,8 +550,10 @@ cudaError_t raise_smem()
 template <auto kernel, typename... Args>
 cudaError_t launch_coop(int ctas, int threads, size_t smem, cudaStream_t s, Args... args)
 {
-    const cudaError_t e = raise_smem<kernel>();
-    if (e != cudaSuccess) return e;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = raise_smem<kernel>();
+        if (e != cudaSuccess) return e;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(threads);

@@ -297,9 +297,7 @@ __device__ __forceinline__ Real adj_mu(const AdjRunArgs<Real> &a, const AdjForwa
     const bool pass = fw.pass >> i & 1u, dom = fw.dom >> i & 1u;
     const Real mv = pass ? lam : (Real)0;
     const double mvd = (double)mv, phd = (double)ph;
-    // without pass mu is 0 and so is the self term; its factor may be NaN
-    // then: kEdge and kPlain take a NaN cell for one inside the domain
-    self = dom && pass ? mvd * fw.factor[i] : 0.;
+    self = dom ? mvd * fw.factor[i] : 0.;
     if (dom && pass) {
         // dt and 1 / Dw are the caller's factors of the sums
         const double tr = mvd * (phd * (1. - phd));

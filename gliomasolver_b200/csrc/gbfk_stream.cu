@@ -1,8 +1,9 @@
 // One RD step of the heavy blocks of a uniform periodic grid that does not fit
 // the SMs' shared memory, for calls of several steps (any number of blocks per
-// direction).  The empty blocks' steps are made up elsewhere
-// (launch_empty_run): nothing couples them to the others.  Results are
-// bit-identical to the other steps.
+// direction).  The empty blocks' steps are made up afterwards (launch_settle):
+// nothing couples them to the others while every value is finite, and with a
+// NaN all steps are taken again there.  Results are bit-identical to the other
+// steps.
 //
 // A persistent CTA per SM; each group of 128 threads takes blocks of its own,
 // four x-consecutive cells per thread, and computes them as the resident runs
@@ -100,11 +101,13 @@ __device__ __forceinline__ void put_faces(Real *faces, int t, const Real (&o)[kC
 }
 
 template <typename Real>
-__global__ void __launch_bounds__(kThreads) stream_faces_kernel(const int *items, const Real *phi, Real *faces)
+__global__ void __launch_bounds__(kThreads) stream_faces_kernel(const int *items, const Real *phi, Real *faces,
+                                                                Real *save)
 {
     Real o[kCells];
     ld_cells(phi + (int64_t)(items[blockIdx.x] >> 2) * kBS3 + threadIdx.x * kCells, o);
     put_faces(faces + (int64_t)blockIdx.x * stream_face_values, threadIdx.x, o);
+    st_cells(save + (int64_t)blockIdx.x * kBS3 + threadIdx.x * kCells, o);
 }
 
 template <typename Real>
@@ -221,7 +224,10 @@ stream_step_kernel(const __grid_constant__ StreamArgs<Real> a)
 #pragma unroll
         for (int q = 0; q < kCells; q++) bad |= o[q] != o[q];
     }
-    if (bad) atomicOr(a.nan_flag, 1u);
+    if (bad) {
+        atomicOr(a.nan_flag, 1u);
+        a.settle->nan = 1;
+    }
     if (lost && t == 0) {
         atomicOr(a.err_flag, kErrStream);
         // the copies in flight land before the CTA's shared memory goes away
@@ -248,10 +254,10 @@ cudaError_t launch_stream_pack(const int *items, int n, int bpd, const Real *H, 
 }
 
 template <typename Real>
-cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, cudaStream_t s)
+cudaError_t launch_stream_faces(const int *items, int n, const Real *phi, Real *faces, Real *save, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    stream_faces_kernel<Real><<<n, kThreads, 0, s>>>(items, phi, faces);
+    stream_faces_kernel<Real><<<n, kThreads, 0, s>>>(items, phi, faces, save);
     return cudaGetLastError();
 }
 
@@ -283,8 +289,8 @@ template cudaError_t launch_stream_pack<float>(const int *, int, int, const floa
                                                int *, int *, cudaStream_t);
 template cudaError_t launch_stream_pack<double>(const int *, int, int, const double *, const unsigned short *, void *,
                                                int *, int *, cudaStream_t);
-template cudaError_t launch_stream_faces<float>(const int *, int, const float *, float *, cudaStream_t);
-template cudaError_t launch_stream_faces<double>(const int *, int, const double *, double *, cudaStream_t);
+template cudaError_t launch_stream_faces<float>(const int *, int, const float *, float *, float *, cudaStream_t);
+template cudaError_t launch_stream_faces<double>(const int *, int, const double *, double *, double *, cudaStream_t);
 template cudaError_t launch_stream_step<float>(const StreamArgs<float> &, bool, int, cudaStream_t);
 template cudaError_t launch_stream_step<double>(const StreamArgs<double> &, bool, int, cudaStream_t);
 

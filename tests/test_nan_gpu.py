@@ -1,7 +1,8 @@
 """Where a NaN goes: every way of taking several steps leaves it in the same
 cells as the one-CTA-per-block kernel, which evaluates the domain test
-p_w + p_g + phi > 0 of every cell as it is written (a CSF cell at +0 is outside
-the domain and keeps its +0 next to a NaN)."""
+p_w + p_g + phi > 0 of every cell as it is written: a CSF cell at +0 is outside
+the domain and keeps its +0 next to a NaN, one with phi > 0 is inside and
+becomes NaN through a coefficient of 0."""
 import numpy as np
 import pytest
 
@@ -13,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 def layered(n, seed, prec, thin=False):
     """p_w, p_g, phi: tissue cut into rooms by CSF sheets one to three cells
-    thick, a corner of CSF (whole blocks of it from 32^3 on), phi in the
+    thick, a corner of CSF (empty blocks in it from 32^3 on), phi in the
     tissue only, NaN in tissue cells of one room in front of a sheet; with
     `thin` also cells whose p_w + p_g is below 0.1."""
     R = np.float64 if prec == "f64" else np.float32
@@ -27,7 +28,7 @@ def layered(n, seed, prec, thin=False):
         tissue[:, :, at:at + width] = False
         tissue[at:at + width, :, :] &= rng.random((width, n, n)) < 0.5
         at += width + 6
-    tissue[: n // 2, : n // 2, : n // 2] = False
+    tissue[: 3 * n // 4, : 3 * n // 4, : 3 * n // 4] = False
     pw = np.where(tissue, rng.uniform(0.3, 0.7, tissue.shape), 0.0)
     pg = np.where(tissue, 1.0 - pw, 0.0)
     if thin:
@@ -76,6 +77,75 @@ def test_nan_beside_csf_in_steps_over_the_heavy_blocks(gbfk_lib, prec, n):
     same_as_block_steps(n, prec, layered(n, n, prec), (8, 13), "pipelined")
 
 
+def outside(fields, kind, seed=0):
+    """The same with values in the CSF too, whole blocks of it among them:
+    positive ones ("positive"), a NaN at the border of an empty block and of
+    the CSF block beside it, each with a positive neighbour across ("nan"), or
+    both."""
+    pw, pg, phi = (f.copy() for f in fields)
+    rng = np.random.default_rng(seed)
+    csf = pw + pg == 0
+    if kind != "nan":
+        phi[csf & (rng.random(phi.shape) < 0.7)] = 0.37
+    if kind != "positive":
+        phi[8, 8, 8], phi[8, 8, 7], phi[8, 8, 9] = np.nan, 0.2, 0.2
+        phi[7, 12, 12], phi[8, 12, 12], phi[9, 12, 12] = np.nan, 0.2, 0.2
+    if kind == "nan":
+        phi[~csf] = np.nan_to_num(phi[~csf])
+    return pw, pg, phi
+
+
+@pytest.mark.parametrize("kind", ["positive", "nan", "both"])
+@pytest.mark.parametrize("prec,n", [("f32", 32), ("f64", 48), ("f32", 104), ("f64", 72)])
+def test_nan_and_tumour_in_empty_blocks_of_a_resident_run(gbfk_lib, prec, n, kind):
+    """A NaN crosses between an empty block and its neighbours through the
+    cells that are inside the domain (phi > 0), both ways."""
+    same_as_block_steps(n, prec, outside(layered(n, n, prec), kind), (8, 13, 40), "run")
+
+
+@pytest.mark.parametrize("kind", ["positive", "nan", "both"])
+@pytest.mark.parametrize("prec,n", [("f32", 152), ("f64", 120)])
+def test_nan_and_tumour_in_empty_blocks_of_streamed_steps(gbfk_lib, prec, n, kind):
+    same_as_block_steps(n, prec, outside(layered(n, n, prec), kind), (8, 13), "pipelined")
+
+
+@pytest.mark.parametrize("n,used", [(32, "run"), (152, "pipelined")])
+def test_nan_that_arises_in_a_run_with_tumour_in_empty_blocks(gbfk_lib, n, used):
+    """Coefficients whose sum over six faces overflows: a cell with six tissue
+    neighbours falls to 0 in the first step and to inf * 0 in the second."""
+    pw, pg, phi = layered(n, n, "f32")
+    tissue = pw + pg > 0
+    pw, pg = tissue.astype(np.float32), np.zeros_like(pg)
+    phi = np.where(tissue, np.float32(0.5), np.float32(0.37))
+    with _pool(n, "f32", (pw, pg, phi)) as a, _pool(n, "f32", (pw, pg, phi)) as b:
+        b.step_kernel = "block"
+        for steps in (1, 1, 8, 9):
+            for p in (a, b):
+                p.upload_dense("phi", phi)
+                p.rd_step(6.2e37, 6.2e36, 0.05, 1e-3, steps)
+            got, want = a.download_dense("phi"), b.download_dense("phi")
+            assert np.array_equal(got, want, equal_nan=True), steps
+            assert np.isnan(want).any() == (steps > 1)
+        assert a.step_kernel == used
+
+
+@pytest.mark.parametrize("kind", ["nan", "both"])
+def test_gradient_with_nan_in_an_empty_block(gbfk_lib, kind):
+    n, steps = 32, 10
+    pw, pg, phi = outside(layered(n, 3, "f32"), kind)
+    rng = np.random.default_rng(1)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
+    s = make_schedule(0.2, 0.1, 100.0, 25.6, n // 8, "f32")
+    out = {}
+    with _pool(n, "f32", (pw, pg, phi)) as pool:
+        pool.set_observations(t1, fl)
+        for k in ("pipelined", "auto"):
+            pool.step_kernel = k
+            out[k] = pool.forward_adjoint(s.Dw, s.Dg, s.rho, min(s.dt, 0.2), steps, sigma=0.0, nsnapshots=4,
+                                          grad_c0=True, t1_uc=0.7, t2_uc=0.25, slope=2.0)
+    assert np.array_equal(out["auto"]["grad_c0"], out["pipelined"]["grad_c0"], equal_nan=True)
+
+
 @pytest.mark.parametrize("prec,bpd", [("f32", 4), ("f64", 3), ("f32", 12)])
 def test_nan_beside_csf_in_a_stage(gbfk_lib, prec, bpd):
     """Initial conditions that are NaN: everywhere in the tissue (a NaN
@@ -100,7 +170,6 @@ def test_nan_beside_csf_in_a_stage(gbfk_lib, prec, bpd):
                 b.run(kind)
             assert e.value.code == 4
             out.append([b.download(i) for i in range(4)])
-        assert b.samples_per_cta == -1
     for i, (want, got) in enumerate(zip(*out)):
         assert np.array_equal(got, want, equal_nan=True), i
         assert np.isnan(want).any() == (i in (1, 2))
