@@ -84,9 +84,11 @@ struct gbfk_batch {
     int chosen_shape = -1;       // pipelined kernel: launch shape code (-1: the default)
     int graph_launches = 0;      // CUDA graphs the last run replayed
     bool ran = false;            // the samples hold their final states
-    // the last run left every final state in phi_all[0] (resident runs) rather
-    // than by the parity of its step count
-    bool final_in_0 = false;
+    // the state buffer that the last run left every final state in (resident
+    // runs; of a sample without steps in phi_all[0]), -1: by the parity of its
+    // step count
+    int final_in = -1;
+    bool ic_clamped = true;      // every initial value is +0 <= phi <= 1 or NaN
     // resident runs: the runs, the teams' offsets, the neighbour tables and
     // the exchange buffers (one allocation), the SM count, and per anatomy its
     // heavy block count
@@ -133,6 +135,13 @@ int bfail(gbfk_batch *b, int code, const char *fmt, ...)
             return bfail(b, e_ == cudaErrorMemoryAllocation ? GBFK_E_OOM : GBFK_E_CUDA, "%s: %s (%s:%d)", \
                          #call, cudaGetErrorString(e_), __FILE__, __LINE__);                              \
     } while (0)
+
+// Which of the two state buffers holds a sample's final state.
+int final_buffer(const gbfk_batch *b, int sample)
+{
+    const int nsteps = b->params[sample].nsteps;
+    return b->final_in < 0 ? nsteps & 1 : nsteps > 0 ? b->final_in : 0;
+}
 
 template <typename Real>
 PoolView<Real> batch_pool(gbfk_batch *b)
@@ -308,6 +317,10 @@ int batch_prepare(gbfk_batch *b)
             boff[k + 1] = bcell.size();
         }
     }
+    // the smoothed ball's profile is slightly negative where psi rounds to 1
+    b->ic_clamped = true;
+    for (const Real v : bval)
+        if (std::signbit(v) || v > (Real)1) b->ic_clamped = false;
     const size_t nball = bcell.size();
     const size_t val_off = (nball * sizeof(int64_t) + 255) & ~(size_t)255;
     if (nball) {
@@ -461,12 +474,16 @@ TeamPlan plan_teams(const std::vector<int> &steps, const std::vector<int> &block
 
 // All samples to their horizons as resident runs, in place in phi_all[0]
 // (whose empty blocks hold the +0 of the initial condition, their final
-// value).  ran: false when the samples do not fit or a coefficient is not
-// finite; nothing has been launched then.
+// value), or, when an initial value is not one that a step leaves (whose sign
+// the runs take for free), after a first step by a launch in phi_all[1].  ran:
+// false when the samples do not fit or a coefficient is not finite; nothing has
+// been launched then.
 template <typename Real>
-int resident_stage(gbfk_batch *b, bool &ran)
+int resident_stage(gbfk_batch *b, const BatchView<Real> &bv, bool &ran)
 {
     ran = false;
+    const int first = b->ic_clamped ? 0 : 1;
+    int nactive = 0;
     std::vector<int> pos, steps, blocks;
     for (int k = 0; k < b->nsamples; k++) {
         const gbfk_sample &p = b->params[b->order[k]];
@@ -475,9 +492,10 @@ int resident_stage(gbfk_batch *b, bool &ran)
             return GBFK_OK;
         const int n = b->h_nheavy[p.anatomy];
         if (n > resident_capacity<Real>(b->sms)) return GBFK_OK;
-        if (p.nsteps > 0 && n > 0) {  // without tissue the state stays 0
+        if (p.nsteps > 0) nactive = k + 1;  // longest first
+        if (p.nsteps > first && n > 0) {    // without tissue the state stays 0
             pos.push_back(k);
-            steps.push_back(p.nsteps);
+            steps.push_back(p.nsteps - first);
             blocks.push_back(n);
         }
     }
@@ -519,15 +537,15 @@ int resident_stage(gbfk_batch *b, bool &ran)
             r.pw = (const Real *)b->pw[a];
             r.pg = (const Real *)b->pg[a];
             r.bpd = bpd;
-            r.in = r.out = pos_field<Real>(b, b->phi_all[0], k, kBS3);
-            r.nsteps = p.nsteps;
+            r.in = r.out = pos_field<Real>(b, b->phi_all[first], k, kBS3);
+            r.nsteps = steps[i];
             r.rho = (Real)p.rho;
             r.dt = p.dt;
             r.ih2 = b->ih2;
             r.nan_flag = b->d_nan + k;
             r.err_flag = b->d_err;
             r.start = carried[a];
-            carried[a] = (carried[a] + (unsigned)p.nsteps) & 3u;
+            carried[a] = (carried[a] + (unsigned)steps[i]) & 3u;
             runs.push_back(r);
             ex_of.push_back(ex[a]);
         }
@@ -563,6 +581,7 @@ int resident_stage(gbfk_batch *b, bool &ran)
     // one graph (a stream that cannot be captured runs it directly)
     auto enqueue = [&] {
         cudaError_t e = cudaMemsetAsync(d + o_ex, 0, ex_len * sizeof(Real), b->stream);
+        if (first && e == cudaSuccess) e = launch_rd_batch_step<Real>(bv, nactive, 0, 4, b->stream);
         if (e == cudaSuccess)
             e = launch_resident_teams<Real>((const ResidentArgs<Real> *)d, (const int *)(d + o_off), plan.teams,
                                             plan.size, plan.per, b->ih2, b->stream);
@@ -588,7 +607,8 @@ int resident_stage(gbfk_batch *b, bool &ran)
     if (ge) cudaGraphExecDestroy(ge);
     if (le != cudaSuccess) return bfail(b, GBFK_E_CUDA, "batch_run: resident runs: %s", cudaGetErrorString(le));
     BK(se);
-    b->launches++;
+    b->launches += 1 + first;
+    b->final_in = first;
     ran = true;
     return GBFK_OK;
 }
@@ -612,26 +632,30 @@ int batch_run(gbfk_batch *b, int spc)
 {
     int rc = batch_prepare<Real>(b);
     if (rc) return rc;
-    b->final_in_0 = false;
+    b->final_in = -1;
+    BatchView<Real> bv;
+    bv.pool = batch_pool<Real>(b);
+    bv.samples = (const SampleView<Real> *)b->d_views;
+    bv.ih2 = b->d_ih2;
+    bv.nan_flags = b->d_nan;
     if (spc == 0) {
         // resident runs wherever the samples fit: faster than every candidate
         // of the autotuner (128^3 FP32: 2.0 us per sample-step against 3.7,
         // 64^3: 0.39 against 0.9)
         bool ran = false;
         b->ran = false;
-        rc = resident_stage<Real>(b, ran);
+        rc = resident_stage<Real>(b, bv, ran);
         if (rc) return rc;
         if (ran) {
             b->chosen_spc = -1;
             b->chosen_shape = -1;
-            b->final_in_0 = true;
             rc = batch_finish(b);
             if (rc != GBFK_E_NAN) return rc;
             // a run's steps are those of finite states only (a NaN would spread
             // through CSF): once more, by launches
             rc = batch_prepare<Real>(b);
             if (rc) return rc;
-            b->final_in_0 = false;
+            b->final_in = -1;
         }
     }
     if (spc == -1 && b->log2_bpd < 0)
@@ -641,11 +665,6 @@ int batch_run(gbfk_batch *b, int spc)
             BK(make_pool_tensor_maps(b->phi_all[q], b->max_samples * b->nblocks, (int)sizeof(Real), b->maps[q]));
         b->maps_ready = true;
     }
-    BatchView<Real> bv;
-    bv.pool = batch_pool<Real>(b);
-    bv.samples = (const SampleView<Real> *)b->d_views;
-    bv.ih2 = b->d_ih2;
-    bv.nan_flags = b->d_nan;
     const int maxsteps = b->nsamples ? b->params[b->order[0]].nsteps : 0;
     // active samples of step k: a prefix of the sorted list
     std::vector<int> sorted_steps(b->nsamples);
@@ -771,7 +790,7 @@ int batch_likelihood(gbfk_batch *b, const gbfk_likelihood_params *params, int pe
         lp.slope = p->slope;
         lp.step_pet = p->step_pet;
         lp.step_mri = p->step_mri;
-        in[s].state = (const Real *)b->phi_all[b->final_in_0 ? 0 : b->params[s].nsteps & 1] + (size_t)b->pos[s] * field;
+        in[s].state = (const Real *)b->phi_all[final_buffer(b, s)] + (size_t)b->pos[s] * field;
     }
     BK(cudaMemcpyAsync(b->d_lik_in, in.data(), in.size() * sizeof(in[0]), cudaMemcpyHostToDevice, b->stream));
     for (int s = 0; s < b->nsamples; s += most) {
@@ -978,8 +997,7 @@ int gbfk_batch_download(gbfk_batch *b, int sample, void *dense_out)
     if (b->pos.size() != (size_t)b->nsamples) return bfail(b, GBFK_E_STATE, "download: the batch has not run");
     if (!b->d_stage) BK(cudaMalloc(&b->d_stage, bytes));
     const size_t field = (size_t)b->nblocks * kBS3 * b->rsize;
-    const void *src = (const char *)b->phi_all[b->final_in_0 ? 0 : b->params[sample].nsteps & 1] +
-                      (size_t)b->pos[sample] * field;
+    const void *src = (const char *)b->phi_all[final_buffer(b, sample)] + (size_t)b->pos[sample] * field;
     if (b->precision == GBFK_F64)
         BK(launch_dense_scatter<double>((const double *)src, (double *)b->d_stage, b->n, false, b->stream));
     else

@@ -203,3 +203,47 @@ def test_steps_over_the_heavy_blocks_equal_the_block_kernel(gbfk_lib, prec, n):
         out[kind] = got
     for a, b in zip(out["auto"], out["block"]):
         assert np.array_equal(a, b)
+
+
+def _ball_value(R, x, centre):
+    """The smoothed ball's value at a cell with the centre's y and z, formed in
+    Real as the reference does."""
+    p = R(R(x) - R(centre))
+    psi = R(R(np.sqrt(R(p * p)) - R(0.005)) * R(64))
+    return R(0.5 * (float(R(R(1) - psi)) - np.sin(np.pi * float(psi)) / np.pi))
+
+
+@pytest.mark.parametrize("prec,bpd", [("f32", 8), ("f64", 8), ("f32", 6), ("f32", 12)])
+def test_stage_of_balls_with_a_negative_value_at_a_block_face(gbfk_lib, prec, bpd):
+    """The ball's profile rounds below 0 where psi is next to 1; the first cell
+    of a block is such a one, and its sign crosses the face like any other's."""
+    from gliomasolver_b200.tmcmc import Batch, StageSample, to_gbfk_samples
+
+    R = np.float64 if prec == "f64" else np.float32
+    n = 8 * bpd
+    spacing = 1 / (8 << int(np.ceil(np.log2(bpd))))
+    centres, x = [], R(16 * spacing + 0.005 + 1 / 64)
+    for _ in range(4000):
+        if _ball_value(R, 16 * spacing, x) < 0:
+            centres.append(float(x))
+        x = np.nextafter(x, R(0))
+    y = 12 * spacing
+    stage = [StageSample(0.2, 0.1, 20.0, (c, y, y)) for c in (centres[0], centres[-1])]
+    stage += [StageSample(0.1, 0.05, 9.0, (0.4, 0.3, 0.3)), stage[0]]
+    recs, _ = to_gbfk_samples(stage, bpd, prec, ic="ball")
+    pw = np.full((n, n, n), 0.7, dtype=R)
+    with Batch(bpd, len(recs), prec, max_anatomies=1) as b:
+        b.set_anatomy(0, pw, (1 - pw).astype(R))
+        for nsteps in ((0, 0, 0, 0), (1, 6, 9, 0), (2, 1, 0, 5)):
+            for r, k in zip(recs, nsteps):
+                r.nsteps = k
+            out = []
+            for kind in (1, 0):
+                b.set_samples(recs)
+                b.run(kind)
+                out.append([b.download(i) for i in range(len(recs))])
+            assert b.samples_per_cta == -1 or max(nsteps) == 0
+            if max(nsteps) == 0:
+                assert out[0][0][12, 12, 16] < 0 and out[0][0][12, 12, 15] == 0
+            for i, (want, got) in enumerate(zip(*out)):
+                assert np.array_equal(got, want), (nsteps, i)
