@@ -260,11 +260,13 @@ void release_topology(gbfk_ctx *c)
     c->topo_cap.clear();
 }
 
-// Something the face coefficients or classes depend on changed.
+// p_w, p_g or the ghost lists changed, on which the face coefficients depend,
+// and the block types and with them the step lists.
 void invalidate_static(gbfk_ctx *c)
 {
     c->static_ghosts_dirty = true;
     c->faces_valid = false;
+    c->lists_valid = false;
 }
 
 // Per-block BlockInfo::origin = index * 2^-level in Real (MRAGrid.inl:208-212).
@@ -510,7 +512,9 @@ int prepare_static(gbfk_ctx *ctx, double Dw, double Dg)
                               ctx->stream));
         ctx->launches++;
         ctx->faces_valid = true;
-        ctx->lists_valid = false;  // block types recomputed
+        // the block types depend on p_w and p_g alone: the step lists, the
+        // tables made from them and the exchange buffers stay; the images do not
+        ctx->stream_ready = false;
         ctx->faces_Dw = kDw;
         ctx->faces_Dg = kDg;
     }
@@ -519,7 +523,7 @@ int prepare_static(gbfk_ctx *ctx, double Dw, double Dg)
 
 // Work lists of the pipelined step from the block types: heavy blocks
 // (entry block * 4 + type; mixed blocks first, then tissue blocks), then
-// empty blocks (entry: block).  Rebuilt whenever the block types change.
+// empty blocks (entry: block).  Rebuilt when p_w, p_g or the topology changed.
 int build_step_lists(gbfk_ctx *ctx)
 {
     if (ctx->lists_valid) return GBFK_OK;

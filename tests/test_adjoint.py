@@ -496,3 +496,34 @@ def test_resident_sweep_equals_launches_per_step(prec, n, steps):
                     assert abs(a[key] - b[key]) <= bound + 1e-13 * abs(b[key]), key
                 if scale == 1.0 and k > 4:
                     assert a["launches"] < steps < b["launches"]
+
+
+@pytest.mark.parametrize("prec,n", [("f64", 64), ("f32", 128)])
+def test_gradient_with_new_coefficients_keeps_its_resident_sweep(gbfk_lib, prec, n):
+    """A calibration's gradients: other coefficients in every call, the same
+    anatomy; every sweep in a few launches, with the bits of a launch per step."""
+    from gliomasolver_b200 import BlockPool
+
+    R = np.float64 if prec == "f64" else np.float32
+    bpd, steps = n // 8, 30
+    pw, pg, _ = make_anatomy(n, 2)
+    rng = np.random.default_rng(n)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
+    with BlockPool(bpd ** 3, prec) as pool:
+        pool.set_uniform(bpd)
+        pool.upload_dense("p_w", pw.astype(R))
+        pool.upload_dense("p_g", pg.astype(R))
+        pool.upload_dense("phi", tumor_ic(n, (0.5, 0.45, 0.5), pw, pg).astype(R))
+        pool.set_observations(t1, fl)
+        for Dw in (0.2, 0.15, 0.1):
+            sched = make_schedule(Dw, 0.1, 100.0, L, bpd, prec)
+            out = {}
+            for kind in ("auto", "pipelined"):
+                pool.step_kernel = kind
+                before = pool.launches
+                out[kind] = pool.forward_adjoint(sched.Dw, sched.Dg, sched.rho, sched.dt, steps, sigma=0.0,
+                                                 nsnapshots=steps + 1, grad_c0=True, **UC)
+                out[kind]["launches"] = pool.launches - before
+            a, b = out["auto"], out["pipelined"]
+            assert np.array_equal(a["grad_c0"], b["grad_c0"]) and a["loss"] == b["loss"]
+            assert a["launches"] < steps < b["launches"], Dw

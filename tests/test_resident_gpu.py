@@ -247,3 +247,54 @@ def test_stage_of_balls_with_a_negative_value_at_a_block_face(gbfk_lib, prec, bp
                 assert out[0][0][12, 12, 16] < 0 and out[0][0][12, 12, 15] == 0
             for i, (want, got) in enumerate(zip(*out)):
                 assert np.array_equal(got, want), (nsteps, i)
+
+
+@pytest.mark.parametrize("prec,n", [("f32", 64), ("f64", 72), ("f32", 152)])
+def test_new_coefficients_keep_the_lists_and_a_new_anatomy_does_not(gbfk_lib, prec, n):
+    """Calls with other coefficients, then with another anatomy too, resident
+    and over the heavy blocks, against the block kernel."""
+    fields, other = _fields(n, 3, prec), _fields(n, 8, prec)
+    other[0][: n // 3] = 0
+    other[1][: n // 3] = 0
+    with _pool(n, prec, fields) as a, _pool(n, prec, fields) as b:
+        b.step_kernel = "block"
+        for k, Dw in enumerate((0.3, 0.1, 0.1, 0.22, 0.05)):
+            s = make_schedule(Dw, 0.2, 300.0, 25.6, n // 8, prec)
+            for p in (a, b):
+                if k == 3:
+                    p.upload_dense("p_w", other[0])
+                    p.upload_dense("p_g", other[1])
+                p.rd_step(s.Dw, s.Dg, s.rho, s.dt, 9, check_nan=True)
+            assert np.array_equal(a.download_dense("phi"), b.download_dense("phi")), k
+
+
+@pytest.mark.parametrize("n", [64, 72])
+def test_new_coefficients_do_not_block_the_host(gbfk_lib, n):
+    """A call with new coefficients on a known anatomy is enqueued behind 0.2 s
+    of other work on the stream without waiting for it."""
+    import time
+
+    import torch
+
+    fields = _fields(n, 1, "f32")
+    st = torch.cuda.Stream()
+    with _pool(n, "f32", fields, st.cuda_stream) as pool:
+        def step(Dw):
+            s = make_schedule(Dw, 0.1, 100.0, 25.6, n // 8, "f32")
+            pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 12)
+
+        step(0.2)
+        step(0.2)
+        pool.sync()
+        done = torch.cuda.Event()
+        t0 = time.perf_counter()
+        with torch.cuda.stream(st):
+            torch.cuda._sleep(400_000_000)  # cycles: at least 0.2 s
+        step(0.1)
+        step(0.15)
+        returned = time.perf_counter() - t0
+        done.record(st)
+        pending = not done.query()
+        pool.sync()
+        assert pending and returned < 0.1 < time.perf_counter() - t0
+        assert pool.step_kernel == "run"
