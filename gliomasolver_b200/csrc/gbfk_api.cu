@@ -714,7 +714,12 @@ int build_run_layout(gbfk_ctx *ctx, const PoolView<Real> &v)
 // step) from 3.  Steps over the heavy blocks alone (256^3: 15.7 us instead of
 // 30) cost 39 us per call (the empty blocks, the faces and state 0, the first
 // launch, launch_settle), and 51 us for the image of new coefficients.
+// A new anatomy's lists and tables cost the host 50-75 us once, on grids that
+// are no power of two, whose block kernel needs neither: even with a launch per
+// step at about 10 steps (24^3, 72^3), at 6 to 8 from 3000 blocks on (120^3 FP64
+// 8, 160^3 FP64 6); 7 and 6 here, as the next call has them.
 constexpr int kResidentSteps = 6, kResidentStepsBlock = 3, kStreamSteps = 3, kStreamStepsNew = 6;
+constexpr int kStepsNewLists = 7, kStepsNewListsLarge = 6, kLargeBlocks = 3000;
 
 template <typename Real>
 int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int nsteps, int check_nan)
@@ -738,8 +743,12 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
                            std::isfinite(dt) && std::isfinite((double)(Real)Dw) && std::isfinite((double)(Real)Dg) &&
                            std::isfinite((double)(Real)rho);
     const int clamped_steps = ctx->phi_clamped ? nsteps : nsteps - 1;
-    bool want_run = uncoupled && clamped_steps >= (pipelined ? kResidentSteps : kResidentStepsBlock);
-    bool want_stream = uncoupled && clamped_steps >= (ctx->lists_valid && ctx->stream_ready ? kStreamSteps : kStreamStepsNew);
+    const bool new_lists = !pipelined && !ctx->lists_valid;
+    const int least_new = ctx->nblocks < kLargeBlocks ? kStepsNewLists : kStepsNewListsLarge;
+    bool want_run = uncoupled && clamped_steps >= (new_lists ? least_new : pipelined ? kResidentSteps : kResidentStepsBlock);
+    bool want_stream = uncoupled && clamped_steps >= (new_lists ? least_new
+                                                      : ctx->lists_valid && ctx->stream_ready ? kStreamSteps
+                                                                                              : kStreamStepsNew);
     // the tables of either cannot be built inside a stream capture
     const bool run_ready = ctx->lists_valid && ctx->res_ready, stream_ready = ctx->lists_valid && ctx->stream_ready;
     if ((want_run && !run_ready) || (want_stream && !stream_ready)) {

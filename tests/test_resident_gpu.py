@@ -298,3 +298,18 @@ def test_new_coefficients_do_not_block_the_host(gbfk_lib, n):
         pool.sync()
         assert pending and returned < 0.1 < time.perf_counter() - t0
         assert pool.step_kernel == "run"
+
+
+def test_a_short_call_on_a_new_anatomy_builds_no_lists(gbfk_lib):
+    """Grids that are no power of two: the block kernel needs no lists, and a
+    few steps do not pay for them; where they are there, they are used."""
+    n = 72
+    fields = _fields(n, 2, "f32")
+    s = make_schedule(0.2, 0.1, 300.0, 25.6, n // 8, "f32")
+    with _pool(n, "f32", fields) as pool:
+        for upload, steps, kernel in ((False, 5, "block"), (False, 9, "run"), (False, 4, "run"), (True, 5, "block"),
+                                      (True, 12, "run"), (False, 3, "run")):
+            if upload:
+                pool.upload_dense("p_w", fields[0])
+            pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, steps)
+            assert pool.step_kernel == kernel
