@@ -772,9 +772,10 @@ int batch_likelihood(gbfk_batch *b, const gbfk_likelihood_params *params, int pe
     const int n = b->n, parts = likelihood_parts(n);
     if (b->nsamples == 0) return GBFK_OK;
     // parameters and results of every sample and the partial sums of as many
-    // as 16 MiB hold (a launch's worth), kept for the next call
+    // as 16 MiB hold (a launch's worth: a grid has at most 65535 rows), kept for
+    // the next call
     const size_t part_bytes = (size_t)parts * kLikelihoodPartBytes;
-    const int most = std::max(1, std::min(b->max_samples, (int)(((size_t)16 << 20) / part_bytes)));
+    const int most = std::max(1, std::min({b->max_samples, 65535, (int)(((size_t)16 << 20) / part_bytes)}));
     if (!b->d_partial) BK(cudaMalloc(&b->d_partial, (size_t)most * part_bytes));
     if (!b->d_lik_in) BK(cudaMalloc(&b->d_lik_in, (size_t)b->max_samples * sizeof(LikelihoodSample)));
     if (!b->d_lik) BK(cudaMalloc(&b->d_lik, (size_t)b->max_samples * 4 * sizeof(double)));

@@ -127,3 +127,32 @@ def test_batch_likelihood_equals_per_sample_likelihood(gbfk_lib, prec):
             pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, s.nsteps)
             assert np.array_equal(got[i], pool.log_likelihood(**kw)), i
     assert np.all(np.isfinite(got)) and len({tuple(r) for r in got}) == 6
+
+
+@pytest.mark.gpu
+def test_likelihoods_of_more_samples_than_a_launch_has_rows(gbfk_lib):
+    """66000 samples of an 8^3 grid, one partial sum each: two launches."""
+    from gliomasolver_b200 import _lib
+    from gliomasolver_b200.tmcmc import Batch
+
+    n, count = 8, 66000
+    rng = np.random.default_rng(5)
+    pw = np.full((n, n, n), 0.6, dtype=np.float32)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.3, 0.5))
+    recs = (_lib.Sample * count)()
+    for i, r in enumerate(recs):
+        r.Dw, r.Dg, r.rho, r.dt, r.nsteps, r.anatomy = 1e-3, 1e-4, 0.05, 1e-3, 0, 0
+        r.x0[0], r.x0[1], r.x0[2] = 0.5, 0.5, 0.1 + 0.1 * (i % 7)
+        r.sigma, r.ic = 0.2, _lib.IC_KINDS["gaussian"]
+    with Batch(1, count, "f32", max_anatomies=1) as b:
+        b.set_anatomy(0, pw, (1 - pw).astype(np.float32))
+        b.set_observations(t1, fl)
+        b.set_samples(recs)
+        b.run(0)
+        many = b.log_likelihood()
+        few = (_lib.Sample * 7)(*recs[:7])
+        b.set_samples(few)
+        b.run(0)
+        want = b.log_likelihood()
+    assert many.shape == (count, 4) and len({float(v) for v in want[:, 1]}) > 3
+    assert np.array_equal(many, want[np.arange(count) % 7])
