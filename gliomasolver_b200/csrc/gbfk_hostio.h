@@ -10,7 +10,8 @@
 // comes down in 4.0 (14.1) on a B200 host of 16 cores.  From 192^3 (28 MB) down,
 // where memory is reused without faults, the plain call is as fast or faster
 // (1.5 ms up against 2.0; 128^3: 0.51 against 0.59).  Pinned, managed and
-// device memory and captured streams take it too.  The caller's buffer is free
+// device memory and captured streams take it too, and the per-thread default
+// stream, which is another stream in every thread.  The caller's buffer is free
 // for reuse (or complete) when the call returns, as with the plain call; the
 // DMA keeps the stream's order.
 #pragma once
@@ -108,7 +109,7 @@ private:
     // threads for a copy of pageable memory; 0: the plain call
     int plan(const void *host, size_t bytes, cudaStream_t s)
     {
-        if (bytes < kSmall) return 0;
+        if (bytes < kSmall || s == cudaStreamPerThread) return 0;
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
             cudaGetLastError();

@@ -335,3 +335,26 @@ def test_copies_of_pageable_memory_round_trip(gbfk_lib, prec, cells, first):
             pool.upload("phi", a, first_cell=first)
             a[:] = -1
             assert np.array_equal(pool.download("phi", cells, first_cell=first), want)
+
+
+def test_large_copies_on_the_per_thread_default_stream(gbfk_lib):
+    """A pool on the calling thread's default stream (the handle 2): large
+    copies keep that stream's order before and after its steps."""
+    n, per_thread = 256, 2
+    rng = np.random.default_rng(3)
+    phi = rng.random((n, n, n), dtype=np.float32)
+    pw = np.full((n, n, n), 0.5, dtype=np.float32)
+    s = make_schedule(0.2, 0.05, 100.0, 25.6, n // 8, "f32")
+    out = []
+    for stream in (None, per_thread):
+        with BlockPool((n // 8) ** 3, "f32", stream=stream) as pool:
+            pool.set_uniform(n // 8)
+            for name, a in (("p_w", pw), ("p_g", pw), ("phi", np.zeros_like(phi))):
+                pool.upload_dense(name, a)
+            for _ in range(2):
+                pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 60)
+                pool.upload_dense("phi", phi)
+                pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 40)
+                out.append(pool.download_dense("phi"))
+    for got in out[1:]:
+        assert np.array_equal(got, out[0])
