@@ -761,7 +761,8 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     }
     if ((want_run || want_stream) && !pipelined) {
         rc = build_step_lists(ctx);
-        if (rc) return rc;
+        if (rc == GBFK_E_OOM) want_run = want_stream = false;  // the block kernel needs none of it
+        else if (rc) return rc;
     }
     double ih2 = 0;
     if (pipelined) {
@@ -1851,12 +1852,22 @@ struct Adjoint {
     AdjRunArgs<Real> run{};  // the arguments that all adjoint runs share
     Real *lam_out = nullptr;
     int64_t total_steps = 0;
+    // Without room for the pointer table (and no adjoint run before it) they
+    // run as a launch per step, and so does what follows (record false then).
     int resident_sweep(double rho_, double dt_)
     {
         record = false;
         std::vector<Op> todo;
         todo.swap(ops);
         const int rc = run_ops(todo, rho_, dt_);
+        if (rc == GBFK_E_OOM && asteps == 0) {
+            for (const Op &o : todo) {
+                if (o.dst) advance(o.src, o.dst, o.k);
+                else adjoint_step(o.src);
+            }
+            CK(err);
+            return GBFK_OK;
+        }
         record = true;
         return rc;
     }
@@ -2208,6 +2219,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
                           ctx->step_pref == GBFK_STEP_AUTO && std::isfinite((double)(Real)p->Dw) &&
                           std::isfinite((double)(Real)p->Dg) && std::isfinite((double)A.rho) &&
                           resident_fits<Real>(ctx) && ctx->n_heavy <= adjoint_run_capacity<Real>(ctx->sms);
+    const bool runs = resident;  // some sweep may run so
     double *run_sums = nullptr;
     const size_t ex = 2 * (size_t)ctx->n_heavy * 384 * 2 * sizeof(Real),
                  acc_bytes = resident ? (size_t)adjoint_run_threads(ctx->n_heavy, ctx->sms) * 6 * sizeof(double) : 0,
@@ -2265,6 +2277,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
                 cleanup();
                 return rc;
             }
+            resident = A.record;
         }
         A.adjoint_reads(F);
         e = A.err;
@@ -2318,7 +2331,8 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
                 cleanup();
                 return rc;
             }
-            A.LAM = A.lam_out;
+            resident = A.record;
+            if (resident) A.LAM = A.lam_out;
         }
         e = A.err;
     }
@@ -2354,12 +2368,12 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         ctx->launches++;
     }
     SettleWords words = {};
-    if (resident && e == cudaSuccess)
+    if (runs && e == cudaSuccess)
         e = cudaMemcpyAsync(&words, ctx->d_nan + 4, sizeof(words), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cleanup();
     if (e != cudaSuccess) return fail(ctx, GBFK_E_CUDA, "forward_adjoint: %s", cudaGetErrorString(e));
-    if (resident) {
+    if (runs) {
         rc = check_stage_timeout(ctx);
         if (rc) return rc;
         if (words.nan) {  // the runs' steps are those of finite states only: once more, a launch per step

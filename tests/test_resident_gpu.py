@@ -313,3 +313,68 @@ def test_a_short_call_on_a_new_anatomy_builds_no_lists(gbfk_lib):
                 pool.upload_dense("p_w", fields[0])
             pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, steps)
             assert pool.step_kernel == kernel
+
+
+class _FullDevice:
+    """Every byte of device memory that cudaMalloc still gives, down to its
+    smallest pieces, held until the end of the block."""
+
+    def __enter__(self):
+        import ctypes
+
+        self.rt = ctypes.CDLL("libcudart.so.12")
+        self.held, size = [], 1 << 36
+        while size >= 256:
+            p = ctypes.c_void_p()
+            if len(self.held) < 20000 and self.rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0:
+                self.held.append(p)
+            else:
+                self.rt.cudaGetLastError()
+                size //= 2
+        return self
+
+    def __exit__(self, *exc):
+        for p in self.held:
+            self.rt.cudaFree(p)
+
+
+def test_runs_without_room_for_their_tables_take_the_launches(gbfk_lib):
+    """No device memory left: a call of several steps on a grid that is no
+    power of two (its lists), and a gradient whose sweep got longer (its
+    pointer table), run with a launch per step, which need neither."""
+    n = 72
+    fields = _fields(n, 2, "f32")
+    s = make_schedule(0.2, 0.1, 300.0, 25.6, n // 8, "f32")
+    g = 32
+    gf = _fields(g, 2, "f32")
+    gf[2] = np.clip(gf[2], 0, 1) * (gf[0] + gf[1] > 0)
+    gs = make_schedule(0.2, 0.1, 300.0, 25.6, g // 8, "f32")
+    masks = (gf[2] > 0.2).astype(float), (gf[2] > 0.1).astype(float)
+
+    def gradient(pool, steps, kind):
+        pool.step_kernel = kind
+        return pool.forward_adjoint(gs.Dw, gs.Dg, gs.rho, 0.2 * gs.dt, steps, sigma=0.0, nsnapshots=4, grad_c0=True,
+                                    t1_uc=0.7, t2_uc=0.25, slope=2.0)
+
+    with _pool(n, "f32", fields) as warm, _pool(n, "f32", fields) as pool, _pool(g, "f32", gf) as grad:
+        grad.set_observations(*masks)
+        want_g = gradient(grad, 150, "pipelined")
+        gradient(grad, 8, "auto")  # the runs' buffers, a short table
+        warm.rd_step(s.Dw, s.Dg, s.rho, s.dt, 20)
+        assert warm.step_kernel == "run"
+        warm.step_kernel = "block"
+        warm.upload_dense("phi", fields[2])
+        warm.rd_step(s.Dw, s.Dg, s.rho, s.dt, 21)
+        want = warm.download_dense("phi")
+        pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 1)  # the coefficients, no lists
+        pool.sync()
+        with _FullDevice():
+            pool.rd_step(s.Dw, s.Dg, s.rho, s.dt, 20)
+            pool.sync()
+            kernel = pool.step_kernel
+            got_g = gradient(grad, 150, "auto")
+        assert kernel == "block"
+        assert np.array_equal(pool.download_dense("phi"), want)
+        again = gradient(grad, 150, "auto")
+    for got in (got_g, again):
+        assert np.array_equal(got["grad_c0"], want_g["grad_c0"]) and got["loss"] == want_g["loss"]
