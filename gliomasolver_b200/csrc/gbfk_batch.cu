@@ -198,7 +198,7 @@ __global__ void ball_ic_kernel(int count, const int64_t *__restrict__ cell, cons
 // Work lists of the pipelined step: per anatomy in use, its heavy blocks
 // (block * 4 + type, mixed first) and empty blocks from the block types the
 // face kernel wrote; per position its anatomy and the prefix sums of the
-// list lengths.  Call after the face kernels of batch_prepare.
+// list lengths.  Call after batch_prepare.
 int batch_lists(gbfk_batch *b)
 {
     const int nb = b->nblocks, na = b->max_anatomies, ns = b->nsamples;
@@ -405,7 +405,7 @@ int batch_prepare(gbfk_batch *b)
     b->empties_static = true;
     for (int k = 0; k < b->nsamples; k++)
         if (!std::isfinite(b->params[b->order[k]].dt)) b->empties_static = false;
-    return batch_lists(b);
+    return GBFK_OK;
 }
 
 // One step of the batch with the chosen kernel: the pipelined step
@@ -632,13 +632,20 @@ int batch_run(gbfk_batch *b, int spc)
 {
     int rc = batch_prepare<Real>(b);
     if (rc) return rc;
+    // the work lists, which the per-block kernel needs none of
+    bool lists = b->log2_bpd >= 0 || spc == 0;
+    if (lists) {
+        rc = batch_lists(b);
+        if (rc == GBFK_E_OOM && b->log2_bpd < 0) lists = false;
+        else if (rc) return rc;
+    }
     b->final_in = -1;
     BatchView<Real> bv;
     bv.pool = batch_pool<Real>(b);
     bv.samples = (const SampleView<Real> *)b->d_views;
     bv.ih2 = b->d_ih2;
     bv.nan_flags = b->d_nan;
-    if (spc == 0) {
+    if (spc == 0 && lists) {
         // resident runs wherever the samples fit: faster than every candidate
         // of the autotuner (128^3 FP32: 2.0 us per sample-step against 3.7,
         // 64^3: 0.39 against 0.9)

@@ -156,3 +156,27 @@ def test_likelihoods_of_more_samples_than_a_launch_has_rows(gbfk_lib):
         want = b.log_likelihood()
     assert many.shape == (count, 4) and len({float(v) for v in want[:, 1]}) > 3
     assert np.array_equal(many, want[np.arange(count) % 7])
+
+
+@pytest.mark.gpu
+def test_the_per_block_kernel_takes_no_work_lists(gbfk_lib):
+    """Where only the per-block kernel runs (a grid that is no power of two, one
+    sample per CTA), a run allocates nothing; the stage of runs does."""
+    import torch
+
+    from gliomasolver_b200.tmcmc import Batch
+
+    n, count = 96, 200
+    pw, pg, _ = make_anatomy(n, 0)
+    stage = sample_stage(count, pw, seed=4, tend_range=(1.0, 2.0))
+    recs, _ = to_gbfk_samples(stage, n // 8, "f32")
+    for r in recs:
+        r.nsteps = 2
+    with Batch(n // 8, count, "f32", max_anatomies=1) as b:
+        b.set_anatomy(0, pw.astype(np.float32), pg.astype(np.float32))
+        b.set_samples(recs)
+        free = [torch.cuda.mem_get_info()[0]]
+        for kind in (1, 0):
+            b.run(kind)
+            free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] == free[1] > free[2]
