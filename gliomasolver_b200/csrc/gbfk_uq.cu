@@ -93,10 +93,12 @@ struct Neumaier {
 
 // Sums of a CTA's threads, the same bits in every run: pairs (sum,
 // compensation) and whole numbers, by warp shuffles, then warp by warp through
-// shared memory; the result is thread 0's.
-template <int kPairs, int kCounts, int kWarps>
-__device__ __forceinline__ void cta_sums(Neumaier (&v)[kPairs], int (&k)[kCounts], double (&red)[kWarps][2 * kPairs],
-                                         int (&cnt)[kWarps][kCounts])
+// shared memory; the result is thread 0's, the whole numbers in `total` (a warp's
+// below 2^32).
+template <int kPairs, int kCounts, int kWarps, typename Total>
+__device__ __forceinline__ void cta_sums(Neumaier (&v)[kPairs], unsigned (&k)[kCounts],
+                                         double (&red)[kWarps][2 * kPairs], unsigned (&cnt)[kWarps][kCounts],
+                                         Total (&total)[kCounts])
 {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
 #pragma unroll
@@ -121,11 +123,13 @@ __device__ __forceinline__ void cta_sums(Neumaier (&v)[kPairs], int (&k)[kCounts
     }
     __syncthreads();
     if (t != 0) return;
+#pragma unroll
+    for (int i = 0; i < kCounts; i++) total[i] = k[i];
     for (int j = 1; j < kWarps; j++) {
 #pragma unroll
         for (int i = 0; i < kPairs; i++) v[i].merge(Neumaier{red[j][2 * i], red[j][2 * i + 1]});
 #pragma unroll
-        for (int i = 0; i < kCounts; i++) k[i] += cnt[j][i];
+        for (int i = 0; i < kCounts; i++) total[i] += cnt[j][i];
     }
 }
 
@@ -230,11 +234,11 @@ struct Bernoulli {
     }
     // the counted terms added to the sum, each count * term as an exact sum of
     // two doubles
-    static __device__ void counted(Neumaier &sum, const int *n, const double *terms)
+    static __device__ void counted(Neumaier &sum, const long long *n, const double *terms)
     {
         for (int i = 0; i < 4; i++)
             if (n[i]) {
-                const double k = n[i], p = k * terms[i];
+                const double k = (double)n[i], p = k * terms[i];
                 sum.add(p);
                 sum.add(__fma_rn(k, terms[i], -p));
             }
@@ -381,17 +385,20 @@ likelihood_partial_kernel(const LikelihoodSample *__restrict__ samples, Likeliho
         }
     }
     Neumaier v[3] = {spet, b1.rest, b2.rest};
-    int k[9] = {npet, b1.zero[0], b1.zero[1], b1.above[0], b1.above[1], b2.zero[0], b2.zero[1], b2.above[0], b2.above[1]};
+    unsigned k[9] = {(unsigned)npet,        (unsigned)b1.zero[0], (unsigned)b1.zero[1],
+                     (unsigned)b1.above[0], (unsigned)b1.above[1], (unsigned)b2.zero[0],
+                     (unsigned)b2.zero[1],  (unsigned)b2.above[0], (unsigned)b2.above[1]};
+    int total[9];
     __shared__ double red[kLikThreads / 32][6];
-    __shared__ int cnt[kLikThreads / 32][9];
-    cta_sums(v, k, red, cnt);
+    __shared__ unsigned cnt[kLikThreads / 32][9];
+    cta_sums(v, k, red, cnt, total);
     if (threadIdx.x != 0) return;
     LikelihoodPart &out = partial[(int64_t)blockIdx.y * gridDim.x + blockIdx.x];
     for (int i = 0; i < 3; i++) {
         out.sum[2 * i] = v[i].s;
         out.sum[2 * i + 1] = v[i].c;
     }
-    for (int i = 0; i < 9; i++) out.count[i] = k[i];
+    for (int i = 0; i < 9; i++) out.count[i] = total[i];
 }
 
 // The sums of the partials and the four results of sample blockIdx.x, each
@@ -409,22 +416,23 @@ likelihood_final_kernel(const LikelihoodPart *__restrict__ partial, int nparts, 
         terms[w] = Bernoulli::term(w & 3, w < 4 ? p.t1_uc : p.t2_uc, is2);
     }
     Neumaier v[3] = {};
-    int k[9] = {};
+    unsigned k[9] = {};
+    long long total[9];  // a dump grid has up to 2^34 voxels, a warp here at most a seventh of them
     for (int i = threadIdx.x; i < nparts; i += kLikThreads) {
         const LikelihoodPart &q = partial[(int64_t)blockIdx.x * nparts + i];
         for (int j = 0; j < 3; j++) v[j].merge(Neumaier{q.sum[2 * j], q.sum[2 * j + 1]});
         for (int j = 0; j < 9; j++) k[j] += q.count[j];
     }
     __shared__ double red[kLikThreads / 32][6];
-    __shared__ int cnt[kLikThreads / 32][9];
-    cta_sums(v, k, red, cnt);
+    __shared__ unsigned cnt[kLikThreads / 32][9];
+    cta_sums(v, k, red, cnt, total);
     if (threadIdx.x != 0) return;
-    Bernoulli::counted(v[1], k + 1, terms);
-    Bernoulli::counted(v[2], k + 5, terms + 4);
+    Bernoulli::counted(v[1], total + 1, terms);
+    Bernoulli::counted(v[2], total + 5, terms + 4);
     const double PI = 3.14159265358979323846;
     double lpet = 0;
     if (have_pet) {
-        const double p1 = -0.5 * (double)k[0] * log(2. * PI * p.pet_sigma2);
+        const double p1 = -0.5 * (double)total[0] * log(2. * PI * p.pet_sigma2);
         const double p2 = -0.5 * (1. / p.pet_sigma2) * (v[0].s + v[0].c);
         lpet = p1 + p2;
     }

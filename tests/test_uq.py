@@ -145,3 +145,18 @@ def test_likelihood_of_a_pool_term_by_term(gbfk_lib, prec, n, slope):
     want = [lpet, float(term(t1, t1uc)), float(term(fl, t2uc))]
     assert np.allclose(got[:3], want, rtol=1e-13, atol=0)
     assert got[3] == pytest.approx(sum(want), rel=1e-12)
+
+
+@pytest.mark.gpu
+def test_likelihood_of_more_voxels_than_an_int_counts(gbfk_lib):
+    """A 1296^3 dump grid: 2.18e9 voxels, all of them 0 and unlabelled."""
+    from gliomasolver_b200 import BlockPool
+
+    n, uc, slope = 1296, 0.25, 2.0
+    none = np.zeros((n, n, n))
+    with BlockPool(1, "f32") as pool:
+        pool.set_uniform(1)
+        pool.set_observations(none, none)
+        got = pool.log_likelihood(t1_uc=uc, t2_uc=uc, slope=slope)
+    want = float(np.longdouble(n) ** 3 * np.log1p(-np.exp(-np.longdouble(uc) ** 2 / slope) / 2))
+    assert got[1] == pytest.approx(want, rel=1e-13) and got[2] == got[1]
