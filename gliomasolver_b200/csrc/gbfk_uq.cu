@@ -225,11 +225,12 @@ struct Bernoulli {
         }
         return true;
     }
-    // the four terms: at u = 0 and above uc, by label
+    // the four terms: at u = 0 and above uc (the same for every uc: uc + 1 may
+    // round to uc), by label
     static __device__ double term(int which, double uc, double is2)
     {
         double a, b;
-        bernoulli_terms(which < 2 ? 0. : uc + 1., uc, is2, a, b);
+        bernoulli_terms(which < 2 ? 0. : 1., which < 2 ? uc : 0., is2, a, b);
         return which & 1 ? a : b;
     }
     // the counted terms added to the sum, each count * term as an exact sum of

@@ -160,3 +160,25 @@ def test_likelihood_of_more_voxels_than_an_int_counts(gbfk_lib):
         got = pool.log_likelihood(t1_uc=uc, t2_uc=uc, slope=slope)
     want = float(np.longdouble(n) ** 3 * np.log1p(-np.exp(-np.longdouble(uc) ** 2 / slope) / 2))
     assert got[1] == pytest.approx(want, rel=1e-13) and got[2] == got[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("uc", [-1e16, -1e150, -3.0, 1e16])
+def test_likelihood_with_a_threshold_that_swallows_one(gbfk_lib, uc):
+    """Thresholds next to which 1 rounds away: every voxel is above (or below) by
+    the term of that side, 1.7 and 1e17 among the values."""
+    from gliomasolver_b200 import BlockPool
+
+    n, slope = 8, 2.0
+    u = np.resize(np.array([0.0, 0.5, 1.7, 1e17 if uc < 0 else 3.0], dtype=np.float64), (n, n, n))
+    t1 = np.resize(np.array([0.0, 1.0, 1.0, 0.0, 1.0]), (n, n, n))
+    with BlockPool(1, "f64") as pool:
+        pool.set_uniform(1)
+        pool.upload_dense("phi", u)
+        pool.set_observations(t1, t1)
+        got = pool.log_likelihood(t1_uc=uc, t2_uc=uc, slope=slope)
+    d = u - uc
+    t = np.where(d > 0, 1.0, d * d) / slope
+    near, far = np.log1p(-np.exp(-t) / 2), np.log(0.5) - t
+    want = np.where(t1 == 1, np.where(d > 0, near, far), np.where(d > 0, far, near)).sum()
+    assert got[1] == pytest.approx(want, rel=1e-12)
