@@ -94,6 +94,7 @@ struct gbfk_batch {
     // heavy block count
     void *d_res = nullptr;
     size_t res_cap = 0;
+    cudaGraphExec_t res_exec = nullptr;  // the last stage's launches; the next one's are put in their place
     int sms = 0;
     std::vector<int> h_nheavy, h_list_off, h_lists;
     // observations of the likelihood step (n^3 grid) and its scratch
@@ -446,17 +447,24 @@ TeamPlan plan_teams(const std::vector<int> &steps, const std::vector<int> &block
     for (int teams = 1; teams * least <= sms && teams <= (int)steps.size(); teams++) {
         const int size = std::min(sms / teams, nmax);
         if (teams < (int)steps.size() && sms / (teams + 1) == sms / teams && (teams + 1) * least <= sms) continue;
-        auto cost = [&](int k) { return overhead + steps[k] * resident_step_us<Real>((blocks[k] + size - 1) / size); };
+        std::vector<double> cost(steps.size());
+        double longest = 0, all = 0;
+        for (size_t k = 0; k < steps.size(); k++) {
+            cost[k] = overhead + steps[k] * resident_step_us<Real>((blocks[k] + size - 1) / size);
+            longest = std::max(longest, cost[k]);
+            all += cost[k];
+        }
+        if (longest >= best_us || all >= best_us * teams) continue;  // it cannot end earlier
         std::vector<int> order(steps.size());
         std::iota(order.begin(), order.end(), 0);
-        std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return cost(i) > cost(j); });
+        std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return cost[i] > cost[j]; });
         std::vector<std::vector<int>> runs(teams);
         std::vector<std::pair<double, int>> heap;  // (time done, team), earliest first
         for (int g = 0; g < teams; g++) heap.push_back({0., g});
         double end = 0;
         for (int k : order) {
             std::pop_heap(heap.begin(), heap.end(), std::greater<>());
-            heap.back().first += cost(k);
+            heap.back().first += cost[k];
             end = std::max(end, heap.back().first);
             runs[heap.back().second].push_back(k);
             std::push_heap(heap.begin(), heap.end(), std::greater<>());
@@ -578,7 +586,8 @@ int resident_stage(gbfk_batch *b, const BatchView<Real> &bv, bool &ran)
     BK(cudaMemcpyAsync(d + o_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     BK(cudaMemcpyAsync(d + o_nbr, nbr.data(), nbr.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     BK(cudaStreamSynchronize(b->stream));
-    // one graph (a stream that cannot be captured runs it directly)
+    // one graph (a stream that cannot be captured runs it directly), put in the
+    // place of the last stage's: to instantiate and destroy one took 115 us
     auto enqueue = [&] {
         cudaError_t e = cudaMemsetAsync(d + o_ex, 0, ex_len * sizeof(Real), b->stream);
         if (first && e == cudaSuccess) e = launch_rd_batch_step<Real>(bv, nactive, 0, 4, b->stream);
@@ -589,22 +598,26 @@ int resident_stage(gbfk_batch *b, const BatchView<Real> &bv, bool &ran)
     };
     b->graph_launches = 0;
     cudaError_t le = cudaSuccess;
-    cudaGraphExec_t ge = nullptr;
     if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
         cudaGraph_t g = nullptr;
         le = enqueue();
         const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
         if (le == cudaSuccess) le = ce;
-        if (le == cudaSuccess) le = cudaGraphInstantiate(&ge, g, 0);
+        cudaGraphExecUpdateResultInfo info;
+        if (le == cudaSuccess && b->res_exec && cudaGraphExecUpdate(b->res_exec, g, &info) != cudaSuccess) {
+            cudaGetLastError();  // other launches than the last stage's
+            cudaGraphExecDestroy(b->res_exec);
+            b->res_exec = nullptr;
+        }
+        if (le == cudaSuccess && !b->res_exec) le = cudaGraphInstantiate(&b->res_exec, g, 0);
         if (g) cudaGraphDestroy(g);
-        if (le == cudaSuccess) le = cudaGraphLaunch(ge, b->stream);
+        if (le == cudaSuccess) le = cudaGraphLaunch(b->res_exec, b->stream);
         b->graph_launches = 1;
     } else {
         cudaGetLastError();
         le = enqueue();
     }
     const cudaError_t se = cudaStreamSynchronize(b->stream);
-    if (ge) cudaGraphExecDestroy(ge);
     if (le != cudaSuccess) return bfail(b, GBFK_E_CUDA, "batch_run: resident runs: %s", cudaGetErrorString(le));
     BK(se);
     b->launches += 1 + first;
@@ -916,6 +929,7 @@ int gbfk_batch_destroy(gbfk_batch *b)
     for (void *p : ptrs)
         if (p) cudaFree(p);
     b->staged.release();
+    if (b->res_exec) cudaGraphExecDestroy(b->res_exec);
     if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return GBFK_OK;
