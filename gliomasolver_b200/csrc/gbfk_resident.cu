@@ -28,13 +28,16 @@
 // No flag accompanies the data: every value of a clamped state is +0 <= phi
 // <= 1 or NaN, so the sign bit of each word is free, and it carries the
 // phase (k / 2) & 1 of the buffer's use.  A reader polls until all its words
-// show the expected phase.  Two buffers are enough: each word has one reader,
-// the thread that owns the cell across the face, and that thread writes the
-// word coming back.  A thread stores state k + 2 over state k only after it
-// has read the mirror thread's word of state k + 1, which that thread stored
-// after its own read of state k.  The phase goes on from launch to launch:
-// the state count lives in device memory (index[0]), advanced by the last CTA
-// to leave, so that a launch replayed from a graph finds it right too.
+// show the expected phase.  Two buffers are enough because of the barrier
+// between a group's polls and its stores, which every thread of the group takes:
+// a group stores state k + 1 of a block only after all its threads have read all
+// faces of state k.  So a block that has read its neighbour's state k + 1 knows
+// that the neighbour has read its own state k, over which it now stores state
+// k + 2.  (The threads that fetch a face are not those that own its cells: a
+// barrier of a warp in the place of the group's would let unread words be
+// overwritten.)  The phase goes on from launch to launch: the state count lives
+// in device memory (index[0]), advanced by the last CTA to leave, so that a
+// launch replayed from a graph finds it right too.
 //
 // Empty blocks (every cell and face-halo cell kEmpty) couple to nothing: all
 // face coefficients of a kEmpty cell are exactly 0 (the harmonic mean with a

@@ -12,11 +12,11 @@
 // travel through L2 as 64-bit words that carry their own tag: mu has any sign,
 // so a word is 32 bits of it and a step count, with one more bit that says
 // whether the cell's coefficient across that face is doubled (FP64: two words).
-// Every word has one reader, the mirror thread, which writes the word coming
-// back, so two buffers are enough (see gbfk_resident.cu).  Between launches mu,
-// self terms and flags are kept in global memory, and each thread's
-// compensated gradient sums too, so that the sums are the same bits however a
-// sweep is cut into launches.
+// Two buffers are enough because of the group's barrier between the polls of a
+// step and its stores (see gbfk_resident.cu).  Between launches mu, self terms
+// and flags are kept in global memory, and each thread's compensated gradient
+// sums too, so that the sums are the same bits however a sweep is cut into
+// launches.
 //
 // What bounds it (128^3 FP32, 8 blocks per CTA, two rounds of four groups): 250
 // warp instructions per 32 cells, 26 of them conversions between float and
