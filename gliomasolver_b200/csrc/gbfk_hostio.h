@@ -106,6 +106,15 @@ private:
 
     char *buffer(int i) const { return buffers_ + i * kChunk; }
 
+    // While another thread captures a stream (in the global mode), a thread may
+    // neither allocate nor wait for an event; the plain call does neither.  The
+    // copies touch no captured stream, so their threads are let off that.
+    struct Relaxed {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    };
+
     // threads for a copy of pageable memory; 0: the plain call
     int plan(const void *host, size_t bytes, cudaStream_t s)
     {
@@ -121,6 +130,7 @@ private:
             return 0;
         }
         if (a.type != cudaMemoryTypeUnregistered) return 0;
+        Relaxed relaxed;
         const int cores = std::max(1, (int)std::thread::hardware_concurrency() / 2);
         const int threads = (int)std::min<size_t>({(size_t)kThreads, (size_t)cores, 1 + (bytes - 1) / kPerThread});
         if (!buffers_ && cudaHostAlloc((void **)&buffers_, 2 * kThreads * kChunk, cudaHostAllocDefault) != cudaSuccess) {
@@ -149,6 +159,7 @@ private:
         for (int t = 1; t < threads; t++) {
             try {
                 pool.emplace_back([&, t] {
+                    Relaxed relaxed;
                     err[t] = cudaSetDevice(device);
                     if (err[t] == cudaSuccess) err[t] = f(t);
                 });
@@ -157,8 +168,11 @@ private:
                 break;
             }
         }
-        for (int t = 0; t < threads; t++)
-            if (mine[t]) err[t] = f(t);
+        {
+            Relaxed relaxed;
+            for (int t = 0; t < threads; t++)
+                if (mine[t]) err[t] = f(t);
+        }
         for (auto &p : pool) p.join();
         for (cudaError_t e : err)
             if (e != cudaSuccess) return e;

@@ -358,3 +358,33 @@ def test_large_copies_on_the_per_thread_default_stream(gbfk_lib):
                 out.append(pool.download_dense("phi"))
     for got in out[1:]:
         assert np.array_equal(got, out[0])
+
+
+@pytest.mark.parametrize("n", [64, 256])
+def test_an_upload_leaves_another_threads_capture_alone(gbfk_lib, n):
+    """gbfk_upload_field while another thread captures a stream in the global
+    mode, staged (its first call allocates) and plain."""
+    import ctypes
+    import threading
+
+    import torch
+
+    phi = np.random.default_rng(n).random(n ** 3, dtype=np.float32)
+    x = torch.zeros(100, device="cuda")
+    with BlockPool((n // 8) ** 3, "f32") as pool:
+        pool.set_uniform(n // 8)
+        rc, graph = [], torch.cuda.CUDAGraph()
+
+        def upload():
+            for _ in range(2):
+                rc.append(pool.lib.gbfk_upload_field(pool.ctx, 0, phi.ctypes.data_as(ctypes.c_void_p),
+                                                     ctypes.c_int64(0), ctypes.c_int64(phi.size)))
+
+        with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+            x.add_(1)
+            thread = threading.Thread(target=upload)
+            thread.start()
+            thread.join()
+        graph.replay()
+        assert rc == [0, 0] and float(x.sum()) == 100
+        assert np.array_equal(pool.download("phi", phi.size), phi)
