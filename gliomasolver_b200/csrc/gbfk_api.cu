@@ -618,6 +618,7 @@ template <typename Real>
 bool build_stream(gbfk_ctx *ctx)
 {
     if (ctx->stream_ready) return true;
+    gbfk_host::Relaxed relaxed;
     const size_t n = (size_t)ctx->n_heavy, record = stream_face_values * sizeof(Real);
     auto zeros = [&](void *faces) {  // the record after the last
         return cudaMemsetAsync((char *)faces + n * record, 0, record, ctx->stream) == cudaSuccess;
@@ -759,7 +760,10 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
             want_stream = want_stream && stream_ready;
         }
     }
+    // a launch per step needs none of these tables, nor may building them
+    // disturb another thread's capture
     if ((want_run || want_stream) && !pipelined) {
+        gbfk_host::Relaxed relaxed;
         rc = build_step_lists(ctx);
         if (rc == GBFK_E_OOM) want_run = want_stream = false;  // the block kernel needs none of it
         else if (rc) return rc;
@@ -790,8 +794,9 @@ int rd_step_impl(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
     const bool fits = (want_run || want_stream) && resident_fits<Real>(ctx);
     bool resident = want_run && fits;
     if (resident) {
+        gbfk_host::Relaxed relaxed;
         rc = build_resident<Real>(ctx);
-        if (rc == GBFK_E_OOM) resident = false;  // one launch per step needs none of it
+        if (rc == GBFK_E_OOM) resident = false;
         else if (rc) return rc;
     }
     // without room for the images, the steps run as they do for short calls

@@ -26,6 +26,17 @@
 
 namespace gbfk_host {
 
+// While another thread captures a stream (in the global mode), a thread may
+// neither allocate nor wait for its own work, or the capture is invalidated.
+// Work that touches no captured stream is let off that in the scope of this.
+struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    Relaxed(const Relaxed &) = delete;
+    Relaxed &operator=(const Relaxed &) = delete;
+};
+
 class StagedCopy {
 public:
     static constexpr size_t kChunk = (size_t)512 << 10;  // bytes of a pinned buffer
@@ -105,15 +116,6 @@ private:
     cudaEvent_t event_[2 * kThreads] = {};
 
     char *buffer(int i) const { return buffers_ + i * kChunk; }
-
-    // While another thread captures a stream (in the global mode), a thread may
-    // neither allocate nor wait for an event; the plain call does neither.  The
-    // copies touch no captured stream, so their threads are let off that.
-    struct Relaxed {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
-        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    };
 
     // threads for a copy of pageable memory; 0: the plain call
     int plan(const void *host, size_t bytes, cudaStream_t s)

@@ -378,3 +378,36 @@ def test_runs_without_room_for_their_tables_take_the_launches(gbfk_lib):
         again = gradient(grad, 150, "auto")
     for got in (got_g, again):
         assert np.array_equal(got["grad_c0"], want_g["grad_c0"]) and got["loss"] == want_g["loss"]
+
+
+@pytest.mark.parametrize("n", [64, 72, 176])
+def test_a_runs_tables_leave_another_threads_capture_alone(gbfk_lib, n):
+    """The first call of several steps on a pool (lists, exchange buffers,
+    images), made while another thread captures a stream in the global mode."""
+    import torch
+
+    fields = _fields(n, 3, "f32")
+    s = make_schedule(0.2, 0.1, 300.0, 25.6, n // 8, "f32")
+    x = torch.zeros(100, device="cuda")
+    with _pool(n, "f32", fields) as a, _pool(n, "f32", fields) as b:
+        b.step_kernel = "block"
+        a.rd_step(s.Dw, s.Dg, s.rho, s.dt, 1)
+        a.sync()
+        errors, graph = [], torch.cuda.CUDAGraph()
+
+        def steps():
+            try:
+                a.rd_step(s.Dw, s.Dg, s.rho, s.dt, 12)
+            except GbfkError as e:
+                errors.append(e)
+
+        with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+            x.add_(1)
+            thread = threading.Thread(target=steps)
+            thread.start()
+            thread.join()
+        graph.replay()
+        b.rd_step(s.Dw, s.Dg, s.rho, s.dt, 13)
+        assert not errors and float(x.sum()) == 100
+        assert a.step_kernel == ("pipelined" if n == 176 else "run")
+        assert np.array_equal(a.download_dense("phi"), b.download_dense("phi"))
