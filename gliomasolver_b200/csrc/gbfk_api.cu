@@ -1082,8 +1082,8 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
     cudaMemset(ctx->pw, 0, bytes);
     cudaMemset(ctx->pg, 0, bytes);
     cudaMemset(ctx->d_nan, 0, 8 * sizeof(unsigned));
-    if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
-        return bail(GBFK_E_CUDA);
+    ctx->sms = gbfk_host::stream_sms(cfg->device, ctx->stream);
+    if (ctx->sms <= 0) return bail(GBFK_E_CUDA);
     if (ensure_table(ctx) != GBFK_OK) return bail(GBFK_E_CUDA);
     *out = ctx;
     return GBFK_OK;

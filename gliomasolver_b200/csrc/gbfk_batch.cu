@@ -850,8 +850,8 @@ int gbfk_batch_create(const gbfk_config *cfg, int bpd, int max_samples, int max_
     };
     if (cudaSetDevice(cfg->device) != cudaSuccess) return bail(GBFK_E_CUDA);
     if (upload_ghost_table() != cudaSuccess) return bail(GBFK_E_CUDA);
-    if (cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
-        return bail(GBFK_E_CUDA);
+    b->sms = gbfk_host::stream_sms(cfg->device, (cudaStream_t)cfg->stream);
+    if (b->sms <= 0) return bail(GBFK_E_CUDA);
     if (cfg->stream) b->stream = (cudaStream_t)cfg->stream;
     else {
         if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(GBFK_E_CUDA);

@@ -16,6 +16,7 @@
 // DMA keeps the stream's order.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,6 +37,33 @@ struct Relaxed {
     Relaxed(const Relaxed &) = delete;
     Relaxed &operator=(const Relaxed &) = delete;
 };
+
+// The SMs that work on stream s of `device` may use: all of them, or its green
+// context's (launches whose CTAs wait for one another must fit them).  0 when
+// the device cannot be asked.
+inline int stream_sms(int device, cudaStream_t s)
+{
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+    if (!s || s == cudaStreamLegacy || s == cudaStreamPerThread) return n;
+    auto entry = [](const char *name) -> void * {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion(name, &p, 12040, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return p;
+        cudaGetLastError();
+        return nullptr;
+    };
+    const auto of_stream = (CUresult(*)(CUstream, CUgreenCtx *))entry("cuStreamGetGreenCtx");
+    const auto resource = (CUresult(*)(CUgreenCtx, CUdevResource *, CUdevResourceType))entry("cuGreenCtxGetDevResource");
+    CUgreenCtx green = nullptr;
+    CUdevResource r;
+    if (of_stream && resource && of_stream((CUstream)s, &green) == CUDA_SUCCESS && green &&
+        resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+        n = std::min(n, (int)r.sm.smCount);
+    return n;
+}
 
 class StagedCopy {
 public:

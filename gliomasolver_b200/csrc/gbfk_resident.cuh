@@ -564,7 +564,9 @@ cudaError_t launch_coop(int ctas, int threads, size_t smem, cudaStream_t s, Args
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch's check
+    return e;
 }
 
 }  // namespace
