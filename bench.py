@@ -61,7 +61,9 @@ def workload_config(n, precision):
                     f"topology, {(n // 8) ** 3} blocks of 8^3, {'FP32' if precision == 'f32' else 'FP64'} storage",
         "n": n, "blocks": (n // 8) ** 3, "precision": precision,
         "Dw_cm2_day": DW, "rho_day": RHO, "L_cm": L_CM, "anatomy_seed": SEED,
-        "l2": "inputs larger than L2: phi in/out + p_w + p_g = %d MB per step" % (16 * n ** 3 // 2 ** 20),
+        "l2": "no flush between steps: phi in/out + p_w + p_g are %d MB (L2: 126 MB); on AUTO a step reads only the "
+              "blocks with tissue, whose state, faces and coefficients stay mostly in L2 (roofline.traffic)"
+              % (16 * n ** 3 // 2 ** 20),
     }
 
 
@@ -136,10 +138,8 @@ def fp64_lines(stream, local, steps):
     per = sec / steps
     out["uniform_n256"] = {
         "workload": f"the headline workload in FP64: {n}^3 uniform frozen topology, {steps} steps",
-        "ms_per_step": 1e3 * per, "cell_updates_per_s": n ** 3 / per,
-        "algorithmic_gbs": 32 * n ** 3 / per / 1e9, "algorithmic_frac": 32 * n ** 3 / per / 1e9 / peak,
-        "minimum_bytes_gbs": 8 * (2 * n ** 3 + 2 * 512 * heavy) / per / 1e9,
-        "minimum_bytes_frac": 8 * (2 * n ** 3 + 2 * 512 * heavy) / per / 1e9 / peak}
+        "ms_per_step": 1e3 * per, "cell_updates_per_s": n ** 3 / per, "heavy_blocks": heavy,
+        "algorithmic_gbs": 32 * n ** 3 / per / 1e9, "algorithmic_frac": 32 * n ** 3 / per / 1e9 / peak}
     return out
 
 
@@ -351,9 +351,9 @@ def batched_stage(args, stream, local, nsamples=512, bpd=16, seed=1):
         "speedup_vs_sequential": t_seq / t_batch,
         "samples_per_cta": spc, "tile_shape": tile, "cuda_graphs": graphs, "batched_launches": batch_launches,
         "ranks": world,
-        "empty_blocks": "the batch steps the empty blocks (no tissue in them or their face halos; +0 from the "
-                        "initial condition on) once, then skips them: both state buffers hold their final +0; "
-                        "the sequential solves step every block",
+        "empty_blocks": "blocks without tissue in them or their face halos stay at the +0 of the initial condition; "
+                        "neither the batch nor the sequential solves step them (where the samples do not fit the SMs, "
+                        "the batch steps them once)",
         "timing": "CUDA events on the stream: batched = face coefficients + initial conditions + all steps; "
                   "sequential = per sample an H2D of c0, face coefficients and its steps",
     }
@@ -441,8 +441,8 @@ def adjoint_sample(stream, local, bpd=16, nsnap=64, check=True):
         "gradient_s": t_adj, "gradient_samples_per_s": 1.0 / t_adj,
         "plain_forward_s": t_fwd, "plain_forward_samples_per_s": 1.0 / t_fwd,
         "gradient_cost_in_forward_solves": t_adj / t_fwd,
-        "forward_steps_note": "the gradient's forward steps run only the blocks with tissue once every empty block "
-                              "holds its final +0; the plain forward solve steps every block",
+        "forward_steps_note": "the gradient's forward steps and the plain forward solve step only the blocks with "
+                              "tissue (an empty block keeps its +0)",
         "all_states": None if all_states is None else dict(
             all_states, gradient_cost_in_forward_solves=all_states["gradient_s"] / t_fwd),
         "loss": res["loss"], "dDw": res["dDw"], "drho": res["drho"], "dx0": list(res["dx0"]),
@@ -703,12 +703,11 @@ def gpu_arm(args):
     achieved = alg_bytes / kernel_s / 1e9
     peak, peak_kind = measured_peak()
     traffic = profiled_traffic(args.step_kernel) if (n, prec) == (N_GRID, "f32") else None
-    # the fewest bytes the exact shortcuts allow: phi in and out for every
-    # cell, p_w and p_g only for blocks with tissue in a cell or a face halo;
-    # on AUTO the other blocks' phi only once for all steps
+    # the fewest bytes a step over all blocks moves with the exact shortcuts:
+    # phi in and out for every cell, p_w and p_g only for blocks with tissue in a
+    # cell or a face halo.  AUTO keeps what it steps in L2: no such count there.
     heavy = heavy_blocks(pw, pg)
-    share = 1 / args.steps if args.step_kernel == "auto" else 1
-    min_bytes = round(word * (4 * 512 * heavy + 2 * (cells - 512 * heavy) * share))
+    min_bytes = None if args.step_kernel == "auto" else word * (2 * cells + 2 * 512 * heavy)
     roofline = {"kernel": KERNEL_NAMES[args.step_kernel, pool.step_kernel].format(real="float" if prec == "f32" else "double"),
                 # AUTO keeps the state and the coefficients in L2 between steps
                 "bound": "issue" if args.step_kernel == "auto" else "hbm", "unit": "GB/s", "peak": peak,
@@ -716,7 +715,7 @@ def gpu_arm(args):
                 "traffic": traffic, "algorithmic_bytes_per_launch": alg_bytes,
                 "algorithmic_achieved": achieved, "algorithmic_frac": achieved / peak,
                 "minimum_bytes_per_launch": min_bytes, "heavy_blocks": heavy,
-                "traffic_over_minimum": (traffic / min_bytes) if traffic else None}
+                "traffic_over_minimum": (traffic / min_bytes) if traffic and min_bytes else None}
     if traffic:
         # DRAM bytes of a warm launch (ncu) over the CUDA-event launch time: the
         # HBM fraction.  The algorithmic figure (4 words per cell-update) exceeds
@@ -848,7 +847,8 @@ def main():
     ap.add_argument("--adaptive-steps", type=int, default=400,
                     help="steps of the config-2 adaptive run on the resident drop-in (0: skip)")
     ap.add_argument("--step-kernel", default="auto", choices=["auto", "block", "pipelined", "run"],
-                    help="step kernel of the resident solve (auto: pipelined on uniform power-of-two grids)")
+                    help="step kernel of the resident solve (auto: the blocks with tissue, resident on the SMs where they "
+                         "fit, else streamed)")
     args = ap.parse_args()
     if args.warmup < 3:
         args.warmup = 3

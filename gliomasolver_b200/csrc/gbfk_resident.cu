@@ -14,14 +14,15 @@
 // What bounds it: a step is one exchange of faces through L2 (about 0.9 us
 // from a block's stores to the end of its neighbours' next step, what an 8-
 // block grid takes) plus the issue of its cells' exact-rounding arithmetic
-// (128^3, FP32, 860 blocks with tissue: 1.35 M warp instructions per step, 61 %
-// of the issue slots).
+// (128^3, FP32, 1033 heavy blocks: 1.35 M warp instructions per step, 61 % of
+// the issue slots).
 // Measured on a B200, us per step over 2000 steps, against one launch per
-// step, a brain of 18 % of its box: 64^3 FP32 1.11 (3.74), FP64 1.37 (3.85);
-// 96^3 FP32 1.32 (9.3, one CTA per block); 128^3 FP32 1.94 (6.41), FP64 3.12
-// (8.82); 160^3 FP32 3.24 (17.5, one CTA per block). A stage by teams of CTAs:
-// 128^3 FP32 1.93 us per sample-step (3.7 in launches over all samples), 64^3
-// 0.42 (0.95).
+// step, the seeded brain of 18 % of its box (64^3 182 heavy blocks, 96^3 484,
+// 128^3 1033, 160^3 1832): 64^3 FP32 1.13 (3.49), FP64 1.30 (3.86); 96^3 FP32
+// 1.30 (9.2, one CTA per block); 128^3 FP32 1.84 (6.36), FP64 2.97 (8.66); 160^3
+// FP32 3.15 (17.1, one CTA per block). A stage by teams of CTAs, setup
+// included: 128^3 FP32 1.78 us per sample-step (3.2 in launches over all
+// samples), 64^3 0.42 (0.96).
 //
 // Faces travel through L2.  After forming state k a block stores its six
 // faces in the exchange buffer k & 1 and its neighbours poll for them there.
@@ -436,13 +437,14 @@ resident_teams_kernel(const ResidentArgs<Real> *runs, const int *off, const int 
 // shorten (64^3 FP32, 2 per CTA: 1.16 us per step against 1.32 with four).
 // Beyond, four cells per thread cost fewer instructions. In FP32 a step takes
 // about 0.70 us per round of the groups over the blocks and 0.155 us per block
-// (4 blocks 1.33 us, 6 1.59, 7 1.73, 8 1.94), so the blocks go in as few
-// rounds as eight groups allow (64 registers a thread, none spilled), with no
-// more groups than those rounds need: 8 blocks 1.94 us with eight groups, 2.58
-// with seven, 2.38 with four; 9 blocks 2.58 with five, 2.76 with eight; 12
-// blocks 2.94 with six, 3.11 with eight, 3.49 with four. FP64 needs 124
-// registers for four cells: four groups (128^3: 3.07; 3.68 with seven, 4.78
-// with two cells per thread).
+// (the seeded brain scaled to fill every SM: 4 blocks 1.36 us, 6 1.69, 7 1.88, 8
+// 2.01, 9 2.57, 12 2.92), so the blocks go in as few rounds as eight groups
+// allow (64 registers a thread, none spilled), with no more groups than those
+// rounds need (on another brain, 8 blocks: 1.94 us with eight groups, 2.58 with
+// seven, 2.38 with four; 9 blocks 2.58 with five, 2.76 with eight; 12 blocks
+// 2.94 with six, 3.11 with eight, 3.49 with four). FP64 needs 126 registers for
+// four cells: four groups (128^3: 3.07; 3.68 with seven, 4.78 with two cells per
+// thread; 4 blocks 1.76, 8 3.19).
 constexpr double kRoundUs = 0.70, kBlockUs = 0.155, kRoundUs64 = 1.5;
 template <typename Real>
 int groups_for(int per, double &us)

@@ -67,7 +67,7 @@ typedef struct {
     int precision;  /* enum gbfk_precision */
     int max_blocks; /* pool capacity in blocks (slots) */
     int device;     /* CUDA device ordinal */
-    void *stream;   /* cudaStream_t to use, or NULL for a context-owned stream */
+    void *stream;   /* cudaStream_t to use (of a green context: on its SMs), or NULL for a context-owned stream */
 } gbfk_config;
 
 /* One leaf block, as MRAG::BlockInfo (MRAG/MRAGcore/MRAGCommon.h:166-260). */
