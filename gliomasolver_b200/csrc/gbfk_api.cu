@@ -1933,7 +1933,6 @@ struct Adjoint {
                 a.out = nullptr;
                 a.stores = d_table + g.table;
                 a.nsteps = g.steps;
-                a.settle = (SettleWords *)(ctx->d_nan + 4);
                 CK(launch_resident_run<Real>(a, ctx->sms, ctx->stream));
                 ctx->launches++;
                 fsteps += g.steps;
@@ -2224,7 +2223,6 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
                           ctx->step_pref == GBFK_STEP_AUTO && std::isfinite((double)(Real)p->Dw) &&
                           std::isfinite((double)(Real)p->Dg) && std::isfinite((double)A.rho) &&
                           resident_fits<Real>(ctx) && ctx->n_heavy <= adjoint_run_capacity<Real>(ctx->sms);
-    const bool runs = resident;  // some sweep may run so
     double *run_sums = nullptr;
     const size_t ex = 2 * (size_t)ctx->n_heavy * 384 * 2 * sizeof(Real),
                  acc_bytes = resident ? (size_t)adjoint_run_threads(ctx->n_heavy, ctx->sms) * 6 * sizeof(double) : 0,
@@ -2239,12 +2237,15 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         if (rc) resident = false;  // one launch per step needs none of it
         rc = GBFK_OK;
     }
+    const bool runs = resident;  // some sweep may run so
     if (resident) {
         char *d = (char *)ctx->d_adj_run;
         if (!ctx->adj_run_ready) {
             CK(cudaMemsetAsync(d, 0, bytes, ctx->stream));
             ctx->adj_run_ready = true;
         }
+        // a NaN in any state, of a run or a launch per step, is noted there
+        CK(cudaMemsetAsync(ctx->d_nan, 0, sizeof(unsigned), ctx->stream));
         A.fs = ctx->stream;
         A.record = true;
         A.total_steps = p->nsteps;
@@ -2372,19 +2373,17 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
         if (e == cudaSuccess) e = ctx->staged.to_host(grad_c0, ctx->d_stage, A.fbytes, ctx->device, ctx->stream);
         ctx->launches++;
     }
-    SettleWords words = {};
+    unsigned nan = 0;
     if (runs && e == cudaSuccess)
-        e = cudaMemcpyAsync(&words, ctx->d_nan + 4, sizeof(words), cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(&nan, ctx->d_nan, sizeof(nan), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cleanup();
     if (e != cudaSuccess) return fail(ctx, GBFK_E_CUDA, "forward_adjoint: %s", cudaGetErrorString(e));
     if (runs) {
         rc = check_stage_timeout(ctx);
         if (rc) return rc;
-        if (words.nan) {  // the runs' steps are those of finite states only: once more, a launch per step
-            CK(cudaMemsetAsync(ctx->d_nan + 4, 0, sizeof(words), ctx->stream));
-            return forward_adjoint_impl<Real>(ctx, p, res, grad_c0, false);
-        }
+        // the runs' steps are those of finite states only: once more, a launch per step
+        if (nan) return forward_adjoint_impl<Real>(ctx, p, res, grad_c0, false);
     }
     auto nsum = [](const double *v, size_t stride, size_t count) {
         double s = 0, c = 0;

@@ -198,3 +198,31 @@ def test_nan_beside_csf_in_a_resident_sweep(gbfk_lib, prec, bpd):
         scale = b[key.replace("_abs", "") + "_abs"]
         assert np.isnan(a[key]) == np.isnan(b[key]), key
         assert np.isnan(b[key]) or abs(a[key] - b[key]) <= 1e-14 * scale + 1e-13 * abs(b[key]), key
+
+
+@pytest.mark.parametrize("steps,ck", [(1, 1), (2, 4), (3, 1), (9, 3)])
+@pytest.mark.parametrize("prec,bpd", [("f64", 4), ("f32", 8)])
+def test_gradient_with_nan_that_arises_in_few_steps(gbfk_lib, prec, bpd, steps, ck):
+    """An infinite tissue fraction: its faces' coefficients are NaN, also those
+    toward CSF, and the states after the first, whether the forward steps are
+    a run or (few) a launch each."""
+    n = 8 * bpd
+    pw, pg, phi = layered(n, 3, prec)
+    phi[np.isnan(phi)] = 0.1
+    for z, y in np.argwhere(pw[:, :, 4] > 0)[:: n][:5]:
+        pw[z, y, 4] = np.inf
+    rng = np.random.default_rng(1)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
+    s = make_schedule(0.2, 0.1, 100.0, 25.6, bpd, prec)
+    out = {}
+    with _pool(n, prec, (pw, pg, phi)) as pool:
+        pool.set_observations(t1, fl)
+        for kind in ("pipelined", "auto"):
+            pool.step_kernel = kind
+            out[kind] = pool.forward_adjoint(s.Dw, s.Dg, s.rho, min(s.dt, 0.2), steps, sigma=0.0, nsnapshots=ck,
+                                             grad_c0=True, term_magnitudes=True, t1_uc=0.7, t2_uc=0.25, slope=2.0)
+    a, b = out["auto"], out["pipelined"]
+    assert np.isnan(b["grad_c0"]).any()
+    assert np.array_equal(a["grad_c0"], b["grad_c0"], equal_nan=True) and a["loss"] == b["loss"]
+    for key in ("dDw", "drho", "dDw_abs", "drho_abs"):
+        assert a[key] == b[key] or np.isnan(a[key]) and np.isnan(b[key]), key
