@@ -2177,7 +2177,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     // and face halos have p_w = p_g = 0, so both diffusivities of such a face
     // are 0 and its harmonic mean is 0), so no neighbour feeds their lambda.
     // They keep status kAdjMuZero in both sets and lambda 0.
-    bool ic_clean = false;    // every empty block of the initial condition holds +0
+    bool ic_clean = false;    // a step makes every empty block of the initial condition +0
     bool ic_clamped = false;  // and every value of it is one of a clamped state, none NaN
     if (e == cudaSuccess && ctx->identity_slots) {
         int *d_list = (int *)ctx->adj_mem[15];
@@ -2192,8 +2192,8 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
             ic_clean = ic_clamped = true;
             for (int b = 0; b < nb; b++) {
                 if (pos[b] & 2) ic_clamped = false;
+                if (bt[b] == kBlockEmpty && (pos[b] & 5)) ic_clean = false;
                 pos[b] &= 1;
-                if (bt[b] == kBlockEmpty && pos[b]) ic_clean = false;
             }
             // blocks with tissue first, then empty blocks with a positive
             // initial value (a tumour outside the anatomy)

@@ -1702,20 +1702,22 @@ cudaError_t upload_ghost_table()
 }
 
 // out[b]: bit 0 a cell of block b (pool order, identity slots) is > 0, bit 1 a
-// cell is negative, -0, above 1 or NaN
+// cell is negative, -0, above 1 or NaN, bit 2 a cell is NaN
 template <typename Real>
 __global__ void block_any_positive_kernel(const Real *__restrict__ phi, int nblocks, unsigned char *__restrict__ out)
 {
     for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
         const Real *q = phi + (int64_t)b * kBS3;
-        bool any = false, off = false;
+        bool any = false, off = false, nan = false;
         for (int c = threadIdx.x; c < kBS3; c += blockDim.x) {
             any |= q[c] > (Real)0;
             off |= !(q[c] <= (Real)1) || signbit(q[c]);
+            nan |= q[c] != q[c];
         }
         any = __syncthreads_or(any);
         off = __syncthreads_or(off);
-        if (threadIdx.x == 0) out[b] = (any ? 1 : 0) | (off ? 2 : 0);
+        nan = __syncthreads_or(nan);
+        if (threadIdx.x == 0) out[b] = (any ? 1 : 0) | (off ? 2 : 0) | (nan ? 4 : 0);
     }
 }
 

@@ -416,7 +416,7 @@ int adjoint_run_threads(int n, int sms);
 template <typename Real>
 cudaError_t launch_adjoint_run(const AdjRunArgs<Real> &a, bool abs_terms, int sms, cudaStream_t s);
 // out[b]: bit 0 a cell of block b (identity slots) is > 0, bit 1 a cell is not
-// in +0 <= phi <= 1
+// in +0 <= phi <= 1, bit 2 a cell is NaN
 template <typename Real>
 cudaError_t launch_block_any_positive(const Real *phi, int nblocks, unsigned char *out, cudaStream_t s);
 // dL/dphi of loss = -(L_T1c + L_FLAIR) in pool order; roi_count: NULL (every

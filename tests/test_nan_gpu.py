@@ -80,11 +80,15 @@ def test_nan_beside_csf_in_steps_over_the_heavy_blocks(gbfk_lib, prec, n):
 def outside(fields, kind, seed=0):
     """The same with values in the CSF too, whole blocks of it among them:
     positive ones ("positive"), a NaN at the border of an empty block and of
-    the CSF block beside it, each with a positive neighbour across ("nan"), or
-    both."""
+    the CSF block beside it, each with a positive neighbour across ("nan"),
+    both, or one NaN inside an empty block that is +0 else ("alone")."""
     pw, pg, phi = (f.copy() for f in fields)
     rng = np.random.default_rng(seed)
     csf = pw + pg == 0
+    if kind == "alone":
+        phi = np.nan_to_num(phi)
+        phi[12, 12, 12] = np.nan
+        return pw, pg, phi
     if kind != "nan":
         phi[csf & (rng.random(phi.shape) < 0.7)] = 0.37
     if kind != "positive":
@@ -129,21 +133,32 @@ def test_nan_that_arises_in_a_run_with_tumour_in_empty_blocks(gbfk_lib, n, used)
         assert a.step_kernel == used
 
 
-@pytest.mark.parametrize("kind", ["nan", "both"])
+@pytest.mark.parametrize("kind", ["nan", "both", "alone"])
 def test_gradient_with_nan_in_an_empty_block(gbfk_lib, kind):
+    """A step keeps such a NaN: the states, the loss and lambda_0 are those of
+    the block kernel whatever the call before was (its buffers' empty blocks
+    may be known to hold +0), with the same coefficients and new ones."""
     n, steps = 32, 10
     pw, pg, phi = outside(layered(n, 3, "f32"), kind)
+    clean = np.where(pw + pg > 0, np.nan_to_num(phi), 0).astype(np.float32)
     rng = np.random.default_rng(1)
     t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
-    s = make_schedule(0.2, 0.1, 100.0, 25.6, n // 8, "f32")
-    out = {}
     with _pool(n, "f32", (pw, pg, phi)) as pool:
         pool.set_observations(t1, fl)
-        for k in ("pipelined", "auto"):
-            pool.step_kernel = k
-            out[k] = pool.forward_adjoint(s.Dw, s.Dg, s.rho, min(s.dt, 0.2), steps, sigma=0.0, nsnapshots=4,
-                                          grad_c0=True, t1_uc=0.7, t2_uc=0.25, slope=2.0)
-    assert np.array_equal(out["auto"]["grad_c0"], out["pipelined"]["grad_c0"], equal_nan=True)
+        for Dw, before in ((0.2, None), (0.2, clean), (0.1, clean), (0.15, None)):
+            s = make_schedule(Dw, 0.1, 100.0, 25.6, n // 8, "f32")
+            out = {}
+            for k in ("block", "pipelined", "auto"):
+                pool.step_kernel = k
+                for field in (before, phi):
+                    if field is None:
+                        continue
+                    pool.upload_dense("phi", field)
+                    out[k] = pool.forward_adjoint(s.Dw, s.Dg, s.rho, min(s.dt, 0.2), steps, sigma=0.0, nsnapshots=4,
+                                                  grad_c0=True, t1_uc=0.7, t2_uc=0.25, slope=2.0)
+            for k in ("pipelined", "auto"):
+                assert np.array_equal(out[k]["grad_c0"], out["block"]["grad_c0"], equal_nan=True), (Dw, k)
+                assert out[k]["loss"] == out["block"]["loss"], (Dw, k)
 
 
 @pytest.mark.parametrize("prec,bpd", [("f32", 4), ("f64", 3), ("f32", 12)])
