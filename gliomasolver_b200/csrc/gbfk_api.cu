@@ -281,10 +281,10 @@ int upload_origin(gbfk_ctx *ctx, const std::vector<int> &level, const std::vecto
         if (rc) return rc;
     }
     if (ctx->precision == GBFK_F64) {
-        CK(cudaMemcpy(ctx->d_origin, o.data(), o.size() * sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_origin, o.data(), o.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     } else {
         std::vector<float> f(o.begin(), o.end());
-        CK(cudaMemcpy(ctx->d_origin, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_origin, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     }
     ctx->have_origin = true;
     return GBFK_OK;
@@ -302,7 +302,7 @@ int upload_ih2(gbfk_ctx *ctx)
         const int rc = topo_alloc(ctx, &ctx->d_ih2, ctx->nblocks * sizeof(double));
         if (rc) return rc;
     }
-    CK(cudaMemcpy(ctx->d_ih2, v.data(), ctx->nblocks * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_ih2, v.data(), ctx->nblocks * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     return GBFK_OK;
 }
 
@@ -433,15 +433,16 @@ int set_csr(gbfk_ctx *ctx, const int64_t *row_ptr, const std::vector<int> &src, 
     if (!rc) rc = topo_alloc(ctx, &ctx->d_gpg, nrows * sizeof(Real));
     if (!rc) rc = topo_alloc(ctx, &ctx->d_gphi, nrows * sizeof(Real));
     if (rc) return rc;
-    CK(cudaMemcpy(ctx->d_row_ptr, row_ptr, (nrows + 1) * sizeof(int64_t), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_row_ptr, row_ptr, (nrows + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     if (nnz) {
-        CK(cudaMemcpy(ctx->d_src, src.data(), nnz * sizeof(int), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(ctx->d_w, w.data(), nnz * sizeof(Real), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_src, src.data(), nnz * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->d_w, w.data(), nnz * sizeof(Real), cudaMemcpyHostToDevice, ctx->stream));
     }
-    CK(cudaMemcpy(ctx->d_nbr, nbr.data(), (size_t)nb * 6 * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_all_rows, all_rows.data(), nrows * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_nbr, nbr.data(), (size_t)nb * 6 * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_all_rows, all_rows.data(), nrows * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     if (!step_rows.empty())
-        CK(cudaMemcpy(ctx->d_step_rows, step_rows.data(), step_rows.size() * sizeof(int), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_step_rows, step_rows.data(), step_rows.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));  // the host arrays are free
     ctx->n_step_rows = (int64_t)step_rows.size();
     ctx->nrows = nrows;
     ctx->have_csr = true;
@@ -1077,11 +1078,11 @@ int gbfk_create(const gbfk_config *cfg, gbfk_ctx **out)
         cudaGetLastError();
         return bail(GBFK_E_OOM);
     }
-    cudaMemset(ctx->phi[0], 0, bytes);
-    cudaMemset(ctx->phi[1], 0, bytes);
-    cudaMemset(ctx->pw, 0, bytes);
-    cudaMemset(ctx->pg, 0, bytes);
-    cudaMemset(ctx->d_nan, 0, 8 * sizeof(unsigned));
+    // here and below: on the context's stream, which the legacy stream of a plain
+    // cudaMemset or cudaMemcpy (whose last piece of pageable memory may still be on
+    // its way when the call returns) is not ordered with
+    for (void *f : {ctx->phi[0], ctx->phi[1], ctx->pw, ctx->pg}) cudaMemsetAsync(f, 0, bytes, ctx->stream);
+    cudaMemsetAsync(ctx->d_nan, 0, 8 * sizeof(unsigned), ctx->stream);
     ctx->sms = gbfk_host::stream_sms(cfg->device, ctx->stream);
     if (ctx->sms <= 0) return bail(GBFK_E_CUDA);
     if (ensure_table(ctx) != GBFK_OK) return bail(GBFK_E_CUDA);
@@ -1200,14 +1201,14 @@ int gbfk_set_uniform(gbfk_ctx *ctx, int bpd)
         if (!rc) rc = topo_alloc(ctx, &ctx->d_h, nb * ctx->rsize);
         if (rc) return rc;
     }
-    CK(cudaMemcpy(ctx->d_slot, ctx->h_slot.data(), nb * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_nbr, nbr.data(), (size_t)nb * 6 * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_slot, ctx->h_slot.data(), nb * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_nbr, nbr.data(), (size_t)nb * 6 * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     if (ctx->precision == GBFK_F64) {
         std::vector<double> hv(nb, h);
-        CK(cudaMemcpy(ctx->d_h, hv.data(), nb * sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_h, hv.data(), nb * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     } else {
         std::vector<float> hv(nb, (float)h);
-        CK(cudaMemcpy(ctx->d_h, hv.data(), nb * sizeof(float), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_h, hv.data(), nb * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     }
     int rc = upload_ih2(ctx);
     if (rc) return rc;
@@ -1223,6 +1224,7 @@ int gbfk_set_uniform(gbfk_ctx *ctx, int bpd)
         if ((1 << L) == bpd) rc = upload_origin(ctx, level, index);
     }
     if (rc) return rc;
+    CK(cudaStreamSynchronize(ctx->stream));
     ctx->have_topology = true;
     return GBFK_OK;
 }
@@ -1269,13 +1271,13 @@ int gbfk_set_topology(gbfk_ctx *ctx, const gbfk_blockinfo *blocks, int nblocks, 
         if (!rc) rc = topo_alloc(ctx, &ctx->d_h, nblocks * ctx->rsize);
         if (rc) return rc;
     }
-    CK(cudaMemcpy(ctx->d_slot, ctx->h_slot.data(), nblocks * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_slot, ctx->h_slot.data(), nblocks * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     if (ctx->precision == GBFK_F64) {
-        CK(cudaMemcpy(ctx->d_h, ctx->h_h.data(), nblocks * sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_h, ctx->h_h.data(), nblocks * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     } else {
         std::vector<float> hv(nblocks);
         for (int i = 0; i < nblocks; i++) hv[i] = (float)ctx->h_h[i];
-        CK(cudaMemcpy(ctx->d_h, hv.data(), nblocks * sizeof(float), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_h, hv.data(), nblocks * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     }
     int rc = ctx->precision == GBFK_F64 ? set_csr<double>(ctx, g->row_ptr, src, g->w0, g->w1, g->w2, true)
                                         : set_csr<float>(ctx, g->row_ptr, src, g->w0, g->w1, g->w2, true);
@@ -1291,6 +1293,7 @@ int gbfk_set_topology(gbfk_ctx *ctx, const gbfk_blockinfo *blocks, int nblocks, 
         rc = upload_origin(ctx, level, index);
         if (rc) return rc;
     }
+    CK(cudaStreamSynchronize(ctx->stream));
     ctx->have_topology = true;
     return GBFK_OK;
 }
@@ -1580,18 +1583,19 @@ int gbfk_set_observations(gbfk_ctx *ctx, int n, const double *t1c, const double 
     }
     CK(cudaMalloc(&ctx->d_t1c, N));
     CK(cudaMalloc(&ctx->d_flair, N));
-    CK(cudaMemcpy(ctx->d_t1c, a.data(), N, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_flair, b.data(), N, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_t1c, a.data(), N, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_flair, b.data(), N, cudaMemcpyHostToDevice, ctx->stream));
     if (pet) {
         CK(cudaMalloc(&ctx->d_pet, N * sizeof(double)));
-        CK(cudaMemcpy(ctx->d_pet, pet, N * sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_pet, pet, N * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     }
     if (roi && nroi > 0) {
         for (int i = 0; i < 3 * nroi; i++)
             if (roi[i] < 0 || roi[i] >= n) return fail(ctx, GBFK_E_INVALID, "set_observations: ROI point out of the grid");
         CK(cudaMalloc(&ctx->d_roi, (size_t)nroi * 3 * sizeof(int)));
-        CK(cudaMemcpy(ctx->d_roi, roi, (size_t)nroi * 3 * sizeof(int), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->d_roi, roi, (size_t)nroi * 3 * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     }
+    CK(cudaStreamSynchronize(ctx->stream));
     ctx->nroi = roi ? nroi : 0;
     ctx->obs_n = n;
     return GBFK_OK;

@@ -890,8 +890,12 @@ int gbfk_batch_create(const gbfk_config *cfg, int bpd, int max_samples, int max_
         cudaGetLastError();
         return bail(GBFK_E_OOM);
     }
-    cudaMemcpy(b->d_nbr, nbr.data(), nbr.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(b->d_ih2, ih2.data(), nb * sizeof(double), cudaMemcpyHostToDevice);
+    // on the batch's stream, which the legacy stream of a plain copy is not ordered with
+    if (cudaMemcpyAsync(b->d_nbr, nbr.data(), nbr.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream) !=
+            cudaSuccess ||
+        cudaMemcpyAsync(b->d_ih2, ih2.data(), nb * sizeof(double), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+        cudaStreamSynchronize(b->stream) != cudaSuccess)
+        return bail(GBFK_E_CUDA);
     const size_t na = (size_t)max_anatomies, ns = (size_t)max_samples;
     if (cudaMalloc(&b->pw_all, na * field) != cudaSuccess || cudaMalloc(&b->pg_all, na * field) != cudaSuccess ||
         cudaMalloc(&b->meta_all, na * nb * kBS3 * sizeof(unsigned short)) != cudaSuccess ||
@@ -1056,16 +1060,17 @@ int gbfk_batch_set_observations(gbfk_batch *b, const double *t1c, const double *
     }
     BK(cudaMalloc(&b->d_t1c, N));
     BK(cudaMalloc(&b->d_flair, N));
-    BK(cudaMemcpy(b->d_t1c, a.data(), N, cudaMemcpyHostToDevice));
-    BK(cudaMemcpy(b->d_flair, c.data(), N, cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(b->d_t1c, a.data(), N, cudaMemcpyHostToDevice, b->stream));
+    BK(cudaMemcpyAsync(b->d_flair, c.data(), N, cudaMemcpyHostToDevice, b->stream));
     if (pet) {
         BK(cudaMalloc(&b->d_pet, N * sizeof(double)));
-        BK(cudaMemcpy(b->d_pet, pet, N * sizeof(double), cudaMemcpyHostToDevice));
+        BK(cudaMemcpyAsync(b->d_pet, pet, N * sizeof(double), cudaMemcpyHostToDevice, b->stream));
     }
     if (roi && nroi > 0) {
         BK(cudaMalloc(&b->d_roi, (size_t)nroi * 3 * sizeof(int)));
-        BK(cudaMemcpy(b->d_roi, roi, (size_t)nroi * 3 * sizeof(int), cudaMemcpyHostToDevice));
+        BK(cudaMemcpyAsync(b->d_roi, roi, (size_t)nroi * 3 * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     }
+    BK(cudaStreamSynchronize(b->stream));
     b->nroi = roi ? nroi : 0;
     b->have_obs = true;
     return GBFK_OK;

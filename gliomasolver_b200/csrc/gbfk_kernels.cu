@@ -1698,7 +1698,9 @@ cudaError_t upload_ghost_table()
 {
     short table[kLab3];
     init_ghost_table_host(table);
-    return cudaMemcpyToSymbol(c_ghost_id, table, sizeof(table));
+    const cudaError_t e = cudaMemcpyToSymbol(c_ghost_id, table, sizeof(table));
+    // there before any stream reads it (the copy returns with its last piece on the way)
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
 }
 
 // out[b]: bit 0 a cell of block b (pool order, identity slots) is > 0, bit 1 a

@@ -200,3 +200,35 @@ def test_run_of_ghost_list_steps_equals_launches(gbfk_lib, prec, bpd):
         assert np.array_equal(a[order], b[order], equal_nan=True)
     assert np.array_equal(out["auto"][-1], out["block"][-1], equal_nan=True)
     assert not np.array_equal(out["auto"][0][order], out["auto"][3][order], equal_nan=True)
+
+
+@pytest.mark.gpu
+def test_topologies_and_observations_are_there_when_the_next_kernel_runs(gbfk_lib):
+    """Ghost lists, slots and observations change and are used at once, many
+    times over on a stream of the context's own, which the legacy stream's
+    copies would not be ordered with."""
+    from gliomasolver_b200 import BlockPool
+
+    n, want = 72, {}
+    r = np.random.default_rng(3)
+    phi = r.random((n, n, n), dtype=np.float32)
+    tissue = np.full_like(phi, 0.5)
+    masks = [(r.random(phi.shape) < f).astype(float) for f in (0.2, 0.6)]
+    for turn in range(40):
+        with BlockPool((n // 8) ** 3, "f32") as pool:
+            for m in (n, n // 3, n):
+                pool.set_uniform(m // 8)
+                for name, a in (("p_w", tissue), ("p_g", tissue), ("phi", phi)):
+                    pool.upload_dense(name, np.ascontiguousarray(a[:m, :m, :m]))
+                pool.rd_step(1e-4, 1e-5, 0.1, 1e-3, 2)
+                got = [pool.fwt_details(), pool.download_dense("phi")]
+                for k in range(2):
+                    assert np.array_equal(got[k], want.setdefault((m, k), got[k])), (turn, m, k)
+        with BlockPool(8, "f32") as pool:
+            pool.set_uniform(2)
+            pool.upload_dense("phi", np.ascontiguousarray(phi[:16, :16, :16]))
+            for k, mask in enumerate(masks):
+                small = np.ascontiguousarray(mask[:16, :16, :16])
+                pool.set_observations(small, small, pet=small * 0.7)
+                got = pool.log_likelihood()
+                assert np.array_equal(got, want.setdefault(("lik", k), got)), (turn, k)
