@@ -2413,7 +2413,7 @@ int forward_adjoint_impl(gbfk_ctx *ctx, const gbfk_adjoint_params *p, gbfk_adjoi
     if (resident) {
         res->drho *= p->dt;
         res->dDw *= p->dt / A.Dw;
-        res->drho_abs *= p->dt;
+        res->drho_abs *= fabs(p->dt);
         res->dDw_abs *= fabs(p->dt / A.Dw);
     }
     for (int d = 0; d < 3; d++) res->dx0[d] = p->sigma > 0 ? nsum(xp.data() + 2 * d, 6, xparts) : 0.0;

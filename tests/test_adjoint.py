@@ -527,3 +527,28 @@ def test_gradient_with_new_coefficients_keeps_its_resident_sweep(gbfk_lib, prec,
             a, b = out["auto"], out["pipelined"]
             assert np.array_equal(a["grad_c0"], b["grad_c0"]) and a["loss"] == b["loss"]
             assert a["launches"] < steps < b["launches"], Dw
+
+
+def test_term_magnitudes_of_a_resident_sweep_with_a_negative_step(gbfk_lib):
+    """Steps back in time: the magnitudes are sums of |term| still."""
+    from gliomasolver_b200 import BlockPool
+
+    n, bpd = 32, 4
+    pw, pg, _ = make_anatomy(n, 2)
+    rng = np.random.default_rng(n)
+    t1, fl = ((rng.random(pw.shape) < f).astype(float) for f in (0.05, 0.1))
+    sched = make_schedule(0.2, 0.1, 100.0, L, bpd, "f64")
+    out = {}
+    with BlockPool(bpd ** 3, "f64") as pool:
+        pool.set_uniform(bpd)
+        for name, a in (("p_w", pw), ("p_g", pg), ("phi", tumor_ic(n, (0.5, 0.45, 0.5), pw, pg))):
+            pool.upload_dense(name, a)
+        pool.set_observations(t1, fl)
+        for kind in ("auto", "pipelined"):
+            pool.step_kernel = kind
+            out[kind] = pool.forward_adjoint(sched.Dw, sched.Dg, sched.rho, -0.05 * sched.dt, 8, sigma=0.0,
+                                             nsnapshots=9, term_magnitudes=True, **UC)
+    a, b = out["auto"], out["pipelined"]
+    assert a["drho_abs"] > 0 and a["dDw_abs"] > 0
+    for key in ("dDw", "drho", "dDw_abs", "drho_abs"):
+        assert a[key] == pytest.approx(b[key], rel=1e-12, abs=1e-14 * b[key.replace("_abs", "") + "_abs"])
