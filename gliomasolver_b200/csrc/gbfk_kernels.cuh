@@ -151,9 +151,10 @@ struct SettleWords {
 // pointers: where the heavy blocks of state s + 1 go (NULL entries: nowhere).
 // empty: the n_empty empty blocks, of which the run only notes in `settle` what
 // launch_settle has to know; settle: NULL, or its words; save: NULL, or where the
-// heavy blocks of state 0 are kept, one after the other.  ex: 2 * n * 384 Real and index: 2 words,
-// both zeroed once per item list and then left to the runs.  dt, Dw and Dg are
-// finite.  err_flag as for the pipelined step (bits 0 and 9: a face never came).
+// heavy blocks of state 0 are kept, one after the other.  ex: 2 * n * 384 Real and
+// index: 2 words, both zeroed once per item list and then left to the runs.  dt,
+// Dw and Dg are finite.  err_flag as for the pipelined step (bits 0 and 9: a face
+// never came).
 template <typename Real>
 struct ResidentArgs {
     const int *items, *nbr;

@@ -254,9 +254,9 @@ int gbfk_batch_set_samples(gbfk_batch *b, int nsamples, const gbfk_sample *sampl
  * 4 for the one-CTA-per-block kernel with that many samples per CTA, or 0:
  * where the blocks with tissue of a sample fit in the SMs' shared memory, all
  * steps of all samples in one launch, each sample resident on a team of SMs;
- * elsewhere the autotuner times the candidates on the first steps and keeps
- * the fastest (the results do not depend on it).  GBFK_E_NAN if a sample
- * became NaN; GBFK_E_STATE for -1 on a grid it does not apply to. */
+ * elsewhere, and again when a sample became NaN there, the autotuner times the
+ * candidates on the first steps and keeps the fastest (the results do not
+ * depend on it).  GBFK_E_NAN if a sample became NaN; GBFK_E_STATE for -1 on a grid it does not apply to. */
 int gbfk_batch_run(gbfk_batch *b, int samples_per_cta);
 /* The samples_per_cta choice the last run used (-1: the pipelined step, or
  * the samples resident in shared memory). */
@@ -331,7 +331,8 @@ int gbfk_batch_log_likelihood(gbfk_batch *b, const gbfk_likelihood_params *param
  * SMs' shared memory with their adjoint state (about 1180 in FP32, 590 in FP64
  * on a B200) and the initial state lies in [0, 1] and is +0 in the others, the
  * steps that follow one another in the sweep run in one cooperative launch,
- * on the context's stream.  Elsewhere the forward steps of the reverse sweep
+ * on the context's stream.  Elsewhere, and again when a state became NaN there,
+ * the forward steps of the reverse sweep
  * run on a second stream of the context (created at the first call, ordered
  * after the work already on the context's stream) next to the adjoint steps;
  * the call returns when both are done.  GBFK_ADJ_STREAMS=1 keeps everything
