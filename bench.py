@@ -41,8 +41,8 @@ from gliomasolver_b200.schedule import make_schedule  # noqa: E402
 METRIC = "RD cell-updates/s & % HBM roofline"
 UNIT = "cell-updates/s"
 # the step kernel behind a choice (--step-kernel) and what the library reports it used
-KERNEL_NAMES = {("auto", "pipelined"): "stream_step_kernel<{real}> (persistent, bulk copies, the blocks with tissue; the "
-                                       "others take all steps in one launch)",
+KERNEL_NAMES = {("auto", "pipelined"): "stream_step_kernel<{real}> (persistent, bulk copies, the blocks with tissue; "
+                                       "what the others hold is settled in one launch at the call's end)",
                 ("auto", "run"): "resident_run_kernel<{real}> (all steps in one launch, blocks in shared memory)",
                 ("pipelined", "pipelined"): "rd_step_tma_kernel<{real}> (persistent, TMA-fed)",
                 ("run", "run"): "rd_step_tma_kernel<{real}> (persistent, TMA-fed, all steps in one launch)",

@@ -144,7 +144,7 @@ int gbfk_rd_step(gbfk_ctx *ctx, double Dw, double Dg, double rho, double dt, int
  * GBFK_STEP_RUN), where they fit: about 2300 blocks in FP32, 1180 in FP64 on
  * a B200. Beyond, each step is a launch over the blocks that hold tissue
  * (reported as GBFK_STEP_PIPELINED); the others, whose cells only react, take
- * all steps in a launch of their own.  Where a NaN turns up in such a call, its
+ * all steps in one launch at the end.  Where a NaN turns up in such a call, its
  * steps are taken again over all blocks, so that the NaN is in the same cells
  * as with a launch per step. Short calls, and the first step after
  * phi was uploaded, run the persistent TMA-fed pipeline on power-of-two grids
